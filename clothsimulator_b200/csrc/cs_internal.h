@@ -375,11 +375,16 @@ struct Collide {
     int* nfill = nullptr;
     int* nlist = nullptr;         // 4 impact + corner, ascending per slot
     float* x1 = nullptr;          // 3N: positions when the collision step began
-    float *cur = nullptr, *next = nullptr, *grad = nullptr;  // 3 per slot
-    float *lambda = nullptr, *coef = nullptr, *cterm = nullptr;  // per constraint
-    float *nterm = nullptr, *gterm = nullptr;                  // per slot
+    float4 *cur = nullptr, *next = nullptr;    // per slot: positions, two buffers
+    float4 *grad = nullptr, *grad2 = nullptr;  // per slot: gradient and its square, two buffers
+    float4* home = nullptr;                    // per slot: position when the step began, mass
+    float4* con = nullptr;                     // 3 per constraint: slots, weights, normal
+    float *lambda = nullptr, *lambda2 = nullptr, *cterm = nullptr;  // per constraint
 };
 
+// threads per CTA of the impact projection and the terms of an ordered sum staged in its shared memory
+#define CS_OPT_THREADS 1024
+#define CS_OPT_STAGE 12288
 #define CS_CONTACT_ITEMS 4096  // keys per compaction block (256 threads x 16)
 #define CS_PAIR_STAGE 16       // candidate pairs staged per thread before appending
 #define CS_SCAN_ITEMS 4096     // ints per block of the exclusive scan (1024 threads x 4)

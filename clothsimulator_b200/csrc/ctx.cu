@@ -952,6 +952,7 @@ struct cs_ctx {
     // collision step (collide.cu)
     Collide coll;
     CollideCaps collCaps;
+    int optCtas = 0;  // CTAs of the projection's cluster (0: not asked yet)
 };
 
 namespace {
@@ -1018,8 +1019,8 @@ void freeBatch(cs_ctx* c) {
     {
         Collide& K = c->coll;
         void* ps[] = {K.found, K.counters, K.sorted, K.all, K.used, K.nodemin, K.alive, K.chosen, K.mark, K.nodes,
-                      K.idx, K.nptr, K.nfill, K.nlist, K.x1, K.cur, K.next, K.grad, K.lambda, K.coef,
-                      K.cterm, K.nterm, K.gterm, K.skey[0], K.skey[1], K.sperm[0], K.sperm[1], K.stmp};
+                      K.idx, K.nptr, K.nfill, K.nlist, K.x1, K.cur, K.next, K.grad, K.grad2, K.home,
+                      K.con, K.lambda, K.lambda2, K.cterm, K.skey[0], K.skey[1], K.sperm[0], K.sperm[1], K.stmp};
         for (void* q : ps)
             if (q) cudaFree(q);
         c->coll = Collide();
@@ -2287,6 +2288,36 @@ cs_status sortImpacts(cs_ctx* c, int nFound, int* pin_out) {
     return CS_OK;
 }
 
+// The projection by one cluster: 16 CTAs, or 8 where a cluster of 16 cannot run (every rank beyond
+// the second evaluates one step length of the line search at a time).
+cs_status launchOpt(cs_ctx* c, int nn, int nc) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(CS_OPT_THREADS);
+    cfg.dynamicSmemBytes = CS_OPT_STAGE * sizeof(float);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (c->optCtas == 0) {
+        CS_CUDA(raiseDynSmem((const void*)cs_opt_kernel, cfg.dynamicSmemBytes));
+        c->optCtas = 8;
+        at[0].val.clusterDim.x = 16;
+        cfg.gridDim = dim3(16);
+        int clusters = 0;
+        if (cudaFuncSetAttribute(cs_opt_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, cs_opt_kernel, &cfg) == cudaSuccess && clusters > 0)
+            c->optCtas = 16;
+        cudaGetLastError();
+    }
+    at[0].val.clusterDim.x = c->optCtas;
+    cfg.gridDim = dim3(c->optCtas);
+    cfg.stream = c->stream;
+    CS_CUDA(cudaLaunchKernelEx(&cfg, cs_opt_kernel, c->B, c->coll, nn, nc));
+    return CS_OK;
+}
+
 cs_status collideScratch(cs_ctx* c, int nFound, int nAll) {
     Batch& B = c->B;
     Collide& K = c->coll;
@@ -2303,9 +2334,9 @@ cs_status collideScratch(cs_ctx* c, int nFound, int nAll) {
         if ((st = once(K.mark, N + 1)) != CS_OK || (st = once(K.used, N)) != CS_OK ||
             (st = once(K.nodes, N)) != CS_OK || (st = once(K.nptr, N + 1)) != CS_OK ||
             (st = once(K.nfill, N + 1)) != CS_OK || (st = once(K.x1, 3 * N)) != CS_OK ||
-            (st = once(K.cur, 3 * N)) != CS_OK || (st = once(K.next, 3 * N)) != CS_OK ||
-            (st = once(K.grad, 3 * N)) != CS_OK || (st = once(K.nterm, N)) != CS_OK ||
-            (st = once(K.gterm, N)) != CS_OK || (st = once(K.counters, 2)) != CS_OK ||
+            (st = once(K.cur, N)) != CS_OK || (st = once(K.next, N)) != CS_OK ||
+            (st = once(K.grad, N)) != CS_OK || (st = once(K.grad2, N)) != CS_OK || (st = once(K.home, N)) != CS_OK ||
+            (st = once(K.counters, 2)) != CS_OK ||
             (st = once(K.nodemin, N)) != CS_OK)
             return st;
         CS_CUDA(cudaMemset(K.used, 0, N * sizeof(int)));
@@ -2363,8 +2394,8 @@ cs_status collideScratch(cs_ctx* c, int nFound, int nAll) {
             return grow(c, q, cap, n);
         };
         if ((st = fresh(K.idx, 4 * P.all)) != CS_OK || (st = fresh(K.nlist, 4 * P.all)) != CS_OK ||
-            (st = fresh(K.lambda, P.all)) != CS_OK || (st = fresh(K.coef, P.all)) != CS_OK ||
-            (st = fresh(K.cterm, P.all)) != CS_OK)
+            (st = fresh(K.lambda, P.all)) != CS_OK || (st = fresh(K.lambda2, P.all)) != CS_OK ||
+            (st = fresh(K.con, 3 * P.all)) != CS_OK || (st = fresh(K.cterm, P.all)) != CS_OK)
             return st;
     }
     return CS_OK;
@@ -2508,8 +2539,7 @@ cs_status cs_collision_step(cs_ctx* c, const cs_collision_params* p, cs_collisio
             if ((st = scanInts(c, K.nptr, nn, nullptr)) != CS_OK) return st;
             cs_opt_fill_kernel<<<nblk(4LL * nAll, 256), 256, 0, c->stream>>>(K, nAll);
             cs_opt_sort_kernel<<<nblk(nn, 256), 256, 0, c->stream>>>(K, nn);
-            cs_opt_kernel<<<1, 1024, 0, c->stream>>>(B, K, nn, nAll);
-            CS_CUDA(cudaGetLastError());
+            if ((st = launchOpt(c, nn, nAll)) != CS_OK) return st;
         }
     }
     C.ccd = 0;

@@ -156,3 +156,23 @@ def test_impact_order_ties_and_signed_zero(ctx_factory):
     ref = sorted(range(n), key=lambda i: (float(t[i]) + 0.0, *(int(v) for v in nodes[i]), int(types[i]), i))
     assert np.array_equal(order, np.array(ref, np.int32))
     assert np.any(np.signbit(t) & (t == 0)) and np.any(~np.signbit(t) & (t == 0))
+
+
+@pytest.mark.parametrize("nq,n_layers,hit", [(4, 2, 1), (8, 2, 12), (40, 2, 10_000), (64, 2, 10_000)])
+def test_projection_sizes_match_oracle(ctx_factory, nq, n_layers, hit):
+    """The projection's ordered sums at their edges: a single impact's four nodes, fewer terms than
+    threads, several terms per thread, more than one chunk (64 x 64 layers: over 7,168 nodes)."""
+    scene = scenes.stacked_sheets(nq, n_layers=n_layers, seed=7)
+    rng = np.random.default_rng(nq)
+    xs = []
+    for k, s in enumerate(scene.sheets):
+        x = s["x"].astype(np.float32).copy()
+        if k == 1:
+            moved = rng.permutation(len(x))[:hit]
+            x[moved, 2] -= (1.5e-3 + 2e-3 * rng.random(len(moved))).astype(np.float32)
+        xs.append(x)
+    g, o = run_both(ctx_factory, scene, xs)
+    assert o[1] > 0, "the case should have impacts"
+    assert (g[0], g[1]) == (o[0], o[1])
+    assert np.array_equal(g[2], o[2].astype(np.float32))
+    assert np.array_equal(g[3], o[3].astype(np.float32))
