@@ -39,7 +39,7 @@ __device__ __forceinline__ T bc_warp_sum(T v) {
 __device__ __forceinline__ bool bc_sheet_on(const Batch& B, int s) {
     if (!B.params->coarse || !B.bc_agg) return false;
     if (B.sheets[s].bc_na <= 0) return false;
-    if (B.sheet_prox && B.sheet_prox[s]) return false;
+    if (B.sheet_prox && B.sheet_prox[s] && !B.bc_resident) return false;
     return true;
 }
 
@@ -57,7 +57,7 @@ __device__ __forceinline__ bool bc_trip_on(const Batch& B, int s) {
 // y over sheets.
 __global__ void __launch_bounds__(256) cs_bc_assemble_kernel(Batch B) {
     const int s = blockIdx.y;
-    if (!bc_sheet_on(B, s) || B.inst[s].phase == PH_RESIDENT) return;
+    if (!bc_sheet_on(B, s) || (B.inst[s].phase == PH_RESIDENT) != (B.bc_resident != 0)) return;
     const SheetDesc& sh = B.sheets[s];
     const int nc = 3 * sh.bc_na;
     float* M = B.bc_mat + sh.bc_mat_off;
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(CS_BC_THREADS) cs_bc_invert_small_kernel(Batch
     extern __shared__ float bc_sm[];
     __shared__ int bad;
     const int s = blockIdx.x;
-    if (!bc_sheet_on(B, s) || B.inst[s].phase == PH_RESIDENT) return;
+    if (!bc_sheet_on(B, s) || (B.inst[s].phase == PH_RESIDENT) != (B.bc_resident != 0)) return;
     const SheetDesc& sh = B.sheets[s];
     const int nc = 3 * sh.bc_na;
     if (nc > CS_BC_SMALL_NC) return;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(CS_BC_THREADS) cs_bc_invert_cluster_kernel(Bat
     const int rank = (int)cluster.block_rank();
     const int s = B.bc_big[blockIdx.x / CS_BC_CLUSTER];
     // the same decision in every CTA of the cluster: all return, or none
-    if (!bc_sheet_on(B, s) || B.inst[s].phase == PH_RESIDENT) return;
+    if (!bc_sheet_on(B, s) || (B.inst[s].phase == PH_RESIDENT) != (B.bc_resident != 0)) return;
     const SheetDesc& sh = B.sheets[s];
     const int nc = 3 * sh.bc_na;
     if (nc <= CS_BC_SMALL_NC || nc > CS_BC_MAX_NC) return;

@@ -52,7 +52,8 @@ struct SheetDesc {
     float wind_density, wind_drag, wind_v[3];
     int nbr_ptr_off, nbr_off;   // this sheet's topology in the one-ring neighbour arrays
     int row2slot_off;           // this sheet's topology in the row -> slot map
-    int resident;               // 1: solved by the cluster-resident kernel (resident.cu)
+    int resident;               // 1: solved by the cluster-resident kernel (resident.cu), 2: by a
+                                // group of CTAs (group.cu)
     int csr_ptr_off;            // this sheet's topology in tcsr_ptr (block CSR for slot lookups)
     int panel_off;              // first value panel: global slot = panel_off * 32 + topology slot
     // coarse space of the batched loop: this sheet's topology in the aggregate arrays, its
@@ -137,6 +138,15 @@ struct SpmvShape {
 struct Batch;
 extern const SpmvShape kSpmvShapes[CS_SPMV_CANDIDATES];
 void launchSpmvShape(const Batch& B, int shape, cudaStream_t st);
+// Group-resident solver (group.cu): block slots per row (column codes live in registers), slices
+// per CTA that a sheet's tiles are planned for, its fewest when a batch would leave the chip idle.
+#define CS_GROUP_MAX_WIDTH 18
+#define CS_GROUP_SLICES 14
+#define CS_GROUP_MAX_WARPS CS_RES_MAX_WARPS
+#define CS_GROUP_CE_PARTS 4    // warps that share a row of the coarse matrix-vector product, at most
+#define CS_GROUP_MIN_SLICES 8
+// coarse unknowns up to which a group's segments are cut finer than one per CTA
+#define CS_GROUP_NC 192
 #define CS_SOLVER_AUTO_DEV 0
 #define CS_SOLVER_BATCHED_DEV 1
 
@@ -202,6 +212,15 @@ struct ProxInst {
 // Per-instance record written by cs_prox_kernel: -dt^2 J of the impulse (12x12), -dt J of
 // the friction (12x12), the impulse right-hand side dt (f + dt J v) (12), the friction one dt f.
 #define CS_PROX_REC 312
+
+// One sheet of the group-resident solver: its CTAs cta0 .. cta0 + ctas - 1, segments per CTA of its
+// coarse space, and where its packets, reduction packets, published-row marks, halo lists and
+// inverse coarse matrix (-1: none) start.
+struct GroupItem {
+    int sheet, cta0, ctas, segs;
+    int slot0, red0, pub0, halo0;
+    long long mat;
+};
 
 struct Batch {
     int N = 0, F = 0, E = 0, S = 0;
@@ -296,6 +315,23 @@ struct Batch {
     int res_cnc = 0;             // largest nc over the resident topologies (0: no coarse correction)
     int res_ck = 0;              // largest K
     int res_coff = 0;            // byte offset of the coarse region in the resident kernel's shared memory
+    // group-resident solver (group.cu): work items, per CTA the items it takes part in (in order);
+    // per topology slot (pub0) whether another CTA reads the row, per CTA (halo0) the slots it reads
+    // from others; exchange packets; the groups' inverse coarse matrices and per sheet their validity;
+    // sizes for the largest group (CTAs, own slots, halo slots, coarse unknowns, 3 segments per CTA,
+    // entries of a CTA's rows of the inverse coarse matrix),
+    // panels per CTA in shared memory and the byte offset of what follows the u array there
+    int n_group = 0, g_max = 0, g_own = 0, g_halo = 0, g_cap = 0, g_coff = 0, g_cnc = 0, g_ck3 = 0, g_cai = 0;
+    GroupItem* gitem = nullptr;
+    int *gcta_ptr = nullptr, *gcta_item = nullptr;
+    unsigned char* gpub = nullptr;
+    int *ghalo_ptr = nullptr, *ghalo = nullptr;
+    uint4 *gupk = nullptr, *grpk = nullptr;
+    float* gc_inv = nullptr;
+    int* gc_ok = nullptr;
+    // the batched coarse set-up kernels (coarse.cu) run on the sheets that the loop solves (0), or,
+    // on a copy of this struct holding the groups' coarse spaces, on those of the groups (1)
+    int bc_resident = 0;
     // per-topology block CSR (local ids, columns ascending) with the SELL slot of each block
     int* tcsr_ptr = nullptr;
     int* tcsr_col = nullptr;
@@ -309,7 +345,7 @@ struct Batch {
     int* xptr = nullptr;          // N + 1: blocks outside the pattern, per row (null: none)
     int* xcol = nullptr;          // their columns (batch nodes), ascending per row
     float* xval = nullptr;        // 9 per block, summed each step
-    int* sheet_prox = nullptr;    // per sheet: 1 if a proximity touches it (batched loop)
+    int* sheet_prox = nullptr;    // per sheet: bit 0 a proximity touches it, bit 1 it has blocks outside the pattern
 };
 
 // Proximity detection (contact.cu, cs_detect_proximities).  Scene-wide ids: nodes and faces as

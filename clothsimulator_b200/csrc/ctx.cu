@@ -19,6 +19,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <string>
@@ -88,6 +89,7 @@ __global__ void cs_opt_idx_kernel(Collide K, int nc);
 __global__ void cs_opt_fill_kernel(Collide K, int nc);
 __global__ void cs_opt_sort_kernel(Collide K, int nn);
 __global__ void cs_opt_kernel(Batch B, Collide K, int nn, int nc);
+__global__ void cs_group_pcg_kernel(Batch B);
 __global__ void cs_collide_velocity_kernel(Batch B, float invDt);
 __global__ void cs_contact_ee_kernel(Batch B, Contact C, int npairs);
 __global__ void cs_contact_count_kernel(Contact C);
@@ -210,6 +212,8 @@ struct Topo {
     // the element's corners, 8 bits per corner
     std::vector<int> rf_ptr, re_ptr;
     std::vector<int2> rf, re;
+    // group-resident solver: CTAs its rows are tiled for (0: not tiled), coarse segments per CTA
+    int group_ctas = 0, group_segs = 0;
     // rest (uv) coordinates of every node, from the first sheet of this connectivity: the
     // geometry the coarse-space segments of the cluster-resident solver are cut along
     std::vector<float> node_uv;
@@ -233,7 +237,48 @@ uint64_t hashInts(const int32_t* a, size_t n, uint64_t h) {
     return h;
 }
 
-std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, std::string& err) {
+// Rows ordered by tiles for the group-resident solver: the slices (32 rows) are dealt evenly to G
+// CTAs and within a CTA to K segments, and recursive bisection of the rest coordinates along the
+// longer axis gives every segment a compact piece of the sheet; rows of a segment by block count
+// (descending, then by index), which keeps its slices' padding low.
+void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, std::vector<int>& order) {
+    const int n = (int)len.size(), ns = (n + CS_SLICE - 1) / CS_SLICE;
+    order.resize(n);
+    for (int i = 0; i < n; i++) order[i] = i;
+    std::vector<int> cut{0};  // first row of every segment
+    for (int c = 0; c < G; c++) {
+        const int lo = (int)((long long)ns * c / G), hi = (int)((long long)ns * (c + 1) / G);
+        for (int k = 0; k < K; k++) cut.push_back(std::min(n, CS_SLICE * (lo + (hi - lo) * (k + 1) / K)));
+    }
+    std::function<void(int, int)> bisect = [&](int a, int b) {  // segments a .. b - 1
+        const int r0 = cut[a], r1 = cut[b];
+        if (r0 >= r1) return;
+        if (b - a == 1) {
+            std::sort(order.begin() + r0, order.begin() + r1,
+                      [&](int x, int y) { return len[x] != len[y] ? len[x] > len[y] : x < y; });
+            return;
+        }
+        float lo[2] = {1e30f, 1e30f}, hi[2] = {-1e30f, -1e30f};
+        for (int i = r0; i < r1; i++)
+            for (int k = 0; k < 2; k++) {
+                lo[k] = std::min(lo[k], uv[2 * order[i] + k]);
+                hi[k] = std::max(hi[k], uv[2 * order[i] + k]);
+            }
+        const int k = hi[1] - lo[1] > hi[0] - lo[0] ? 1 : 0;
+        // tiles are halved before their segments are
+        const int m = b - a > K ? a + ((b - a) / K + 1) / 2 * K : a + (b - a) / 2;
+        if (cut[m] > r0 && cut[m] < r1)
+            std::nth_element(order.begin() + r0, order.begin() + cut[m], order.begin() + r1, [&](int x, int y) {
+                return uv[2 * x + k] != uv[2 * y + k] ? uv[2 * x + k] < uv[2 * y + k] : x < y;
+            });
+        bisect(a, m);
+        bisect(m, b);
+    };
+    bisect(0, G * K);
+}
+
+// groupCtas: CTAs to tile the rows for (the group-resident solver), 0 for none.
+std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int groupCtas, std::string& err) {
     auto t = std::make_shared<Topo>();
     const int nn = s.n_nodes, nv = s.n_verts, nf = s.n_faces;
     t->n_nodes = nn;
@@ -427,6 +472,11 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, std::string& err) {
         }
     }
     t->n_slices = (nn + CS_SLICE - 1) / CS_SLICE;
+    if (groupCtas > 0) {
+        t->group_ctas = groupCtas;
+        t->group_segs = std::max(1, std::min({CS_COARSE_MAX_K, CS_GROUP_NC / (3 * groupCtas), t->n_slices / groupCtas}));
+        tileOrder(t->node_uv, len, t->group_ctas, t->group_segs, order);
+    }
     t->rowmap.assign((size_t)t->n_slices * CS_SLICE, 0);
     t->row2slot.assign(nn, 0);
     for (int r = 0; r < nn; r++) {
@@ -663,6 +713,28 @@ struct BCPlan {
     std::vector<int4> pairs;
 };
 
+// The pairs of aggregates and their stored blocks (slots with contributors; padding has none).
+void coarsePairs(const Topo& T, BCPlan& P) {
+    std::vector<std::pair<uint64_t, int>> blk;
+    blk.reserve(T.nnzb);
+    for (int sl = 0; sl < T.n_slices; sl++)
+        for (int k = 0; k < T.slice_width[sl]; k++)
+            for (int l = 0; l < T.slice_rows[sl]; l++) {
+                const int slot = (T.slice_tpanel0[sl] + k) * CS_SLICE + l;
+                if (T.tcptr[slot + 1] == T.tcptr[slot]) continue;
+                blk.emplace_back((uint64_t)P.agg[T.rowmap[sl * CS_SLICE + l]] << 32 | (uint32_t)P.agg[T.tcol[slot]], slot);
+            }
+    std::sort(blk.begin(), blk.end());
+    for (size_t i = 0; i < blk.size();) {
+        size_t j = i;
+        while (j < blk.size() && blk[j].first == blk[i].first) j++;
+        P.pairs.push_back(make_int4((int)(blk[i].first >> 32), (int)(uint32_t)blk[i].first, (int)P.contrib.size(),
+                                    (int)(P.contrib.size() + (j - i))));
+        for (size_t q = i; q < j; q++) P.contrib.push_back(blk[q].second);
+        i = j;
+    }
+}
+
 void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
     P = BCPlan();
     const int n = T.n_nodes;
@@ -696,24 +768,7 @@ void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
     P.mem.resize(n);
     std::vector<int> fill(P.mptr.begin(), P.mptr.end() - 1);
     for (int i = 0; i < n; i++) P.mem[fill[P.agg[i]]++] = i;
-    // coarse pattern: every stored block (slots with contributors; padding has none)
-    std::vector<std::tuple<int, int, int>> blk;
-    for (int sl = 0; sl < T.n_slices; sl++)
-        for (int k = 0; k < T.slice_width[sl]; k++)
-            for (int l = 0; l < T.slice_rows[sl]; l++) {
-                const int slot = (T.slice_tpanel0[sl] + k) * CS_SLICE + l;
-                if (T.tcptr[slot + 1] == T.tcptr[slot]) continue;
-                blk.emplace_back(P.agg[T.rowmap[sl * CS_SLICE + l]], P.agg[T.tcol[slot]], slot);
-            }
-    std::sort(blk.begin(), blk.end());
-    for (size_t i = 0; i < blk.size();) {
-        size_t j = i;
-        while (j < blk.size() && std::get<0>(blk[j]) == std::get<0>(blk[i]) && std::get<1>(blk[j]) == std::get<1>(blk[i])) j++;
-        P.pairs.push_back(make_int4(std::get<0>(blk[i]), std::get<1>(blk[i]), (int)P.contrib.size(),
-                                    (int)(P.contrib.size() + (j - i))));
-        for (size_t q = i; q < j; q++) P.contrib.push_back(std::get<2>(blk[q]));
-        i = j;
-    }
+    coarsePairs(T, P);
 }
 
 // Coarse-space plan of one topology on a cluster of `ncta` CTAs: each CTA's strip of rows is cut
@@ -855,6 +910,72 @@ ResidentPlan residentPlan(const Topo& T, int ncta) {
     return P;
 }
 
+// Halo plan of one topology on its group of CTAs (group.cu): per panel slot the index of its column
+// in the reading CTA's u array (own slot, or CS_RES_HALO_BIT | halo index), per slot whether another
+// CTA reads it, per CTA the topology slots it reads from others.
+struct GroupPlan {
+    std::vector<int> code, halo_ptr, halo;
+    std::vector<unsigned char> pub;
+    int max_own = 0, max_halo = 0, max_panels = 0, max_width = 0;
+    BCPlan coarse;
+};
+
+GroupPlan groupPlan(const Topo& T) {
+    GroupPlan P;
+    const int G = T.group_ctas, K = T.group_segs, ns = T.n_slices;
+    std::vector<int> owner(T.n_nodes), first(G + 1);
+    for (int c = 0; c <= G; c++) first[c] = (int)((long long)ns * c / G);
+    P.coarse.agg.resize(T.n_nodes);
+    for (int c = 0; c < G; c++) {
+        const int nsl = first[c + 1] - first[c];
+        P.max_own = std::max(P.max_own, nsl);
+        for (int sl = first[c], seg = 0; sl < first[c + 1]; sl++) {
+            while (seg + 1 < K && sl - first[c] >= nsl * (seg + 1) / K) seg++;
+            for (int l = 0; l < T.slice_rows[sl]; l++) {
+                owner[T.rowmap[sl * CS_SLICE + l]] = c;
+                P.coarse.agg[T.rowmap[sl * CS_SLICE + l]] = c * K + seg;
+            }
+        }
+    }
+    P.coarse.na = G * K;
+    P.code.assign(T.tcol.size(), 0);
+    P.pub.assign((size_t)ns * CS_SLICE, 0);
+    P.halo_ptr.push_back(0);
+    std::vector<int> need, at(T.n_nodes, -1);
+    for (int c = 0; c < G; c++) {
+        need.clear();
+        int np = 0;
+        for (int sl = first[c]; sl < first[c + 1]; sl++) {
+            np += T.slice_width[sl];
+            P.max_width = std::max(P.max_width, T.slice_width[sl]);
+            for (int k = 0; k < T.slice_width[sl]; k++)
+                for (int l = 0; l < T.slice_rows[sl]; l++) {
+                    const int col = T.tcol[(size_t)(T.slice_tpanel0[sl] + k) * CS_SLICE + l];
+                    if (owner[col] != c) need.push_back(T.row2slot[col]);
+                }
+        }
+        P.max_panels = std::max(P.max_panels, np);
+        std::sort(need.begin(), need.end());
+        need.erase(std::unique(need.begin(), need.end()), need.end());
+        P.max_halo = std::max(P.max_halo, (int)need.size());
+        for (size_t h = 0; h < need.size(); h++) {
+            P.pub[need[h]] = 1;
+            at[T.rowmap[need[h]]] = (int)h;
+        }
+        P.halo.insert(P.halo.end(), need.begin(), need.end());
+        P.halo_ptr.push_back((int)P.halo.size());
+        for (int sl = first[c]; sl < first[c + 1]; sl++)
+            for (int k = 0; k < T.slice_width[sl]; k++)
+                for (int l = 0; l < T.slice_rows[sl]; l++) {
+                    const size_t slot = (size_t)(T.slice_tpanel0[sl] + k) * CS_SLICE + l;
+                    const int col = T.tcol[slot];
+                    P.code[slot] = owner[col] == c ? T.row2slot[col] - first[c] * CS_SLICE : CS_RES_HALO_BIT | at[col];
+                }
+    }
+    coarsePairs(T, P.coarse);
+    return P;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -938,6 +1059,12 @@ struct cs_ctx {
     std::vector<int> handleNode;  // batch node of every handle, in load order (cs_set_handle_motions)
     int maxHandleMotion = -1;     // largest motion a handle follows (-1: none)
     size_t resSmem = 0;
+    // group-resident solver launch (group.cu): CTAs, threads and dynamic shared memory per CTA; its
+    // coarse spaces, in a copy of B's coarse fields; the exchange packets' bytes
+    int groupCtas = 0, groupThreads = 0;
+    size_t groupSmem = 0, groupPkBytes = 0;
+    long long groupMatFloats = 0;
+    Batch groupCoarse;
     std::vector<int> rlistAll;  // resident sheets before the proximity filter
     std::vector<int> rlistCur;  // resident sheets now
     std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, strip-local ones
@@ -1031,6 +1158,9 @@ void freeBatch(cs_ctx* c) {
     c->sheetGroupDev = nullptr;
     c->rlistAll.clear();
     c->rlistCur.clear();
+    c->groupCtas = c->groupThreads = 0;
+    c->groupSmem = c->groupPkBytes = 0;
+    c->groupCoarse = Batch();
     c->B = Batch();
     c->loaded = false;
     c->lastStepValid = false;
@@ -1068,10 +1198,12 @@ int launchAssembly(cs_ctx* c) {
 
 // The batched loop's coarse matrices of this step's systems, inverted (coarse.cu; the kernels
 // return at once for sheets the loop does not solve or when the step asks for no correction).
+int launchCoarseInverses(cs_ctx* c, const Batch& B, long long matFloats);
 int launchBatchedCoarseSetup(cs_ctx* c) {
-    Batch& B = c->B;
-    if (B.bc_total_agg <= 0) return 0;
-    cudaMemsetAsync(B.bc_mat, 0, (size_t)c->bcMatFloats * sizeof(float), c->stream);
+    return c->B.bc_total_agg > 0 ? launchCoarseInverses(c, c->B, c->bcMatFloats) : 0;
+}
+int launchCoarseInverses(cs_ctx* c, const Batch& B, long long matFloats) {
+    cudaMemsetAsync(B.bc_mat, 0, (size_t)matFloats * sizeof(float), c->stream);
     const int gx = std::max(1, std::min(256, nblk(B.bc_max_npair, 8)));
     cs_bc_assemble_kernel<<<dim3(gx, B.S), 256, 0, c->stream>>>(B);
     cs_bc_invert_small_kernel<<<B.S, CS_BC_THREADS, (CS_BC_SMALL_NC * CS_BC_SMALL_NC + 4 + 2 * CS_BC_KB * CS_BC_SMALL_NC + CS_BC_KB * CS_BC_KB) * sizeof(float),
@@ -1102,7 +1234,8 @@ int launchBatchedCoarseSetup(cs_ctx* c) {
 int assemblyKernels(const cs_ctx* c) { return (c->B.E ? 1 : 0) + 1 + (c->B.n_pinst > 0 ? 3 : 0); }
 int bcSetupKernels(const cs_ctx* c) { return c->B.bc_total_agg > 0 ? 2 + (c->B.bc_n_big > 0 ? 1 : 0) : 0; }
 int residentKernels(const cs_ctx* c) {
-    return c->resClusters > 0 ? 1 + (c->B.res_cnc > 0 && c->B.n_resident > 0 ? 1 : 0) : 0;
+    return (c->resClusters > 0 ? 1 + (c->B.res_cnc > 0 && c->B.n_resident > 0 ? 1 : 0) : 0) +
+           (c->groupCtas > 0 ? 3 + (c->groupCoarse.bc_n_big > 0 ? 1 : 0) : 0);
 }
 int tripKernels(const cs_ctx* c) { return 4 + (c->B.bc_total_agg > 0 && c->tripCoarse ? 3 : 0); }
 
@@ -1162,6 +1295,28 @@ void launchResident(cs_ctx* c, bool setup = true) {
     cudaLaunchKernelEx(&cfg, cs_resident_pcg_kernel, c->B);
 }
 
+// Sheets solved by groups of CTAs: their coarse matrices, the packets cleared, one cooperative launch
+// (its CTAs wait on one another).
+void launchGroup(cs_ctx* c) {
+    if (c->groupCtas <= 0) return;
+    Batch G = c->groupCoarse;
+    G.inst = c->B.inst;
+    G.sheet_prox = c->B.sheet_prox;
+    launchCoarseInverses(c, G, c->groupMatFloats);
+    cudaMemsetAsync(c->B.gupk, 0, c->groupPkBytes, c->stream);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3(c->groupCtas);
+    cfg.blockDim = dim3(c->groupThreads);
+    cfg.dynamicSmemBytes = c->groupSmem;
+    cfg.stream = c->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, cs_group_pcg_kernel, c->B);
+}
+
 int launchMlpInference(cs_ctx* c, float* pred);
 
 // The step up to its solve loop: assembly; the resident sheets' coarse matrices on the side
@@ -1180,6 +1335,7 @@ void launchPrelude(cs_ctx* c, bool learned) {
     launchSolvePrologue(c);
     if (fork) cudaStreamWaitEvent(c->stream, c->evJoin, 0);
     launchResident(c, false);
+    launchGroup(c);
 }
 
 // Learned warm start: features of the assembled system, layer 1, layers 2-3 + output; the
@@ -1339,6 +1495,27 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     }
     if (N >= (1LL << 31) / 9 || F >= (1LL << 31) / 32) return fail(c, CS_ERR_INVALID_ARG, "batch too large");
 
+    // Sheets of more slices than a cluster of 10 CTAs holds are tiled for the group-resident solver
+    // where the chip's CTAs hold them: up to CS_GROUP_SLICES slices a CTA (their panels about fill
+    // its shared memory), fewer while the batch's large sheets would not fill the chip.
+    cudaDeviceProp devProp;
+    CS_CUDA(cudaGetDeviceProperties(&devProp, c->device));
+    const int maxCtas = devProp.multiProcessorCount;
+    const char* clEnv = std::getenv("CS_RESIDENT_CL");
+    const bool groupsOn = !(clEnv && std::atoi(clEnv) == 0);
+    const int clusterSlices = 10 * CS_RES_MAX_WARPS;
+    long long groupSlices = 0;
+    for (int s = 0; s < n_sheets; s++) {
+        const int ns = nblk(sheets[s].n_nodes, CS_SLICE);
+        if (ns > clusterSlices && ns <= CS_GROUP_MAX_WARPS * maxCtas) groupSlices += ns;
+    }
+    const int groupTarget = (int)std::max<long long>(CS_GROUP_MIN_SLICES, std::min<long long>(CS_GROUP_SLICES, groupSlices / maxCtas));
+    auto groupCtasFor = [&](int n_nodes) {
+        const int ns = nblk(n_nodes, CS_SLICE);
+        if (!groupsOn || ns <= clusterSlices || ns > CS_GROUP_MAX_WARPS * maxCtas) return 0;
+        return std::min(maxCtas, nblk(ns, groupTarget));
+    };
+
     // topologies (shared)
     std::map<TopoKey, int> topoIndex;
     std::vector<std::shared_ptr<Topo>> topos;
@@ -1356,7 +1533,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             sheetTopoId[s] = it->second;
         } else {
             std::string err;
-            auto t = buildTopo(d, err);
+            auto t = buildTopo(d, groupCtasFor(d.n_nodes), err);
             if (!t) return fail(c, CS_ERR_INVALID_ARG, "sheet %d: %s", s, err.c_str());
             sheetTopoId[s] = (int)topos.size();
             topoIndex[k] = (int)topos.size();
@@ -1427,8 +1604,6 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         std::vector<ResidentPlan> plans;
         std::vector<char> resident;
     };
-    cudaDeviceProp devProp;
-    CS_CUDA(cudaGetDeviceProperties(&devProp, c->device));
     cudaFuncAttributes resAttr;
     CS_CUDA(cudaFuncGetAttributes(&resAttr, cs_resident_pcg_kernel));
     auto planFor = [&](int cl) {
@@ -1437,6 +1612,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         R.plans.resize(topos.size());
         R.resident.assign(topos.size(), 0);
         for (size_t t = 0; t < topos.size() && cl > 0; t++) {
+            if (topos[t]->n_slices > CS_RES_MAX_WARPS * cl) continue;  // no split fits
             R.plans[t] = residentPlan(*topos[t], cl);
             const ResidentPlan& P = R.plans[t];
             // p indices (own slots + halo) are 12-bit in the kernel's packed column codes
@@ -1591,6 +1767,51 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         for (const int4& q : P.pairs) hbc_pair.push_back(make_int4(q.x, q.y, q.z + c0, q.w + c0));
         hbc_contrib.insert(hbc_contrib.end(), P.contrib.begin(), P.contrib.end());
     }
+    // group-resident plans: the topologies tiled for a group whose rows and panels fit
+    std::vector<GroupPlan> gplans(topos.size());
+    std::vector<char> topoGroup(topos.size(), 0);
+    {
+        cudaFuncAttributes ga;
+        CS_CUDA(cudaFuncGetAttributes(&ga, cs_group_pcg_kernel));
+        const size_t optin = devProp.sharedMemPerBlockOptin - ga.sharedSizeBytes;
+        auto r2 = [](size_t n) { return (n + 1) & ~(size_t)1; };
+        auto r4 = [](size_t n) { return (n + 3) & ~(size_t)3; };
+        int warps = 0, panels = 0;
+        for (size_t t = 0; t < topos.size(); t++) {
+            const Topo& T = *topos[t];
+            if (T.group_ctas <= 0 || topoResident[t]) continue;
+            gplans[t] = groupPlan(T);
+            const GroupPlan& P = gplans[t];
+            const int nc = 3 * P.coarse.na;
+            // a quarter of the panels or more beyond shared memory: the loop streams as fast
+            if (P.max_own > CS_GROUP_MAX_WARPS || P.max_width > CS_GROUP_MAX_WIDTH || nc > CS_BC_MAX_NC ||
+                (size_t)P.max_panels * 3 / 4 * CS_PANEL_FLOATS * sizeof(float) +
+                        (2 * (size_t)P.max_own * CS_SLICE + P.max_halo) * sizeof(float4) + 24 * 1024 > optin)
+                continue;
+            topoGroup[t] = 1;
+            B.g_max = std::max(B.g_max, T.group_ctas);
+            warps = std::max(warps, P.max_own);
+            panels = std::max(panels, P.max_panels);
+            B.g_halo = std::max(B.g_halo, P.max_halo);
+            B.g_cnc = std::max(B.g_cnc, nc);
+            B.g_ck3 = std::max(B.g_ck3, 3 * T.group_segs);
+            B.g_cai = std::max(B.g_cai, 3 * T.group_segs * nc);
+        }
+        if (warps > 0) {
+            B.g_own = warps * CS_SLICE;
+            const size_t u = (2 * (size_t)B.g_own + B.g_halo) * sizeof(float4);
+            const size_t rest = (r2(3 * (size_t)B.g_max) + 2 * r2(B.g_cnc)) * sizeof(double) +
+                                (2 * r4(B.g_cnc) + r4(CS_GROUP_CE_PARTS * (size_t)B.g_ck3) + r4(B.g_cai)) * sizeof(float);
+            B.g_cap = (int)std::min<size_t>(panels, (optin - u - rest) / (CS_PANEL_FLOATS * sizeof(float)));
+            B.g_coff = (int)(B.g_cap * CS_PANEL_FLOATS * sizeof(float) + u);
+            c->groupSmem = B.g_coff + rest;
+            c->groupThreads = B.g_own;
+            CS_CUDA(raiseDynSmem((const void*)cs_group_pcg_kernel, c->groupSmem));
+            int perSM = 0;
+            CS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, cs_group_pcg_kernel, c->groupThreads, c->groupSmem));
+            if (perSM < 1) std::fill(topoGroup.begin(), topoGroup.end(), 0);
+        }
+    }
     c->resCL = c->resThreads = c->resClusters = 0;
     c->resSmem = 0;
     B.res_cnc = B.res_ck = B.res_coff = 0;
@@ -1622,6 +1843,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                 const int base = (int)hrsend.size();
                 for (int k = 0; k <= CS_RES_MAX_CL; k++) hrsendptr[t * (CS_RES_MAX_CL + 1) + k] = base + plans[t].sendptr[k];
                 hrsend.insert(hrsend.end(), plans[t].send.begin(), plans[t].send.end());
+            } else if (topoGroup[t]) {
+                for (int code : gplans[t].code) hrcode.push_back(code & CS_RES_HALO_BIT ? B.g_own + (code & ~CS_RES_HALO_BIT) : code);
             } else {
                 hrcode.insert(hrcode.end(), T.tcol.size(), 0);
             }
@@ -1675,7 +1898,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         sd.nbr_ptr_off = topoNbrPtr0[sheetTopoId[s]];
         sd.row2slot_off = topoRow2Slot0[sheetTopoId[s]];
         sd.nbr_off = topoNbr0[sheetTopoId[s]];
-        sd.resident = topoResident[sheetTopoId[s]];
+        sd.resident = topoResident[sheetTopoId[s]] ? 1 : topoGroup[sheetTopoId[s]] ? 2 : 0;
         sd.csr_ptr_off = topoCsrPtr0[sheetTopoId[s]];
         sd.panel_off = panel_off;
         {
@@ -1786,7 +2009,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     // resident sheets, largest first (the persistent clusters take them in this order)
     std::vector<int> hrlist;
     for (int s = 0; s < n_sheets; s++)
-        if (hs[s].resident) hrlist.push_back(s);
+        if (hs[s].resident == 1) hrlist.push_back(s);
     std::stable_sort(hrlist.begin(), hrlist.end(), [&](int a, int b) { return hs[a].n_slices > hs[b].n_slices; });
     B.n_resident = (int)hrlist.size();
     B.res_cap = resCap;
@@ -1802,6 +2025,77 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         c->sheetBlocks[s] = plans[sheetTopoId[s]].blocks;
         c->sheetLocalBlocks[s] = plans[sheetTopoId[s]].local_blocks;
     }
+    // Work items of the group-resident solver: sheets of the most CTAs first, each on the range of
+    // CTAs where it can start soonest (a solve's time taken as the square root of its nodes, as its
+    // CG iterations grow).  Every CTA takes its sheets in this order, so no two sheets wait on one
+    // another.
+    std::vector<GroupItem> hgitem;
+    std::vector<std::vector<int>> ctaItems(maxCtas);
+    std::vector<unsigned char> hgpub;
+    std::vector<int> hghalo_ptr, hghalo, hgcta_ptr, hgcta_item, topoPub0(topos.size(), 0), topoHalo0(topos.size(), 0);
+    std::vector<SheetDesc> hgs = hs;
+    std::vector<int4> hgc_pair;
+    std::vector<int> hgc_contrib, topoGc0(topos.size(), 0), hgc_big;
+    int gSlots = 0, gRed = 0, gMaxPair = 0;
+    long long gMat = 0;
+    {
+        for (size_t t = 0; t < topos.size(); t++) {
+            if (!topoGroup[t]) continue;
+            const GroupPlan& P = gplans[t];
+            topoPub0[t] = (int)hgpub.size();
+            hgpub.insert(hgpub.end(), P.pub.begin(), P.pub.end());
+            topoHalo0[t] = (int)hghalo_ptr.size();
+            for (int v : P.halo_ptr) hghalo_ptr.push_back(v + (int)hghalo.size());
+            hghalo.insert(hghalo.end(), P.halo.begin(), P.halo.end());
+            topoGc0[t] = (int)hgc_pair.size();
+            const int c0 = (int)hgc_contrib.size();
+            for (const int4& q : P.coarse.pairs) hgc_pair.push_back(make_int4(q.x, q.y, q.z + c0, q.w + c0));
+            hgc_contrib.insert(hgc_contrib.end(), P.coarse.contrib.begin(), P.coarse.contrib.end());
+        }
+        for (SheetDesc& d : hgs) d.bc_na = 0;
+        std::vector<int> gl;
+        for (int s = 0; s < n_sheets; s++)
+            if (hs[s].resident == 2) gl.push_back(s);
+        auto ctasOf = [&](int s) { return topos[sheetTopoId[s]]->group_ctas; };
+        std::stable_sort(gl.begin(), gl.end(), [&](int a, int b) { return ctasOf(a) > ctasOf(b); });
+        std::vector<double> busy(maxCtas, 0.0);
+        for (int s : gl) {
+            const int t = sheetTopoId[s], G = ctasOf(s), K = topos[t]->group_segs;
+            int best = 0;
+            double when = 1e300;
+            for (int o = 0; o + G <= maxCtas; o++) {
+                const double b = *std::max_element(busy.begin() + o, busy.begin() + o + G);
+                if (b < when) {
+                    when = b;
+                    best = o;
+                }
+            }
+            GroupItem gi{s, best, G, K, gSlots, gRed, topoPub0[t], topoHalo0[t], gMat};
+            for (int k = best; k < best + G; k++) {
+                busy[k] = when + std::sqrt((double)hs[s].n_nodes);
+                ctaItems[k].push_back((int)hgitem.size());
+            }
+            hgitem.push_back(gi);
+            c->groupCtas = std::max(c->groupCtas, best + G);
+            gSlots += hs[s].n_slices * CS_SLICE;
+            gRed += 2 * G * (K + 2);
+            SheetDesc& d = hgs[s];
+            const BCPlan& P = gplans[t].coarse;
+            d.bc_na = P.na;
+            d.bc_pair_off = topoGc0[t];
+            d.bc_npair = (int)P.pairs.size();
+            d.bc_mat_off = gMat;
+            gMat += (long long)(3 * P.na) * (3 * P.na);
+            gMaxPair = std::max(gMaxPair, (int)P.pairs.size());
+            if (3 * P.na > CS_BC_SMALL_NC) hgc_big.push_back(s);
+        }
+        hgcta_ptr.push_back(0);
+        for (int k = 0; k < maxCtas; k++) {
+            hgcta_item.insert(hgcta_item.end(), ctaItems[k].begin(), ctaItems[k].end());
+            hgcta_ptr.push_back((int)hgcta_item.size());
+        }
+    }
+    B.n_group = (int)hgitem.size();
     c->sheets = hs;
     c->slices = hslices;
 
@@ -1866,6 +2160,20 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     UP(rwmask, hrwmask);
     UP(cpair, hcpair);
     UP(ccontrib, hccontrib);
+    if (B.n_group > 0) {
+        UP(gitem, hgitem);
+        UP(gcta_ptr, hgcta_ptr);
+        UP(gcta_item, hgcta_item);
+        UP(gpub, hgpub);
+        UP(ghalo_ptr, hghalo_ptr);
+        UP(ghalo, hghalo);
+        UP(gc_ok, std::vector<int>(n_sheets, 0));
+        // row packets, then the reduction packets
+        if ((st = dalloc(c, &B.gupk, (size_t)gSlots + gRed)) != CS_OK) return st;
+        B.grpk = B.gupk + gSlots;
+        c->groupPkBytes = ((size_t)gSlots + gRed) * sizeof(uint4);
+        if ((st = dalloc(c, &B.gc_inv, (size_t)gMat)) != CS_OK) return st;
+    }
 #undef UP
 #define AL(field, n) \
     if ((st = dalloc(c, &B.field, (size_t)(n))) != CS_OK) return st;
@@ -1890,6 +2198,21 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     AL(cinv, B.res_cnc > 0 ? (long long)hrlist.size() * B.res_cnc * B.res_cnc : 1);
     AL(cvalid, std::max<size_t>(hrlist.size(), 1));
 #undef AL
+    if (B.n_group > 0) {
+        // the groups' coarse spaces, as the batched coarse set-up reads them
+        Batch& G = c->groupCoarse;
+        G = B;
+        G.bc_resident = 1;
+        G.bc_max_npair = gMaxPair;
+        G.bc_n_big = (int)hgc_big.size();
+        if ((st = upload(c, &G.sheets, hgs)) != CS_OK || (st = upload(c, &G.bc_pair, hgc_pair)) != CS_OK ||
+            (st = upload(c, &G.bc_contrib, hgc_contrib)) != CS_OK || (st = upload(c, &G.bc_big, hgc_big)) != CS_OK ||
+            (st = dalloc(c, &G.bc_mat, (size_t)gMat)) != CS_OK)
+            return st;
+        G.bc_inv = B.gc_inv;
+        G.bc_ok = B.gc_ok;
+        c->groupMatFloats = gMat;
+    }
     CS_CUDA(cudaMemset(B.dv, 0, 3LL * B.N * sizeof(float)));
     CS_CUDA(cudaMemcpy(B.x0, B.x, 3LL * B.N * sizeof(float), cudaMemcpyDeviceToDevice));  // Node::Node
     CS_CUDA(cudaMemset(B.warm, 0, 3LL * B.N * sizeof(float)));
@@ -2690,7 +3013,7 @@ static cs_status fillStepStats(cs_ctx* c, cs_step_stats* stats, int loop_cap, bo
     if (timed) CS_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     stats->ms = ms;
     if (loopv[0] >= loop_cap) return fail(c, CS_ERR_TIMEOUT, "solve loop hit its trip bound (%d)", loop_cap);
-    if (loopv[6]) return fail(c, CS_ERR_TIMEOUT, "cluster-resident solve: a wait on another CTA ran out");
+    if (loopv[6]) return fail(c, CS_ERR_TIMEOUT, "resident solve: a wait on another CTA ran out");
     if (capped) return fail(c, breakdown ? CS_ERR_NON_SPD : CS_ERR_NOT_CONVERGED, "%d of %d sheets did not converge",
                             c->B.S - stats->converged, c->B.S);
     return CS_OK;
@@ -2998,6 +3321,7 @@ static float timeWholeSolve(cs_ctx* c, const cs_step_params& q) {
     launchSolvePrologueAgain(c);
     cudaEventRecord(c->ev0, c->stream);
     launchResident(c);
+    launchGroup(c);
     int go = 1, trips = 0;
     while (go) {
         for (int t = 0; t < 8; t++) launchTrip(c, 0);
@@ -3111,7 +3435,7 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
         float ms[2] = {0.f, 0.f};
         for (int k = 0; k < 2; k++) {
             q.solver = k == 0 ? CS_SOLVER_AUTO : CS_SOLVER_BATCHED;
-            if (k == 0 && c->resClusters <= 0) continue;
+            if (k == 0 && c->resClusters <= 0 && c->groupCtas <= 0) continue;
             const int nrep = reps < 2 ? reps : 2;
             for (int r = 0; r <= nrep; r++) {
                 const float t = timeWholeSolve(c, q);
@@ -3119,7 +3443,7 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
                 if (r > 0) ms[k] += t / nrep;
             }
         }
-        const int bestS = (c->resClusters > 0 && ms[0] <= ms[1]) ? CS_SOLVER_AUTO : CS_SOLVER_BATCHED;
+        const int bestS = ((c->resClusters > 0 || c->groupCtas > 0) && ms[0] <= ms[1]) ? CS_SOLVER_AUTO : CS_SOLVER_BATCHED;
         c->tunedSolver = bestS;
         if (out) {
             out->solver_ms[0] = ms[0];
@@ -3261,6 +3585,7 @@ cs_status mlpEnergyPrepare(cs_ctx* c, const cs_step_params* p) {
     cs_mlp_features_kernel<<<nblk(B.N, 256), 256, 0, c->stream>>>(B, M, M.feat);
     launchSolvePrologue(c);
     launchResident(c);
+    launchGroup(c);
     int go = 1, trips = 0;
     while (go) {
         for (int t = 0; t < 8; t++) launchTrip(c, 0);

@@ -91,7 +91,7 @@ typedef struct cs_step_params {
     int advance;              /* 1: v += dv and x += dt v (a full step); 0: solve only */
     int use_graph;            /* 1: run the captured CUDA graph; 0: host-driven launches */
     int solver;               /* CS_SOLVER_*: which PCG kernels solve the sheets */
-    int precond_degree;       /* cluster-resident solver's preconditioner: 0 or 1 the 3x3
+    int precond_degree;       /* on-chip solvers' preconditioner: 0 or 1 the 3x3
                                  block-Jacobi inverse; an odd degree 3..CS_PRECOND_MAX_DEGREE a
                                  Chebyshev polynomial of that degree in the block-Jacobi-scaled
                                  matrix of each CTA's strip of rows (no exchange between CTAs).
@@ -128,8 +128,9 @@ typedef struct cs_step_params {
 #define CS_PRECOND_MAX_DEGREE 15
 
 /* CS_SOLVER_AUTO: sheets whose system fits one thread-block cluster's shared memory are
- * solved by a cluster each, the system resident on chip for the whole solve; the others by
- * the batched loop.  CS_SOLVER_BATCHED: every sheet by the batched loop (the system streamed
+ * solved by a cluster each, the system resident on chip for the whole solve; larger ones, in mixed
+ * precision, by a group of CTAs over the whole chip while their rows and panels fit its shared
+ * memory (about 80,000 nodes of a grid); the others by the batched loop.  CS_SOLVER_BATCHED: every sheet by the batched loop (the system streamed
  * from HBM every iteration).  Both run the same mixed/plain PCG to the same FP64-checked
  * tolerance. */
 #define CS_SOLVER_AUTO 0
