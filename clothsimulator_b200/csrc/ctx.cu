@@ -67,7 +67,7 @@ __global__ void cs_prox_rowcount_kernel(const ProxInst* inst, int T, int* rowCou
 __global__ void cs_prox_rowfill_kernel(const ProxInst* inst, int T, const int* rowPtr, int* rowFill, int* rowInst);
 __global__ void cs_prox_rowsort_kernel(int N, const int* rowPtr, int* rowInst);
 __global__ void cs_prox_outside_kernel(Batch B, const int* rowPtr, const int* rowInst, const ProxInst* inst,
-                                       const int* xptr, int* out);
+                                       const int* xptr, int* out, int* sheet_prox);
 __global__ void cs_contact_face_kernel(Batch B, Contact C);
 __global__ void cs_contact_node_kernel(Batch B, Contact C);
 __global__ void cs_contact_grid_kernel(Batch B, Contact C, const int* sheet_group);
@@ -1067,6 +1067,7 @@ struct cs_ctx {
     Batch groupCoarse;
     std::vector<int> rlistAll;  // resident sheets before the proximity filter
     std::vector<int> rlistCur;  // resident sheets now
+    int residentProx = 0;       // those of them that a proximity touches
     std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, strip-local ones
     // proximities (cs_set_proximities): their device lists, and the host copies of the
     // blocks outside the pattern that cs_get_system merges
@@ -1158,6 +1159,7 @@ void freeBatch(cs_ctx* c) {
     c->sheetGroupDev = nullptr;
     c->rlistAll.clear();
     c->rlistCur.clear();
+    c->residentProx = 0;
     c->groupCtas = c->groupThreads = 0;
     c->groupSmem = c->groupPkBytes = 0;
     c->groupCoarse = Batch();
@@ -2247,7 +2249,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
 cs_status cs_get_solver_info(const cs_ctx* c, int* info) {
     if (!c || !info) return CS_ERR_INVALID_ARG;
     if (!c->loaded) return CS_ERR_STATE;
-    info[0] = c->B.n_resident;
+    info[0] = c->B.n_resident - c->residentProx;
     info[1] = c->resCL;
     info[2] = c->resThreads;
     info[3] = c->resClusters;
@@ -2390,14 +2392,15 @@ cs_status applyProximities(cs_ctx* c, int n, float thickness) {
         // the lists cs_prox_outside_kernel reads through B
         B.prow_ptr = P.rowPtr;
         B.prow_inst = P.rowInst;
-        cs_prox_outside_kernel<<<nblk(B.N, 128), 128, 0, c->stream>>>(B, P.rowPtr, P.rowInst, P.inst, nullptr, P.xptr);
+        cs_prox_outside_kernel<<<nblk(B.N, 128), 128, 0, c->stream>>>(B, P.rowPtr, P.rowInst, P.inst, nullptr, P.xptr,
+                                                                       P.sheetProx);
         int X = 0;
         if ((st = scanInts(c, P.xptr, B.N, &X)) != CS_OK) return st;
         if (X > 0) {
             if ((st = grow(c, P.xcol, P.xcolCap, (size_t)X)) != CS_OK) return st;
             if ((st = grow(c, P.xval, P.xvalCap, 9 * (size_t)X)) != CS_OK) return st;
             cs_prox_outside_kernel<<<nblk(B.N, 128), 128, 0, c->stream>>>(B, P.rowPtr, P.rowInst, P.inst, P.xptr,
-                                                                           P.xcol);
+                                                                           P.xcol, nullptr);
             CS_CUDA(cudaMemsetAsync(P.xval, 0, 9 * (size_t)X * sizeof(float), c->stream));
         }
         CS_CUDA(cudaGetLastError());
@@ -2415,11 +2418,15 @@ cs_status applyProximities(cs_ctx* c, int n, float thickness) {
         B.sheet_prox = P.sheetProx;
         P.n = n;
     }
-    // sheets with proximities leave the cluster-resident kernel's work list for the batched
-    // loop (their systems carry blocks outside the pattern, which only its SpMV reads)
+    // sheets whose proximities couple nodes outside the mesh pattern leave the resident kernels for
+    // the batched loop (only its SpMV reads such blocks); others keep the pattern and stay
     std::vector<int> rl;
+    c->residentProx = 0;
     for (int s : c->rlistAll)
-        if (!touched[s]) rl.push_back(s);
+        if (!(touched[s] & 2)) {
+            rl.push_back(s);
+            c->residentProx += touched[s] ? 1 : 0;
+        }
     if (!rl.empty()) CS_CUDA(cudaMemcpy(B.rlist, rl.data(), rl.size() * sizeof(int), cudaMemcpyHostToDevice));
     B.n_resident = (int)rl.size();
     c->rlistCur = rl;

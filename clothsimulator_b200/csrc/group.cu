@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         const GroupItem gi = B.gitem[B.gcta_item[it]];
         const int s = gi.sheet;
         // sheets with proximity blocks outside the pattern are the batched loop's
-        if (B.sheet_prox && B.sheet_prox[s]) continue;
+        if (B.sheet_prox && (B.sheet_prox[s] & 2)) continue;
         const SheetDesc& sh = B.sheets[s];
         const int G = gi.ctas, rank = (int)blockIdx.x - gi.cta0, K = gi.segs, ns = sh.n_slices;
         const int lo = (int)((long long)ns * rank / G), hi = (int)((long long)ns * (rank + 1) / G), nsl = hi - lo;

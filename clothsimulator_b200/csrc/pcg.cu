@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(128) cs_solve_setup_kernel(Batch B) {
         I.scaled = 0;
         I.wscale = 1.0;
         if (sh.resident && B.params->solver == CS_SOLVER_AUTO_DEV && (sh.resident == 1 || B.params->mixed) &&
-            !(B.sheet_prox && B.sheet_prox[s]))
+            !(B.sheet_prox && (B.sheet_prox[s] & 2)))
             I.phase = PH_RESIDENT;  // solved by cs_resident_pcg_kernel or cs_group_pcg_kernel before the loop
         else
             I.phase = B.params->warm ? PH_RES : PH_INIT;

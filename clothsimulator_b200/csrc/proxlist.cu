@@ -214,9 +214,9 @@ __global__ void cs_prox_rowsort_kernel(int N, const int* rowPtr, int* rowInst) {
 }
 
 // Columns of blocks outside the mesh pattern per row: with xptr null, their number into
-// out[row]; otherwise the columns, ascending, into out[xptr[row]...].
+// out[row], and bit 1 of the sheet's mark where there are any; otherwise the columns, ascending, into out[xptr[row]...].
 __global__ void cs_prox_outside_kernel(Batch B, const int* rowPtr, const int* rowInst, const ProxInst* inst,
-                                       const int* xptr, int* out) {
+                                       const int* xptr, int* out, int* sheet_prox) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= B.N) return;
     const int q0 = rowPtr[row], q1 = rowPtr[row + 1];
@@ -242,6 +242,7 @@ __global__ void cs_prox_outside_kernel(Batch B, const int* rowPtr, const int* ro
         }
     if (!xptr) {
         out[row] = count;
+        if (count > 0) atomicOr(&sheet_prox[B.node_sheet[row]], 2);
         return;
     }
     int* seg = out + xptr[row];

@@ -164,7 +164,7 @@ cs_status cs_load_batch(cs_ctx* ctx, const cs_material_desc* materials, int n_ma
  * it while proximities are set). */
 cs_status cs_get_sizes(const cs_ctx* ctx, long long* sizes);
 
-/* info[0..10] = sheets solved cluster-resident, CTAs per cluster, threads per CTA, clusters
+/* info[0..10] = sheets solved cluster-resident (that no proximity touches), CTAs per cluster, threads per CTA, clusters
  * in the persistent grid, SELL panels per CTA in shared memory, dynamic shared memory bytes
  * per CTA; the batched SpMV's launch shape (threads per block, slices per warp, slots loaded
  * together; cs_tune); the fastest resident preconditioner cs_tune found (degree, coarse
@@ -244,8 +244,8 @@ typedef struct cs_proximity_desc {
  * nodes of other sheets enter a sheet's terms through their state at the start of the step
  * (the reference steps cloths one after another, so a later cloth there sees an earlier
  * cloth's updated velocities).  Blocks outside the mesh's pattern are kept beside it;
- * cs_get_system returns them merged.  Sheets with proximities are solved by the batched
- * loop. */
+ * cs_get_system returns them merged.  Sheets with such blocks are solved by the batched loop,
+ * the others as without proximities. */
 cs_status cs_set_proximities(cs_ctx* ctx, const cs_proximity_desc* proximities, int n, float thickness);
 
 /* Proximity detection: what Simulator::physicsStep runs before stepping the cloths
