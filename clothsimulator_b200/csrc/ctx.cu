@@ -3568,8 +3568,8 @@ void mlpEnergyForwardBackward(cs_ctx* c, int s0, int s1) {
     cs_mlp_l23_kernel<<<c->mlpGridTile, 128, MLP_SMEM_L23, c->stream>>>(B, M, n0, n1, M.z2, M.z3, M.y, M.pred);
     cs_mlp_energy_kernel<<<nblk((long long)(sl1 - sl0) * 32, 128), 128, 0, c->stream>>>(B, M, sl0, sl1);
     cs_mlp_energy_sheet_kernel<<<s1 - s0, 128, 0, c->stream>>>(B, M, s0, s1, 1);
-    cs_mlp_bwd23_kernel<<<c->mlpGridTrain, 128, MLP_SMEM_BWD23, c->stream>>>(B, M, n0, n1, nullptr);
-    cs_mlp_bwd1_kernel<<<c->mlpGridTrain, 128, MLP_SMEM_BWD1, c->stream>>>(B, M, M.feat, n0, n1);
+    cs_mlp_bwd23_kernel<<<c->mlpGridTrain, MLP_BWD_THREADS, MLP_SMEM_BWD23, c->stream>>>(B, M, n0, n1, nullptr);
+    cs_mlp_bwd1_kernel<<<c->mlpGridTrain, MLP_BWD_THREADS, MLP_SMEM_BWD1, c->stream>>>(B, M, M.feat, n0, n1);
 }
 
 // The first half of a training step: assembly for the current state, the features of that
@@ -3616,8 +3616,8 @@ void mlpForwardBackward(cs_ctx* c, int slot, int s0, int s1) {
     const float* tg = M.dtarget + (size_t)slot * B.N * 3;
     cs_mlp_l1_kernel<<<c->mlpGridTile, 128, MLP_SMEM_L1, c->stream>>>(B, M, f, n0, n1, M.z1);
     cs_mlp_l23_kernel<<<c->mlpGridTile, 128, MLP_SMEM_L23, c->stream>>>(B, M, n0, n1, M.z2, M.z3, M.y, nullptr);
-    cs_mlp_bwd23_kernel<<<c->mlpGridTrain, 128, MLP_SMEM_BWD23, c->stream>>>(B, M, n0, n1, tg);
-    cs_mlp_bwd1_kernel<<<c->mlpGridTrain, 128, MLP_SMEM_BWD1, c->stream>>>(B, M, f, n0, n1);
+    cs_mlp_bwd23_kernel<<<c->mlpGridTrain, MLP_BWD_THREADS, MLP_SMEM_BWD23, c->stream>>>(B, M, n0, n1, tg);
+    cs_mlp_bwd1_kernel<<<c->mlpGridTrain, MLP_BWD_THREADS, MLP_SMEM_BWD1, c->stream>>>(B, M, f, n0, n1);
 }
 
 }  // namespace

@@ -460,23 +460,34 @@ __global__ void __launch_bounds__(128, 4) cs_mlp_l23_kernel(Batch B, MlpDev M, i
 // M.dy, ga and gb per sheet in M.sheet_scale; dL/dy = sigma_y dL/dp); its value comes from those
 // kernels.  Writes du2 (N x 128) for
 // layer 1's backward and this CTA's gradient partials of W2, b2, W3, b3, W4, b4 and of the loss.
-__global__ void __launch_bounds__(128) cs_mlp_bwd23_kernel(Batch B, MlpDev M, int n0, int n1,
-                                                         const float* __restrict__ target) {
+//
+// 512 threads per CTA (one CTA per SM: the tile's FP32 operands fill its shared memory).  What
+// bounds it: the FP32 products of the weight gradients (12,288 multiply-adds a node) and their
+// shared-memory reads, so a warp owns four rows of dW2 and dW3 (one broadcast 16-byte read of dz
+// per node) and a lane 4 or 2 of their columns; element-wise phases run over contiguous memory, and
+// TMEM rows are read by four warps each, a quarter of the columns per warp.  With 128 threads, a
+// node per thread in the element-wise phases and a row per thread pair in the products, a minibatch
+// of 16 sheets of 64 x 64 took 499 us on a B200.  Every sum runs over the tile's nodes in order.
+#define MLP_BWD_LD 68  // floats per node row of the shared operands: 16-byte rows, 4 banks apart
+__global__ void __launch_bounds__(MLP_BWD_THREADS, 1) cs_mlp_bwd23_kernel(Batch B, MlpDev M, int n0, int n1,
+                                                                        const float* __restrict__ target) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    float* sDZ = reinterpret_cast<float*>(smem);                 // 128 x 65 fp32 (dz3, then dz2)
-    float* sX = reinterpret_cast<float*>(smem + 33280);          // 128 x 65 fp32 (h3, then h2)
-    __nv_bfloat16* sU = reinterpret_cast<__nv_bfloat16*>(smem + 66560);  // 128 x 136 bf16 (u2)
-    unsigned char* sA = smem + 101376;                           // 128 x 64 bf16 MMA operand
-    unsigned char* sW3t = smem + 117760;                         // 64 x 64 bf16 (W3^T)
-    unsigned char* sW2t = smem + 125952;                         // 128 x 64 bf16 (W2^T)
-    float* sf = reinterpret_cast<float*>(smem + 142336);         // W4 (192), mu_y, sigma_y, dy (128 x 4)
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 142336 + 2880);
+    constexpr int LD = MLP_BWD_LD, TILE = 128 * LD * 4;
+    float* sDZ = reinterpret_cast<float*>(smem);                 // 128 x 64 fp32 (dz3, then dz2)
+    float* sX = reinterpret_cast<float*>(smem + TILE);           // 128 x 64 fp32 (h3, then h2)
+    __nv_bfloat16* sU = reinterpret_cast<__nv_bfloat16*>(smem + 2 * TILE);  // 128 x 128 bf16 (u2), rows of 136
+    unsigned char* sA = smem + 3 * TILE;                         // 128 x 64 bf16 MMA operand
+    unsigned char* sW3t = sA + 16384;                            // 64 x 64 bf16 (W3^T)
+    unsigned char* sW2t = sW3t + 8192;                           // 128 x 64 bf16 (W2^T)
+    float* sf = reinterpret_cast<float*>(sW2t + 16384);          // W4 (192), mu_y, sigma_y, dy (128 x 4), loss (128)
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sf + 840);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 1);
     float* sDY = sf + 200;
-    const int t = threadIdx.x, warp = t >> 5;
+    float* sL = sf + 712;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     load_weight_tile(M.wb + MLP_W3, 64, 64, true, sW3t);
     load_weight_tile(M.wb + MLP_W2, 64, 128, true, sW2t);
-    for (int e = t; e < 192; e += 128) sf[e] = __bfloat162float(M.wb[MLP_W4 + e]);
+    for (int e = t; e < 192; e += MLP_BWD_THREADS) sf[e] = __bfloat162float(M.wb[MLP_W4 + e]);
     if (t < 3) {
         sf[192 + t] = M.stats[32 + t];
         sf[195 + t] = M.stats[35 + t];
@@ -489,42 +500,58 @@ __global__ void __launch_bounds__(128) cs_mlp_bwd23_kernel(Batch B, MlpDev M, in
     uint32_t phase = 0;
     bool ok = true;
     const float scale = 2.0f / (float)max(n1 - n0, 1);
-    // owned accumulators: row r of W2/W3 (columns half h), column t of W4, biases
-    const int r = t >> 1, hf = t & 1;
-    float acc2[64], acc3[32];
+    // rows 4 warp .. 4 warp + 3 of W2 (columns 4 lane ..) and W3 (columns 2 lane ..)
+    float acc2[4][4], acc3[4][2];
 #pragma unroll
-    for (int c = 0; c < 64; c++) acc2[c] = 0.f;
+    for (int i = 0; i < 4; i++) {
 #pragma unroll
-    for (int c = 0; c < 32; c++) acc3[c] = 0.f;
-    float acc4[3] = {0.f, 0.f, 0.f}, accb2 = 0.f, accb3 = 0.f, accb4 = 0.f, loss = 0.f;
+        for (int c = 0; c < 4; c++) acc2[i][c] = 0.f;
+        acc3[i][0] = acc3[i][1] = 0.f;
+    }
+    float acc4 = 0.f, accb2 = 0.f, accb3 = 0.f, accb4 = 0.f, loss = 0.f;
+    // this thread's TMEM row (a node of the tile) and quarter of the columns
+    const int trow = 32 * (warp & 3) + lane, tq = warp >> 2;
     const int ntiles = (n1 - n0 + 127) / 128;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const int node = n0 + tile * 128 + t;
-        const bool valid = node < n1;
+        const int base = n0 + tile * 128, rows = min(128, n1 - base);
         // 1. dy, h3, dz3
-        float dy[3] = {0.f, 0.f, 0.f};
-        if (valid && target) {
-            for (int i = 0; i < 3; i++) {
-                const float tt = (target[3 * (size_t)node + i] - sf[192 + i]) / sf[195 + i];
-                const float d = M.y[3 * (size_t)node + i] - tt;
-                loss += d * d;
-                dy[i] = scale * d;
+        if (t < 128) {
+            const int node = base + t;
+            float dy[3] = {0.f, 0.f, 0.f};
+            if (t < rows && target) {
+                for (int i = 0; i < 3; i++) {
+                    const float tt = (target[3 * (size_t)node + i] - sf[192 + i]) / sf[195 + i];
+                    const float d = M.y[3 * (size_t)node + i] - tt;
+                    loss += d * d;
+                    dy[i] = scale * d;
+                }
+            } else if (t < rows) {
+                const int sh = B.node_sheet[node];
+                const float ga = M.sheet_scale[2 * sh], gb = M.sheet_scale[2 * sh + 1];
+                for (int i = 0; i < 3; i++)
+                    dy[i] = (ga * M.dy[3 * (size_t)node + i] - gb * B.b[3 * (size_t)node + i]) * sf[195 + i];
             }
-        } else if (valid) {
-            const int sh = B.node_sheet[node];
-            const float ga = M.sheet_scale[2 * sh], gb = M.sheet_scale[2 * sh + 1];
-            for (int i = 0; i < 3; i++)
-                dy[i] = (ga * M.dy[3 * (size_t)node + i] - gb * B.b[3 * (size_t)node + i]) * sf[195 + i];
+            for (int i = 0; i < 3; i++) sDY[4 * t + i] = dy[i];
         }
-        for (int i = 0; i < 3; i++) sDY[4 * t + i] = dy[i];
-        for (int j = 0; j < 64; j++) {
-            const float z = valid ? M.z3[64 * (size_t)node + j] : 0.f;
-            const float h = valid ? silu(z) : 0.f;
-            const float dh = dy[0] * sf[j] + dy[1] * sf[64 + j] + dy[2] * sf[128 + j];
-            const float dz = valid ? dh * silu_grad(z) : 0.f;
-            sX[65 * t + j] = h;
-            sDZ[65 * t + j] = dz;
-            tc::st_bf16(sA, 128, t, j, dz);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int e = t + MLP_BWD_THREADS * k, n = e >> 4, j = 4 * (e & 15);
+            const float4 z = n < rows ? __ldg(reinterpret_cast<const float4*>(M.z3 + 64 * (size_t)(base + n) + j))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float zz[4] = {z.x, z.y, z.z, z.w};
+            float h[4], dz[4];
+            __align__(8) __nv_bfloat16 db[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                h[c] = n < rows ? silu(zz[c]) : 0.f;
+                const float dh = sDY[4 * n] * sf[j + c] + sDY[4 * n + 1] * sf[64 + j + c] + sDY[4 * n + 2] * sf[128 + j + c];
+                dz[c] = n < rows ? dh * silu_grad(zz[c]) : 0.f;
+                db[c] = __float2bfloat16_rn(dz[c]);
+            }
+            *reinterpret_cast<float4*>(sX + LD * n + j) = make_float4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<float4*>(sDZ + LD * n + j) = make_float4(dz[0], dz[1], dz[2], dz[3]);
+            *reinterpret_cast<uint2*>(sA + tc::kmajor_offset(128, n, j)) = *reinterpret_cast<const uint2*>(db);
         }
         tc::fence_async_shared();
         sync_tmem();
@@ -533,66 +560,111 @@ __global__ void __launch_bounds__(128) cs_mlp_bwd23_kernel(Batch B, MlpDev M, in
             tc::gemm_tile(tmem, tc::smem_u32(sA), tc::smem_u32(sW3t), 64, 64, false);
             tc::mma_commit(bar);
         }
-        if (t < 64) {
-            for (int n = 0; n < 128; n++) {
-                const float h = sX[65 * n + t];
-                acc4[0] += sDY[4 * n] * h;
-                acc4[1] += sDY[4 * n + 1] * h;
-                acc4[2] += sDY[4 * n + 2] * h;
-            }
-        } else if (t < 67) {
-            for (int n = 0; n < 128; n++) accb4 += sDY[4 * n + (t - 64)];
+        if (t < 192) {
+            const int i = t >> 6, j = t & 63;
+#pragma unroll 8
+            for (int n = 0; n < 128; n++) acc4 += sDY[4 * n + i] * sX[LD * n + j];
+        } else if (t < 195) {
+            for (int n = 0; n < 128; n++) accb4 += sDY[4 * n + (t - 192)];
+        } else if (t >= 256 && t < 320) {
+#pragma unroll 8
+            for (int n = 0; n < 128; n++) accb3 += sDZ[LD * n + (t - 256)];
         }
-        if (hf == 0)
-            for (int n = 0; n < 128; n++) accb3 += sDZ[65 * n + r];
         __syncthreads();
         // 3. h2 = bf16(SiLU(z2)) and dW3
-        for (int j = 0; j < 64; j++) sX[65 * t + j] = valid ? bf(silu(M.z2[64 * (size_t)node + j])) : 0.f;
-        __syncthreads();
-        for (int n = 0; n < 128; n++) {
-            const float d = sDZ[65 * n + r];
 #pragma unroll
-            for (int c = 0; c < 32; c++) acc3[c] += d * sX[65 * n + 32 * hf + c];
+        for (int k = 0; k < 4; k++) {
+            const int e = t + MLP_BWD_THREADS * k, n = e >> 4, j = 4 * (e & 15);
+            float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (n < rows) {
+                z = __ldg(reinterpret_cast<const float4*>(M.z2 + 64 * (size_t)(base + n) + j));
+                z = make_float4(bf(silu(z.x)), bf(silu(z.y)), bf(silu(z.z)), bf(silu(z.w)));
+            }
+            *reinterpret_cast<float4*>(sX + LD * n + j) = z;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int n = 0; n < 128; n++) {
+            const float4 d = *reinterpret_cast<const float4*>(sDZ + LD * n + 4 * warp);
+            const float2 x = *reinterpret_cast<const float2*>(sX + LD * n + 2 * lane);
+            const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                acc3[i][0] += dd[i] * x.x;
+                acc3[i][1] += dd[i] * x.y;
+            }
         }
         ok = __syncthreads_and(tc::mbar_wait(bar, phase) ? 1 : 0) != 0;
         phase ^= 1;
         tc::fence_after_sync();
         if (!ok) break;
-        // 4. dz2 = dh2 * SiLU'(z2); u2 rebuilt
-        float dz2[64];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
+        // 4. dz2 = dh2 * SiLU'(z2); u2 rebuilt, four threads per node
+        float dz2[16];
+        {
             float dh[16];
-            tc::tmem_ld16(tc::tmem_addr(tmem, warp, 16 * q), dh);
+            tc::tmem_ld16(tc::tmem_addr(tmem, warp & 3, 16 * tq), dh);
+            const float4* z = reinterpret_cast<const float4*>(M.z2 + 64 * (size_t)(base + trow) + 16 * tq);
 #pragma unroll
-            for (int c = 0; c < 16; c++)
-                dz2[16 * q + c] = valid ? dh[c] * silu_grad(M.z2[64 * (size_t)node + 16 * q + c]) : 0.f;
-        }
-        if (valid) {
-            const __nv_bfloat16* hi = M.h1 + 64 * (size_t)node;
-            Nbr nb = neighbours(B, node);
-            const float inv = nb.end > nb.beg ? 1.0f / (nb.end - nb.beg) : 0.f;
-            for (int j = 0; j < 64; j++) sU[136 * t + j] = hi[j];
-            for (int q = 0; q < 4; q++) {
-                float acc[16];
-#pragma unroll
-                for (int c = 0; c < 16; c++) acc[c] = 0.f;
-                for (int k = nb.beg; k < nb.end; k++) {
-                    const __nv_bfloat16* hj = M.h1 + 64 * (size_t)(B.nbr[k] + nb.off) + 16 * q;
-#pragma unroll
-                    for (int c = 0; c < 16; c++) acc[c] += __bfloat162float(hj[c]);
-                }
-#pragma unroll
-                for (int c = 0; c < 16; c++) sU[136 * t + 64 + 16 * q + c] = __float2bfloat16_rn(acc[c] * inv);
+            for (int c = 0; c < 4; c++) {
+                const float4 v = trow < rows ? __ldg(z + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                dz2[4 * c] = trow < rows ? dh[4 * c] * silu_grad(v.x) : 0.f;
+                dz2[4 * c + 1] = trow < rows ? dh[4 * c + 1] * silu_grad(v.y) : 0.f;
+                dz2[4 * c + 2] = trow < rows ? dh[4 * c + 2] * silu_grad(v.z) : 0.f;
+                dz2[4 * c + 3] = trow < rows ? dh[4 * c + 3] * silu_grad(v.w) : 0.f;
             }
-        } else {
-            for (int j = 0; j < 128; j++) sU[136 * t + j] = __float2bfloat16_rn(0.f);
+        }
+        {
+            const int n = t >> 2, q = t & 3;
+            uint4 own[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+            float acc[16];
+#pragma unroll
+            for (int c = 0; c < 16; c++) acc[c] = 0.f;
+            float inv = 0.f;
+            if (n < rows) {
+                const uint4* hi = reinterpret_cast<const uint4*>(M.h1 + 64 * (size_t)(base + n) + 16 * q);
+                own[0] = __ldg(hi);
+                own[1] = __ldg(hi + 1);
+                const Nbr nb = neighbours(B, base + n);
+                inv = nb.end > nb.beg ? 1.0f / (nb.end - nb.beg) : 0.f;
+                for (int k0 = nb.beg; k0 < nb.end; k0 += 4) {
+                    uint4 v[4][2];
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (k0 + k < nb.end) {
+                            const uint4* hj =
+                                reinterpret_cast<const uint4*>(M.h1 + 64 * (size_t)(__ldg(B.nbr + k0 + k) + nb.off) + 16 * q);
+                            v[k][0] = __ldg(hj);
+                            v[k][1] = __ldg(hj + 1);
+                        }
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (k0 + k < nb.end) {
+                            const __nv_bfloat16* hv = reinterpret_cast<const __nv_bfloat16*>(v[k]);
+#pragma unroll
+                            for (int c = 0; c < 16; c++) acc[c] += __bfloat162float(hv[c]);
+                        }
+                }
+            }
+            __align__(16) __nv_bfloat16 ab[16];
+#pragma unroll
+            for (int c = 0; c < 16; c++) ab[c] = __float2bfloat16_rn(acc[c] * inv);
+            uint4* u = reinterpret_cast<uint4*>(sU + 136 * n + 16 * q);
+            u[0] = own[0];
+            u[1] = own[1];
+            u[8] = reinterpret_cast<const uint4*>(ab)[0];
+            u[9] = reinterpret_cast<const uint4*>(ab)[1];
         }
         sync_tmem();  // every thread is done reading dz3 (sDZ) for dW3
+        {
+            __align__(16) __nv_bfloat16 db[16];
 #pragma unroll
-        for (int j = 0; j < 64; j++) {
-            sDZ[65 * t + j] = dz2[j];
-            tc::st_bf16(sA, 128, t, j, dz2[j]);
+            for (int c = 0; c < 4; c++)
+                *reinterpret_cast<float4*>(sDZ + LD * trow + 16 * tq + 4 * c) =
+                    make_float4(dz2[4 * c], dz2[4 * c + 1], dz2[4 * c + 2], dz2[4 * c + 3]);
+#pragma unroll
+            for (int c = 0; c < 16; c++) db[c] = __float2bfloat16_rn(dz2[c]);
+            *reinterpret_cast<uint4*>(sA + tc::kmajor_offset(128, trow, 16 * tq)) = reinterpret_cast<const uint4*>(db)[0];
+            *reinterpret_cast<uint4*>(sA + tc::kmajor_offset(128, trow, 16 * tq + 8)) = reinterpret_cast<const uint4*>(db)[1];
         }
         tc::fence_async_shared();
         sync_tmem();
@@ -601,23 +673,33 @@ __global__ void __launch_bounds__(128) cs_mlp_bwd23_kernel(Batch B, MlpDev M, in
             tc::gemm_tile(tmem + 64, tc::smem_u32(sA), tc::smem_u32(sW2t), 64, 128, false);
             tc::mma_commit(bar);
         }
+#pragma unroll 4
         for (int n = 0; n < 128; n++) {
-            const float d = sDZ[65 * n + r];
+            const float4 d = *reinterpret_cast<const float4*>(sDZ + LD * n + 4 * warp);
+            const uint2 xb = *reinterpret_cast<const uint2*>(sU + 136 * n + 4 * lane);
+            const __nv_bfloat16* xv = reinterpret_cast<const __nv_bfloat16*>(&xb);
+            const float dd[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-            for (int c = 0; c < 64; c++) acc2[c] += d * __bfloat162float(sU[136 * n + 64 * hf + c]);
-            if (hf == 0) accb2 += d;
+            for (int c = 0; c < 4; c++) {
+                const float x = __bfloat162float(xv[c]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc2[i][c] += dd[i] * x;
+            }
         }
+        if (t < 64)
+#pragma unroll 8
+            for (int n = 0; n < 128; n++) accb2 += sDZ[LD * n + t];
         ok = __syncthreads_and(tc::mbar_wait(bar, phase) ? 1 : 0) != 0;
         phase ^= 1;
         tc::fence_after_sync();
         if (!ok) break;
         // 6. du2 out
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
+        for (int h = 0; h < 2; h++) {
             float du[16];
-            tc::tmem_ld16(tc::tmem_addr(tmem, warp, 64 + 16 * q), du);
-            if (valid) {
-                float4* dst = reinterpret_cast<float4*>(M.du2 + 128 * (size_t)node + 16 * q);
+            tc::tmem_ld16(tc::tmem_addr(tmem, warp & 3, 64 + 32 * tq + 16 * h), du);
+            if (trow < rows) {
+                float4* dst = reinterpret_cast<float4*>(M.du2 + 128 * (size_t)(base + trow) + 32 * tq + 16 * h);
 #pragma unroll
                 for (int c = 0; c < 4; c++) dst[c] = make_float4(du[4 * c], du[4 * c + 1], du[4 * c + 2], du[4 * c + 3]);
             }
@@ -630,92 +712,136 @@ __global__ void __launch_bounds__(128) cs_mlp_bwd23_kernel(Batch B, MlpDev M, in
     // this CTA's partials
     float* gp = M.gpart + (size_t)blockIdx.x * MLP_P;
 #pragma unroll
-    for (int c = 0; c < 64; c++) gp[MLP_W2 + 128 * r + 64 * hf + c] = acc2[c];
+    for (int i = 0; i < 4; i++) {
 #pragma unroll
-    for (int c = 0; c < 32; c++) gp[MLP_W3 + 64 * r + 32 * hf + c] = acc3[c];
-    if (hf == 0) {
-        gp[MLP_B2 + r] = accb2;
-        gp[MLP_B3 + r] = accb3;
+        for (int c = 0; c < 4; c++) gp[MLP_W2 + 128 * (4 * warp + i) + 4 * lane + c] = acc2[i][c];
+#pragma unroll
+        for (int c = 0; c < 2; c++) gp[MLP_W3 + 64 * (4 * warp + i) + 2 * lane + c] = acc3[i][c];
     }
-    if (t < 64)
-        for (int i = 0; i < 3; i++) gp[MLP_W4 + 64 * i + t] = acc4[i];
-    else if (t < 67)
-        gp[MLP_B4 + t - 64] = accb4;
+    if (t < 64) gp[MLP_B2 + t] = accb2;
+    if (t >= 256 && t < 320) gp[MLP_B3 + t - 256] = accb3;
+    if (t < 192) gp[MLP_W4 + t] = acc4;
+    else if (t < 195) gp[MLP_B4 + t - 192] = accb4;
     // loss partial (fixed-order block sum)
-    __shared__ float sl[128];
-    sl[t] = loss;
+    if (t < 128) sL[t] = loss;
     __syncthreads();
     if (t == 0) {
         float s = 0.f;
-        for (int i = 0; i < 128; i++) s += sl[i];
+        for (int i = 0; i < 128; i++) s += sL[i];
         M.loss_part[blockIdx.x] = s / (float)max(n1 - n0, 1);
     }
 }
 
 // Backward into layer 1 over nodes [n0, n1): dh1_i = du2_i[0:64] + sum over neighbours j of
 // du2_j[64:128] / deg_j (the transpose of the mean aggregation), dz1 = dh1 * SiLU'(z1),
-// and this CTA's partials of W1, b1.
-__global__ void __launch_bounds__(128) cs_mlp_bwd1_kernel(Batch B, MlpDev M, const float* __restrict__ fsrc, int n0,
-                                                        int n1) {
+// and this CTA's partials of W1, b1.  Four threads per node gather 16 of its 64 columns each; a warp
+// owns four rows of dW1, a lane one column (as in cs_mlp_bwd23_kernel; 233 us before, with a node
+// per thread, for a minibatch of 16 sheets of 64 x 64).
+__global__ void __launch_bounds__(MLP_BWD_THREADS) cs_mlp_bwd1_kernel(Batch B, MlpDev M, const float* __restrict__ fsrc,
+                                                                    int n0, int n1) {
     extern __shared__ __align__(16) float dyn[];
-    float* sDZ = dyn;                 // 128 x 65
-    float* sU = dyn + 128 * 65;       // 128 x 33
-    float* sst = sU + 128 * 33;       // 32
-    const int t = threadIdx.x;
+    constexpr int LD = MLP_BWD_LD, LU = 36;
+    float* sDZ = dyn;               // 128 x 64
+    float* sU = dyn + 128 * LD;     // 128 x 32
+    float* sst = sU + 128 * LU;     // 32
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     if (t < 32) sst[t] = M.stats[t];
     __syncthreads();
-    const int r = t >> 1, hf = t & 1;
-    float acc1[16], accb1 = 0.f;
-#pragma unroll
-    for (int c = 0; c < 16; c++) acc1[c] = 0.f;
+    float acc1[4] = {0.f, 0.f, 0.f, 0.f}, accb1 = 0.f;
+    const int n = t >> 2, q = t & 3;
     const int ntiles = (n1 - n0 + 127) / 128;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int node = n0 + tile * 128 + t;
+        const int node = n0 + tile * 128 + n;
         const bool valid = node < n1;
         if (valid) {
-            Nbr nb = neighbours(B, node);
-            float dh[64];
-            for (int j = 0; j < 64; j++) dh[j] = M.du2[128 * (size_t)node + j];
-            for (int k = nb.beg; k < nb.end; k++) {
-                const int g = B.nbr[k] + nb.off;
-                const SheetDesc& sh = B.sheets[B.node_sheet[g]];
-                const int lg = g - sh.node_off;
-                const int deg = B.nbr_ptr[sh.nbr_ptr_off + lg + 1] - B.nbr_ptr[sh.nbr_ptr_off + lg];
-                const float w = 1.0f / (float)deg;
-                for (int j = 0; j < 64; j++) dh[j] += M.du2[128 * (size_t)g + 64 + j] * w;
+            const SheetDesc& sh = B.sheets[B.node_sheet[node]];
+            const int* np = B.nbr_ptr + sh.nbr_ptr_off;  // the neighbours are of the same sheet
+            const int beg = sh.nbr_off + np[node - sh.node_off], end = sh.nbr_off + np[node - sh.node_off + 1];
+            float dh[16];
+            {
+                const float4* d = reinterpret_cast<const float4*>(M.du2 + 128 * (size_t)node + 16 * q);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const float4 v = __ldg(d + c);
+                    dh[4 * c] = v.x;
+                    dh[4 * c + 1] = v.y;
+                    dh[4 * c + 2] = v.z;
+                    dh[4 * c + 3] = v.w;
+                }
             }
-            for (int j = 0; j < 64; j++) sDZ[65 * t + j] = dh[j] * silu_grad(M.z1[64 * (size_t)node + j]);
+            const float4 x = __ldg(reinterpret_cast<const float4*>(fsrc + 16 * (size_t)node) + q);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int k0 = beg; k0 < end; k0 += 2) {
+                float4 v[2][4], xj[2];
+                float w[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    if (k0 + k < end) {
+                        const int lg = __ldg(B.nbr + k0 + k);
+                        w[k] = 1.0f / (float)(__ldg(np + lg + 1) - __ldg(np + lg));
+                        const float4* d = reinterpret_cast<const float4*>(M.du2 + 128 * (size_t)(lg + sh.node_off) + 64 + 16 * q);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) v[k][c] = __ldg(d + c);
+                        xj[k] = __ldg(reinterpret_cast<const float4*>(fsrc + 16 * (size_t)(lg + sh.node_off)) + q);
+                    }
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    if (k0 + k < end) {
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            dh[4 * c] += v[k][c].x * w[k];
+                            dh[4 * c + 1] += v[k][c].y * w[k];
+                            dh[4 * c + 2] += v[k][c].z * w[k];
+                            dh[4 * c + 3] += v[k][c].w * w[k];
+                        }
+                        acc[0] += xj[k].x;
+                        acc[1] += xj[k].y;
+                        acc[2] += xj[k].z;
+                        acc[3] += xj[k].w;
+                    }
+            }
+            const float4* z = reinterpret_cast<const float4*>(M.z1 + 64 * (size_t)node + 16 * q);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float4 v = __ldg(z + c);
+                *reinterpret_cast<float4*>(sDZ + LD * n + 16 * q + 4 * c) =
+                    make_float4(dh[4 * c] * silu_grad(v.x), dh[4 * c + 1] * silu_grad(v.y), dh[4 * c + 2] * silu_grad(v.z),
+                                dh[4 * c + 3] * silu_grad(v.w));
+            }
             // u1 = bf16([x, agg(x)]) as in the forward pass
-            const float* x = fsrc + 16 * (size_t)node;
-            float acc[16];
-            for (int c = 0; c < 16; c++) {
-                sU[33 * t + c] = bf((x[c] - sst[c]) / sst[16 + c]);
-                acc[c] = 0.f;
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+            const float inv = end > beg ? 1.0f / (end - beg) : 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float mu = sst[4 * q + c], sg = sst[16 + 4 * q + c];
+                sU[LU * n + 4 * q + c] = bf((xs[c] - mu) / sg);
+                sU[LU * n + 16 + 4 * q + c] = end > beg ? bf((acc[c] * inv - mu) / sg) : 0.f;
             }
-            for (int k = nb.beg; k < nb.end; k++) {
-                const float* xj = fsrc + 16 * (size_t)(B.nbr[k] + nb.off);
-                for (int c = 0; c < 16; c++) acc[c] += xj[c];
-            }
-            const float inv = nb.end > nb.beg ? 1.0f / (nb.end - nb.beg) : 0.f;
-            for (int c = 0; c < 16; c++)
-                sU[33 * t + 16 + c] = nb.end > nb.beg ? bf((acc[c] * inv - sst[c]) / sst[16 + c]) : 0.f;
         } else {
-            for (int j = 0; j < 64; j++) sDZ[65 * t + j] = 0.f;
-            for (int c = 0; c < 32; c++) sU[33 * t + c] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 16; c++) sDZ[LD * n + 16 * q + c] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; c++) sU[LU * n + 8 * q + c] = 0.f;
         }
         __syncthreads();
-        for (int n = 0; n < 128; n++) {
-            const float d = sDZ[65 * n + r];
-#pragma unroll
-            for (int c = 0; c < 16; c++) acc1[c] += d * sU[33 * n + 16 * hf + c];
-            if (hf == 0) accb1 += d;
+#pragma unroll 8
+        for (int k = 0; k < 128; k++) {
+            const float4 d = *reinterpret_cast<const float4*>(sDZ + LD * k + 4 * warp);
+            const float u = sU[LU * k + lane];
+            acc1[0] += d.x * u;
+            acc1[1] += d.y * u;
+            acc1[2] += d.z * u;
+            acc1[3] += d.w * u;
         }
+        if (t < 64)
+#pragma unroll 8
+            for (int k = 0; k < 128; k++) accb1 += sDZ[LD * k + t];
         __syncthreads();
     }
     float* gp = M.gpart + (size_t)blockIdx.x * MLP_P;
 #pragma unroll
-    for (int c = 0; c < 16; c++) gp[MLP_W1 + 32 * r + 16 * hf + c] = acc1[c];
-    if (hf == 0) gp[MLP_B1 + r] = accb1;
+    for (int i = 0; i < 4; i++) gp[MLP_W1 + 32 * (4 * warp + i) + lane] = acc1[i];
+    if (t < 64) gp[MLP_B1 + t] = accb1;
 }
 
 // Sums the per-CTA gradient partials in CTA order (deterministic), then one Adam step

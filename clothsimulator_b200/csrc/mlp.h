@@ -58,10 +58,12 @@ __global__ void cs_mlp_energy_norm_kernel(Batch B, MlpDev M, int sl0, int sl1);
 __global__ void cs_mlp_energy_sheet_kernel(Batch B, MlpDev M, int s0, int s1, int mode);
 __global__ void cs_mlp_energy_loss_kernel(MlpDev M, int s0, int s1, float* acc);
 
+// threads per CTA of the backward kernels
+#define MLP_BWD_THREADS 512
 // dynamic shared memory of the tile kernels (bytes)
 #define MLP_SMEM_L1 12816
 #define MLP_SMEM_L23 51216
-#define MLP_SMEM_BWD23 145232
-#define MLP_SMEM_BWD1 50304
+#define MLP_SMEM_BWD23 (3 * 128 * 68 * 4 + 16384 + 8192 + 16384 + 840 * 4 + 16)
+#define MLP_SMEM_BWD1 ((128 * 68 + 128 * 36 + 32) * 4)
 
 #endif
