@@ -285,7 +285,10 @@ struct Batch {
     double* part = nullptr;      // 2 per slice
     InstState* inst = nullptr;
     DevParams* params = nullptr;
-    int* loop = nullptr;         // [0] loop trip counter, [1] instances not done, [5] resident work counter
+    // [0] loop trip counter, [1] instances not done, [2] a trip's finished blocks, [3] go on, [4] trips
+    // since load, [5] resident work counter, [6] error word, [7] checksum (cs_tune), [8], [9] the solve
+    // set-up's finished blocks and instances that the loop solves
+    int* loop = nullptr;
     // cluster-resident solver (resident.cu)
     int n_resident = 0;          // sheets listed in rlist
     int res_cap = 0;             // panels per CTA held in shared memory

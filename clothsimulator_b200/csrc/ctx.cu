@@ -41,7 +41,7 @@ __global__ void cs_reduce1_kernel(Batch B);
 __global__ void cs_vector_kernel(Batch B);
 __global__ void cs_reduce2_kernel(Batch B, cudaGraphConditionalHandle handle);
 __global__ void cs_solve_prologue_kernel(Batch B);
-__global__ void cs_solve_setup_kernel(Batch B);
+__global__ void cs_solve_setup_kernel(Batch B, cudaGraphConditionalHandle handle);
 __global__ void cs_advance_kernel(Batch B);
 __global__ void cs_spmv_plain_kernel(Batch B, const float* x, float* y);
 __global__ void cs_profile_setup_kernel(Batch B, int phase);
@@ -1256,9 +1256,9 @@ cs_status setTripCoarse(cs_ctx* c, bool on) {
     return CS_OK;
 }
 
-void launchSolvePrologue(cs_ctx* c) {
+void launchSolvePrologue(cs_ctx* c, cudaGraphConditionalHandle h = 0) {
     Batch& B = c->B;
-    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B);
+    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B, h);
     launchBatchedCoarseSetup(c);
     cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
 }
@@ -1324,7 +1324,7 @@ int launchMlpInference(cs_ctx* c, float* pred);
 // The step up to its solve loop: assembly; the resident sheets' coarse matrices on the side
 // stream while the learned inference (when asked) and the solve set-up run on the main stream;
 // the join; the cluster-resident solve.  Captured into the step graph, or launched directly.
-void launchPrelude(cs_ctx* c, bool learned) {
+void launchPrelude(cs_ctx* c, bool learned, cudaGraphConditionalHandle h = 0) {
     launchAssembly(c);
     const bool fork = c->resClusters > 0 && c->B.res_cnc > 0 && c->B.n_resident > 0;
     if (fork) {
@@ -1334,7 +1334,7 @@ void launchPrelude(cs_ctx* c, bool learned) {
         cudaEventRecord(c->evJoin, c->side);
     }
     if (learned) launchMlpInference(c, c->B.warm);
-    launchSolvePrologue(c);
+    launchSolvePrologue(c, h);
     if (fork) cudaStreamWaitEvent(c->stream, c->evJoin, 0);
     launchResident(c, false);
     launchGroup(c);
@@ -1366,15 +1366,32 @@ void launchTrip(cs_ctx* c, cudaGraphConditionalHandle h) {
     cs_reduce2_kernel<<<B.S, CS_REDUCE_THREADS, 0, c->stream>>>(B, h);
 }
 
+// The solve loop launched from the host: eight trips between looks at the device's condition, the
+// first look before any (no trip when every sheet is solved on chip).
+cs_status hostLoop(cs_ctx* c, int loop_cap) {
+    for (int trips = 0; trips <= loop_cap + 16; trips += 8) {
+        int go = 0;
+        CS_CUDA(cudaMemcpyAsync(&go, c->B.loop + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CS_CUDA(cudaStreamSynchronize(c->stream));
+        if (!go) break;
+        for (int t = 0; t < 8; t++) launchTrip(c, 0);
+    }
+    return CS_OK;
+}
+
 cs_status buildGraph(cs_ctx* c, bool learned) {
     cudaGraphExec_t& exec = c->gexec[learned][c->tripCoarse];
     if (exec) return CS_OK;
     cudaGraph_t graph;
     CS_CUDA(cudaGraphCreate(&graph, 0));
     c->gph[learned][c->tripCoarse] = graph;
+    // the loop's condition: set by the solve set-up (no trip when every sheet is solved on chip) and
+    // by each trip
+    cudaGraphConditionalHandle handle;
+    CS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
     // prelude: assembly (+ learned warm start) + solve setup, captured into the graph
     CS_CUDA(cudaStreamBeginCaptureToGraph(c->stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launchPrelude(c, learned);
+    launchPrelude(c, learned, handle);
     cudaStreamCaptureStatus cst;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
@@ -1382,8 +1399,6 @@ cs_status buildGraph(cs_ctx* c, bool learned) {
     std::vector<cudaGraphNode_t> prelude(deps, deps + ndeps);
     CS_CUDA(cudaStreamEndCapture(c->stream, &graph));
     // while loop over solve trips
-    cudaGraphConditionalHandle handle;
-    CS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
@@ -2196,7 +2211,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     AL(part, 2LL * B.n_slices);
     AL(inst, B.S);
     AL(params, 1);
-    AL(loop, 8);
+    AL(loop, 10);
     AL(cinv, B.res_cnc > 0 ? (long long)hrlist.size() * B.res_cnc * B.res_cnc : 1);
     AL(cvalid, std::max<size_t>(hrlist.size(), 1));
 #undef AL
@@ -2220,7 +2235,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     CS_CUDA(cudaMemset(B.warm, 0, 3LL * B.N * sizeof(float)));
     CS_CUDA(cudaMemset(B.A, 0, (size_t)B.n_panels * CS_PANEL_FLOATS * sizeof(float)));
     CS_CUDA(cudaMemset(B.inst, 0, B.S * sizeof(InstState)));
-    CS_CUDA(cudaMemset(B.loop, 0, 8 * sizeof(int)));
+    CS_CUDA(cudaMemset(B.loop, 0, 10 * sizeof(int)));
     CS_CUDA(cudaDeviceSynchronize());
     {
         cudaDeviceProp prop;
@@ -3044,15 +3059,7 @@ cs_status cs_step(cs_ctx* c, const cs_step_params* p, cs_step_stats* stats) {
     } else {
         c->hostLaunches += assemblyKernels(c) + 3 + bcSetupKernels(c) + residentKernels(c) + (learned ? 3 : 0);
         launchPrelude(c, learned);
-        int go = 1;
-        int trips = 0;
-        while (go) {
-            for (int t = 0; t < 8; t++) launchTrip(c, 0);
-            trips += 8;
-            CS_CUDA(cudaMemcpyAsync(&go, c->B.loop + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            CS_CUDA(cudaStreamSynchronize(c->stream));
-            if (trips > d.loop_cap + 16) break;
-        }
+        if ((st = hostLoop(c, d.loop_cap)) != CS_OK) return st;
         cs_advance_kernel<<<nblk(3LL * c->B.N, 256), 256, 0, c->stream>>>(c->B);
     }
     CS_CUDA(cudaGetLastError());
@@ -3236,7 +3243,7 @@ cs_status cs_profile_kernels(cs_ctx* c, const cs_step_params* p, int reps, float
     ms[1] = timeIt(1);
     ms[2] = timeIt(2);
     // solver kernels with every instance held in one phase
-    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B);
+    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B, 0);
     cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
     cs_profile_setup_kernel<<<nblk(B.S, 128), 128, 0, c->stream>>>(B, PH_CG);
     ms[3] = timeIt(3);
@@ -3249,7 +3256,7 @@ cs_status cs_profile_kernels(cs_ctx* c, const cs_step_params* p, int reps, float
     ms[9] = ms[10] = 0.f;
     if (B.bc_total_agg > 0 && p->coarse) {
         cs_slice_bnorm_kernel<<<nblk((long long)B.n_slices * 32, 128), 128, 0, c->stream>>>(B);
-        cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B);
+        cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B, 0);
         float t = 0.f;
         cudaEventRecord(c->ev0, c->stream);
         for (int r = 0; r < reps; r++) launchBatchedCoarseSetup(c);
@@ -3329,15 +3336,7 @@ static float timeWholeSolve(cs_ctx* c, const cs_step_params& q) {
     cudaEventRecord(c->ev0, c->stream);
     launchResident(c);
     launchGroup(c);
-    int go = 1, trips = 0;
-    while (go) {
-        for (int t = 0; t < 8; t++) launchTrip(c, 0);
-        trips += 8;
-        if (cudaMemcpyAsync(&go, B.loop + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
-            cudaStreamSynchronize(c->stream) != cudaSuccess)
-            return -1.f;
-        if (trips > d.loop_cap + 16) break;
-    }
+    if (hostLoop(c, d.loop_cap) != CS_OK) return -1.f;
     cudaEventRecord(c->ev1, c->stream);
     if (cudaEventSynchronize(c->ev1) != cudaSuccess) return -1.f;
     float ms = 0.f;
@@ -3356,7 +3355,7 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
     CS_CUDA(cudaMemcpyAsync(B.params, &d, sizeof(d), cudaMemcpyHostToDevice, c->stream));
     launchAssembly(c);
     // the SpMV's shapes on one fixed CG product (every instance in PH_CG, as cs_profile_kernels sets it)
-    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B);
+    cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B, 0);
     cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
     cs_profile_setup_kernel<<<nblk(B.S, 128), 128, 0, c->stream>>>(B, PH_CG);
     unsigned* sum = reinterpret_cast<unsigned*>(B.loop + 7);
@@ -3593,14 +3592,7 @@ cs_status mlpEnergyPrepare(cs_ctx* c, const cs_step_params* p) {
     launchSolvePrologue(c);
     launchResident(c);
     launchGroup(c);
-    int go = 1, trips = 0;
-    while (go) {
-        for (int t = 0; t < 8; t++) launchTrip(c, 0);
-        trips += 8;
-        CS_CUDA(cudaMemcpyAsync(&go, B.loop + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        CS_CUDA(cudaStreamSynchronize(c->stream));
-        if (trips > d.loop_cap + 16) break;
-    }
+    if ((st = hostLoop(c, d.loop_cap)) != CS_OK) return st;
     cs_mlp_energy_norm_kernel<<<nblk((long long)B.n_slices * 32, 128), 128, 0, c->stream>>>(B, M, 0, B.n_slices);
     cs_mlp_energy_sheet_kernel<<<B.S, 128, 0, c->stream>>>(B, M, 0, B.S, 0);
     CS_CUDA(cudaGetLastError());

@@ -580,8 +580,9 @@ __global__ void cs_solve_prologue_kernel(Batch B) {
     B.pB[i] = 0.f;
 }
 
-// Per instance: ||b||^2 from the assembly's slice partials, and the initial phase.
-__global__ void __launch_bounds__(128) cs_solve_setup_kernel(Batch B) {
+// Per instance: ||b||^2 from the assembly's slice partials, and the initial phase.  The last block
+// decides whether the loop runs at all (not when every sheet is solved on chip).
+__global__ void __launch_bounds__(128) cs_solve_setup_kernel(Batch B, cudaGraphConditionalHandle handle) {
     __shared__ double shd[4];
     const int s = blockIdx.x;
     const SheetDesc& sh = B.sheets[s];
@@ -608,9 +609,17 @@ __global__ void __launch_bounds__(128) cs_solve_setup_kernel(Batch B) {
             B.loop[0] = 0;
             B.loop[1] = 0;
             B.loop[2] = 0;
-            B.loop[3] = 1;
             B.loop[5] = 0;
             B.loop[6] = 0;
+        }
+        if (I.phase != PH_RESIDENT) atomicAdd(&B.loop[9], 1);
+        __threadfence();
+        if (atomicAdd(&B.loop[8], 1) == (int)gridDim.x - 1) {
+            __threadfence();
+            const int go = atomicExch(&B.loop[9], 0) > 0 ? 1 : 0;
+            B.loop[8] = 0;
+            B.loop[3] = go;
+            if (handle) cudaGraphSetConditional(handle, go);
         }
     }
 }
