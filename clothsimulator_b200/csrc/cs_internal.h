@@ -134,7 +134,10 @@ struct SpmvShape {
     int threads, spw, unroll;
 };
 #define CS_SPMV_CANDIDATES 24
-#define CS_SPMV_DEFAULT 1  // 128 threads, one slice per warp, no unrolling
+// 64 threads, one slice per warp, four slots' loads issued together: at the sizes where the loop is
+// bound by the latency of a row's loads one slot at a time costs most (128 threads, no unrolling: 26 us
+// for a sheet of 66,049 nodes in L2), and the large ones stream as fast
+#define CS_SPMV_DEFAULT 12
 struct Batch;
 extern const SpmvShape kSpmvShapes[CS_SPMV_CANDIDATES];
 void launchSpmvShape(const Batch& B, int shape, cudaStream_t st);
