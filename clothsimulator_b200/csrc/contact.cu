@@ -16,7 +16,7 @@
 //   cs_contact_grid_kernel   thread per face: pushes the face onto the bucket of every cell
 //                            its bounds touch (lock-free singly linked lists; buckets by the
 //                            spatial hash of Teschner et al. 2003 with a final bit mix)
-//   cs_contact_pair_kernel   thread per face f: walks the cells of its dilated bounds and
+//   cs_contact_pair_kernel   lanes per face f walk the cells of its dilated bounds and
 //                            appends each face g > f of its collision group whose bounds
 //                            overlap, once per pair (in the lowest cell the two share)
 //   cs_contact_vf/ee_kernel  thread per (pair, vertex-face test) and per (pair, edge-edge
@@ -249,60 +249,64 @@ __global__ void __launch_bounds__(128) cs_contact_grid_kernel(Batch B, Contact C
             }
 }
 
-// Candidate face pairs: thread per face f, walking the cells of its dilated bounds; each pair
-// (f, g > f) of one collision group whose bounds overlap is appended once (in the lowest cell
-// the two share).  Pairs are staged per thread and appended with one atomic per warp.
+// Candidate face pairs: CS_PAIR_LANES lanes per face f share out the cells of its dilated bounds; each
+// pair (f, g > f) of one collision group whose bounds overlap is appended once (in the lowest cell
+// the two share).  Pairs are staged per thread and appended with one atomic per warp.  What bounds it is
+// the latency of the buckets' linked lists (a dependent load per entry): one thread walking all of a
+// face's cells took 166 us for two 64 x 64 layers.
 __global__ void __launch_bounds__(128) cs_contact_pair_kernel(Batch B, Contact C, const int* sheet_group) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = t / CS_PAIR_LANES, part = t % CS_PAIR_LANES;
     int2 buf[CS_PAIR_STAGE];
     int nb = 0;
     if (f < B.F && !C.ext[1]) {
         const float c = cell_size(C);
-        const float t = C.dilate;  // 2 x repulsionThickness (Simulator.cu:274) or the collision thickness
+        const float th = C.dilate;  // 2 x repulsionThickness (Simulator.cu:274) or the collision thickness
         const int group = sheet_group[B.face_nodes[f].w];
         float dlo[3], dhi[3];
-        int qlo[3], qhi[3];
+        int qlo[3], qn[3];
         bool ok = true;
         for (int k = 0; k < 3; k++) {
-            dlo[k] = C.box[6 * (size_t)f + k] - t;  // Bounds::dilate (Bounds.cu:60-68)
-            dhi[k] = C.box[6 * (size_t)f + 3 + k] + t;
+            dlo[k] = C.box[6 * (size_t)f + k] - th;  // Bounds::dilate (Bounds.cu:60-68)
+            dhi[k] = C.box[6 * (size_t)f + 3 + k] + th;
             qlo[k] = cell_of(dlo[k], c);
-            qhi[k] = cell_of(dhi[k], c);
-            ok &= qhi[k] - qlo[k] <= 2;
+            qn[k] = cell_of(dhi[k], c) - qlo[k] + 1;
+            ok &= qn[k] <= 3;
         }
         if (!ok) atomicOr(&C.ext[1], 4u);
         const long long walk_cap = 8LL * B.F + 8;
-        for (int ix = qlo[0]; ok && ix <= qhi[0]; ix++)
-            for (int iy = qlo[1]; ok && iy <= qhi[1]; iy++)
-                for (int iz = qlo[2]; ok && iz <= qhi[2]; iz++) {
-                    long long walked = 0;
-                    for (int e = C.head[bucket(C, group, ix, iy, iz)]; e >= 0; e = C.next[e]) {
-                        if (++walked > walk_cap) {
-                            atomicOr(&C.ext[1], 8u);
-                            ok = false;
-                            break;
-                        }
-                        const int g = e >> 3;
-                        if (g <= f) continue;
-                        if (sheet_group[B.face_nodes[g].w] != group) continue;
-                        const float* gb = C.box + 6 * (size_t)g;
-                        // Bounds::overlap(b, thickness) (Bounds.cu:85-101): g against f dilated
-                        if (gb[0] > dhi[0] || gb[3] < dlo[0] || gb[1] > dhi[1] || gb[4] < dlo[1] || gb[2] > dhi[2] ||
-                            gb[5] < dlo[2])
-                            continue;
-                        // one test per pair: in the lowest cell both cover
-                        if (max(qlo[0], cell_of(gb[0], c)) != ix || max(qlo[1], cell_of(gb[1], c)) != iy ||
-                            max(qlo[2], cell_of(gb[2], c)) != iz)
-                            continue;
-                        if (nb == CS_PAIR_STAGE) {
-                            const int base = atomicAdd(C.pair_count, nb);
-                            for (int k = 0; k < nb; k++)
-                                if (base + k < C.pair_cap) C.pairs[base + k] = buf[k];
-                            nb = 0;
-                        }
-                        buf[nb++] = make_int2(f, g);
-                    }
+        const int cells = ok ? qn[0] * qn[1] * qn[2] : 0;
+        for (int q = part; q < cells; q += CS_PAIR_LANES) {
+            const int ix = qlo[0] + q / (qn[1] * qn[2]), iy = qlo[1] + q / qn[2] % qn[1], iz = qlo[2] + q % qn[2];
+            long long walked = 0;
+            for (int e = C.head[bucket(C, group, ix, iy, iz)]; e >= 0;) {
+                const int at = e;
+                e = C.next[at];  // requested before the entry's tests
+                if (++walked > walk_cap) {
+                    atomicOr(&C.ext[1], 8u);
+                    q = cells;
+                    break;
                 }
+                const int g = at >> 3;
+                if (g <= f) continue;
+                if (sheet_group[B.face_nodes[g].w] != group) continue;
+                const float* gb = C.box + 6 * (size_t)g;
+                // Bounds::overlap(b, thickness) (Bounds.cu:85-101): g against f dilated
+                if (gb[0] > dhi[0] || gb[3] < dlo[0] || gb[1] > dhi[1] || gb[4] < dlo[1] || gb[2] > dhi[2] || gb[5] < dlo[2])
+                    continue;
+                // one test per pair: in the lowest cell both cover
+                if (max(qlo[0], cell_of(gb[0], c)) != ix || max(qlo[1], cell_of(gb[1], c)) != iy ||
+                    max(qlo[2], cell_of(gb[2], c)) != iz)
+                    continue;
+                if (nb == CS_PAIR_STAGE) {
+                    const int base = atomicAdd(C.pair_count, nb);
+                    for (int k = 0; k < nb; k++)
+                        if (base + k < C.pair_cap) C.pairs[base + k] = buf[k];
+                    nb = 0;
+                }
+                buf[nb++] = make_int2(f, g);
+            }
+        }
     }
     // warp-aggregated append of the staged pairs
     const int lane = threadIdx.x & 31;

@@ -40,6 +40,9 @@ __host__ __device__ inline uint32_t cs_code(int is_edge, int elem, int a, int b)
 // fit four warps in a CTA's shared memory gets fewer.  (One-warp CTAs, 15 warps per SM instead
 // of 12, measured slower on the windy batch: 3.82 against 3.35 ms.)
 #define CS_GATHER_THREADS 128
+// threads (rows) per block of the proximity row kernel, and its shared memory: a row's blocks and columns
+#define CS_PROX_ROW_THREADS 32
+inline size_t cs_prox_row_smem(int width) { return (size_t)width * 10 * CS_PROX_ROW_THREADS * sizeof(float); }
 
 struct SheetDesc {
     int node_off, n_nodes;
@@ -428,6 +431,7 @@ struct Collide {
 #define CS_OPT_THREADS 1024
 #define CS_OPT_STAGE 12288
 #define CS_CONTACT_ITEMS 4096  // keys per compaction block (256 threads x 16)
+#define CS_PAIR_LANES 8        // lanes that share out the cells of a face
 #define CS_PAIR_STAGE 16       // candidate pairs staged per thread before appending
 #define CS_SCAN_ITEMS 4096     // ints per block of the exclusive scan (1024 threads x 4)
 

@@ -1191,7 +1191,7 @@ int launchAssembly(cs_ctx* c) {
         // proximity terms after the handles (Cloth.cu:676-684): records, then per row the
         // blocks, right-hand side and block-Jacobi inverse, then the ||b|| partials
         cs_prox_kernel<<<nblk(B.n_pinst, 128), 128, 0, c->stream>>>(B);
-        cs_prox_row_kernel<<<nblk(B.N, 128), 128, 0, c->stream>>>(B);
+        cs_prox_row_kernel<<<nblk(B.N, CS_PROX_ROW_THREADS), CS_PROX_ROW_THREADS, cs_prox_row_smem(B.gather_width), c->stream>>>(B);
         cs_slice_bnorm_kernel<<<nblk((long long)B.n_slices * 32, 128), 128, 0, c->stream>>>(B);
         n += 3;
     }
@@ -2250,6 +2250,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             return fail(c, CS_ERR_INVALID_ARG, "slices of %d block slots exceed the assembly's shared memory", B.gather_width);
         c->gatherSmem = (size_t)c->gatherWarps * perWarp;
         CS_CUDA(raiseDynSmem((const void*)cs_gather_kernel, c->gatherSmem));
+        CS_CUDA(raiseDynSmem((const void*)cs_prox_row_kernel, cs_prox_row_smem(B.gather_width)));
         const int threads = 32 * c->gatherWarps;
         int perSM = 0;
         CS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, cs_gather_kernel, threads, c->gatherSmem));
@@ -2599,7 +2600,7 @@ cs_status candidatePairs(cs_ctx* c, const int* sheetGroup, int& npairs) {
             C.pair_cap = (int)std::min<size_t>(cap, INT32_MAX);
         }
         CS_CUDA(cudaMemsetAsync(C.pair_count, 0, sizeof(int), c->stream));
-        cs_contact_pair_kernel<<<nblk(B.F, 128), 128, 0, c->stream>>>(B, C, c->sheetGroupDev);
+        cs_contact_pair_kernel<<<nblk((long long)B.F * CS_PAIR_LANES, 128), 128, 0, c->stream>>>(B, C, c->sheetGroupDev);
         CS_CUDA(cudaMemcpyAsync(&npairs, C.pair_count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CS_CUDA(cudaStreamSynchronize(c->stream));
         if (npairs <= C.pair_cap) break;

@@ -655,7 +655,12 @@ __global__ void __launch_bounds__(128) cs_prox_kernel(Batch B) {
 // Cloth.cu:42-76): instances ascending, impulse before friction, row corner, column corner;
 // after the gather's handle terms.  Blocks on the mesh pattern are summed onto their slot,
 // others onto the row's side list (zeroed first); the row's block-Jacobi inverse is redone.
-__global__ void __launch_bounds__(128) cs_prox_row_kernel(Batch B) {
+// The sums are a serial chain per row, so the row's blocks and columns are copied to shared memory
+// first (entry e of slot k of a thread at [(9 k + e) * CS_PROX_ROW_THREADS + thread]: no conflicts),
+// summed there and written back: summed in place through L2, a step of two 64 x 64 layers (18,600
+// proximities) took 317 us.
+extern __shared__ float cs_prox_acc[];
+__global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch B) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= B.N) return;
     const int q0 = B.prow_ptr[row], q1 = B.prow_ptr[row + 1];
@@ -663,18 +668,19 @@ __global__ void __launch_bounds__(128) cs_prox_row_kernel(Batch B) {
     const SheetDesc& sd = B.sheets[B.node_sheet[row]];
     const int* cp = B.tcsr_ptr + sd.csr_ptr_off;
     const int li = row - sd.node_off;
-    const int c0 = cp[li], c1 = cp[li + 1];
-    // SELL slot of block (row, col) on the mesh pattern, or -1
-    auto slot_of = [&](int col) {
-        const int lj = col - sd.node_off;
-        int lo = c0, hi = c1;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (B.tcsr_col[mid] < lj) lo = mid + 1;
-            else hi = mid;
-        }
-        return (lo < c1 && B.tcsr_col[lo] == lj) ? sd.panel_off * CS_SLICE + B.tcsr_slot[lo] : -1;
-    };
+    const int c0 = cp[li], nc = cp[li + 1] - c0;
+    float* const acc = cs_prox_acc + threadIdx.x;
+    int* const cols = reinterpret_cast<int*>(cs_prox_acc + 9 * (size_t)B.gather_width * CS_PROX_ROW_THREADS) + threadIdx.x;
+    int diag = 0;
+    for (int k = 0; k < nc; k++) {
+        const int col = B.tcsr_col[c0 + k] + sd.node_off;
+        cols[k * CS_PROX_ROW_THREADS] = col;
+        if (col == row) diag = k;
+        float a[9];
+        load_slot(B.A, sd.panel_off * CS_SLICE + B.tcsr_slot[c0 + k], a);
+#pragma unroll
+        for (int e = 0; e < 9; e++) acc[(9 * k + e) * CS_PROX_ROW_THREADS] = a[e];
+    }
     const int x0 = B.xptr ? B.xptr[row] : 0, x1 = B.xptr ? B.xptr[row + 1] : 0;
     for (int m = x0; m < x1; m++)
         for (int e = 0; e < 9; e++) B.xval[9 * (size_t)m + e] = 0.0f;
@@ -683,6 +689,21 @@ __global__ void __launch_bounds__(128) cs_prox_row_kernel(Batch B) {
         const int inst = B.prow_inst[q];
         const ProxInst& P = B.pinst[inst];
         const float* rec = B.prec + (size_t)inst * CS_PROX_REC;
+        // the position in the row of each of the instance's columns (-1: outside the pattern, -2: none)
+        int at[4];
+#pragma unroll
+        for (int bb = 0; bb < 4; bb++) {
+            at[bb] = -2;
+            if (!((P.local >> bb) & 1)) continue;
+            const int col = P.node[bb];
+            int lo = 0, hi = nc;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (cols[mid * CS_PROX_ROW_THREADS] < col) lo = mid + 1;
+                else hi = mid;
+            }
+            at[bb] = lo < nc && cols[lo * CS_PROX_ROW_THREADS] == col ? lo : -1;
+        }
         for (int fr = 0; fr < 2; fr++)
             for (int a = 0; a < 4; a++) {
                 if (!((P.local >> a) & 1) || P.node[a] != row) continue;
@@ -690,38 +711,36 @@ __global__ void __launch_bounds__(128) cs_prox_row_kernel(Batch B) {
                 b0 += r[0];
                 b1 += r[1];
                 b2 += r[2];
+#pragma unroll
                 for (int bb = 0; bb < 4; bb++) {
-                    if (!((P.local >> bb) & 1)) continue;
-                    const int col = P.node[bb];
+                    if (at[bb] == -2) continue;
                     const float* blk = rec + fr * 144 + (3 * a) * 12 + 3 * bb;
-                    const int slot = slot_of(col);
-                    float acc[9];
-                    float* dst = nullptr;
-                    if (slot >= 0) {
-                        load_slot(B.A, slot, acc);
-                    } else {
-                        int m = x0;
-                        while (m < x1 && B.xcol[m] != col) m++;
-                        if (m == x1) continue;  // not listed: cannot happen for a consistent list
-                        dst = B.xval + 9 * (size_t)m;
-                        for (int e = 0; e < 9; e++) acc[e] = dst[e];
+                    if (at[bb] >= 0) {
+                        float* d = acc + 9 * at[bb] * CS_PROX_ROW_THREADS;
+#pragma unroll
+                        for (int k = 0; k < 3; k++)
+#pragma unroll
+                            for (int h = 0; h < 3; h++) d[(3 * k + h) * CS_PROX_ROW_THREADS] += blk[k * 12 + h];
+                        continue;
                     }
+                    int m = x0;
+                    while (m < x1 && B.xcol[m] != P.node[bb]) m++;
+                    if (m == x1) continue;  // not listed: cannot happen for a consistent list
+                    float* dst = B.xval + 9 * (size_t)m;
                     for (int k = 0; k < 3; k++)
-                        for (int h = 0; h < 3; h++) acc[3 * k + h] += blk[k * 12 + h];
-                    if (slot >= 0) store_slot(B.A, slot, acc);
-                    else
-                        for (int e = 0; e < 9; e++) dst[e] = acc[e];
+                        for (int h = 0; h < 3; h++) dst[3 * k + h] += blk[k * 12 + h];
                 }
             }
     }
     B.b[3 * row] = b0;
     B.b[3 * row + 1] = b1;
     B.b[3 * row + 2] = b2;
-    const int ds = slot_of(row);
-    if (ds >= 0) {
+    for (int k = 0; k < nc; k++) {
         float a[9];
-        load_slot(B.A, ds, a);
-        block_inverse(a, B.Pinv + 9 * (size_t)row);
+#pragma unroll
+        for (int e = 0; e < 9; e++) a[e] = acc[(9 * k + e) * CS_PROX_ROW_THREADS];
+        store_slot(B.A, sd.panel_off * CS_SLICE + B.tcsr_slot[c0 + k], a);
+        if (k == diag) block_inverse(a, B.Pinv + 9 * (size_t)row);
     }
 }
 
