@@ -1068,6 +1068,8 @@ struct cs_ctx {
     std::vector<int> rlistAll;  // resident sheets before the proximity filter
     std::vector<int> rlistCur;  // resident sheets now
     int residentProx = 0;       // those of them that a proximity touches
+    int loopSheets = 0;         // sheets that the batched loop solves on the AUTO route
+    int proxSteps = 0;          // steps since the proximities last changed
     std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, strip-local ones
     // proximities (cs_set_proximities): their device lists, and the host copies of the
     // blocks outside the pattern that cs_get_system merges
@@ -2443,6 +2445,9 @@ cs_status applyProximities(cs_ctx* c, int n, float thickness) {
             rl.push_back(s);
             c->residentProx += touched[s] ? 1 : 0;
         }
+    c->proxSteps = 0;
+    c->loopSheets = 0;
+    for (int s = 0; s < B.S; s++) c->loopSheets += (c->sheets[s].resident == 0 || (touched[s] & 2)) ? 1 : 0;
     if (!rl.empty()) CS_CUDA(cudaMemcpy(B.rlist, rl.data(), rl.size() * sizeof(int), cudaMemcpyHostToDevice));
     B.n_resident = (int)rl.size();
     c->rlistCur = rl;
@@ -3054,7 +3059,16 @@ cs_status cs_step(cs_ctx* c, const cs_step_params* p, cs_step_stats* stats) {
     if ((st = setTripCoarse(c, p->coarse != 0)) != CS_OK) return st;
     CS_CUDA(cudaEventRecord(c->ev0, c->stream));
     const bool learned = p->warm_start == CS_WARM_LEARNED;
-    if (p->use_graph) {
+    // A graph holds the proximity lists it was captured with.  While they change from step to step
+    // (detection before every step), capturing one per step would cost more than it saves: such a
+    // step launches its kernels directly, where none of its sheets needs the loop.
+    const bool direct = p->use_graph && c->prox.n > 0 && c->proxSteps == 0 && p->precision == CS_PREC_MIXED &&
+                        p->solver == CS_SOLVER_AUTO && c->loopSheets == 0;
+    c->proxSteps++;
+    if (direct) {
+        launchPrelude(c, learned);
+        cs_advance_kernel<<<nblk(3LL * c->B.N, 256), 256, 0, c->stream>>>(c->B);
+    } else if (p->use_graph) {
         if ((st = buildGraph(c, learned)) != CS_OK) return st;
         CS_CUDA(cudaGraphLaunch(c->gexec[learned][c->tripCoarse], c->stream));
     } else {

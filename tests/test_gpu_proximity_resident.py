@@ -37,3 +37,19 @@ def test_in_pattern_proximities_stay_on_chip(ctx_factory, nq, touched):
     ctx.set_proximities(None, THICKNESS)
     ctx.step(params_for(scene, advance=0))
     assert np.array_equal(ctx.get_dv(), dv0)
+
+
+@pytest.mark.parametrize("touched", [(), (1,)])
+def test_steps_after_a_change_of_the_proximities_agree(ctx_factory, touched):
+    """The first step after a change launches its kernels directly (where no sheet needs the loop), the
+    next ones run the graph captured with the new lists: the same bits."""
+    scene, prox = make_case(seed=33, n_sheets=4, nq=12, touched=touched, pairs=((0, 3), (1, 2)))
+    ctx = ctx_factory(scene.sheets)
+    for lists in (prox, {k: v[:-1] for k, v in prox.items()}):
+        ctx.set_proximities(lists, THICKNESS)
+        out = []
+        for graph in (1, 1, 1, 0):
+            ctx.step(params_for(scene, advance=0, precond_degree=3, use_graph=graph))
+            out.append(ctx.get_dv().copy())
+        for dv in out[1:]:
+            assert np.array_equal(dv, out[0])
