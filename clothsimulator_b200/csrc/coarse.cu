@@ -4,18 +4,25 @@
 // Block-Jacobi PCG needs many iterations on a large sheet (1,700 on a 1,000 x 1,000 grid): the
 // smooth error spans the sheet and the diagonal blocks cannot move it.  Each sheet's nodes are
 // grouped into aggregates (its rest (u, v) coordinates binned into g x g cells, the non-empty
-// cells), and the preconditioner becomes additive two-level,
-//     z = D^-1 r + R^T A_c^-1 R r,
+// cells), and the preconditioner becomes additive multilevel,
+//     z = D^-1 r + F^T D_F^-1 F r + G^T D_G^-1 G r + R^T A_c^-1 R r,
 // R summing a vector over each aggregate (one value per aggregate and component) and
-// A_c = R A R^T.  Per step: A_c is summed from per-pair contributor lists (a fixed order, so
+// A_c = R A R^T.  F and G sum over the cells of two finer grids nested in the aggregates' (about
+// CS_BC_NODES_PER_FINE nodes a cell, and up to CS_BC_FINE_SPLIT times wider), of whose matrices
+// F A F^T and G A G^T only the 3x3 diagonal blocks are used: the errors as wide as a few nodes,
+// which neither D^-1 nor aggregates of hundreds of nodes reach, cost no coarse solve.  On the
+// B200 (tol 1e-6): an irregular sheet of 301 x 301 nodes 136 -> 98 iterations and, with 192 coarse unknowns
+// instead of 768, 7.9 -> 6.3 ms; one of 1,001 x 1,001 nodes 481 -> 355 iterations, 116 -> 90 ms (a trip
+// 11 us longer).  Per step: A_c is summed from per-pair contributor lists (a fixed order, so
 // the result is deterministic) and inverted by Gauss-Jordan in FP32 -- one CTA with the matrix
 // in shared memory up to CS_BC_SMALL_NC unknowns, else a cluster of CS_BC_CLUSTER CTAs with its
 // rows spread over their shared memory and each pivot row read through distributed shared
 // memory -- then symmetrised.  A_c is SPD (A is), so no pivoting is needed; the pivots are
 // diagonal blocks of CS_BC_PB aggregates (CS_BC_KB rows, a twelfth of the barriers of scalar
 // pivots), and a non-positive pivot inside one disables the sheet's correction for the step.  Per CG trip, after the vector
-// update: R r (a block per aggregate), e_c = A_c^-1 R r (a warp per coarse row), then
-// z += R^T e_c with the r.z and r.r partials recomputed (a warp per 32 rows in natural order,
+// update: F r, G r and R r (a block per aggregate, reading r once) and the finer cells' own
+// corrections; e_c = A_c^-1 R r, added to those of the cells inside (a block per aggregate); then
+// z += the cell's correction with the r.z and r.r partials recomputed (a warp per 32 rows in natural order,
 // as cs_vector_kernel lays them out).  Sheets solved cluster-resident (their own coarse
 // correction, resident.cu) and sheets with proximities (blocks outside the pattern) skip it.
 #include <cooperative_groups.h>
@@ -33,6 +40,85 @@ __device__ __forceinline__ T bc_warp_sum(T v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// Lanes 0-7 return the warp's sum of a, 8-15 of b, 16-23 of c: 6 exchanges instead of 15.
+__device__ __forceinline__ double bc_warp_sum3(double a, double b, double c, int lane) {
+    const bool up = lane & 16, odd = lane & 8;
+    double x = __shfl_xor_sync(0xffffffffu, up ? a : c, 16), y = __shfl_xor_sync(0xffffffffu, up ? b : 0.0, 16);
+    x += up ? c : a;
+    y += up ? 0.0 : b;
+    double v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ void coarse_load_block(const Batch& B, const SheetDesc& sh, int slot, float (&a)[9]) {
+    const float* pk = B.A + (size_t)(sh.panel_off + slot / CS_SLICE) * CS_PANEL_FLOATS;
+    const int l = slot % CS_SLICE;
+    const float4 a0 = __ldg(reinterpret_cast<const float4*>(pk) + l);
+    const float4 a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + l);
+    a[0] = a0.x;
+    a[1] = a0.y;
+    a[2] = a0.z;
+    a[3] = a0.w;
+    a[4] = a1.x;
+    a[5] = a1.y;
+    a[6] = a1.z;
+    a[7] = a1.w;
+    a[8] = __ldg(pk + 256 + l);
+}
+
+// The warp's sum of a 3x3 block per lane, symmetrised and inverted into out[9] (FP64 inside): zeros,
+// that is no correction by the cell, unless `on` and the block is positive definite.
+__device__ __forceinline__ void bc_cell_inverse(const float (&a)[9], bool on, float* out, int lane) {
+    double m[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) m[k] = bc_warp_sum((double)a[k]);
+    if (lane != 0) return;
+    const double a00 = m[0], a11 = m[4], a22 = m[8];
+    const double a01 = 0.5 * (m[1] + m[3]), a02 = 0.5 * (m[2] + m[6]), a12 = 0.5 * (m[5] + m[7]);
+    const double c00 = a11 * a22 - a12 * a12, c01 = a02 * a12 - a01 * a22, c02 = a01 * a12 - a02 * a11;
+    const double m2 = a00 * a11 - a01 * a01, det = a00 * c00 + a01 * c01 + a02 * c02, id = 1.0 / det;
+    on = on && a00 > 0.0 && m2 > 0.0 && det > 0.0 && isfinite((float)id);
+    const double inv[9] = {c00, c01, c02, c01, a00 * a22 - a02 * a02, a01 * a02 - a00 * a12, c02, a01 * a02 - a00 * a12, m2};
+#pragma unroll
+    for (int k = 0; k < 9; k++) out[k] = on ? (float)(inv[k] * id) : 0.f;
+}
+
+// The diagonal blocks of F A F^T for the fine cells of middle cell `mid` of a sheet, and of G A G^T for
+// itself, inverted: a lane per node of a fine cell walks the node's row.
+__device__ __noinline__ void bc_cell_blocks(const Batch& B, const SheetDesc& sh, int mid, int lane) {
+    const int* fptr = B.bc_fptr + sh.bc_mid_off + mid;
+    const int* mptr = B.bc_mptr + sh.bc_fine_off;
+    const int* cp = B.tcsr_ptr + sh.csr_ptr_off;
+    const int f0 = fptr[0], f1 = fptr[1];
+    float am[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) am[k] = 0.f;
+    for (int f = f0; f < f1; f++) {
+        float af[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) af[k] = 0.f;
+        for (int m = mptr[f] + lane; m < mptr[f + 1]; m += 32) {
+            const int node = B.bc_mem[sh.bc_node_off + m];
+#pragma unroll 4
+            for (int q = cp[node]; q < cp[node + 1]; q++) {
+                const int fc = B.bc_node_fine[sh.bc_node_off + B.tcsr_col[q]];
+                if (fc < f0 || fc >= f1) continue;
+                float a[9];
+                coarse_load_block(B, sh, B.tcsr_slot[q], a);
+#pragma unroll
+                for (int k = 0; k < 9; k++) {
+                    am[k] += a[k];
+                    af[k] += fc == f ? a[k] : 0.f;
+                }
+            }
+        }
+        bc_cell_inverse(af, sh.bc_levels & 1, B.bc_finv + 9 * (size_t)(sh.bc_fvec_off + f), lane);
+    }
+    bc_cell_inverse(am, sh.bc_levels & 2, B.bc_minv + 9 * (size_t)(sh.bc_mvec_off + mid), lane);
 }
 
 // The sheet takes the correction this step (independent of its phase).
@@ -53,8 +139,8 @@ __device__ __forceinline__ bool bc_trip_on(const Batch& B, int s) {
 
 // A_c of every sheet the loop solves: a warp per coarse pair (a, b) sums the 3x3 blocks of its
 // contributor slots (lane-strided, then a butterfly: a fixed order) into rows 3a..3a+2,
-// columns 3b..3b+2 of the sheet's dense coarse matrix (zeroed before).  Grid: x over pairs,
-// y over sheets.
+// columns 3b..3b+2 of the sheet's dense coarse matrix (zeroed before); further warps take the middle
+// cells and the fine cells in them.  Grid: x over pairs and middle cells, y over sheets.
 __global__ void __launch_bounds__(256) cs_bc_assemble_kernel(Batch B) {
     const int s = blockIdx.y;
     if (!bc_sheet_on(B, s) || (B.inst[s].phase == PH_RESIDENT) != (B.bc_resident != 0)) return;
@@ -63,7 +149,11 @@ __global__ void __launch_bounds__(256) cs_bc_assemble_kernel(Batch B) {
     float* M = B.bc_mat + sh.bc_mat_off;
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
-    for (int q = blockIdx.x * wpb + (threadIdx.x >> 5); q < sh.bc_npair; q += gridDim.x * wpb) {
+    for (int q = blockIdx.x * wpb + (threadIdx.x >> 5); q < sh.bc_npair + sh.bc_nmid; q += gridDim.x * wpb) {
+        if (q >= sh.bc_npair) {
+            bc_cell_blocks(B, sh, q - sh.bc_npair, lane);
+            continue;
+        }
         const int4 pr = B.bc_pair[sh.bc_pair_off + q];
         float a[9];
 #pragma unroll
@@ -395,56 +485,104 @@ __global__ void __launch_bounds__(CS_BC_THREADS) cs_bc_invert_cluster_kernel(Bat
     if (rank == 0 && threadIdx.x == 0) B.bc_ok[s] = bad ? 0 : 1;
 }
 
-// R r: a block per aggregate sums r over its member nodes (thread-strided over the ascending
-// members, then a fixed-order block sum) in FP64, stored in FP32.
-__global__ void __launch_bounds__(256) cs_bc_restrict_kernel(Batch B) {
-    __shared__ double sh3[3 * 8];
-    const int w = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (w >= B.bc_total_agg) return;
-    const int2 sa = B.bc_agg[w];
+// F r, G r and R r: a block per aggregate, a warp per middle cell in it.  The warp sums r over the nodes
+// of a fine cell in FP64 (lane-strided, then a butterfly; CS_BC_UNROLL cells' loads together), the fine
+// cells' sums over the middle cell, and the block the middle cells' over the aggregate, each in a fixed
+// order; R r is stored in FP32, and the cells' D_F^-1 F r and D_G^-1 G r as the cells' corrections.
+__global__ void __launch_bounds__(CS_BC_RESTRICT_THREADS) cs_bc_restrict_kernel(Batch B) {
+    __shared__ double sh3[CS_BC_RESTRICT_THREADS / 32][3];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int2 sa = B.bc_agg[blockIdx.x];
     if (!bc_trip_on(B, sa.x)) return;
     const SheetDesc& sh = B.sheets[sa.x];
-    const int m0 = B.bc_mptr[sh.bc_agg_off + sa.y], m1 = B.bc_mptr[sh.bc_agg_off + sa.y + 1];
-    double r0 = 0.0, r1 = 0.0, r2 = 0.0;
-    for (int m = m0 + (int)threadIdx.x; m < m1; m += blockDim.x) {
-        const int node = sh.node_off + B.bc_mem[sh.bc_mem_off + m];
-        r0 += (double)B.r[3 * node];
-        r1 += (double)B.r[3 * node + 1];
-        r2 += (double)B.r[3 * node + 2];
+    const int* aptr = B.bc_aptr + sh.bc_agg_off + sa.y;
+    const int* mptr = B.bc_mptr + sh.bc_fine_off;
+    double t[3] = {0.0, 0.0, 0.0};
+    for (int mid = aptr[0] + wid; mid < aptr[1]; mid += CS_BC_RESTRICT_THREADS / 32) {
+        const int f0 = B.bc_fptr[sh.bc_mid_off + mid], f1 = B.bc_fptr[sh.bc_mid_off + mid + 1];
+        double g[3] = {0.0, 0.0, 0.0};
+        for (int f = f0; f < f1; f += CS_BC_UNROLL) {
+            double a[CS_BC_UNROLL][3];
+            int m0[CS_BC_UNROLL], m1[CS_BC_UNROLL];
+#pragma unroll
+            for (int u = 0; u < CS_BC_UNROLL; u++) {
+                m0[u] = f + u < f1 ? mptr[f + u] + lane : 0;
+                m1[u] = f + u < f1 ? mptr[f + u + 1] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < CS_BC_UNROLL; u++) {
+                const float* r = B.r + 3 * (size_t)(sh.node_off + (m0[u] < m1[u] ? B.bc_mem[sh.bc_node_off + m0[u]] : 0));
+#pragma unroll
+                for (int c = 0; c < 3; c++) a[u][c] = m0[u] < m1[u] ? (double)r[c] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < CS_BC_UNROLL; u++) {
+                if (f + u >= f1) break;
+                for (int m = m0[u] + 32; m < m1[u]; m += 32) {
+                    const float* r = B.r + 3 * (size_t)(sh.node_off + B.bc_mem[sh.bc_node_off + m]);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) a[u][c] += (double)r[c];
+                }
+                const double v = bc_warp_sum3(a[u][0], a[u][1], a[u][2], lane);
+                double s[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    s[c] = __shfl_sync(0xffffffffu, v, 8 * c);
+                    g[c] += s[c];
+                }
+                if (lane < 3) {
+                    const float* d = B.bc_finv + 9 * (size_t)(sh.bc_fvec_off + f + u) + 3 * lane;
+                    B.bc_ef[3 * (size_t)(sh.bc_fvec_off + f + u) + lane] = d[0] * (float)s[0] + d[1] * (float)s[1] + d[2] * (float)s[2];
+                }
+            }
+        }
+        if (lane < 3) {
+            const float* d = B.bc_minv + 9 * (size_t)(sh.bc_mvec_off + mid) + 3 * lane;
+            B.bc_em[3 * (size_t)(sh.bc_mvec_off + mid) + lane] = d[0] * (float)g[0] + d[1] * (float)g[1] + d[2] * (float)g[2];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) t[c] += g[c];
     }
-    r0 = bc_warp_sum(r0);
-    r1 = bc_warp_sum(r1);
-    r2 = bc_warp_sum(r2);
-    if (lane == 0) {
-        sh3[3 * wid] = r0;
-        sh3[3 * wid + 1] = r1;
-        sh3[3 * wid + 2] = r2;
-    }
+    if (lane < 3) sh3[wid][lane] = lane == 0 ? t[0] : lane == 1 ? t[1] : t[2];
     __syncthreads();
     if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) t += sh3[3 * q + threadIdx.x];
-        B.bc_rc[sh.bc_vec_off + 3 * sa.y + threadIdx.x] = (float)t;
+        double x = 0.0;
+        for (int q = 0; q < CS_BC_RESTRICT_THREADS / 32; q++) x += sh3[q][threadIdx.x];
+        B.bc_rc[sh.bc_vec_off + 3 * sa.y + threadIdx.x] = (float)x;
     }
 }
 
-// e_c = A_c^-1 R r: a warp per coarse row (lane-strided columns, then a butterfly).
-__global__ void __launch_bounds__(256) cs_bc_apply_kernel(Batch B) {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (w >= 3 * B.bc_total_agg) return;
-    const int2 sa = B.bc_agg[w / 3];
+// e_c = A_c^-1 R r: a block per aggregate, a warp for each of its three rows (lane-strided columns, then
+// a butterfly); then the aggregate's and the middle cells' corrections are added to the fine cells'.
+__global__ void __launch_bounds__(CS_BC_APPLY_THREADS) cs_bc_apply_kernel(Batch B) {
+    __shared__ float ec[3];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int2 sa = B.bc_agg[blockIdx.x];
     if (!bc_trip_on(B, sa.x)) return;
     const SheetDesc& sh = B.sheets[sa.x];
-    const int nc = 3 * sh.bc_na, i = 3 * sa.y + w % 3;
-    const float* row = B.bc_inv + sh.bc_mat_off + (size_t)i * nc;
-    const float* rc = B.bc_rc + sh.bc_vec_off;
-    float acc = 0.f;
-    for (int j = lane; j < nc; j += 32) acc = __fmaf_rn(row[j], rc[j], acc);
-    acc = bc_warp_sum(acc);
-    if (lane == 0) B.bc_ec[sh.bc_vec_off + i] = acc;
+    if (wid < 3) {
+        const int nc = 3 * sh.bc_na, i = 3 * sa.y + wid;
+        const float* row = B.bc_inv + sh.bc_mat_off + (size_t)i * nc;
+        const float* rc = B.bc_rc + sh.bc_vec_off;
+        float acc = 0.f;
+#pragma unroll 8
+        for (int j = lane; j < nc; j += 32) acc = __fmaf_rn(row[j], rc[j], acc);
+        acc = bc_warp_sum(acc);
+        if (lane == 0) ec[wid] = acc;
+    }
+    __syncthreads();
+    const int* aptr = B.bc_aptr + sh.bc_agg_off + sa.y;
+    for (int mid = aptr[0] + wid; mid < aptr[1]; mid += CS_BC_APPLY_THREADS / 32) {
+        const float* em = B.bc_em + 3 * (size_t)(sh.bc_mvec_off + mid);
+        const int f0 = 3 * B.bc_fptr[sh.bc_mid_off + mid], f1 = 3 * B.bc_fptr[sh.bc_mid_off + mid + 1];
+        for (int q = f0 + lane; q < f1; q += 32) {
+            const int c = q % 3;
+            B.bc_ef[3 * (size_t)sh.bc_fvec_off + q] += em[c] + ec[c];
+        }
+    }
 }
 
-// z += R^T e_c over the rows of the slice index's natural-order chunk (as cs_vector_kernel takes
+// z += the fine cells' corrections over the rows of the slice index's natural-order chunk (as cs_vector_kernel takes
 // them), and that chunk's r.z and r.r partials recomputed with the corrected z.
 __global__ void __launch_bounds__(128) cs_bc_finish_kernel(Batch B) {
     const int slice = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
@@ -459,7 +597,7 @@ __global__ void __launch_bounds__(128) cs_bc_finish_kernel(Batch B) {
     float rzf = 0.f, rrf = 0.f;
     if (live) {
         const int row = sh.node_off + local;
-        const float* ec = B.bc_ec + sh.bc_vec_off + 3 * B.bc_node_agg[sh.bc_node_off + local];
+        const float* ec = B.bc_ef + 3 * (size_t)(sh.bc_fvec_off + B.bc_node_fine[sh.bc_node_off + local]);
         float r[3], z[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -504,26 +642,6 @@ __global__ void __launch_bounds__(128) cs_bc_finish_kernel(Batch B) {
 // resident kernel, which applies its CTA's rows each CG iteration.  A non-positive or
 // non-finite pivot marks the work item's coarse matrix invalid and the solve runs without the
 // correction.  One CTA per resident work item; dynamic shared memory cs_coarse_setup_smem(nc).
-namespace {
-
-__device__ __forceinline__ void coarse_load_block(const Batch& B, const SheetDesc& sh, int slot, float (&a)[9]) {
-    const float* pk = B.A + (size_t)(sh.panel_off + slot / CS_SLICE) * CS_PANEL_FLOATS;
-    const int l = slot % CS_SLICE;
-    const float4 a0 = __ldg(reinterpret_cast<const float4*>(pk) + l);
-    const float4 a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + l);
-    a[0] = a0.x;
-    a[1] = a0.y;
-    a[2] = a0.z;
-    a[3] = a0.w;
-    a[4] = a1.x;
-    a[5] = a1.y;
-    a[6] = a1.z;
-    a[7] = a1.w;
-    a[8] = __ldg(pk + 256 + l);
-}
-
-}  // namespace
-
 __global__ void __launch_bounds__(CS_COARSE_THREADS) cs_coarse_setup_kernel(Batch B) {
     extern __shared__ __align__(16) float cs_coarse_sm[];
     __shared__ int bad;

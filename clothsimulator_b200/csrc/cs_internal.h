@@ -61,7 +61,11 @@ struct SheetDesc {
     int panel_off;              // first value panel: global slot = panel_off * 32 + topology slot
     // coarse space of the batched loop: this sheet's topology in the aggregate arrays, its
     // aggregates, its coarse unknowns' offset in the per-sheet vectors and its matrices' offset
-    int bc_node_off, bc_agg_off, bc_mem_off, bc_pair_off, bc_npair, bc_na, bc_vec_off;
+    int bc_node_off, bc_agg_off, bc_pair_off, bc_npair, bc_na, bc_vec_off;
+    // the finer cells: the topology's middle and fine cells in their pointer arrays, the middle cells'
+    // number, this sheet's offset among the middle and the fine cells of all sheets; levels in use
+    // (bit 0: fine, bit 1: middle)
+    int bc_mid_off, bc_fine_off, bc_nmid, bc_mvec_off, bc_fvec_off, bc_levels;
     long long bc_mat_off;
 };
 
@@ -115,6 +119,13 @@ enum InstPhase : int {
 // one CTA in shared memory, larger ones by a cluster of CS_BC_CLUSTER CTAs
 #define CS_BC_NODES_PER_AGG 256
 #define CS_BC_MAX_G 16
+#define CS_BC_BIG_NODES (1 << 18)  // sheets up to this size take at most 8 x 8 cells
+// the finer grids' cells (coarse.cu): nodes of a fine cell, fine cells along the side of a middle one
+#define CS_BC_NODES_PER_FINE 30
+#define CS_BC_FINE_SPLIT 4
+#define CS_BC_RESTRICT_THREADS 512
+#define CS_BC_APPLY_THREADS 128
+#define CS_BC_UNROLL 4
 #define CS_BC_MAX_NC (3 * CS_BC_MAX_G * CS_BC_MAX_G)
 #define CS_BC_SMALL_NC 192
 #define CS_BC_CLUSTER 16
@@ -236,15 +247,21 @@ struct Batch {
     int bc_n_big = 0;            // sheets whose coarse system exceeds CS_BC_SMALL_NC
     int2* bc_agg = nullptr;      // per global aggregate: (sheet, local aggregate)
     int* bc_big = nullptr;       // the sheets inverted by a cluster
-    int* bc_node_agg = nullptr;  // per topology node: its aggregate
-    int* bc_mptr = nullptr;      // per topology aggregate: member range (na + 1 per topology)
-    int* bc_mem = nullptr;       // per topology: member nodes, by aggregate, ascending
+    int* bc_node_fine = nullptr; // per topology node: its fine cell
+    int* bc_aptr = nullptr;      // per topology aggregate: its middle cells (na + 1 per topology)
+    int* bc_fptr = nullptr;      // per topology middle cell: its fine cells (one more per topology)
+    int* bc_mptr = nullptr;      // per topology fine cell: its nodes in bc_mem (one more per topology)
+    int* bc_mem = nullptr;       // per topology: the nodes by fine cell, ascending
+    float* bc_finv = nullptr;    // per sheet fine cell: its diagonal block's inverse (9)
+    float* bc_minv = nullptr;    // the same of the middle cells
+    float* bc_ef = nullptr;      // per sheet fine cell: its correction, then the sum of all levels' (3)
+    float* bc_em = nullptr;      // per sheet middle cell: its correction (3)
+    int bc_max_nmid = 0;         // largest number of middle cells of a sheet
     int4* bc_pair = nullptr;     // per topology coarse pair: (a, b, contributor begin, end)
     int* bc_contrib = nullptr;   // topology slots (panel * 32 + lane) of the stored blocks of each pair
     float* bc_mat = nullptr;     // per sheet nc x nc: the coarse matrix R A R^T (then GJ's work)
     float* bc_inv = nullptr;     // per sheet nc x nc: its inverse, symmetrised
     float* bc_rc = nullptr;      // per sheet nc: R r
-    float* bc_ec = nullptr;      // per sheet nc: A_c^-1 R r
     int* bc_ok = nullptr;        // per sheet: the coarse inverse of this step is valid
     int n_slices = 0, n_panels = 0, n_tpanels = 0, n_tables = 0;
     // nodes

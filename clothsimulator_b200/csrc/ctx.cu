@@ -705,11 +705,14 @@ void permuteLanesByAggregate(Topo& T, const std::vector<int>& agg) {
 
 // Coarse space of the batched loop for one topology (coarse.cu): the nodes binned by their rest
 // (u, v) into g x g cells of the bounding box (g = round(sqrt(nodes / CS_BC_NODES_PER_AGG)),
-// 1..gmax), the non-empty cells numbered in cell order as aggregates; members of each
-// aggregate ascending; per pair of aggregates, the stored blocks coupling them in slot order.
+// 1..gmax), the non-empty cells numbered in cell order as aggregates; per pair of aggregates, the
+// stored blocks coupling them in slot order.  A cell's side is cut into s middle cells and each of
+// theirs into t fine ones, s t = round(sqrt(nodes per aggregate / CS_BC_NODES_PER_FINE)) as nearly as
+// s and t allow; the non-empty ones are numbered aggregate by aggregate and middle cell by middle cell.
 struct BCPlan {
     int na = 0;
-    std::vector<int> agg, mptr, mem, contrib;
+    int levels = 0;  // bit 0: fine cells smaller than the middle ones, bit 1: middle smaller than the aggregates
+    std::vector<int> agg, fine, aptr, fptr, mptr, mem, contrib;
     std::vector<int4> pairs;
 };
 
@@ -740,7 +743,9 @@ void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
     const int n = T.n_nodes;
     if (n <= 0 || (int)T.node_uv.size() < 2 * n) return;
     int g = (int)std::lround(std::sqrt((double)n / CS_BC_NODES_PER_AGG));
-    g = std::max(1, std::min(g, gmax));
+    // beyond 8 x 8 the inversion takes a cluster and 2 ms (768 unknowns): at 301 x 301 nodes it saved 15 of
+    // 98 iterations and cost 0.8 ms more than they, at 1,001 x 1,001 it is 3 of 90 ms
+    g = std::max(1, std::min(g, n <= CS_BC_BIG_NODES ? std::min(gmax, 8) : gmax));
     float u0 = T.node_uv[0], u1 = u0, v0 = T.node_uv[1], v1 = v0;
     for (int i = 0; i < n; i++) {
         u0 = std::min(u0, T.node_uv[2 * i]);
@@ -749,25 +754,37 @@ void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
         v1 = std::max(v1, T.node_uv[2 * i + 1]);
     }
     const double du = u1 > u0 ? (double)(u1 - u0) : 1.0, dv = v1 > v0 ? (double)(v1 - v0) : 1.0;
-    std::vector<int> cell(n), id(g * g, -1);
+    const double side = std::max(1.0, std::sqrt((double)n / ((double)g * g * CS_BC_NODES_PER_FINE)));
+    const int sm = std::max(1, (int)std::ceil(side / CS_BC_FINE_SPLIT - 0.25)), tf = std::max(1, (int)std::lround(side / sm));
+    P.levels = (tf > 1 ? 1 : 0) | (sm > 1 ? 2 : 0);
+    const int gf = g * sm * tf;
+    // a node's aggregate cell, middle cell in it and fine cell in that, as one key
+    std::vector<std::pair<long long, int>> key(n);
     for (int i = 0; i < n; i++) {
-        const int cu = std::min(g - 1, std::max(0, (int)((T.node_uv[2 * i] - u0) / du * g)));
-        const int cv = std::min(g - 1, std::max(0, (int)((T.node_uv[2 * i + 1] - v0) / dv * g)));
-        cell[i] = cu * g + cv;
-        id[cell[i]] = 0;
+        const int fu = std::min(gf - 1, std::max(0, (int)((T.node_uv[2 * i] - u0) / du * gf)));
+        const int fv = std::min(gf - 1, std::max(0, (int)((T.node_uv[2 * i + 1] - v0) / dv * gf)));
+        const int mu = fu / tf, mv = fv / tf;
+        const long long a = (long long)(mu / sm) * g + mv / sm, m = (a * sm + mu % sm) * sm + mv % sm;
+        key[i] = {(m * tf + fu % tf) * tf + fv % tf, i};
     }
-    for (int k = 0; k < g * g; k++)
-        if (id[k] == 0) id[k] = P.na++;
+    std::sort(key.begin(), key.end());
     P.agg.resize(n);
-    P.mptr.assign(P.na + 1, 0);
-    for (int i = 0; i < n; i++) {
-        P.agg[i] = id[cell[i]];
-        P.mptr[P.agg[i] + 1]++;
-    }
-    for (int a = 0; a < P.na; a++) P.mptr[a + 1] += P.mptr[a];
+    P.fine.resize(n);
     P.mem.resize(n);
-    std::vector<int> fill(P.mptr.begin(), P.mptr.end() - 1);
-    for (int i = 0; i < n; i++) P.mem[fill[P.agg[i]]++] = i;
+    const long long perMid = (long long)tf * tf, perAgg = perMid * sm * sm;
+    for (int i = 0; i < n; i++) {
+        const long long k = key[i].first, last = i ? key[i - 1].first : -1;
+        if (!i || k / perAgg != last / perAgg) P.aptr.push_back((int)P.fptr.size());
+        if (!i || k / perMid != last / perMid) P.fptr.push_back((int)P.mptr.size());
+        if (k != last) P.mptr.push_back(i);
+        P.mem[i] = key[i].second;
+        P.agg[P.mem[i]] = (int)P.aptr.size() - 1;
+        P.fine[P.mem[i]] = (int)P.mptr.size() - 1;
+    }
+    P.na = (int)P.aptr.size();
+    P.aptr.push_back((int)P.fptr.size());
+    P.fptr.push_back((int)P.mptr.size());
+    P.mptr.push_back(n);
     coarsePairs(T, P);
 }
 
@@ -1208,7 +1225,7 @@ int launchBatchedCoarseSetup(cs_ctx* c) {
 }
 int launchCoarseInverses(cs_ctx* c, const Batch& B, long long matFloats) {
     cudaMemsetAsync(B.bc_mat, 0, (size_t)matFloats * sizeof(float), c->stream);
-    const int gx = std::max(1, std::min(256, nblk(B.bc_max_npair, 8)));
+    const int gx = std::max(1, std::min(256, nblk(B.bc_max_npair + B.bc_max_nmid, 8)));
     cs_bc_assemble_kernel<<<dim3(gx, B.S), 256, 0, c->stream>>>(B);
     cs_bc_invert_small_kernel<<<B.S, CS_BC_THREADS, (CS_BC_SMALL_NC * CS_BC_SMALL_NC + 4 + 2 * CS_BC_KB * CS_BC_SMALL_NC + CS_BC_KB * CS_BC_KB) * sizeof(float),
                                 c->stream>>>(B);
@@ -1361,8 +1378,8 @@ void launchTrip(cs_ctx* c, cudaGraphConditionalHandle h) {
     cs_vector_kernel<<<g, 128, 0, c->stream>>>(B);
     if (B.bc_total_agg > 0 && c->tripCoarse) {
         // the coarse correction of z and the r.z, r.r partials it changes (coarse.cu)
-        cs_bc_restrict_kernel<<<B.bc_total_agg, 256, 0, c->stream>>>(B);
-        cs_bc_apply_kernel<<<nblk((long long)B.bc_total_agg * 96, 256), 256, 0, c->stream>>>(B);
+        cs_bc_restrict_kernel<<<B.bc_total_agg, CS_BC_RESTRICT_THREADS, 0, c->stream>>>(B);
+        cs_bc_apply_kernel<<<B.bc_total_agg, CS_BC_APPLY_THREADS, 0, c->stream>>>(B);
         cs_bc_finish_kernel<<<g, 128, 0, c->stream>>>(B);
     }
     cs_reduce2_kernel<<<B.S, CS_REDUCE_THREADS, 0, c->stream>>>(B, h);
@@ -1769,17 +1786,20 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     }
     std::vector<BCPlan> bcplans(topos.size());
     for (size_t t = 0; t < topos.size(); t++) batchedCoarsePlan(*topos[t], bcGmax, bcplans[t]);
-    std::vector<int> hbc_node_agg, hbc_mptr, hbc_mem, hbc_contrib;
+    std::vector<int> hbc_fine, hbc_aptr, hbc_fptr, hbc_mptr, hbc_mem, hbc_contrib;
     std::vector<int4> hbc_pair;
-    std::vector<int> topoBcNode0(topos.size()), topoBcAgg0(topos.size()), topoBcMem0(topos.size()),
-        topoBcPair0(topos.size());
+    std::vector<int> topoBcNode0(topos.size()), topoBcAgg0(topos.size()), topoBcMid0(topos.size()),
+        topoBcFine0(topos.size()), topoBcPair0(topos.size());
     for (size_t t = 0; t < topos.size(); t++) {
         const BCPlan& P = bcplans[t];
-        topoBcNode0[t] = (int)hbc_node_agg.size();
-        topoBcAgg0[t] = (int)hbc_mptr.size();
-        topoBcMem0[t] = (int)hbc_mem.size();
+        topoBcNode0[t] = (int)hbc_fine.size();
+        topoBcAgg0[t] = (int)hbc_aptr.size();
+        topoBcMid0[t] = (int)hbc_fptr.size();
+        topoBcFine0[t] = (int)hbc_mptr.size();
         topoBcPair0[t] = (int)hbc_pair.size();
-        hbc_node_agg.insert(hbc_node_agg.end(), P.agg.begin(), P.agg.end());
+        hbc_fine.insert(hbc_fine.end(), P.fine.begin(), P.fine.end());
+        hbc_aptr.insert(hbc_aptr.end(), P.aptr.begin(), P.aptr.end());
+        hbc_fptr.insert(hbc_fptr.end(), P.fptr.begin(), P.fptr.end());
         hbc_mptr.insert(hbc_mptr.end(), P.mptr.begin(), P.mptr.end());
         hbc_mem.insert(hbc_mem.end(), P.mem.begin(), P.mem.end());
         const int c0 = (int)hbc_contrib.size();
@@ -1895,7 +1915,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     }
     int node_off = 0, face_off = 0, edge_off = 0, slice_off = 0, panel_off = 0;
     long long nnzb = 0;
-    int bcVec = 0, bcMaxPair = 0;
+    int bcVec = 0, bcMaxPair = 0, bcMid = 0, bcFine = 0, bcMaxMid = 0;
     long long bcMat = 0;
     std::vector<int2> hbc_agg;
     std::vector<int> hbc_big;
@@ -1925,7 +1945,15 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             const BCPlan& P = bcplans[t];
             sd.bc_node_off = topoBcNode0[t];
             sd.bc_agg_off = topoBcAgg0[t];
-            sd.bc_mem_off = topoBcMem0[t];
+            sd.bc_mid_off = topoBcMid0[t];
+            sd.bc_fine_off = topoBcFine0[t];
+            sd.bc_nmid = P.na > 0 ? (int)P.fptr.size() - 1 : 0;
+            sd.bc_mvec_off = bcMid;
+            sd.bc_fvec_off = bcFine;
+            sd.bc_levels = P.levels;
+            bcMid += sd.bc_nmid;
+            bcFine += P.na > 0 ? (int)P.mptr.size() - 1 : 0;
+            bcMaxMid = std::max(bcMaxMid, sd.bc_nmid);
             sd.bc_pair_off = topoBcPair0[t];
             sd.bc_npair = (int)P.pairs.size();
             sd.bc_na = P.na;
@@ -2071,7 +2099,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             for (const int4& q : P.coarse.pairs) hgc_pair.push_back(make_int4(q.x, q.y, q.z + c0, q.w + c0));
             hgc_contrib.insert(hgc_contrib.end(), P.coarse.contrib.begin(), P.coarse.contrib.end());
         }
-        for (SheetDesc& d : hgs) d.bc_na = 0;
+        for (SheetDesc& d : hgs) d.bc_na = d.bc_nmid = 0;
         std::vector<int> gl;
         for (int s = 0; s < n_sheets; s++)
             if (hs[s].resident == 2) gl.push_back(s);
@@ -2149,7 +2177,9 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     UP(rowmap, hrowmap);
     UP(bc_agg, hbc_agg);
     UP(bc_big, hbc_big);
-    UP(bc_node_agg, hbc_node_agg);
+    UP(bc_node_fine, hbc_fine);
+    UP(bc_aptr, hbc_aptr);
+    UP(bc_fptr, hbc_fptr);
     UP(bc_mptr, hbc_mptr);
     UP(bc_mem, hbc_mem);
     UP(bc_pair, hbc_pair);
@@ -2157,10 +2187,14 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     if ((st = dalloc(c, &B.bc_mat, (size_t)std::max(1LL, bcMat))) != CS_OK) return st;
     if ((st = dalloc(c, &B.bc_inv, (size_t)std::max(1LL, bcMat))) != CS_OK) return st;
     if ((st = dalloc(c, &B.bc_rc, (size_t)std::max(1, bcVec))) != CS_OK) return st;
-    if ((st = dalloc(c, &B.bc_ec, (size_t)std::max(1, bcVec))) != CS_OK) return st;
+    if ((st = dalloc(c, &B.bc_finv, 9 * (size_t)std::max(1, bcFine))) != CS_OK) return st;
+    if ((st = dalloc(c, &B.bc_minv, 9 * (size_t)std::max(1, bcMid))) != CS_OK) return st;
+    if ((st = dalloc(c, &B.bc_ef, 3 * (size_t)std::max(1, bcFine))) != CS_OK) return st;
+    if ((st = dalloc(c, &B.bc_em, 3 * (size_t)std::max(1, bcMid))) != CS_OK) return st;
     UP(bc_ok, std::vector<int>(n_sheets, 0));
     B.bc_total_agg = (int)hbc_agg.size();
     B.bc_max_npair = bcMaxPair;
+    B.bc_max_nmid = bcMaxMid;
     B.bc_n_big = (int)hbc_big.size();
     c->bcMatFloats = bcMat;
     UP(row2slot, hrow2slot);
@@ -2223,6 +2257,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         G = B;
         G.bc_resident = 1;
         G.bc_max_npair = gMaxPair;
+        G.bc_max_nmid = 0;
         G.bc_n_big = (int)hgc_big.size();
         if ((st = upload(c, &G.sheets, hgs)) != CS_OK || (st = upload(c, &G.bc_pair, hgc_pair)) != CS_OK ||
             (st = upload(c, &G.bc_contrib, hgc_contrib)) != CS_OK || (st = upload(c, &G.bc_big, hgc_big)) != CS_OK ||
@@ -3282,8 +3317,8 @@ cs_status cs_profile_kernels(cs_ctx* c, const cs_step_params* p, int reps, float
         cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
         cudaEventRecord(c->ev0, c->stream);
         for (int r = 0; r < reps; r++) {
-            cs_bc_restrict_kernel<<<B.bc_total_agg, 256, 0, c->stream>>>(B);
-            cs_bc_apply_kernel<<<nblk((long long)B.bc_total_agg * 96, 256), 256, 0, c->stream>>>(B);
+            cs_bc_restrict_kernel<<<B.bc_total_agg, CS_BC_RESTRICT_THREADS, 0, c->stream>>>(B);
+            cs_bc_apply_kernel<<<B.bc_total_agg, CS_BC_APPLY_THREADS, 0, c->stream>>>(B);
             cs_bc_finish_kernel<<<g, 128, 0, c->stream>>>(B);
         }
         cudaEventRecord(c->ev1, c->stream);

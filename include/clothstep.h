@@ -100,9 +100,9 @@ typedef struct cs_step_params {
     int coarse;               /* 1 adds a coarse-space correction, 0 leaves it out.  Cluster-resident
                                  solver with the Chebyshev preconditioner: one constant per
                                  component on each of a few geometric segments of every CTA's
-                                 strip.  Batched loop: one per aggregate of about 256 nodes (the
-                                 rest (u, v) binned into at most 16 x 16 cells), added to
-                                 block-Jacobi; sheets with proximities keep block-Jacobi alone.
+                                 strip.  Batched loop: one per aggregate of 256 nodes or more
+                                 (the rest (u, v) binned into at most 16 x 16 cells) and one
+                                 per finer cell inside them, added to block-Jacobi; sheets with proximities keep block-Jacobi alone.
                                  Either way the coarse matrix R A R^T is inverted per sheet and
                                  step. */
     /* Cloth::physicsStep's `transformations` (Cloth.cuh:91-92): the motions' transformations at
