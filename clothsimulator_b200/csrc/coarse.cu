@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(128) cs_bc_finish_kernel(Batch B) {
 // ---------------------------------------------------------------------------------------
 // Coarse matrix of each resident sheet, for the coarse-space correction of the cluster-resident
 // solver (resident.cu): A_c = R A R^T, where R sums the rows of each aggregate (a segment of a
-// CTA's strip) per component, so block (a, b) of A_c is the sum of the stored blocks A_ij with
+// CTA's tile) per component, so block (a, b) of A_c is the sum of the stored blocks A_ij with
 // row i in aggregate a and column j in aggregate b.  The loader lists those blocks per pair
 // (a, b) in slot order; a warp sums a pair, lane l taking the blocks l, l + 32, ... in order,
 // and a butterfly combines the lanes (a fixed order: deterministic, no atomics).  A_c is SPD (A
@@ -690,6 +690,10 @@ __global__ void __launch_bounds__(CS_COARSE_THREADS) cs_coarse_setup_kernel(Batc
             for (int e = 0; e < 9; e++) M[(size_t)(3 * pr.x + e / 3) * ld + 3 * pr.y + e % 3] = acc[e];
         }
     }
+    __syncthreads();
+    // a segment without rows (a tile of fewer slices than segments) has an empty row: its unknown is 0
+    for (int q = tid; q < nc; q += blockDim.x)
+        if (M[(size_t)q * ld + q] == 0.f) M[(size_t)q * ld + q] = 1.f;
     __syncthreads();
     const int rs = blockDim.x / nc;  // rows whose updates run together (nc <= blockDim)
     const int j = tid % nc, i0 = tid / nc;

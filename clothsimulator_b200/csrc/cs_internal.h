@@ -100,17 +100,20 @@ enum InstPhase : int {
 // Reliable updates keep the search direction only while the recursive residual has drifted
 // from the FP64 one by at most this fraction of the latter (larger drift: restart).
 #define CS_RELIABLE_DRIFT 0.1
+#define CS_LAST_SWEEP 0.3  // on-chip solvers: recursive residual that ends the last sweep, of the tolerance
+// power iterations per sheet solve for the tile-local Chebyshev bound
 #define CS_CHEB_POWER_ITERS 10
-// A sheet uses the strip-local Chebyshev preconditioner only if at least this share of its
-// blocks couple rows of one strip.  Small sheets split into thin strips do better with
-// block-Jacobi; measured on the B200 (hanging and windy sheets, tol 1e-6): 24x24 (0.54 of the
+// A sheet uses the tile-local Chebyshev preconditioner only if at least this share of its
+// blocks couple rows of one CTA.  Small sheets split into thin strips do better with
+// block-Jacobi; measured on the B200 (hanging and windy sheets in strips, tol 1e-6): 24x24 (0.54 of the
 // blocks strip-local) and 28x28 (0.59) need fewer or as many iterations with block-Jacobi, 32x32
 // (0.71), 40x40 (0.65), 48x48 (0.84) and 64x64 (0.89) fewer with the Chebyshev polynomial.
-#define CS_CHEB_MIN_LOCAL 0.62  // power iterations per sheet solve for the strip-local Chebyshev bound
-// Coarse-space correction of the cluster-resident solver (with the strip-local Chebyshev
-// preconditioner): each CTA's strip of rows is cut into K segments along the principal axis of
-// its nodes' rest (uv) coordinates, K = min(CS_COARSE_MAX_K, CS_COARSE_AGGS / CTAs per cluster);
-// the coarse space holds one constant per (segment, component).
+#define CS_CHEB_MIN_LOCAL 0.62
+// Coarse-space correction of the cluster-resident solver: each CTA's tile of rows is cut into K
+// segments of whole slices, K = min(CS_COARSE_SEGS, CS_COARSE_AGGS / CTAs per cluster), and the coarse
+// space holds one constant per (segment, component): at most 64 unknowns, two per lane of a warp.  With
+// the levels below it (levels.cuh) more segments save little: 1, 2, 3 or 6 take 82, 76, 77 or 76
+// iterations on a 64 x 64 sheet.
 // threads of the per-instance reduction kernels of the batched loop
 #define CS_REDUCE_THREADS 256
 // coarse-space correction of the batched loop (coarse.cu): a sheet's nodes binned by their rest
@@ -134,7 +137,11 @@ enum InstPhase : int {
 #define CS_BC_PB 4
 #define CS_BC_KB (3 * CS_BC_PB)
 #define CS_COARSE_MAX_K 8
-#define CS_COARSE_AGGS 54
+#define CS_COARSE_SEGS 2
+#define CS_COARSE_AGGS 21
+// slices per CTA from which the coarse correction is worth its set-up: with 7.6 (48 x 48 quads) it saves
+// 15 of 79 iterations, with 3.5 (32 x 32) one of 58
+#define CS_COARSE_MIN_SLICES 5
 // Threads of the per-sheet set-up kernel that forms and inverts the coarse matrix, and its
 // dynamic shared memory: the nc x nc matrix with rows padded to 16 bytes, then one pivot block.
 #define CS_COARSE_THREADS 512
@@ -209,7 +216,7 @@ struct DevParams {
     int advance;           // 1: v += dv, x += dt v at the end of the step
     int warm_scale;        // 1: the warm start replaced by its Galerkin multiple before the guard
     int solver;            // CS_SOLVER_AUTO_DEV: resident sheets on the cluster kernel; BATCHED: loop only
-    int cheb_degree;       // resident solver: 1 block-Jacobi; odd >= 3 strip-local Chebyshev of that degree
+    int cheb_degree;       // resident solver: 1 block-Jacobi; odd >= 3 levels, or tile-local Chebyshev of that degree without `coarse`
     int coarse;            // resident solver with the Chebyshev preconditioner: 1 adds the coarse-space correction
     int n_motions;         // transformations of this step (cs_step_params.transformations)
     float motion[CS_MAX_MOTIONS][CS_TRANSFORM_FLOATS];
@@ -236,6 +243,7 @@ struct ProxInst {
 struct GroupItem {
     int sheet, cta0, ctas, segs;
     int slot0, red0, pub0, halo0;
+    int octets;  // its rows are in octet order (levels.cuh)
     long long mat;
 };
 
@@ -321,19 +329,15 @@ struct Batch {
     int* rsendptr = nullptr;     // per topology: CS_RES_MAX_CL + 1 offsets into rsend per owner rank
     uint32_t* rsend = nullptr;   // halo sends: src slot | dst rank << 12 | dst halo index << 16
     int* rhalo = nullptr;        // per topology: CS_RES_MAX_CL + 1 halo slot counts per rank
-    int* rcheb = nullptr;        // per topology and rank: 1 if the strip uses the Chebyshev preconditioner when asked
-    int res_halo0 = 0;           // first halo slot of every CTA's p array (= own slots per CTA)
-    int res_alt = 0;             // first slot of the second own-row buffer (strip-local Chebyshev)
+    int* rcheb = nullptr;        // per topology and rank: bit 0, the Chebyshev preconditioner when asked; bit 1, rows tiled (levels)
+    int res_halo0 = 0;           // first halo slot of every CTA's u array (after the own slots and a zero entry)
+    int res_alt = 0;             // first slot of the second own-row buffer (tile-local Chebyshev)
     // coarse-space correction (resident.cu): per topology {coarse unknowns nc (0: none), segments
-    // per strip K, first and last entry of the coarse pattern in cpair}; per topology row its
-    // sheet-local aggregate (rank * K + segment; at row2slot offsets); per topology, rank and
-    // warp the segments among the warp's rows (bit k: segment k); the coarse pattern's block
+    // per tile K, first and last entry of the coarse pattern in cpair}; the coarse pattern's block
     // pairs {aggregate a, aggregate b, first, last contributor in ccontrib} with their stored
     // blocks as topology slots; per resident work item the inverse coarse matrix (nc x nc) and
     // whether it was formed.
     int4* rcoarse = nullptr;
-    int* ragg = nullptr;
-    int* rwmask = nullptr;       // per topology: CS_RES_MAX_CL x CS_RES_MAX_WARPS
     int4* cpair = nullptr;
     int* ccontrib = nullptr;
     float* cinv = nullptr;

@@ -212,8 +212,10 @@ struct Topo {
     // the element's corners, 8 bits per corner
     std::vector<int> rf_ptr, re_ptr;
     std::vector<int2> rf, re;
-    // group-resident solver: CTAs its rows are tiled for (0: not tiled), coarse segments per CTA
-    int group_ctas = 0, group_segs = 0;
+    // CTAs its rows are tiled for (a cluster's, or a group's where `group`; 0: not tiled) and the
+    // segments each tile is ordered by
+    int tile_ctas = 0, tile_segs = 0;
+    bool group = false, octets = false;
     // rest (uv) coordinates of every node, from the first sheet of this connectivity: the
     // geometry the coarse-space segments of the cluster-resident solver are cut along
     std::vector<float> node_uv;
@@ -237,11 +239,12 @@ uint64_t hashInts(const int32_t* a, size_t n, uint64_t h) {
     return h;
 }
 
-// Rows ordered by tiles for the group-resident solver: the slices (32 rows) are dealt evenly to G
+// Rows ordered by tiles for the solvers that hold a sheet on chip: the slices (32 rows) are dealt evenly to G
 // CTAs and within a CTA to K segments, and recursive bisection of the rest coordinates along the
-// longer axis gives every segment a compact piece of the sheet; rows of a segment by block count
+// longer axis gives every segment a compact piece of the sheet.  With `octets` the bisection goes on to
+// slices and to eights of rows, each compact; else the rows of a segment are ordered by block count
 // (descending, then by index), which keeps its slices' padding low.
-void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, std::vector<int>& order) {
+void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, bool octets, std::vector<int>& order) {
     const int n = (int)len.size(), ns = (n + CS_SLICE - 1) / CS_SLICE;
     order.resize(n);
     for (int i = 0; i < n; i++) order[i] = i;
@@ -250,14 +253,8 @@ void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G,
         const int lo = (int)((long long)ns * c / G), hi = (int)((long long)ns * (c + 1) / G);
         for (int k = 0; k < K; k++) cut.push_back(std::min(n, CS_SLICE * (lo + (hi - lo) * (k + 1) / K)));
     }
-    std::function<void(int, int)> bisect = [&](int a, int b) {  // segments a .. b - 1
-        const int r0 = cut[a], r1 = cut[b];
-        if (r0 >= r1) return;
-        if (b - a == 1) {
-            std::sort(order.begin() + r0, order.begin() + r1,
-                      [&](int x, int y) { return len[x] != len[y] ? len[x] > len[y] : x < y; });
-            return;
-        }
+    // rows r0 .. r1 - 1 split at `at` along the longer axis of their bounds
+    auto split = [&](int r0, int at, int r1) {
         float lo[2] = {1e30f, 1e30f}, hi[2] = {-1e30f, -1e30f};
         for (int i = r0; i < r1; i++)
             for (int k = 0; k < 2; k++) {
@@ -265,20 +262,42 @@ void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G,
                 hi[k] = std::max(hi[k], uv[2 * order[i] + k]);
             }
         const int k = hi[1] - lo[1] > hi[0] - lo[0] ? 1 : 0;
-        // tiles are halved before their segments are
-        const int m = b - a > K ? a + ((b - a) / K + 1) / 2 * K : a + (b - a) / 2;
-        if (cut[m] > r0 && cut[m] < r1)
-            std::nth_element(order.begin() + r0, order.begin() + cut[m], order.begin() + r1, [&](int x, int y) {
+        if (at > r0 && at < r1)
+            std::nth_element(order.begin() + r0, order.begin() + at, order.begin() + r1, [&](int x, int y) {
                 return uv[2 * x + k] != uv[2 * y + k] ? uv[2 * x + k] < uv[2 * y + k] : x < y;
             });
+    };
+    std::function<void(int, int)> patches = [&](int r0, int r1) {
+        const int rows = r1 - r0, unit = rows > CS_SLICE ? CS_SLICE : 8, units = (rows + unit - 1) / unit;
+        if (units < 2) return;
+        const int at = r0 + (units / 2) * unit;
+        split(r0, at, r1);
+        patches(r0, at);
+        patches(at, r1);
+    };
+    std::function<void(int, int)> bisect = [&](int a, int b) {  // segments a .. b - 1
+        const int r0 = cut[a], r1 = cut[b];
+        if (r0 >= r1) return;
+        if (b - a == 1) {
+            if (octets)
+                patches(r0, r1);
+            else
+                std::sort(order.begin() + r0, order.begin() + r1,
+                          [&](int x, int y) { return len[x] != len[y] ? len[x] > len[y] : x < y; });
+            return;
+        }
+        // tiles are halved before their segments are
+        const int m = b - a > K ? a + ((b - a) / K + 1) / 2 * K : a + (b - a) / 2;
+        split(r0, cut[m], r1);
         bisect(a, m);
         bisect(m, b);
     };
     bisect(0, G * K);
 }
 
-// groupCtas: CTAs to tile the rows for (the group-resident solver), 0 for none.
-std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int groupCtas, std::string& err) {
+// tileCtas: CTAs to tile the rows for (0: none), at most `segs` segments per tile; octets: in
+// octet order whatever it pads.
+std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, bool octets, std::string& err) {
     auto t = std::make_shared<Topo>();
     const int nn = s.n_nodes, nv = s.n_verts, nf = s.n_faces;
     t->n_nodes = nn;
@@ -472,10 +491,32 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int groupCtas, std::stri
         }
     }
     t->n_slices = (nn + CS_SLICE - 1) / CS_SLICE;
-    if (groupCtas > 0) {
-        t->group_ctas = groupCtas;
-        t->group_segs = std::max(1, std::min({CS_COARSE_MAX_K, CS_GROUP_NC / (3 * groupCtas), t->n_slices / groupCtas}));
-        tileOrder(t->node_uv, len, t->group_ctas, t->group_segs, order);
+    if (tileCtas > 0) {
+        t->tile_ctas = tileCtas;
+        t->tile_segs = std::max(1, std::min(segs, t->n_slices / tileCtas));
+        // Octet order mixes long and short rows in a slice: little on a grid, a quarter more panels on an
+        // irregular mesh.  A group, whose tiles fill the shared memory, takes it up to a tenth more.
+        const int few = std::min(t->tile_segs, CS_COARSE_SEGS);
+        tileOrder(t->node_uv, len, t->tile_ctas, few, true, order);
+        t->octets = true;
+        if (!octets) {
+            std::vector<int> sorted;
+            tileOrder(t->node_uv, len, t->tile_ctas, t->tile_segs, false, sorted);
+            auto panels = [&](const std::vector<int>& o) {
+                long long n = 0;
+                for (int i = 0; i < nn; i += CS_SLICE) {
+                    int w = 0;
+                    for (int l = i; l < std::min(nn, i + CS_SLICE); l++) w = std::max(w, len[o[l]]);
+                    n += w;
+                }
+                return n;
+            };
+            if (10 * panels(order) > 11 * panels(sorted)) {
+                order.swap(sorted);
+                t->octets = false;
+            }
+        }
+        if (t->octets) t->tile_segs = few;
     }
     t->rowmap.assign((size_t)t->n_slices * CS_SLICE, 0);
     t->row2slot.assign(nn, 0);
@@ -597,23 +638,14 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int groupCtas, std::stri
     return t;
 }
 
-// Cluster-resident solve plan for one topology: contiguous slice ranges per CTA rank with
-// balanced panel counts.  Returns the largest number of slices a rank gets.
-int residentSplit(const Topo& T, int ncta, std::vector<int>& split) {
-    split.assign(CS_RES_MAX_CL + 1, T.n_slices);
-    std::vector<long long> pre(T.n_slices + 1, 0);
-    for (int i = 0; i < T.n_slices; i++) pre[i + 1] = pre[i] + T.slice_width[i];
-    split[0] = 0;
-    for (int c = 1; c < ncta; c++) {
-        const double target = (double)pre[T.n_slices] * c / ncta;
-        int sl = (int)(std::lower_bound(pre.begin(), pre.end(), (long long)std::ceil(target)) - pre.begin());
-        if (sl > 0 && target - pre[sl - 1] < pre[sl] - target) sl--;
-        split[c] = std::max(split[c - 1], std::min(sl, T.n_slices));
-    }
-    int w = 0;
-    for (int c = 0; c < ncta; c++) w = std::max(w, split[c + 1] - split[c]);
-    return w;
-}
+// Coarse space of one topology: each node's aggregate and, per pair of aggregates, the stored blocks
+// (topology slots) coupling them, in slot order; the batched loop's finer cells (batchedCoarsePlan).
+struct BCPlan {
+    int na = 0;
+    int levels = 0;  // bit 0: fine cells smaller than the middle ones, bit 1: middle smaller than the aggregates
+    std::vector<int> agg, fine, aptr, fptr, mptr, mem, contrib;
+    std::vector<int4> pairs;
+};
 
 // Halo plan of one topology on a cluster of `ncta` CTAs.  CTA c owns the rows of slices
 // [split[c], split[c+1]) at local slots (slice - split[c]) * 32 + lane.  Every column a CTA's
@@ -621,100 +653,27 @@ int residentSplit(const Topo& T, int ncta, std::vector<int>& split) {
 // (owner rank, owner slot).  code: per panel slot, the local p index of its column (own slot,
 // or CS_RES_HALO_BIT | halo index, rebased once the batch's own-slot count is known).  send:
 // per owner CTA (sendptr), the entries src slot | dst rank << 12 | dst halo index << 16.
-struct CoarsePlan {
-    int K = 0, nc = 0;             // segments per strip, coarse unknowns (3 per aggregate)
-    std::vector<int> agg;          // per local row: rank * K + segment
-    std::vector<int> wmask;        // CS_RES_MAX_CL x CS_RES_MAX_WARPS: segments among each warp's rows (bits)
-    std::vector<int4> pairs;       // coarse block pairs {a, b, first, last contributor}
-    std::vector<int> contrib;      // topology slots of the stored blocks, per pair ascending
-};
-
 struct ResidentPlan {
     std::vector<int> split, code, sendptr, halo_count;
     std::vector<uint32_t> send;
     int w = 0, max_halo = 0, max_panels = 0, max_width = 0;
     long long blocks = 0, local_blocks = 0;  // pattern blocks; those with row and column on one CTA
-    CoarsePlan coarse;
+    BCPlan coarse;
 };
 
-// Segments per strip of the coarse-space correction on a cluster of `ncta` CTAs; CS_COARSE_SEGMENTS
+// Segments per tile of the coarse-space correction on a cluster of `ncta` CTAs; CS_COARSE_SEGMENTS
 // (0..CS_COARSE_MAX_K, at most CS_COARSE_AGGS / ncta) sets it, 0 turns the correction off.
 int coarseSegments(int ncta) {
     const int cap = CS_COARSE_AGGS / std::max(ncta, 1);
     if (const char* ev = std::getenv("CS_COARSE_SEGMENTS")) return std::max(0, std::min({std::atoi(ev), CS_COARSE_MAX_K, cap}));
-    return std::min(CS_COARSE_MAX_K, cap);
+    return std::min(CS_COARSE_SEGS, cap);
 }
 
-// Shared memory of the coarse region of the resident kernel (resident.cu lays it out the same
-// way, each part rounded up to 4 floats): the CTA's rows of the inverse coarse matrix (3K x nc
-// floats), the coarse residual in FP32 (nc), the
-// correction of the CTA's aggregates and its partial sums (CP = 3K rounded up to 4, each), the
-// partials of every CTA in two buffers (2 x ncta x CP), then the coarse residual and search
-// direction in FP64 (nc each).
+// Shared memory of the coarse vectors of the resident kernel (resident.cu): a CTA's partial sums (CP =
+// 3K rounded up to 4 floats), every CTA's in two buffers, and the CTA's rows of A_c^-1.
 size_t coarseSmemBytes(int ncta, int K) {
-    if (K <= 0) return 0;
-    auto r4 = [](size_t n) { return (n + 3) / 4 * 4; };  // every part starts on 16 bytes
-    const size_t nc = 3 * (size_t)ncta * K, cp = r4(3 * (size_t)K);
-    const size_t f = r4(3 * (size_t)K * nc) + r4(nc) + 2 * cp + 2 * (size_t)ncta * cp;
-    return f * sizeof(float) + 2 * nc * sizeof(double);
+    return K <= 0 ? 0 : ((3 * (size_t)K + 3) / 4 * 4 * (1 + 2 * (size_t)ncta) + 3 * (size_t)K * 64) * sizeof(float);
 }
-
-// Reorders the lanes of every SELL slice of a topology so that rows of one coarse aggregate sit
-// in consecutive lanes (stable within an aggregate).  A slice keeps its rows and width; only
-// which lane holds which row changes, with every slot-indexed array (columns, contributor
-// lists, the block-CSR view's slots) moved along.  Per warp, the resident solver then sums a
-// vector over each aggregate with one segmented scan.
-void permuteLanesByAggregate(Topo& T, const std::vector<int>& agg) {
-    const size_t nslot = (size_t)T.n_tpanels * CS_SLICE;
-    std::vector<int> newOf(nslot), rowmap = T.rowmap;
-    for (int s = 0; s < T.n_slices; s++) {
-        const int rows = T.slice_rows[s];
-        std::vector<int> perm(rows), lnew(CS_SLICE);
-        for (int l = 0; l < rows; l++) perm[l] = l;
-        std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) {
-            return agg[T.rowmap[s * CS_SLICE + a]] < agg[T.rowmap[s * CS_SLICE + b]];
-        });
-        for (int l = 0; l < CS_SLICE; l++) lnew[l] = l;
-        for (int pos = 0; pos < rows; pos++) {
-            lnew[perm[pos]] = pos;
-            rowmap[s * CS_SLICE + pos] = T.rowmap[s * CS_SLICE + perm[pos]];
-        }
-        for (int k = 0; k < T.slice_width[s]; k++)
-            for (int l = 0; l < CS_SLICE; l++)
-                newOf[(size_t)(T.slice_tpanel0[s] + k) * CS_SLICE + l] = (T.slice_tpanel0[s] + k) * CS_SLICE + lnew[l];
-    }
-    std::vector<int> oldOf(nslot), tcol(nslot), tcptr(nslot + 1);
-    for (size_t o = 0; o < nslot; o++) oldOf[newOf[o]] = (int)o;
-    std::vector<uint32_t> tcontrib;
-    tcontrib.reserve(T.tcontrib.size());
-    for (size_t q = 0; q < nslot; q++) {
-        const int o = oldOf[q];
-        tcol[q] = T.tcol[o];
-        tcptr[q] = (int)tcontrib.size();
-        tcontrib.insert(tcontrib.end(), T.tcontrib.begin() + T.tcptr[o], T.tcontrib.begin() + T.tcptr[o + 1]);
-    }
-    tcptr[nslot] = (int)tcontrib.size();
-    for (int& q : T.csr_slot) q = newOf[q];
-    T.rowmap = rowmap;
-    for (int s = 0; s < T.n_slices; s++)
-        for (int l = 0; l < T.slice_rows[s]; l++) T.row2slot[rowmap[s * CS_SLICE + l]] = s * CS_SLICE + l;
-    T.tcol.swap(tcol);
-    T.tcptr.swap(tcptr);
-    T.tcontrib.swap(tcontrib);
-}
-
-// Coarse space of the batched loop for one topology (coarse.cu): the nodes binned by their rest
-// (u, v) into g x g cells of the bounding box (g = round(sqrt(nodes / CS_BC_NODES_PER_AGG)),
-// 1..gmax), the non-empty cells numbered in cell order as aggregates; per pair of aggregates, the
-// stored blocks coupling them in slot order.  A cell's side is cut into s middle cells and each of
-// theirs into t fine ones, s t = round(sqrt(nodes per aggregate / CS_BC_NODES_PER_FINE)) as nearly as
-// s and t allow; the non-empty ones are numbered aggregate by aggregate and middle cell by middle cell.
-struct BCPlan {
-    int na = 0;
-    int levels = 0;  // bit 0: fine cells smaller than the middle ones, bit 1: middle smaller than the aggregates
-    std::vector<int> agg, fine, aptr, fptr, mptr, mem, contrib;
-    std::vector<int4> pairs;
-};
 
 // The pairs of aggregates and their stored blocks (slots with contributors; padding has none).
 void coarsePairs(const Topo& T, BCPlan& P) {
@@ -738,6 +697,12 @@ void coarsePairs(const Topo& T, BCPlan& P) {
     }
 }
 
+// Coarse space of the batched loop for one topology (coarse.cu): the nodes binned by their rest
+// (u, v) into g x g cells of the bounding box (g = round(sqrt(nodes / CS_BC_NODES_PER_AGG)),
+// 1..gmax), the non-empty cells numbered in cell order as aggregates; per pair of aggregates, the
+// stored blocks coupling them in slot order.  A cell's side is cut into s middle cells and each of
+// theirs into t fine ones, s t = round(sqrt(nodes per aggregate / CS_BC_NODES_PER_FINE)) as nearly as
+// s and t allow; the non-empty ones are numbered aggregate by aggregate and middle cell by middle cell.
 void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
     P = BCPlan();
     const int n = T.n_nodes;
@@ -788,86 +753,49 @@ void batchedCoarsePlan(const Topo& T, int gmax, BCPlan& P) {
     coarsePairs(T, P);
 }
 
-// Coarse-space plan of one topology on a cluster of `ncta` CTAs: each CTA's strip of rows is cut
-// into K segments of equal row count along the principal axis of the rows' rest coordinates (a
-// strip of a grid sheet is a band of grid rows; its segments are blocks side by side), and the
-// coarse pattern lists, per pair of aggregates, the stored blocks coupling them in slot order.
-void coarsePlan(const Topo& T, ResidentPlan& P, int ncta, int K) {
-    CoarsePlan& C = P.coarse;
-    C = CoarsePlan();
-    C.K = K;
-    C.nc = 3 * ncta * K;
-    C.agg.assign(T.n_nodes, -1);
-    C.wmask.assign(CS_RES_MAX_CL * CS_RES_MAX_WARPS, 0);
+// Coarse space of a tiled topology on `ncta` CTAs: the slices of each CTA cut into K segments.
+void tileCoarse(const Topo& T, int ncta, int K, BCPlan& P) {
+    P = BCPlan();
+    P.na = ncta * K;
+    P.agg.resize(T.n_nodes);
     for (int c = 0; c < ncta; c++) {
-        std::vector<std::pair<int, int>> rows;  // (local row, own slot)
-        for (int sl = P.split[c]; sl < P.split[c + 1]; sl++)
-            for (int l = 0; l < T.slice_rows[sl]; l++)
-                rows.push_back({T.rowmap[sl * CS_SLICE + l], (sl - P.split[c]) * CS_SLICE + l});
-        const int n = (int)rows.size();
-        double mx = 0.0, my = 0.0;
-        for (auto& r : rows) {
-            mx += T.node_uv[2 * r.first];
-            my += T.node_uv[2 * r.first + 1];
-        }
-        mx /= std::max(n, 1);
-        my /= std::max(n, 1);
-        double sxx = 0.0, sxy = 0.0, syy = 0.0;
-        for (auto& r : rows) {
-            const double dx = T.node_uv[2 * r.first] - mx, dy = T.node_uv[2 * r.first + 1] - my;
-            sxx += dx * dx;
-            sxy += dx * dy;
-            syy += dy * dy;
-        }
-        // principal axis: eigenvector of the larger eigenvalue of the 2x2 scatter matrix
-        const double tr = sxx + syy, det = sxx * syy - sxy * sxy;
-        const double l1 = 0.5 * tr + std::sqrt(std::max(0.0, 0.25 * tr * tr - det));
-        double ax = 1.0, ay = 0.0;
-        if (std::fabs(sxy) > 0.0) {
-            ax = l1 - syy;
-            ay = sxy;
-        } else if (syy > sxx) {
-            ax = 0.0;
-            ay = 1.0;
-        }
-        std::vector<std::pair<double, int>> key(n);
-        for (int i = 0; i < n; i++) {
-            const int r = rows[i].first;
-            key[i] = {(T.node_uv[2 * r] - mx) * ax + (T.node_uv[2 * r + 1] - my) * ay, i};
-        }
-        std::sort(key.begin(), key.end());
+        const int lo = (int)((long long)T.n_slices * c / ncta), hi = (int)((long long)T.n_slices * (c + 1) / ncta);
         for (int k = 0; k < K; k++)
-            for (int i = (int)((long long)k * n / K); i < (int)((long long)(k + 1) * n / K); i++) {
-                const auto& r = rows[key[i].second];
-                C.agg[r.first] = c * K + k;
-                C.wmask[c * CS_RES_MAX_WARPS + r.second / CS_SLICE] |= 1 << k;  // own slot / 32 = warp
-            }
+            for (int sl = lo + (hi - lo) * k / K; sl < lo + (hi - lo) * (k + 1) / K; sl++)
+                for (int l = 0; l < T.slice_rows[sl]; l++) P.agg[T.rowmap[sl * CS_SLICE + l]] = c * K + k;
     }
-    // coarse pattern: every stored block (slots with contributors; padding has none)
-    std::vector<std::tuple<int, int, int>> blk;  // (a, b, slot)
-    for (int sl = 0; sl < T.n_slices; sl++)
-        for (int k = 0; k < T.slice_width[sl]; k++)
-            for (int l = 0; l < T.slice_rows[sl]; l++) {
-                const int slot = (T.slice_tpanel0[sl] + k) * CS_SLICE + l;
-                if (T.tcptr[slot + 1] == T.tcptr[slot]) continue;
-                blk.emplace_back(C.agg[T.rowmap[sl * CS_SLICE + l]], C.agg[T.tcol[slot]], slot);
-            }
-    std::sort(blk.begin(), blk.end());
-    for (size_t i = 0; i < blk.size();) {
-        size_t j = i;
-        while (j < blk.size() && std::get<0>(blk[j]) == std::get<0>(blk[i]) && std::get<1>(blk[j]) == std::get<1>(blk[i])) j++;
-        C.pairs.push_back(make_int4(std::get<0>(blk[i]), std::get<1>(blk[i]), (int)C.contrib.size(),
-                                    (int)(C.contrib.size() + (j - i))));
-        for (size_t q = i; q < j; q++) C.contrib.push_back(std::get<2>(blk[q]));
-        i = j;
-    }
+    coarsePairs(T, P);
 }
 
 #define CS_RES_HALO_BIT 0x40000000
 
+// The slices of each CTA: an even share of them where the rows are tiled for it, else contiguous
+// ranges of balanced panel counts.
+void residentSplit(const Topo& T, int ncta, bool tiled, ResidentPlan& P) {
+    std::vector<long long> pre(T.n_slices + 1, 0);
+    for (int i = 0; i < T.n_slices; i++) pre[i + 1] = pre[i] + T.slice_width[i];
+    P.split.assign(CS_RES_MAX_CL + 1, T.n_slices);
+    P.split[0] = 0;
+    for (int c = 1; c < ncta; c++) {
+        if (tiled) {
+            P.split[c] = (int)((long long)T.n_slices * c / ncta);
+            continue;
+        }
+        const double target = (double)pre[T.n_slices] * c / ncta;
+        int sl = (int)(std::lower_bound(pre.begin(), pre.end(), (long long)std::ceil(target)) - pre.begin());
+        if (sl > 0 && target - pre[sl - 1] < pre[sl] - target) sl--;
+        P.split[c] = std::max(P.split[c - 1], std::min(sl, T.n_slices));
+    }
+    P.w = P.max_panels = 0;
+    for (int c = 0; c < ncta; c++) {
+        P.w = std::max(P.w, P.split[c + 1] - P.split[c]);
+        P.max_panels = std::max(P.max_panels, (int)(pre[P.split[c + 1]] - pre[P.split[c]]));
+    }
+}
+
 ResidentPlan residentPlan(const Topo& T, int ncta) {
     ResidentPlan P;
-    P.w = residentSplit(T, ncta, P.split);
+    residentSplit(T, ncta, T.tile_ctas > 0, P);
     const int nn = T.n_nodes;
     std::vector<int> owner(nn, 0), oslot(nn, 0);
     for (int c = 0; c < ncta; c++)
@@ -939,22 +867,14 @@ struct GroupPlan {
 
 GroupPlan groupPlan(const Topo& T) {
     GroupPlan P;
-    const int G = T.group_ctas, K = T.group_segs, ns = T.n_slices;
+    const int G = T.tile_ctas, K = T.tile_segs, ns = T.n_slices;
     std::vector<int> owner(T.n_nodes), first(G + 1);
     for (int c = 0; c <= G; c++) first[c] = (int)((long long)ns * c / G);
-    P.coarse.agg.resize(T.n_nodes);
     for (int c = 0; c < G; c++) {
-        const int nsl = first[c + 1] - first[c];
-        P.max_own = std::max(P.max_own, nsl);
-        for (int sl = first[c], seg = 0; sl < first[c + 1]; sl++) {
-            while (seg + 1 < K && sl - first[c] >= nsl * (seg + 1) / K) seg++;
-            for (int l = 0; l < T.slice_rows[sl]; l++) {
-                owner[T.rowmap[sl * CS_SLICE + l]] = c;
-                P.coarse.agg[T.rowmap[sl * CS_SLICE + l]] = c * K + seg;
-            }
-        }
+        P.max_own = std::max(P.max_own, first[c + 1] - first[c]);
+        for (int sl = first[c]; sl < first[c + 1]; sl++)
+            for (int l = 0; l < T.slice_rows[sl]; l++) owner[T.rowmap[sl * CS_SLICE + l]] = c;
     }
-    P.coarse.na = G * K;
     P.code.assign(T.tcol.size(), 0);
     P.pub.assign((size_t)ns * CS_SLICE, 0);
     P.halo_ptr.push_back(0);
@@ -989,7 +909,7 @@ GroupPlan groupPlan(const Topo& T) {
                     P.code[slot] = owner[col] == c ? T.row2slot[col] - first[c] * CS_SLICE : CS_RES_HALO_BIT | at[col];
                 }
     }
-    coarsePairs(T, P.coarse);
+    tileCoarse(T, G, K, P.coarse);
     return P;
 }
 
@@ -1087,7 +1007,7 @@ struct cs_ctx {
     int residentProx = 0;       // those of them that a proximity touches
     int loopSheets = 0;         // sheets that the batched loop solves on the AUTO route
     int proxSteps = 0;          // steps since the proximities last changed
-    std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, strip-local ones
+    std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, tile-local ones
     // proximities (cs_set_proximities): their device lists, and the host copies of the
     // blocks outside the pattern that cs_get_system merges
     ProxBuffers prox;
@@ -1537,9 +1457,15 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     cudaDeviceProp devProp;
     CS_CUDA(cudaGetDeviceProperties(&devProp, c->device));
     const int maxCtas = devProp.multiProcessorCount;
-    const char* clEnv = std::getenv("CS_RESIDENT_CL");
-    const bool groupsOn = !(clEnv && std::atoi(clEnv) == 0);
-    const int clusterSlices = 10 * CS_RES_MAX_WARPS;
+    // CS_RESIDENT_CL (2..16) forces a cluster size; 0 solves every sheet in the batched loop
+    int forcedCl = -1;
+    if (const char* ev = std::getenv("CS_RESIDENT_CL")) {
+        forcedCl = std::atoi(ev);
+        if (forcedCl != 0 && (forcedCl < 2 || forcedCl > CS_RES_MAX_CL))
+            return fail(c, CS_ERR_INVALID_ARG, "CS_RESIDENT_CL must be 0 or 2..16");
+    }
+    const bool groupsOn = forcedCl != 0;
+    const int clusterSlices = (forcedCl > 0 ? forcedCl : 10) * CS_RES_MAX_WARPS;
     long long groupSlices = 0;
     for (int s = 0; s < n_sheets; s++) {
         const int ns = nblk(sheets[s].n_nodes, CS_SLICE);
@@ -1555,6 +1481,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     // topologies (shared)
     std::map<TopoKey, int> topoIndex;
     std::vector<std::shared_ptr<Topo>> topos;
+    std::vector<int> topoSheet;  // a sheet of each
     c->sheetTopo.assign(n_sheets, nullptr);
     std::vector<int> sheetTopoId(n_sheets);
     for (int s = 0; s < n_sheets; s++) {
@@ -1569,13 +1496,15 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             sheetTopoId[s] = it->second;
         } else {
             std::string err;
-            auto t = buildTopo(d, groupCtasFor(d.n_nodes), err);
+            const int G = groupCtasFor(d.n_nodes);
+            auto t = buildTopo(d, G, G > 0 ? std::min(CS_COARSE_MAX_K, CS_GROUP_NC / (3 * G)) : 0, false, err);
             if (!t) return fail(c, CS_ERR_INVALID_ARG, "sheet %d: %s", s, err.c_str());
+            t->group = G > 0;
             sheetTopoId[s] = (int)topos.size();
             topoIndex[k] = (int)topos.size();
             topos.push_back(t);
+            topoSheet.push_back(s);
         }
-        c->sheetTopo[s] = topos[sheetTopoId[s]];
     }
     // materials: scaled stretching tables per distinct (rows, multiplier)
     std::map<std::vector<float>, std::vector<float>> baseSamples;
@@ -1621,18 +1550,10 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     std::vector<int> topoNbrPtr0(topos.size()), topoNbr0(topos.size());
     std::vector<int> topoPanel0(topos.size()), topoSlice0(topos.size());
     std::vector<int> htcsr_ptr, htcsr_col, htcsr_slot, topoCsrPtr0(topos.size());
-    // Cluster-resident solve plan (resident.cu).  Clusters must fit a GPC, so the number of
-    // SMs a cluster size keeps busy varies: 8- and 9-CTA clusters are planned and the one that
-    // makes the most sheets resident, then keeps the most SMs busy, is taken (on the B200, 15
-    // clusters of 8 occupy 120 SMs, 15 clusters of 9 occupy 135, 11 of 10 occupy 110).
-    // CS_RESIDENT_CL (2..16) forces a size; 0 solves every sheet in the batched loop.
-    std::vector<int> candidates = {8, 9, 10};
-    if (const char* ev = std::getenv("CS_RESIDENT_CL")) {
-        const int v = std::atoi(ev);
-        if (v != 0 && (v < 2 || v > CS_RES_MAX_CL))
-            return fail(c, CS_ERR_INVALID_ARG, "CS_RESIDENT_CL must be 0 or 2..16");
-        candidates = {v};
-    }
+    // Cluster-resident solve plan (resident.cu).  Clusters must fit a GPC, so the number of SMs a
+    // cluster size keeps busy varies: the one of 8, 9 and 10 CTAs that makes the most sheets resident,
+    // then keeps the most SMs busy, is taken (on the B200, 15 clusters of 8 occupy 120 SMs, 15 clusters
+    // of 9 occupy 135, 11 of 10 occupy 110), by estimates of each sheet's share of a CTA.
     struct ResChoice {
         int cl = 0, w = 0, panels = 0, halo = 0, cap = 0, clusters = 0, ck = 0;
         long long sheets = 0;
@@ -1642,15 +1563,25 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     };
     cudaFuncAttributes resAttr;
     CS_CUDA(cudaFuncGetAttributes(&resAttr, cs_resident_pcg_kernel));
-    auto planFor = [&](int cl) {
+    // The plan for clusters of `cl` CTAs: exact once the topologies are tiled for them, before that with the
+    // rows' present order and a halo estimated from a square tile's perimeter.
+    auto planFor = [&](int cl, bool exact) {
         ResChoice R;
         R.cl = cl;
         R.plans.resize(topos.size());
         R.resident.assign(topos.size(), 0);
         for (size_t t = 0; t < topos.size() && cl > 0; t++) {
-            if (topos[t]->n_slices > CS_RES_MAX_WARPS * cl) continue;  // no split fits
-            R.plans[t] = residentPlan(*topos[t], cl);
-            const ResidentPlan& P = R.plans[t];
+            const Topo& T = *topos[t];
+            if (T.n_slices > CS_RES_MAX_WARPS * cl || T.group) continue;
+            ResidentPlan& P = R.plans[t];
+            if (exact) {
+                P = residentPlan(T, cl);
+            } else {
+                residentSplit(T, cl, T.n_slices >= 2 * cl, P);
+                P.max_width = *std::max_element(T.slice_width.begin(), T.slice_width.end());
+                P.max_halo = cl > 1 ? (int)(8.0 * std::sqrt(32.0 * P.w)) + 32 : 0;
+                P.blocks = P.local_blocks = 1;
+            }
             // p indices (own slots + halo) are 12-bit in the kernel's packed column codes
             if (P.w > CS_RES_MAX_WARPS || P.max_width > CS_RES_MAX_WIDTH || P.max_halo + CS_RES_MAX_WARPS * CS_SLICE >= 4096)
                 continue;
@@ -1660,23 +1591,24 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             R.halo = std::max(R.halo, P.max_halo);
         }
         if (R.w == 0) return R;
-        // coarse-space correction for the topologies with the strip-local Chebyshev
-        // preconditioner (it needs a second warp for the segment sums)
+        // coarse-space correction for the topologies of enough slices (it needs a second warp for the
+        // segment sums, which they have)
         R.ck = coarseSegments(cl);
         bool anyCoarse = false;
         for (size_t t = 0; t < topos.size(); t++)
-            anyCoarse |= R.resident[t] && R.plans[t].blocks > 0 &&
-                         (double)R.plans[t].local_blocks >= CS_CHEB_MIN_LOCAL * (double)R.plans[t].blocks;
-        if (!anyCoarse || R.ck < 2 || R.w < 2) R.ck = 0;
-        // p array: own slots, halo slots, then a second own-slot buffer (strip-local Chebyshev),
+            anyCoarse |= R.resident[t] && topos[t]->n_slices >= CS_COARSE_MIN_SLICES * cl;
+        if (!anyCoarse) R.ck = 0;
+        // p array: own slots, halo slots, then a second own-slot buffer (tile-local Chebyshev),
         // then the coarse region
-        const size_t ubytes = ((size_t)2 * R.w * CS_SLICE + R.halo) * sizeof(float4);
+        const size_t ubytes = (2 * ((size_t)R.w * CS_SLICE + 1) + R.halo) * sizeof(float4);
         const size_t pbytes = ubytes + coarseSmemBytes(cl, R.ck);
         const size_t budget = devProp.sharedMemPerBlockOptin > resAttr.sharedSizeBytes + pbytes
                                   ? devProp.sharedMemPerBlockOptin - resAttr.sharedSizeBytes - pbytes : 0;
         R.cap = (int)std::min<size_t>((size_t)R.panels, budget / (CS_PANEL_FLOATS * sizeof(float)));
-        R.smem = (size_t)R.cap * CS_PANEL_FLOATS * sizeof(float) + pbytes;
-        if (budget > 0) {
+        // Clusters at a time with `cap` panels per CTA in shared memory
+        auto clustersWith = [&](int cap) {
+            R.smem = (size_t)cap * CS_PANEL_FLOATS * sizeof(float) + pbytes;
+            int n = 0;
             raiseDynSmem((const void*)cs_resident_pcg_kernel, R.smem);
             if (cl > 8) cudaFuncSetAttribute(cs_resident_pcg_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             cudaLaunchConfig_t cfg = {};
@@ -1690,8 +1622,26 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             cfg.dynamicSmemBytes = R.smem;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&R.clusters, cs_resident_pcg_kernel, &cfg) != cudaSuccess) R.clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, cs_resident_pcg_kernel, &cfg) != cudaSuccess) n = 0;
             cudaGetLastError();
+            return n;
+        };
+        if (budget > 0) {
+            // Two CTAs per SM hide each other's waits: where all but a quarter of the panels fit half an
+            // SM's shared memory and there are sheets for it, the others are read from L2
+            const size_t half = devProp.sharedMemPerMultiprocessor / 2 - devProp.reservedSharedMemPerBlock - resAttr.sharedSizeBytes;
+            const int cap2 = half > pbytes ? (int)((half - pbytes) / (CS_PANEL_FLOATS * sizeof(float))) : 0;
+            long long n = 0;
+            for (int sh = 0; sh < n_sheets; sh++) n += R.resident[sheetTopoId[sh]];
+            R.clusters = clustersWith(R.cap);
+            if (cap2 < R.cap && 4 * cap2 >= 3 * R.panels && n > R.clusters) {
+                const int two = clustersWith(cap2);
+                if (two > R.clusters) {
+                    R.clusters = two;
+                    R.cap = cap2;
+                }
+                R.smem = (size_t)R.cap * CS_PANEL_FLOATS * sizeof(float) + pbytes;
+            }
         }
         if (R.clusters <= 0) {
             R.clusters = 0;
@@ -1701,16 +1651,41 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         return R;
     };
     ResChoice res;
-    for (int cl : candidates) {
-        ResChoice R = planFor(cl);
-        const bool better = res.cl == 0 || R.sheets > res.sheets ||
-                            (R.sheets == res.sheets && (long long)R.clusters * R.cl > (long long)res.clusters * res.cl);
-        if (better) res = std::move(R);
+    {
+        ResChoice est;
+        if (forcedCl >= 0) {
+            est = planFor(forcedCl, false);
+        } else {
+            for (int cl : {8, 9, 10}) {
+                ResChoice R = planFor(cl, false);
+                if (est.cl == 0 || R.sheets > est.sheets ||
+                    (R.sheets == est.sheets && (long long)R.clusters * R.cl > (long long)est.clusters * est.cl))
+                    est = std::move(R);
+            }
+        }
+        const int best = est.cl;
+        if (best > 0) {
+            for (size_t t = 0; t < topos.size(); t++) {
+                // sheets of fewer than two slices per CTA keep the rows' own order: tiles of one slice have no
+                // patches within to correct, their strips are too thin for the Chebyshev preconditioner
+                // (CS_CHEB_MIN_LOCAL), they take block-Jacobi
+                if (!est.resident[t] || topos[t]->n_slices < 2 * best) continue;
+                std::string err;
+                auto T = buildTopo(sheets[topoSheet[t]], best, std::max(1, coarseSegments(best)), true, err);
+                if (!T) return fail(c, CS_ERR_INVALID_ARG, "sheet %d: %s", topoSheet[t], err.c_str());
+                topos[t] = T;
+            }
+            res = planFor(best, true);
+        } else {
+            res.resident.assign(topos.size(), 0);
+            res.plans.resize(topos.size());
+        }
     }
+    for (int s = 0; s < n_sheets; s++) c->sheetTopo[s] = topos[sheetTopoId[s]];
     std::vector<int> hrsplit(topos.size() * (CS_RES_MAX_CL + 1), 0), hrcode;
     std::vector<int> hrsendptr(topos.size() * (CS_RES_MAX_CL + 1), 0);
     std::vector<int> hrhalo(topos.size() * (CS_RES_MAX_CL + 1), 0);
-    // sheets whose strips keep enough of the couplings use the strip-local Chebyshev
+    // sheets whose tiles keep enough of the couplings use the tile-local Chebyshev
     // preconditioner (when asked for); the others stay with block-Jacobi
     std::vector<int> hrcheb(topos.size() * (CS_RES_MAX_CL + 1), 0);
     std::vector<uint32_t> hrsend;
@@ -1723,35 +1698,24 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             std::copy(plans[t].halo_count.begin(), plans[t].halo_count.end(), hrhalo.begin() + t * (CS_RES_MAX_CL + 1));
             const bool cheb = plans[t].blocks > 0 &&
                               (double)plans[t].local_blocks >= CS_CHEB_MIN_LOCAL * (double)plans[t].blocks;
-            for (int r = 0; r <= CS_RES_MAX_CL; r++) hrcheb[t * (CS_RES_MAX_CL + 1) + r] = cheb;
-            if (cheb && res.ck > 0) {
-                // segments, then the lanes of each slice grouped by segment, then the plans
-                // again over the moved slots (the slices and their rows stay)
-                coarsePlan(*topos[t], plans[t], res.cl, res.ck);
-                permuteLanesByAggregate(*topos[t], plans[t].coarse.agg);
-                plans[t] = residentPlan(*topos[t], res.cl);
-                coarsePlan(*topos[t], plans[t], res.cl, res.ck);
-            }
+            const bool tiled = topos[t]->tile_ctas > 0;
+            for (int r = 0; r <= CS_RES_MAX_CL; r++) hrcheb[t * (CS_RES_MAX_CL + 1) + r] = (cheb ? 1 : 0) | (tiled ? 2 : 0);
+            if (tiled && res.ck > 0 && topos[t]->n_slices >= CS_COARSE_MIN_SLICES * res.cl)
+                tileCoarse(*topos[t], res.cl, res.ck, plans[t].coarse);
         }
     // coarse-space arrays, per topology concatenated
     std::vector<int4> hrcoarse(topos.size(), make_int4(0, 0, 0, 0)), hcpair;
-    std::vector<int> hragg, hrwmask(topos.size() * CS_RES_MAX_CL * CS_RES_MAX_WARPS, 0), hccontrib;
+    std::vector<int> hccontrib;
     for (size_t t = 0; t < topos.size(); t++) {
-        static const CoarsePlan none;
-        const CoarsePlan& C = t < plans.size() ? plans[t].coarse : none;
-        if (topoResident[t] && C.nc > 0) {
+        const BCPlan& C = plans[t].coarse;
+        if (topoResident[t] && C.na > 0) {
             const int p0 = (int)hcpair.size(), c0 = (int)hccontrib.size();
             for (const int4& q : C.pairs) hcpair.push_back(make_int4(q.x, q.y, q.z + c0, q.w + c0));
             hccontrib.insert(hccontrib.end(), C.contrib.begin(), C.contrib.end());
-            std::copy(C.wmask.begin(), C.wmask.end(), hrwmask.begin() + t * CS_RES_MAX_CL * CS_RES_MAX_WARPS);
-            hrcoarse[t] = make_int4(C.nc, C.K, p0, (int)hcpair.size());
-            hragg.insert(hragg.end(), C.agg.begin(), C.agg.end());
-        } else {
-            hragg.insert(hragg.end(), topos[t]->n_nodes, -1);
+            hrcoarse[t] = make_int4(3 * C.na, res.ck, p0, (int)hcpair.size());
         }
     }
-    // the batched loop's coarse spaces (after the lane moves above: the contributor slots refer
-    // to the final slot numbering); up to CS_BC_MAX_G^2 aggregates when 16-CTA clusters can run
+    // the batched loop's coarse spaces; up to CS_BC_MAX_G^2 aggregates when 16-CTA clusters can run
     // the larger inversions, else as many as one CTA inverts
     int bcGmax = CS_BC_MAX_G;
     {
@@ -1818,7 +1782,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         int warps = 0, panels = 0;
         for (size_t t = 0; t < topos.size(); t++) {
             const Topo& T = *topos[t];
-            if (T.group_ctas <= 0 || topoResident[t]) continue;
+            if (!T.group || topoResident[t]) continue;
             gplans[t] = groupPlan(T);
             const GroupPlan& P = gplans[t];
             const int nc = 3 * P.coarse.na;
@@ -1828,13 +1792,13 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                         (2 * (size_t)P.max_own * CS_SLICE + P.max_halo) * sizeof(float4) + 24 * 1024 > optin)
                 continue;
             topoGroup[t] = 1;
-            B.g_max = std::max(B.g_max, T.group_ctas);
+            B.g_max = std::max(B.g_max, T.tile_ctas);
             warps = std::max(warps, P.max_own);
             panels = std::max(panels, P.max_panels);
             B.g_halo = std::max(B.g_halo, P.max_halo);
             B.g_cnc = std::max(B.g_cnc, nc);
-            B.g_ck3 = std::max(B.g_ck3, 3 * T.group_segs);
-            B.g_cai = std::max(B.g_cai, 3 * T.group_segs * nc);
+            B.g_ck3 = std::max(B.g_ck3, 3 * T.tile_segs);
+            B.g_cai = std::max(B.g_cai, 3 * T.tile_segs * nc);
         }
         if (warps > 0) {
             B.g_own = warps * CS_SLICE;
@@ -1878,7 +1842,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             if (topoResident[t]) {
                 // halo slots follow the batch's own slots in every CTA's p array
                 for (int code : plans[t].code)
-                    hrcode.push_back(code & CS_RES_HALO_BIT ? resW * CS_SLICE + (code & ~CS_RES_HALO_BIT) : code);
+                    hrcode.push_back(code & CS_RES_HALO_BIT ? resW * CS_SLICE + 1 + (code & ~CS_RES_HALO_BIT) : code);
                 const int base = (int)hrsend.size();
                 for (int k = 0; k <= CS_RES_MAX_CL; k++) hrsendptr[t * (CS_RES_MAX_CL + 1) + k] = base + plans[t].sendptr[k];
                 hrsend.insert(hrsend.end(), plans[t].send.begin(), plans[t].send.end());
@@ -2060,8 +2024,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     std::stable_sort(hrlist.begin(), hrlist.end(), [&](int a, int b) { return hs[a].n_slices > hs[b].n_slices; });
     B.n_resident = (int)hrlist.size();
     B.res_cap = resCap;
-    B.res_halo0 = resW * CS_SLICE;
-    B.res_alt = resW * CS_SLICE + res.halo;
+    B.res_halo0 = resW * CS_SLICE + 1;  // a zero entry before the halo
+    B.res_alt = B.res_halo0 + res.halo;
     c->resClustersMax = c->resClusters;
     c->resClusters = std::min(c->resClusters, B.n_resident);
     c->rlistAll = hrlist;
@@ -2103,11 +2067,11 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         std::vector<int> gl;
         for (int s = 0; s < n_sheets; s++)
             if (hs[s].resident == 2) gl.push_back(s);
-        auto ctasOf = [&](int s) { return topos[sheetTopoId[s]]->group_ctas; };
+        auto ctasOf = [&](int s) { return topos[sheetTopoId[s]]->tile_ctas; };
         std::stable_sort(gl.begin(), gl.end(), [&](int a, int b) { return ctasOf(a) > ctasOf(b); });
         std::vector<double> busy(maxCtas, 0.0);
         for (int s : gl) {
-            const int t = sheetTopoId[s], G = ctasOf(s), K = topos[t]->group_segs;
+            const int t = sheetTopoId[s], G = ctasOf(s), K = topos[t]->tile_segs;
             int best = 0;
             double when = 1e300;
             for (int o = 0; o + G <= maxCtas; o++) {
@@ -2117,7 +2081,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                     best = o;
                 }
             }
-            GroupItem gi{s, best, G, K, gSlots, gRed, topoPub0[t], topoHalo0[t], gMat};
+            GroupItem gi{s, best, G, K, gSlots, gRed, topoPub0[t], topoHalo0[t], topos[t]->octets ? 1 : 0, gMat};
             for (int k = best; k < best + G; k++) {
                 busy[k] = when + std::sqrt((double)hs[s].n_nodes);
                 ctaItems[k].push_back((int)hgitem.size());
@@ -2209,8 +2173,6 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     UP(rhalo, hrhalo);
     UP(rcheb, hrcheb);
     UP(rcoarse, hrcoarse);
-    UP(ragg, hragg);
-    UP(rwmask, hrwmask);
     UP(cpair, hcpair);
     UP(ccontrib, hccontrib);
     if (B.n_group > 0) {

@@ -34,6 +34,7 @@
 // 72 x 72 quads 8.1 -> 1.8 ms, an irregular sheet of 261 x 261 nodes 13.0 -> 4.3 ms, 64 sheets of 4 to
 // 128 quads a side 15.5 -> 9.9 ms.
 #include "cs_internal.h"
+#include "levels.cuh"
 
 namespace {
 
@@ -93,6 +94,7 @@ struct __align__(16) GroupShared {
     int cheb_deg;
     float cheb_inv_th;
     float cheb_a[CS_PRECOND_MAX_DEGREE], cheb_b[CS_PRECOND_MAX_DEGREE];
+    alignas(16) float lev[CS_GROUP_MAX_WARPS][5][8];
 };
 
 // The dynamic shared memory after the panels and the three parts of the u array, each part
@@ -392,8 +394,10 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         };
         // The tile-local Chebyshev polynomial's interval: power iteration for P^-1 A_loc, as in
         // resident.cu (an odd degree keeps the preconditioner SPD whatever the estimate).
+        const bool levels = P.coarse && P.cheb_degree >= 3 && gi.octets;
         __syncthreads();
-        if (P.cheb_degree >= 3) {
+        if (levels) level_blocks(spn, gpn, ks, width, code, w, lane, live, S.lev[w]);
+        if (!levels && P.cheb_degree >= 3) {
             float v[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -610,6 +614,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                 coarse_matvec();
                 __syncthreads();
             }
+            if (levels) level_correction(S.lev[w], r, lane, u);
             if (coarse && live) {
                 // u = C r + R^T A_c^-1 R r: the additive coarse-space correction
 #pragma unroll

@@ -6,31 +6,39 @@
 // the shared memory of a cluster of 8 to 10 CTAs (227 KB each), so here each cluster
 //   * takes the next sheet from a device work counter (persistent clusters; a sheet that
 //     converges early frees its cluster at once, there is no batch-wide tail),
-//   * copies its share of the sheet's SELL-32 panels (a contiguous strip of slices) into
-//     shared memory once per solve,
+//   * copies its tile of the sheet's SELL-32 panels (a contiguous range of slices; the loader orders
+//     the rows by tiles) into shared memory once per solve (what exceeds the budget, spread evenly
+//     over the slices, is read from L2),
 //   * runs the per-instance state machine of the batched loop (FP32 CG on the correction
 //     system, FP64 dot products and norms, FP64 residual replacements with the search
 //     direction kept (reliable updates), warm-start guard, inner and outer stopping tests)
 //     with the FP32 vectors in registers, one thread per row.  The CG recurrence is the
 //     Chronopoulos-Gear form: per iteration one SpMV w = A u and ONE fused reduction of
 //     (r.u, w.u, r.r), instead of two reductions;
-//   * preconditions with the 3x3 block-Jacobi inverse or, when asked and the sheet's strips
-//     keep enough of its couplings, with a Chebyshev polynomial in the block-Jacobi-scaled
-//     strip of rows each CTA holds (its SpMVs read only the CTA's own shared memory);
+//   * preconditions with the 3x3 block-Jacobi inverse; when asked, for a sheet whose rows are ordered
+//     by tiles, together with the levels of levels.cuh and, on larger sheets, a coarse-space
+//     correction (one constant per component on CS_COARSE_SEGS segments of every tile), or, without
+//     that correction, with a Chebyshev polynomial in the block-Jacobi-scaled tile each CTA holds (its
+//     SpMVs read only the CTA's own shared memory) if the tiles keep enough of the couplings;
 //   * exchanges data without cluster barriers: after u = P^-1 r each CTA pushes the values
-//     of its strip's boundary rows into the halo slots of the CTAs that read them with
+//     of its tile's boundary rows into the halo slots of the CTAs that read them with
 //     st.async remote stores, which complete bytes on the receiver's mbarrier; reduction
 //     partials travel the same way.  A CTA waits only on its own mbarriers.  Sends for step
 //     k+1 depend on every CTA's step-k partial, so one halo buffer and two reduction buffers
 //     suffice (a sender is never two steps ahead of a receiver);
-//   * sums deterministically: a butterfly within each warp (IEEE addition is commutative, so
-//     every lane ends with the same bits), then warp and CTA partials in a fixed order, every
-//     CTA summing the same partials: all CTAs take identical decisions;
-//   * runs the SpMV's local slots while the halo values travel, the halo slots after.
+//   * sums deterministically: lanes, warps and CTAs in fixed orders, every CTA summing the same
+//     partials: all CTAs take identical decisions;
+//   * forms the sums r.u and r.r while the halo values travel.
 // Every wait is bounded.  A CTA whose wait runs out raises an abort flag in all CTAs and an
 // error word for the host, and all CTAs leave through the kernel's final cluster barrier (the
 // only one after start-up), so no CTA exits while another may still address its memory.
-// Rows of a slice beyond the shared-memory panel budget are read from global memory.
+//
+// What bounds it: the chain of latencies of one iteration -- its instructions in the slowest warp, two
+// exchanges through the cluster (halo, reduction), FP64 sums -- about 6 us for a 64 x 64 sheet on 9 CTAs
+// of 15 warps, 4 us for a 16 x 16 one.  Measured on the B200 (tol 1e-6, whole steps) against strips of
+// rows with a strip-local Chebyshev-3, 162 coarse unknowns and sums by every thread: a lone sheet of 64 x
+// 64 quads 1.14 -> 0.82 ms, 48 x 48 0.92 -> 0.52, 32 x 32 0.85 -> 0.34, 16 x 16 0.38 -> 0.30; 96 sheets of
+// 45 x 45 4.3 -> 2.9 ms, 700 of 64 x 64 46.0 -> 39.9 ms.
 //
 // Replaces the reference's per-cloth GPU solve (Cloth.cu:766-809) like pcg.cu does; the
 // block-Jacobi preconditioner is the 3x3 block inverse from the gather kernel (the reference
@@ -38,6 +46,7 @@
 #include <cooperative_groups.h>
 
 #include "cs_internal.h"
+#include "levels.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -130,24 +139,29 @@ __device__ __forceinline__ bool rfinite(double x) { return x == x && x < 1e300 &
 struct __align__(16) ResShared {
     double red[2][CS_RES_MAX_CL][4];   // reduction partials by sender rank, two buffers
     double wsum[CS_RES_MAX_WARPS][4];  // warp partials
+    float wy[CS_RES_MAX_WARPS][4];     // warp sums of the coarse restriction
+    double tot[6];                     // a reduction's sums and the scalars derived from them
     uint64_t bar[5];                   // 0 halo, 1-2 reduction buffers, 3 residual signal, 4 work item
     int next;                          // work item sent by rank 0
     int abort_flag;                    // raised by any CTA whose wait ran out
-    // strip-local Chebyshev preconditioner of the current sheet: degree (1: block-Jacobi),
+    // tile-local Chebyshev preconditioner of the current sheet: degree (1: block-Jacobi),
     // 1/theta, and per step k the coefficients of d_k = a_k d_{k-1} + b_k P^-1 (r - A_loc x)
     int cheb_deg;
     float cheb_inv_th;
     float cheb_a[CS_PRECOND_MAX_DEGREE], cheb_b[CS_PRECOND_MAX_DEGREE];
+    // inverse diagonal blocks of the levels: per warp its four octets, then the slice (six entries)
+    alignas(16) float lev[CS_RES_MAX_WARPS][5][8];
+    double sc[CS_RES_MAX_WARPS][7];    // scalars of the solve, per warp
 };
 
 constexpr float CHEB_LMAX_MARGIN = 1.1f; // the estimate approaches lambda_max from below
 constexpr float CHEB_LMIN_RATIO = 1.0f / 30.0f;
 
-// Waits for `parity` of `bar` on every thread, at most RES_WAIT_TRIES polls, giving up early
-// once another CTA raised the abort flag.  Returns true on every thread only if the whole
-// CTA saw the phase complete.
+// Waits for `parity` of `bar`, at most RES_WAIT_TRIES polls, giving up early once another CTA raised
+// the abort flag (res_poll); on every thread, returning true only if the whole CTA saw the phase
+// complete (res_wait).
 template <bool CLUSTER = false>
-__device__ __forceinline__ bool res_wait(ResShared& S, uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool res_poll(ResShared& S, uint32_t bar, uint32_t parity) {
     bool ok = false;
     for (uint32_t t = 0; t < RES_WAIT_TRIES; t++) {
         if (rbar_test<CLUSTER>(bar, parity)) {
@@ -158,7 +172,12 @@ __device__ __forceinline__ bool res_wait(ResShared& S, uint32_t bar, uint32_t pa
         // back off: polls share the shared-memory pipe with the remote stores being awaited
         __nanosleep(RES_POLL_NS);
     }
-    return __syncthreads_and(ok ? 1 : 0) != 0;
+    __syncwarp();
+    return ok;
+}
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool res_wait(ResShared& S, uint32_t bar, uint32_t parity) {
+    return __syncthreads_and(res_poll<CLUSTER>(S, bar, parity) ? 1 : 0) != 0;
 }
 
 // Raises the abort flag in every CTA of the cluster and the error word for the host.
@@ -169,196 +188,148 @@ __device__ __forceinline__ void res_abort(const cg::cluster_group& cl, ResShared
     }
 }
 
-// Cluster-wide sum of three values (fp32: in float, the plain FP32 solver; else double).
-// Order: a butterfly within each warp, then the warp partials in warp order, then the CTA
-// partials in rank order.  The last two are serial sums over broadcast shared-memory reads,
-// done redundantly by every thread that needs the result (no shuffles: with ~20 warps per SM
-// the shuffle pipe is the bottleneck of a butterfly).  Every CTA sums the same partials in
-// the same order, so all threads of the cluster return identical sums.  Partials travel by
-// st.async into buffer `nred & 1` of every CTA.  Returns false if the wait gave up (the
-// caller aborts).
-__device__ __forceinline__ bool cluster_sum3(ResShared& S, int rank, int ncta, uint32_t& nred, double (&v)[3], bool fp32) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int b = (int)(nred & 1u);
-#pragma unroll
-    for (int i = 0; i < 3; i++) v[i] = fp32 ? (double)rwarp_sum((float)v[i]) : rwarp_sum(v[i]);
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 3; i++) S.wsum[w][i] = v[i];
-    }
-    __syncthreads();
-    if (w == 0 && lane < ncta) {
-        // unrolled to the compile-time bound so every load issues before the add chain
-        double t[3];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            if (fp32) {
-                float a = 0.f;
-#pragma unroll
-                for (int j = 0; j < CS_RES_MAX_WARPS; j++)
-                    if (j < nw) a += (float)S.wsum[j][i];
-                t[i] = (double)a;
-            } else {
-                double a = 0.0;
-#pragma unroll
-                for (int j = 0; j < CS_RES_MAX_WARPS; j++)
-                    if (j < nw) a += S.wsum[j][i];
-                t[i] = a;
-            }
-        }
-        const uint32_t bar = saddr(&S.bar[1 + b]);
-        if (lane == 0) rbar_expect(bar, (uint32_t)ncta * 32u);
-        const uint32_t dst = mapa(saddr(&S.red[b][rank][0]), lane);
-        const uint32_t dbar = mapa(bar, lane);
-        st_async_d2(dst, t[0], t[1], dbar);
-        st_async_d2(dst + 16, t[2], 0.0, dbar);
-    }
-    const bool ok = res_wait(S, saddr(&S.bar[1 + b]), (nred >> 1) & 1u);
-    nred++;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        if (fp32) {
-            float a = 0.f;
-#pragma unroll
-            for (int c = 0; c < CS_RES_MAX_CL; c++)
-                if (c < ncta) a += (float)S.red[b][c][i];
-            v[i] = (double)a;
-        } else {
-            double a = 0.0;
-#pragma unroll
-            for (int c = 0; c < CS_RES_MAX_CL; c++)
-                if (c < ncta) a += S.red[b][c][i];
-            v[i] = a;
-        }
-    }
-    return ok;
-}
-
-// The coarse-space correction's state in one CTA's shared memory: the coarse region the loader
-// sizes with coarseSmemBytes, each part rounded up to 4 floats.  Offsets come from the kernel
-// parameters (res_cnc = nc, res_ck = K), so they hold no registers.
-//   ai   this CTA's rows of the inverse coarse matrix, 3K x nc
-//   r32  the coarse residual R r in FP32 (the matrix-vector product's input), nc
-//   ce   the correction of this CTA's aggregates, 3K (CP = 3K rounded up to 4)
-//   part this CTA's segment sums before they are sent, CP
-//   red  every CTA's segment sums: [buffer][rank][CP]
-//   r64, s64  the coarse residual R r and search direction R s in FP64, nc each
+// The coarse vectors in one CTA's shared memory, sized by the loader with coarseSmemBytes (CP = 3K
+// rounded up to 4 floats):
+//   part  this CTA's segment sums before they are sent, CP
+//   red   every CTA's segment sums: [buffer][rank][CP]
+//   ai    the rows of A_c^-1 of this CTA's segments, 3K x 64 (nc <= 64)
 struct CoarseSm {
     unsigned char* base;
     int nc, k3, cp;
     __device__ __forceinline__ CoarseSm(unsigned char* b, int nc_, int k) : base(b), nc(nc_), k3(3 * k), cp((3 * k + 3) / 4 * 4) {}
-    __device__ __forceinline__ static int r4(int n) { return (n + 3) / 4 * 4; }
-    __device__ __forceinline__ float* ai() const { return reinterpret_cast<float*>(base); }
-    __device__ __forceinline__ float* r32() const { return ai() + r4(k3 * nc); }
-    __device__ __forceinline__ float* ce() const { return r32() + r4(nc); }
-    __device__ __forceinline__ float* part() const { return ce() + cp; }
+    __device__ __forceinline__ float* part() const { return reinterpret_cast<float*>(base); }
     __device__ __forceinline__ float* red() const { return part() + cp; }
-    __device__ __forceinline__ double* r64(int ncta) const { return reinterpret_cast<double*>(red() + 2 * ncta * cp); }
-    __device__ __forceinline__ double* s64(int ncta) const { return r64(ncta) + nc; }
+    __device__ __forceinline__ float* ai(int ncta) const { return red() + 2 * ncta * cp; }
     // entry q of the coarse vector in one buffer of `red` (rank q / 3K, segment and component
     // q % 3K)
     __device__ __forceinline__ int off(int q) const { return (q / k3) * cp + q % k3; }
 };
 
-// cluster_sum3 that also carries the coarse vector R y of a per-row vector y.  The lanes of a
-// slice hold the rows of one segment consecutively (the loader orders them so); `cseg` packs this
-// lane's run: the run's first lane (bits 0-4), whether this lane ends it (bit 5), the segment + 1
-// (bits 8-15; 0 for a lane without a row) and, for the gathering lanes of warp 1, the warps
-// holding the lane's segment (bits 16-31); bit 6 is the caller's.  A segmented inclusive scan (5 shuffle steps per
-// component) leaves each run's sum in its last lane, which stages it in `wp` (warp-major, CP
-// floats per warp); after the first barrier lane 3k + c of warp 1 adds component c of segment
-// k over the warps holding it (bits 16-31 of its cseg), in warp order, and those sums travel
-// with the three values to every CTA.  On return buffer (nred - 1) & 1 of C.red holds R y, entry
-// q at C.off(q) (q = 3 (rank K + k) + c); it may be overwritten by the reduction after next.
-// Deterministic like cluster_sum3.
-__device__ __forceinline__ bool cluster_sum3c(ResShared& S, int rank, int ncta, uint32_t& nred, double (&v)[3], bool fp32,
-                                              const float (&y)[3], bool live, int cseg, float* wp, const CoarseSm& C) {
+// Warp sums of two (lanes 0-15 return the first, 16-31 the second) and of three values (lanes 0-7, 8-15,
+// 16-23), by exchanges that halve the values a lane carries: 5 and 8 additions instead of 10 and 15.
+template <class T>
+__device__ __forceinline__ T rwarp_sum2(T a, T b) {
+    const bool up = threadIdx.x & 16;
+    T v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <class T>
+__device__ __forceinline__ T rwarp_sum3(T a, T b, T c) {
+    const bool up = threadIdx.x & 16, odd = threadIdx.x & 8;
+    T x = __shfl_xor_sync(0xffffffffu, up ? a : c, 16), y = __shfl_xor_sync(0xffffffffu, up ? b : T(0), 16);
+    x += up ? c : a;
+    y += up ? T(0) : b;
+    T v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// The warp's part of a reduction: sums 0 and 2, sum 1, or the coarse restriction of y, in shared memory.
+__device__ __forceinline__ void put_sum02(ResShared& S, double a, double c, bool fp32) {
+    const int lane = threadIdx.x & 31;
+    const double t = fp32 ? (double)rwarp_sum2((float)a, (float)c) : rwarp_sum2(a, c);
+    if ((lane & 15) == 0) S.wsum[threadIdx.x >> 5][lane >> 3] = t;  // lane 0: sum 0, lane 16: sum 2
+}
+__device__ __forceinline__ void put_sum1(ResShared& S, double a, bool fp32) {
+    const double t = fp32 ? (double)rwarp_sum((float)a) : rwarp_sum(a);
+    if ((threadIdx.x & 31) == 0) S.wsum[threadIdx.x >> 5][1] = t;
+}
+__device__ __forceinline__ void put_coarse(ResShared& S, const float (&y)[3]) {
+    const int lane = threadIdx.x & 31;
+    const float t = rwarp_sum3(y[0], y[1], y[2]);
+    if ((lane & 7) == 0 && lane < 24) S.wy[threadIdx.x >> 5][lane >> 3] = t;
+}
+// The sums over 16 lanes (each half of the warp) of three values, in FP64 or (fp32) in float.
+__device__ __forceinline__ void half_sum3(double (&t)[3], bool fp32) {
+    if (fp32) {
+        float f[3] = {(float)t[0], (float)t[1], (float)t[2]};
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 3; i++) f[i] += __shfl_xor_sync(0xffffffffu, f[i], o);
+#pragma unroll
+        for (int i = 0; i < 3; i++) t[i] = (double)f[i];
+        return;
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 3; i++) t[i] += __shfl_xor_sync(0xffffffffu, t[i], o);
+}
+
+// Cluster-wide sum of three values (fp32: in float, the plain FP32 solver; else double) and, with
+// COARSE, the coarse vector R y of a per-row vector y, of the warps' sums that put_* stored.  Its time is a chain of latencies, so the stages
+// are short and only warp 0 works on the cluster's: a barrier; warp 0 adds the warps' sums
+//  (a lane per warp) and sends the CTA's partials by st.async to buffer `nred & 1` of every CTA,
+// waits for everyone's, adds them (a lane per CTA), calls `post` on the sums for the scalars that
+// depend on them, and publishes both; a barrier.  Fixed orders, the same in every CTA: all threads of
+// the cluster return identical sums.  (Sums added serially by every thread and divisions done by every
+// thread took 5,900 of the 12,500 cycles of an iteration on a 64 x 64 sheet.)
+// R y: every warp's rows are of one segment (the loader cuts a tile's slices into K ranges); after the
+// first barrier lane 3k + c of warp 1 adds component c over segment k's warps, in warp order, and sends
+// the sums.  On return buffer (nred - 1) & 1 of C.red holds R y, entry q at C.off(q) (q = 3 (rank K + k)
+// + c); it may be overwritten by the reduction after next.
+// Returns false if the wait gave up (the caller aborts).
+template <bool COARSE, class Post>
+__device__ __forceinline__ bool cluster_reduce(ResShared& S, int rank, int ncta, uint32_t& nred, double (&v)[3], bool fp32,
+                                               int nsl, const CoarseSm& C, Post post) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int b = (int)(nred & 1u);
-    {
-        const int rs = cseg & 31, sg = ((cseg >> 8) & 0xff) - 1;
-        float a0 = live ? y[0] : 0.f, a1 = live ? y[1] : 0.f, a2 = live ? y[2] : 0.f;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const float t0 = __shfl_up_sync(0xffffffffu, a0, d), t1 = __shfl_up_sync(0xffffffffu, a1, d),
-                        t2 = __shfl_up_sync(0xffffffffu, a2, d);
-            if (lane - d >= rs) {
-                a0 += t0;
-                a1 += t1;
-                a2 += t2;
-            }
-        }
-        if (((cseg >> 5) & 1) && sg >= 0 && 3 * sg < C.k3) {
-            wp[w * C.cp + 3 * sg] = a0;
-            wp[w * C.cp + 3 * sg + 1] = a1;
-            wp[w * C.cp + 3 * sg + 2] = a2;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++) v[i] = fp32 ? (double)rwarp_sum((float)v[i]) : rwarp_sum(v[i]);
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 3; i++) S.wsum[w][i] = v[i];
-    }
     __syncthreads();
-    double t[3] = {0.0, 0.0, 0.0};
-    if (w == 0 && lane < ncta) {
+    bool ok = true;
+    if (w == 0) {
+        const uint32_t bar = saddr(&S.bar[1 + b]);
+        if (lane == 0) rbar_expect(bar, (uint32_t)ncta * (32u + (COARSE ? 4u * (uint32_t)C.cp : 0u)));
+        const int h = lane & 15;
+        double t[3] = {0.0, 0.0, 0.0};
+        if (h < nw)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            if (fp32) {
-                float a = 0.f;
+            for (int i = 0; i < 3; i++) t[i] = S.wsum[h][i];
+        half_sum3(t, fp32);
+        if (lane < ncta) {
+            const uint32_t dst = mapa(saddr(&S.red[b][rank][0]), lane);
+            const uint32_t dbar = mapa(bar, lane);
+            st_async_d2(dst, t[0], t[1], dbar);
+            st_async_d2(dst + 16, t[2], 0.0, dbar);
+        }
+        ok = res_poll(S, bar, (nred >> 1) & 1u);
+        t[0] = t[1] = t[2] = 0.0;
+        if (h < ncta)
 #pragma unroll
-                for (int j = 0; j < CS_RES_MAX_WARPS; j++)
-                    if (j < nw) a += (float)S.wsum[j][i];
-                t[i] = (double)a;
-            } else {
-                double a = 0.0;
+            for (int i = 0; i < 3; i++) t[i] = S.red[b][h][i];
+        half_sum3(t, fp32);
+        double x[3] = {0.0, 0.0, 0.0};
+        post(t, x);
+        if (lane == 0) {
 #pragma unroll
-                for (int j = 0; j < CS_RES_MAX_WARPS; j++)
-                    if (j < nw) a += S.wsum[j][i];
-                t[i] = a;
+            for (int i = 0; i < 3; i++) {
+                S.tot[i] = t[i];
+                S.tot[3 + i] = x[i];
             }
         }
-    }
-    if (w == 1 && lane < C.cp) {
-        float a = 0.f;
-        const unsigned wk = (unsigned)cseg >> 16;  // the warps holding this lane's segment
-#pragma unroll
-        for (int j = 0; j < CS_RES_MAX_WARPS; j++)
-            if ((wk >> j) & 1u) a += wp[j * C.cp + lane];
-        C.part()[lane] = a;
-    }
-    // warps 0 and 1 only (named barrier 1 of 64 threads): the segment sums are in place before
-    // warp 0 sends them; the other warps go straight to the wait
-    if (w < 2) asm volatile("bar.sync 1, 64;" ::: "memory");
-    if (w == 0 && lane < ncta) {
+    } else if (COARSE && w == 1) {
         const uint32_t bar = saddr(&S.bar[1 + b]);
-        if (lane == 0) rbar_expect(bar, (uint32_t)ncta * (32u + 4u * (uint32_t)C.cp));
-        const uint32_t dst = mapa(saddr(&S.red[b][rank][0]), lane);
-        const uint32_t dbar = mapa(bar, lane);
-        st_async_d2(dst, t[0], t[1], dbar);
-        st_async_d2(dst + 16, t[2], 0.0, dbar);
-        const uint32_t cdst = mapa(saddr(C.red() + ((size_t)b * ncta + rank) * C.cp), lane);
-        for (int q = 0; q < C.cp / 4; q++) st_async_f4(cdst + 16u * q, reinterpret_cast<const float4*>(C.part())[q], dbar);
+        if (lane < C.cp) {
+            float a = 0.f;
+            const int K = C.k3 / 3, k = lane / 3, c = lane - 3 * k, q0 = (nsl * k) / K, q1 = k < K ? (nsl * (k + 1)) / K : q0;
+#pragma unroll 8
+            for (int q = q0; q < q1; q++) a += S.wy[q][c];
+            C.part()[lane] = a;
+        }
+        __syncwarp();
+        if (lane < ncta) {
+            const uint32_t cdst = mapa(saddr(C.red() + ((size_t)b * ncta + rank) * C.cp), lane);
+            const uint32_t dbar = mapa(bar, lane);
+            for (int q = 0; q < C.cp / 4; q++)
+                st_async_f4(cdst + 16u * q, reinterpret_cast<const float4*>(C.part())[q], dbar);
+        }
     }
-    const bool ok = res_wait(S, saddr(&S.bar[1 + b]), (nred >> 1) & 1u);
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
     nred++;
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-        if (fp32) {
-            float a = 0.f;
-#pragma unroll
-            for (int c = 0; c < CS_RES_MAX_CL; c++)
-                if (c < ncta) a += (float)S.red[b][c][i];
-            v[i] = (double)a;
-        } else {
-            double a = 0.0;
-#pragma unroll
-            for (int c = 0; c < CS_RES_MAX_CL; c++)
-                if (c < ncta) a += S.red[b][c][i];
-            v[i] = a;
-        }
-    }
+    for (int i = 0; i < 3; i++) v[i] = S.tot[i];
     return ok;
 }
 
@@ -389,27 +360,74 @@ __device__ __forceinline__ void mat3_vec(const float (&M)[9], const float (&x)[3
     y[2] = M[6] * x[0] + M[7] * x[1] + M[8] * x[2];
 }
 
-// w += (row of A) u over the row's block slots whose u entry is local (HALO = false: own
-// rows) or a halo copy (HALO = true), fully unrolled so that every slot's panel and u loads
-// are in flight together.  The local pass runs while the halo values travel.  `cw` holds the
-// slots' indices into this CTA's u array (own rows below `halo0`, then the halo slots), two
-// 16-bit indices per word.  `pn` points at the row's first panel, in shared memory or
-// (beyond the shared-memory budget) in global memory.
-template <bool HALO>
-__device__ __forceinline__ void row_times_u(const float* __restrict__ pn, int width, const uint32_t (&cw)[CS_RES_MAX_WIDTH / 2],
-                                            const float4* su, int halo0, int lane, float& q0, float& q1, float& q2) {
+__device__ __forceinline__ void block_times(const float4 a0, const float4 a1, const float a8, const float4 pv, float& q0,
+                                            float& q1, float& q2) {
+    q0 = fmaf(a0.z, pv.z, fmaf(a0.y, pv.y, fmaf(a0.x, pv.x, q0)));
+    q1 = fmaf(a1.y, pv.z, fmaf(a1.x, pv.y, fmaf(a0.w, pv.x, q1)));
+    q2 = fmaf(a8, pv.z, fmaf(a1.w, pv.y, fmaf(a1.z, pv.x, q2)));
+}
+
+// w += (row of A) u.  The first ks slots of a slice (uniform in the warp) are in shared memory, slots ks ..
+// width - 1 (beyond the budget, spread evenly over the slices) in global memory, the first of those
+// requested by row_tail_load before the halo wait.  A warp's time is its count of instructions and the
+// latencies between them, so the slots go RES_CHUNK at a time without branches, a chunk's loads in flight
+// together, over own rows and halo copies alike (a pass over the own rows while the halo values travel
+// and a second over the halo's took longer than the wait it hid).  `cw`: the byte offsets of the slots'
+// entries in the u array, two 16-bit ones per word.
+#define RES_CHUNK 4
+struct RowTail {
+    float4 a0, a1;
+    float a8;
+    int idx;
+};
+__device__ __forceinline__ RowTail row_tail_load(const float* __restrict__ gp, int ks, int width, const int* __restrict__ code,
+                                                 int lane) {
+    RowTail t;
+    t.a0 = t.a1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    t.a8 = 0.f;
+    t.idx = 0;
+    if (ks < width) {
+        const float* pk = gp + (size_t)ks * CS_PANEL_FLOATS;
+        t.a0 = __ldg(reinterpret_cast<const float4*>(pk) + lane);
+        t.a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + lane);
+        t.a8 = __ldg(pk + 256 + lane);
+        t.idx = __ldg(code + ks * CS_SLICE + lane);
+    }
+    return t;
+}
+// LOCAL: only the columns that are the CTA's own rows (entries below `halo0`; the one before it is zero).
+template <bool LOCAL>
+__device__ __forceinline__ void row_times(const float* __restrict__ sp, const float* __restrict__ gp, int ks, int width,
+                                          const uint32_t (&cw)[CS_RES_MAX_WIDTH / 2], const int* __restrict__ code,
+                                          const RowTail& t, const float4* su, int halo0, int lane, bool live, float& q0, float& q1,
+                                          float& q2) {
+    const unsigned char* const sb = reinterpret_cast<const unsigned char*>(su);
 #pragma unroll
-    for (int k = 0; k < CS_RES_MAX_WIDTH; k++) {
-        const int idx = (int)((cw[k >> 1] >> ((k & 1) * 16)) & 0xffffu);
-        if (k < width && (idx >= halo0) == HALO) {
-            const float* pk = pn + k * CS_PANEL_FLOATS;
-            const float4 a0 = reinterpret_cast<const float4*>(pk)[lane];
-            const float4 a1 = reinterpret_cast<const float4*>(pk + 128)[lane];
-            const float a8 = pk[256 + lane];
-            const float4 pv = su[idx];
-            q0 += a0.x * pv.x + a0.y * pv.y + a0.z * pv.z;
-            q1 += a0.w * pv.x + a1.x * pv.y + a1.y * pv.z;
-            q2 += a1.z * pv.x + a1.w * pv.y + a8 * pv.z;
+    for (int k0 = 0; k0 < CS_RES_MAX_WIDTH; k0 += RES_CHUNK) {
+        if (k0 >= ks) break;
+        float4 a0[RES_CHUNK], a1[RES_CHUNK], pv[RES_CHUNK];
+        float a8[RES_CHUNK];
+#pragma unroll
+        for (int j = 0; j < RES_CHUNK; j++) {
+            const int k = k0 + j;
+            const float* pk = sp + (k < ks ? k : k0) * CS_PANEL_FLOATS;
+            const uint32_t at = (k & 1) ? cw[k >> 1] >> 16 : cw[k >> 1] & 0xffffu;
+            a0[j] = reinterpret_cast<const float4*>(pk)[lane];
+            a1[j] = reinterpret_cast<const float4*>(pk + 128)[lane];
+            a8[j] = pk[256 + lane];
+            pv[j] = *reinterpret_cast<const float4*>(sb + (LOCAL ? min(at, 16u * (halo0 - 1)) : at));
+        }
+#pragma unroll
+        for (int j = 0; j < RES_CHUNK; j++) block_times(a0[j], a1[j], a8[j], pv[j], q0, q1, q2);
+    }
+    if (ks < width) {
+        if (live && (!LOCAL || t.idx < halo0)) block_times(t.a0, t.a1, t.a8, su[t.idx], q0, q1, q2);
+        for (int k = ks + 1; k < width; k++) {
+            const int idx = __ldg(code + k * CS_SLICE + lane);
+            if (!live || (LOCAL && idx >= halo0)) continue;
+            const float* pk = gp + (size_t)k * CS_PANEL_FLOATS;
+            block_times(__ldg(reinterpret_cast<const float4*>(pk) + lane), __ldg(reinterpret_cast<const float4*>(pk + 128) + lane),
+                        __ldg(pk + 256 + lane), su[idx], q0, q1, q2);
         }
     }
 }
@@ -424,7 +442,7 @@ extern __shared__ __align__(16) unsigned char cs_res_smem[];
 // none is left).  B.loop[5] is the work counter (zeroed by the solve setup), B.loop[6] the
 // error word (set when a wait ran out).
 __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kernel(Batch B) {
-    const DevParams P = *B.params;
+    const DevParams& P = *B.params;
     if (P.solver != CS_SOLVER_AUTO_DEV || B.n_resident == 0) return;  // uniform over the grid
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -469,77 +487,79 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         const SheetDesc sh = B.sheets[s];
         const int tb = sh.topo * (CS_RES_MAX_CL + 1);
         const int lo = B.rsplit[tb + rank], hi = B.rsplit[tb + rank + 1];
-        int cta_p0 = 0, cta_p1 = 0;
-        if (hi > lo) {
-            cta_p0 = B.slices[sh.slice_off + lo].panel0;
-            const SliceDesc& last = B.slices[sh.slice_off + hi - 1];
-            cta_p1 = last.panel0 + last.width;
-        }
-        // this CTA's panels (contiguous) into shared memory, up to the budget
+        const int nsl = hi - lo;
+        // this CTA's panels into shared memory, up to the budget: what exceeds it are
+        // the last slots of the slices, spread evenly
+        bool live = false;
+        int width = 0, ks = 0, lp = 0, gp = 0, tp = 0, row = 0;
         {
-            const int ncopy = min(cta_p1 - cta_p0, cap) * (CS_PANEL_FLOATS / 4);
-            const float4* src = reinterpret_cast<const float4*>(B.A + (size_t)cta_p0 * CS_PANEL_FLOATS);
-            float4* dst = reinterpret_cast<float4*>(cs_res_smem);
-            for (int i = tid; i < ncopy; i += blockDim.x) dst[i] = __ldg(src + i);
+            const SliceDesc* sl = B.slices + sh.slice_off + lo;
+            const int panels = nsl > 0 ? sl[nsl - 1].panel0 + sl[nsl - 1].width - sl[0].panel0 : 0;
+            const int over = max(panels - cap, 0);
+            int at = 0;
+            for (int j = 0; j < nsl; j++) {
+                const int wd = sl[j].width, p0 = sl[j].panel0;
+                const int out = min(wd, (over * (j + 1)) / nsl - (over * j) / nsl), keep = wd - out;
+                const float4* src = reinterpret_cast<const float4*>(B.A + (size_t)p0 * CS_PANEL_FLOATS);
+                float4* dst = reinterpret_cast<float4*>(cs_res_smem) + (size_t)at * (CS_PANEL_FLOATS / 4);
+                for (int i = tid; i < keep * (CS_PANEL_FLOATS / 4); i += blockDim.x) dst[i] = __ldg(src + i);
+                if (j == w) {
+                    lp = at;
+                    ks = keep;
+                    width = wd;
+                }
+                at += keep;
+            }
         }
         // this thread's row: slice lo + w, lane
-        bool live = false;
-        int width = 0, lp = 0, gp = 0, tp = 0, row = 0;
-        if (lo + w < hi) {
+        if (w < nsl) {
             const SliceDesc d = B.slices[sh.slice_off + lo + w];
             live = lane < d.rows;
-            width = d.width;
             gp = d.panel0;
             tp = d.tpanel0;
-            lp = d.panel0 - cta_p0;
             if (live) row = B.rowmap[d.topo_slice * CS_SLICE + lane];
         }
-        if (!live) width = 0;
-        const bool in_smem = lp + width <= cap;
+        const float* const spn = sm_panels + (size_t)lp * CS_PANEL_FLOATS;
+        const float* const gpn = B.A + (size_t)gp * CS_PANEL_FLOATS;
+        const int* const code = B.rcode + (size_t)tp * CS_SLICE;
         const int g = sh.node_off + row;
-        // u-array indices of the row's slots, packed 16-bit, for the whole solve
+        // byte offsets of the u entries of the slots in shared memory (fewer than 4,096 entries), for the
+        // whole solve; others point at the zero entry between the own rows and the halo
+        if (tid == 0) su[halo0 - 1] = su[B.res_alt + halo0 - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t cw[CS_RES_MAX_WIDTH / 2];
 #pragma unroll
-        for (int j = 0; j < CS_RES_MAX_WIDTH / 2; j++) {
-            uint32_t lo16 = 0, hi16 = 0;
-            if (2 * j < width) lo16 = (uint32_t)__ldg(&B.rcode[(tp + 2 * j) * CS_SLICE + lane]) & 0xfffu;
-            if (2 * j + 1 < width) hi16 = (uint32_t)__ldg(&B.rcode[(tp + 2 * j + 1) * CS_SLICE + lane]) & 0xfffu;
-            cw[j] = lo16 | (hi16 << 16);
+        for (int j = 0; j < CS_RES_MAX_WIDTH; j++) {
+            const uint32_t at = 16u * (live && j < ks ? __ldg(code + j * CS_SLICE + lane) & 0xfff : halo0 - 1);
+            cw[j >> 1] = (j & 1) ? cw[j >> 1] | at << 16 : at;
         }
         // halo sends of this CTA (the first one per thread in a register) and bytes it receives
         const int snd0 = B.rsendptr[tb + rank], snd1 = B.rsendptr[tb + rank + 1];
         const uint32_t my_send = snd0 + tid < snd1 ? __ldg(&B.rsend[snd0 + tid]) : 0u;
         const uint32_t halo_bytes = (uint32_t)B.rhalo[tb + rank] * 16u;
 
-        // coarse-space correction (uniform over the cluster): its shared-memory region, this
-        // CTA's rows of the inverse coarse matrix, this thread's segment and, for the lanes of
-        // warp 1 that sum segments, their slot ranges
+        // the multilevel preconditioner, and its coarse-space correction (both uniform over the cluster)
+        const bool levels = P.coarse && P.cheb_degree >= 3 && (B.rcheb[tb + rank] & 2);
         const int4 cinfo = B.rcoarse[sh.topo];
-        const bool coarse = P.coarse && P.cheb_degree >= 3 && B.rcheb[tb + rank] && cinfo.x == B.res_cnc &&
-                            cinfo.x > 0 && B.cvalid[idx] && nw >= 2;
+        const bool coarse = levels && cinfo.x == B.res_cnc && cinfo.x > 0 && B.cvalid[idx] && nw >= 2;
 #define C CoarseSm(cs_res_smem + B.res_coff, B.res_cnc, B.res_ck)
-        // the segment masks of this CTA's warps (tb = topology x (CS_RES_MAX_CL + 1))
-#define WMASKS (B.rwmask + (tb / (CS_RES_MAX_CL + 1)) * CS_RES_MAX_CL * CS_RES_MAX_WARPS + rank * CS_RES_MAX_WARPS)
-        int cseg = 0;  // this lane's segment run, the warps holding its segment (cluster_sum3c)
-        // this thread's entry of the coarse vectors in a buffer of C.red (q = tid, the common case)
-        const int coff = coarse && tid < C.nc ? C.off(tid) : 0;
+        // Every warp keeps the whole coarse residual R r and direction R s (FP64), entries `lane` and
+        // `lane + 32` per lane (nc <= 64): applying and updating the correction takes no barrier.  `coff`:
+        // those entries' places in a buffer of C.red (16 bits each), `rw` R w of the last CG reduction
+        // there (read at once: a reduction later, the buffer may be overwritten).
+        int coff = 0;
+        float rw[2] = {0.f, 0.f};
+        const float* cai = C.ai(ncta) + lane;  // this warp's segment's rows of A_c^-1
+        double cr[2] = {0.0, 0.0}, cs[2] = {0.0, 0.0};
         if (coarse) {
+            int seg = 0;
+            while (seg + 1 < B.res_ck && w >= (nsl * (seg + 1)) / B.res_ck) seg++;
+            cai += 3 * 64 * seg;
             const float* src = B.cinv + (size_t)idx * B.res_cnc * B.res_cnc + (size_t)rank * C.k3 * C.nc;
-            for (int i = tid; i < C.k3 * C.nc; i += blockDim.x) C.ai()[i] = __ldcg(src + i);
-            for (int i = tid; i < C.nc; i += blockDim.x) C.s64(ncta)[i] = 0.0;
-            const int myseg = live ? B.ragg[sh.row2slot_off + row] - rank * B.res_ck : -1;
-            // this lane's run of equal segments (consecutive lanes; -1: no row)
-            const unsigned same = __match_any_sync(0xffffffffu, myseg);
-            cseg = (__ffs(same) - 1) | ((lane == 31 || !((same >> (lane + 1)) & 1u)) ? 32 : 0) |
-                   ((live ? myseg + 1 : 0) << 8);
-            if (w == 1 && lane < C.k3) {
-                // the warps whose rows include this lane's segment (the gather of cluster_sum3c)
-                int wk = 0;
-                for (int j = 0; j < nw; j++) wk |= ((__ldg(&WMASKS[j]) >> (lane / 3)) & 1) << j;
-                cseg |= wk << 16;
-            }
+            for (int i = tid; i < C.k3 * 64; i += blockDim.x) C.ai(ncta)[i] = (i & 63) < C.nc ? __ldcg(src + (i >> 6) * C.nc + (i & 63)) : 0.f;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (lane + 32 * h < C.nc) coff |= C.off(lane + 32 * h) << (16 * h);
         }
-        // bit 6 of cseg: the buffer of C.red holding the last coarse vector received
 
         float Pi[9];
         float e[3] = {0.f, 0.f, 0.f}, r[3] = {0.f, 0.f, 0.f}, u[3], wv[3], p[3] = {0.f, 0.f, 0.f},
@@ -553,9 +573,14 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
 #pragma unroll
             for (int k = 0; k < 9; k++) Pi[k] = 0.f;
         }
-        const double bn = sqrt(B.inst[s].bnorm2);
-        double gam = 0.0, gam_prev = 0.0, rr = 0.0, delta = 0.0, alpha_d = 0.0, res0 = bn, resnorm = -1.0,
-               first_res = -1.0;
+        // scalars used once per iteration or less live in shared memory, a copy per warp (every lane
+        // writes the same value and reads its own write)
+        double &bn = S.sc[w][0], &res0 = S.sc[w][1], &resnorm = S.sc[w][2], &first_res = S.sc[w][3], &rr = S.sc[w][4],
+               &delta = S.sc[w][5], &thr = S.sc[w][6];
+        bn = res0 = sqrt(B.inst[s].bnorm2);
+        rr = delta = thr = 0.0;
+        resnorm = first_res = -1.0;
+        double gam = 0.0, gam_prev = 0.0, alpha_d = 0.0;
         bool cont = false;  // the next PH_INIT keeps the search direction (reliable update)
         // dv64 and e are known to be zero (zero guess before its first CG step, or a rejected
         // warm start just cleared): the next FP64 residual is b itself and needs no SpMV
@@ -576,63 +601,46 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         int phase = (P.warm || coarse) ? PH_RES : PH_INIT;
         bool ok = true;
 
-        // q = A_loc x over this CTA's own rows (the strip's diagonal block of A), x in `buf`
+        // The next iteration's scalars from the reduction's sums (r.u, w.u, r.r), by warp 0: the step
+        // length alpha = gnew / (dnew - beta gnew / alpha_prev), 1 / gnew and 1 / (gnew alpha)
+        auto no_post = [](const double (&)[3], double (&)[3]) {};
+        auto next_step = [&](const double (&t)[3], double (&x)[3]) {
+            if (!mixed || phase != PH_CG) return;
+            x[0] = t[0] / (t[1] - t[0] * t[0] * inv_ga);
+            x[1] = 1.0 / t[0];
+            x[2] = 1.0 / (t[0] * x[0]);
+        };
+        // q = A_loc x over this CTA's own rows and columns (the tile's diagonal block of A), x in `buf`
         float4* const su_alt = su + B.res_alt;
         auto local_spmv = [&](const float4* buf, float (&q)[3]) {
             q[0] = q[1] = q[2] = 0.f;
-            if (in_smem)
-                row_times_u<false>(sm_panels + (size_t)lp * CS_PANEL_FLOATS, width, cw, buf, halo0, lane, q[0], q[1], q[2]);
-            else
-                row_times_u<false>(B.A + (size_t)gp * CS_PANEL_FLOATS, width, cw, buf, halo0, lane, q[0], q[1], q[2]);
+            row_times<true>(spn, gpn, ks, width, cw, code, row_tail_load(gpn, ks, width, code, lane), buf, halo0, lane, live,
+                            q[0], q[1], q[2]);
         };
-        // ce = this CTA's rows of A_c^-1 times the coarse residual (a warp per row, lanes over
-        // the columns, butterfly sum: a fixed order)
-        auto coarse_matvec = [&]() {
-            const float* ai = C.ai();
-            const float* r32 = C.r32();
-            // rows j and j + nw together (their loads in flight at once), columns fully unrolled
-            for (int j = w; j < C.k3; j += 2 * nw) {
-                const int j1 = j + nw;
-                float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-                for (int n = 0; n < 6; n++) {
-                    const int t = lane + 32 * n;
-                    if (t < C.nc) {
-                        const float rt = r32[t];
-                        a0 = fmaf(ai[j * C.nc + t], rt, a0);
-                        if (j1 < C.k3) a1 = fmaf(ai[j1 * C.nc + t], rt, a1);
-                    }
-                }
-                a0 = rwarp_sum(a0);
-                if (lane == 0) C.ce()[j] = a0;
-                if (j1 < C.k3) {
-                    a1 = rwarp_sum(a1);
-                    if (lane == 0) C.ce()[j1] = a1;
-                }
-            }
-        };
-        // The coarse images of the CG recurrences, replicated in every CTA: with s = w + beta s
-        // and the next iteration's r -= alpha s, R s = R w + beta R s and R r -= alpha R s
-        // (R w from the reduction just done); R r is what the next preconditioner application
-        // reads.  An FP64 residual replaces R r exactly (PH_RES).
+        // The coarse images of the CG recurrences: with s = w + beta s and the next iteration's
+        // r -= alpha s, R s = R w + beta R s and R r -= alpha R s (R w from the reduction just done); R r
+        // is what the next preconditioner application reads.  An FP64 residual replaces R r exactly
+        // (PH_RES).
         auto coarse_step = [&](double beta_c, double alpha_c) {
-            double* s64 = C.s64(ncta);
-            double* r64 = C.r64(ncta);
-            const float* red = C.red() + (size_t)((cseg >> 6) & 1) * ncta * C.cp;  // R w of the last CG reduction
-            for (int q = tid; q < C.nc; q += blockDim.x) {
-                const double sq = (double)red[q == tid ? coff : C.off(q)] + beta_c * s64[q];
-                s64[q] = sq;
-                const double rq = r64[q] - alpha_c * sq;
-                r64[q] = rq;
-                C.r32()[q] = (float)rq;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                cs[h] = (double)rw[h] + beta_c * cs[h];
+                cr[h] -= alpha_c * cs[h];
             }
         };
-        // Strip-local Chebyshev preconditioner: the largest eigenvalue of P^-1 A_loc by power
+        // The levels' diagonal blocks: sums of the row's stored blocks whose column lies in the same octet
+        // or slice (of a tile's rows, every eight and every 32 are a compact patch of the sheet).
+        if (levels) {
+            __syncthreads();  // the panels are in place
+            level_blocks(spn, gpn, ks, width, code, w, lane, live, S.lev[w]);
+            __syncwarp();
+        }
+        // Tile-local Chebyshev preconditioner: the largest eigenvalue of P^-1 A_loc by power
         // iteration from a hashed +-1 vector (the first barrier also covers the panel copy),
         // then the coefficients of the Chebyshev iteration on [lmax / 30, lmax].  An odd
         // degree keeps the polynomial positive on all of (0, inf), so the preconditioner is
         // SPD whatever the estimate.
-        if (P.cheb_degree >= 3 && B.rcheb[tb + rank]) {
+        if (!levels && P.cheb_degree >= 3 && (B.rcheb[tb + rank] & 1)) {
             float v[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -641,7 +649,7 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
             }
             double lam = 0.0;
             for (int it = 0; it < CS_CHEB_POWER_ITERS; it++) {
-                if (live) su_alt[myslot] = make_float4(v[0], v[1], v[2], 0.f);
+                su_alt[myslot] = make_float4(v[0], v[1], v[2], 0.f);
                 __syncthreads();
                 float q[3], z[3];
                 local_spmv(su_alt, q);
@@ -706,7 +714,6 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 }
                 double v[3] = {0.0, 0.0, 0.0};
                 if (live) {
-                    const float* pn = in_smem ? sm_panels + (size_t)lp * CS_PANEL_FLOATS : B.A + (size_t)gp * CS_PANEL_FLOATS;
                     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
                     // four slots' column and dv64 loads in flight at a time; sums in slot order
 #pragma unroll
@@ -724,7 +731,8 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             if (k0 + j >= width) break;
-                            const float* pk = pn + (size_t)(k0 + j) * CS_PANEL_FLOATS;
+                            const int k = k0 + j;
+                            const float* pk = k < ks ? spn + k * CS_PANEL_FLOATS : gpn + (size_t)k * CS_PANEL_FLOATS;
                             const float4 a0 = reinterpret_cast<const float4*>(pk)[lane];
                             const float4 a1 = reinterpret_cast<const float4*>(pk + 128)[lane];
                             const float a8 = pk[256 + lane];
@@ -753,17 +761,18 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                         v[1] = q0 * q0 + q1 * q1 + q2 * q2;
                     }
                 }
+                put_sum02(S, v[0], v[2], false);
+                put_sum1(S, v[1], false);
                 if (coarse) {
                     // the coarse residual R r of the replaced r travels with the norms
-                    ok = cluster_sum3c(S, rank, ncta, nred, v, false, r, live, cseg, reinterpret_cast<float*>(su_alt), C);
+                    put_coarse(S, r);
+                    ok = cluster_reduce<true>(S, rank, ncta, nred, v, false, nsl, C, no_post);
                     const float* red = C.red() + (size_t)((nred - 1) & 1u) * ncta * C.cp;
-                    for (int q = tid; q < C.nc; q += blockDim.x) {
-                        const float rq = red[q == tid ? coff : C.off(q)];
-                        C.r64(ncta)[q] = (double)rq;
-                        C.r32()[q] = rq;
-                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        if (lane + 32 * h < C.nc) cr[h] = (double)red[(coff >> (16 * h)) & 0xffff];
                 } else {
-                    ok = cluster_sum3(S, rank, ncta, nred, v, false);
+                    ok = cluster_reduce<false>(S, rank, ncta, nred, v, false, nsl, C, no_post);
                 }
                 if (!ok) break;
                 if (scale_pass) {
@@ -875,10 +884,8 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 }
                 for (int k = 1; k < cdeg; k++) {
                     float4* const buf = (k & 1) ? su : su_alt;
-                    if (live) buf[myslot] = make_float4(u[0], u[1], u[2], 0.f);
+                    buf[myslot] = make_float4(u[0], u[1], u[2], 0.f);
                     __syncthreads();
-                    // the coarse correction of this CTA's aggregates, read after the next barrier
-                    if (coarse && k == 1) coarse_matvec();
                     float q[3], t[3];
                     local_spmv(buf, q);
 #pragma unroll
@@ -892,20 +899,17 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                     }
                 }
             }
-            if (coarse) {
-                if (cdeg < 3) {
-                    // this CTA's spectrum bound failed (block-Jacobi): barriers of its own
-                    __syncthreads();
-                    coarse_matvec();
-                    __syncthreads();
-                }
-                // u = C r + R^T A_c^-1 R r: the additive coarse-space correction
-                if (live) {
+            if (levels) {
+                // + the octet's, the slice's and the segment's corrections (additive)
+                level_correction(S.lev[w], r, lane, u);
+                if (coarse) {
+                    const float r0 = (float)cr[0], r1 = (float)cr[1];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) u[c] += C.ce()[3 * (((cseg >> 8) & 0xff) - 1) + c];
+                    for (int c = 0; c < 3; c++) u[c] += rwarp_sum(fmaf(cai[64 * c + 32], r1, cai[64 * c] * r0));
                 }
             }
-            if (live) su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
+            if (!live) u[0] = u[1] = u[2] = 0.f;  // an octet's correction reaches lanes without a row
+            su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
             __syncthreads();
             if (tid == 0) rbar_expect(hbar, halo_bytes);
             for (int i = snd0 + tid; i < snd1; i += blockDim.x) {
@@ -913,41 +917,43 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 const int d = (int)((m >> 12) & 0xfu);
                 st_async_f4(mapa(saddr(&su[halo0 + (int)(m >> 16)]), d), su[m & 0xfffu], mapa(hbar, d));
             }
-            wv[0] = wv[1] = wv[2] = 0.f;
-            const float* pn = in_smem ? sm_panels + (size_t)lp * CS_PANEL_FLOATS : B.A + (size_t)gp * CS_PANEL_FLOATS;
-            if (in_smem)
-                row_times_u<false>(sm_panels + (size_t)lp * CS_PANEL_FLOATS, width, cw, su, halo0, lane, wv[0], wv[1], wv[2]);
+            // while the halo values travel: the sums r.u and r.r, the first slot in global memory
+            const RowTail tail = row_tail_load(gpn, ks, width, code, lane);
+            if (mixed)
+                put_sum02(S, (double)r[0] * u[0] + (double)r[1] * u[1] + (double)r[2] * u[2],
+                          (double)r[0] * r[0] + (double)r[1] * r[1] + (double)r[2] * r[2], false);
             else
-                row_times_u<false>(pn, width, cw, su, halo0, lane, wv[0], wv[1], wv[2]);
+                put_sum02(S, (double)(r[0] * u[0] + r[1] * u[1] + r[2] * u[2]), (double)(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]), true);
             ok = res_wait(S, hbar, nhalo & 1u);
             nhalo++;
             if (!ok) break;
-            if (in_smem)
-                row_times_u<true>(sm_panels + (size_t)lp * CS_PANEL_FLOATS, width, cw, su, halo0, lane, wv[0], wv[1], wv[2]);
-            else
-                row_times_u<true>(pn, width, cw, su, halo0, lane, wv[0], wv[1], wv[2]);
+            wv[0] = wv[1] = wv[2] = 0.f;
+            row_times<false>(spn, gpn, ks, width, cw, code, tail, su, halo0, lane, live, wv[0], wv[1], wv[2]);
             double v[3] = {0.0, 0.0, 0.0};
-            if (live) {
-                if (mixed) {
-                    v[0] = (double)r[0] * u[0] + (double)r[1] * u[1] + (double)r[2] * u[2];
-                    v[1] = (double)wv[0] * u[0] + (double)wv[1] * u[1] + (double)wv[2] * u[2];
-                    v[2] = (double)r[0] * r[0] + (double)r[1] * r[1] + (double)r[2] * r[2];
-                } else {
-                    v[0] = (double)(r[0] * u[0] + r[1] * u[1] + r[2] * u[2]);
-                    v[1] = (double)(wv[0] * u[0] + wv[1] * u[1] + wv[2] * u[2]);
-                    v[2] = (double)(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-                }
-            }
+            if (mixed)
+                put_sum1(S, (double)wv[0] * u[0] + (double)wv[1] * u[1] + (double)wv[2] * u[2], false);
+            else
+                put_sum1(S, (double)(wv[0] * u[0] + wv[1] * u[1] + wv[2] * u[2]), true);
             if (coarse) {
                 // R w travels with the dot products (the coarse recurrences below)
-                ok = cluster_sum3c(S, rank, ncta, nred, v, fp32, wv, live, cseg, reinterpret_cast<float*>(su_alt), C);
-                cseg = (cseg & ~64) | (int)(((nred - 1) & 1u) << 6);
+                put_coarse(S, wv);
+                ok = cluster_reduce<true>(S, rank, ncta, nred, v, fp32, nsl, C, next_step);
+                const float* red = C.red() + (size_t)((nred - 1) & 1u) * ncta * C.cp;
+#pragma unroll
+                for (int h = 0; h < 2; h++) rw[h] = lane + 32 * h < C.nc ? red[(coff >> (16 * h)) & 0xffff] : 0.f;
             } else {
-                ok = cluster_sum3(S, rank, ncta, nred, v, fp32);
+                ok = cluster_reduce<false>(S, rank, ncta, nred, v, fp32, nsl, C, next_step);
             }
             if (!ok) break;
             const double gnew = v[0], dnew = v[1];
             rr = v[2];
+            if (phase == PH_INIT) {
+                // the last sweep goes to CS_LAST_SWEEP of the tolerance: at equal residuals the levels leave
+                // up to 1.6 times the error in dv that a larger coarse space did (32 x 32 quads)
+                const double ti = mixed ? P.inner_tol * res0 : 0.0, tt = P.tol * bn;
+                const double t = ti > tt ? ti : (mixed ? CS_LAST_SWEEP : 1.0) * tt;
+                thr = t * t;
+            }
             if (phase == PH_INIT && cont) {
                 // p = u + beta p and s = w + beta s with beta = (r.u) / (the last iteration's
                 // r.u); r no longer follows the recursion that the Chronopoulos-Gear step
@@ -963,7 +969,9 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                     }
                     double v2[3] = {0.0, 0.0, 0.0};
                     if (live) v2[0] = (double)p[0] * sv3[0] + (double)p[1] * sv3[1] + (double)p[2] * sv3[2];
-                    ok = cluster_sum3(S, rank, ncta, nred, v2, false);
+                    put_sum02(S, v2[0], 0.0, false);
+                    put_sum1(S, 0.0, false);
+                    ok = cluster_reduce<false>(S, rank, ncta, nred, v2, false, nsl, C, no_post);
                     if (!ok) break;
                     if (v2[0] > 0.0 && rfinite(v2[0]) && rfinite(gnew / v2[0])) {
                         gam = gnew;
@@ -1016,21 +1024,14 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
             // PH_CG: the iteration's x and r updates are done; stopping test on ||r||
             iters += 1;
             sweep_iters += 1;
-            // ||r|| against the thresholds, squared (no square root on the critical path)
-            bool stop;
-            if (mixed) {
-                const double ti = P.inner_tol * res0, tt = 0.5 * P.tol * bn;
-                stop = rr <= ti * ti || rr <= tt * tt || sweep_iters >= P.sweep_cap;
-            } else {
-                const double tt = P.tol * bn;
-                stop = rr <= tt * tt;
-            }
+            // ||r|| against the sweep's threshold, squared (no square root on the critical path)
+            bool stop = v[2] <= thr || (mixed && sweep_iters >= P.sweep_cap);
             float nb, na;
             double na_d;
             if (mixed) {
                 // beta = gnew / gam; alpha = gnew / (dnew - beta gnew / alpha_prev)
                 const double bd = gnew * inv_gam;
-                na_d = gnew / (dnew - gnew * gnew * inv_ga);
+                na_d = S.tot[3];
                 nb = (float)bd;
                 na = (float)na_d;
             } else {
@@ -1038,7 +1039,7 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 na = (float)gnew / ((float)dnew - nb * (float)gnew / alpha);
                 na_d = (double)na;
             }
-            if (!rfinite((double)nb) || !rfinite((double)na) || !(gnew > 0.0) || !(na > 0.f)) {
+            if (!isfinite(nb) || !isfinite(na) || !(gnew > 0.0) || !(na > 0.f)) {
                 flags |= CS_IF_BREAKDOWN;
                 stop = true;
             }
@@ -1059,8 +1060,8 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
             }
             if (coarse) coarse_step((double)beta, alpha_d);
             if (mixed) {
-                inv_gam = 1.0 / gam;
-                inv_ga = 1.0 / (gam * alpha_d);
+                inv_gam = S.tot[4];
+                inv_ga = S.tot[5];
             }
         }
         if (!ok) {
@@ -1090,6 +1091,5 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         if (!ok) break;
     }
 #undef C
-#undef WMASKS
     cl.sync();  // no CTA leaves while another may still address its shared memory
 }

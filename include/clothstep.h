@@ -91,18 +91,22 @@ typedef struct cs_step_params {
     int advance;              /* 1: v += dv and x += dt v (a full step); 0: solve only */
     int use_graph;            /* 1: run the captured CUDA graph; 0: host-driven launches */
     int solver;               /* CS_SOLVER_*: which PCG kernels solve the sheets */
-    int precond_degree;       /* on-chip solvers' preconditioner: 0 or 1 the 3x3
-                                 block-Jacobi inverse; an odd degree 3..CS_PRECOND_MAX_DEGREE a
-                                 Chebyshev polynomial of that degree in the block-Jacobi-scaled
-                                 matrix of each CTA's strip of rows (no exchange between CTAs).
+    int precond_degree;       /* on-chip solvers' preconditioner: 0 or 1 the 3x3 block-Jacobi
+                                 inverse; an odd degree 3..CS_PRECOND_MAX_DEGREE, with `coarse`,
+                                 a multilevel one (block-Jacobi, patches of 8 and of 32 rows, the
+                                 coarse space) for sheets whose rows are ordered by tiles;
+                                 otherwise a Chebyshev polynomial of that degree in the
+                                 block-Jacobi-scaled matrix of each CTA's rows (no exchange
+                                 between CTAs), except where those rows are too thin a strip.
                                  The batched loop uses block-Jacobi (with the coarse
                                  correction when `coarse`). */
-    int coarse;               /* 1 adds a coarse-space correction, 0 leaves it out.  Cluster-resident
-                                 solver with the Chebyshev preconditioner: one constant per
-                                 component on each of a few geometric segments of every CTA's
-                                 strip.  Batched loop: one per aggregate of 256 nodes or more
-                                 (the rest (u, v) binned into at most 16 x 16 cells) and one
-                                 per finer cell inside them, added to block-Jacobi; sheets with proximities keep block-Jacobi alone.
+    int coarse;               /* 1 adds a coarse-space correction, 0 leaves it out.  On-chip
+                                 solvers with a degree of 3 or more: one constant per component
+                                 on each of a few segments of every CTA's tile of rows, on sheets
+                                 large enough for it.  Batched loop: one per aggregate of 256
+                                 nodes or more (the rest (u, v) binned into at most 16 x 16
+                                 cells) and one per finer cell inside them, added to
+                                 block-Jacobi; sheets with proximities keep block-Jacobi alone.
                                  Either way the coarse matrix R A R^T is inverted per sheet and
                                  step. */
     /* Cloth::physicsStep's `transformations` (Cloth.cuh:91-92): the motions' transformations at
@@ -203,8 +207,8 @@ typedef struct cs_tune_result {
 cs_status cs_tune(cs_ctx* ctx, const cs_step_params* params, int reps, cs_tune_result* out);
 
 /* out[0..2] = 3x3 blocks of the systems of the sheets now solved cluster-resident (the mesh
- * pattern's), those among them whose row and column belong to the same CTA's strip of rows
- * (what one strip-local SpMV of the Chebyshev preconditioner reads), and the power iterations
+ * pattern's), those among them whose row and column belong to the same CTA's rows
+ * (what one tile-local SpMV of the Chebyshev preconditioner reads), and the power iterations
  * each resident solve runs for that preconditioner's eigenvalue bound.  For work accounting
  * (rooflines); no counterpart in the reference. */
 cs_status cs_get_resident_blocks(const cs_ctx* ctx, long long* out);
