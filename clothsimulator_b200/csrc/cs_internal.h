@@ -165,6 +165,7 @@ void launchSpmvShape(const Batch& B, int shape, cudaStream_t st);
 // Group-resident solver (group.cu): block slots per row (column codes live in registers), slices
 // per CTA that a sheet's tiles are planned for, its fewest when a batch would leave the chip idle.
 #define CS_GROUP_MAX_WIDTH 18
+#define CS_GROUP_OCTET_PANELS 190  // a tile's panels up to which a group's rows take the octet order
 #define CS_GROUP_SLICES 14
 #define CS_GROUP_MAX_WARPS CS_RES_MAX_WARPS
 #define CS_GROUP_CE_PARTS 4    // warps that share a row of the coarse matrix-vector product, at most

@@ -494,25 +494,28 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     if (tileCtas > 0) {
         t->tile_ctas = tileCtas;
         t->tile_segs = std::max(1, std::min(segs, t->n_slices / tileCtas));
-        // Octet order mixes long and short rows in a slice: little on a grid, a quarter more panels on an
-        // irregular mesh.  A group, whose tiles fill the shared memory, takes it up to a tenth more.
+        // Octet order mixes long and short rows in a slice: 1.2 times the panels on a grid of alternating
+        // diagonals, 1.3 times on an irregular mesh.  A group, whose tiles can fill the shared memory, takes
+        // it while a tile's panels about fit.
         const int few = std::min(t->tile_segs, CS_COARSE_SEGS);
         tileOrder(t->node_uv, len, t->tile_ctas, few, true, order);
         t->octets = true;
         if (!octets) {
-            std::vector<int> sorted;
-            tileOrder(t->node_uv, len, t->tile_ctas, t->tile_segs, false, sorted);
-            auto panels = [&](const std::vector<int>& o) {
-                long long n = 0;
-                for (int i = 0; i < nn; i += CS_SLICE) {
-                    int w = 0;
-                    for (int l = i; l < std::min(nn, i + CS_SLICE); l++) w = std::max(w, len[o[l]]);
-                    n += w;
+            auto mostPanels = [&](const std::vector<int>& o) {
+                int most = 0;
+                for (int c = 0; c < tileCtas; c++) {
+                    int n = 0;
+                    for (int sl = (int)((long long)t->n_slices * c / tileCtas); sl < (int)((long long)t->n_slices * (c + 1) / tileCtas); sl++) {
+                        int w = 0;
+                        for (int l = sl * CS_SLICE; l < std::min(nn, (sl + 1) * CS_SLICE); l++) w = std::max(w, len[o[l]]);
+                        n += w;
+                    }
+                    most = std::max(most, n);
                 }
-                return n;
+                return most;
             };
-            if (10 * panels(order) > 11 * panels(sorted)) {
-                order.swap(sorted);
+            if (mostPanels(order) > CS_GROUP_OCTET_PANELS) {
+                tileOrder(t->node_uv, len, t->tile_ctas, t->tile_segs, false, order);
                 t->octets = false;
             }
         }
@@ -1788,6 +1791,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             const int nc = 3 * P.coarse.na;
             // a quarter of the panels or more beyond shared memory: the loop streams as fast
             if (P.max_own > CS_GROUP_MAX_WARPS || P.max_width > CS_GROUP_MAX_WIDTH || nc > CS_BC_MAX_NC ||
+                P.max_own * CS_SLICE + 1 + P.max_halo >= 4096 ||  // 16-bit byte offsets of the u entries
                 (size_t)P.max_panels * 3 / 4 * CS_PANEL_FLOATS * sizeof(float) +
                         (2 * (size_t)P.max_own * CS_SLICE + P.max_halo) * sizeof(float4) + 24 * 1024 > optin)
                 continue;
@@ -1801,14 +1805,14 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             B.g_cai = std::max(B.g_cai, 3 * T.tile_segs * nc);
         }
         if (warps > 0) {
-            B.g_own = warps * CS_SLICE;
+            B.g_own = warps * CS_SLICE + 1;  // a zero entry before the halo
             const size_t u = (2 * (size_t)B.g_own + B.g_halo) * sizeof(float4);
             const size_t rest = (r2(3 * (size_t)B.g_max) + 2 * r2(B.g_cnc)) * sizeof(double) +
                                 (2 * r4(B.g_cnc) + r4(CS_GROUP_CE_PARTS * (size_t)B.g_ck3) + r4(B.g_cai)) * sizeof(float);
             B.g_cap = (int)std::min<size_t>(panels, (optin - u - rest) / (CS_PANEL_FLOATS * sizeof(float)));
             B.g_coff = (int)(B.g_cap * CS_PANEL_FLOATS * sizeof(float) + u);
             c->groupSmem = B.g_coff + rest;
-            c->groupThreads = B.g_own;
+            c->groupThreads = warps * CS_SLICE;
             CS_CUDA(raiseDynSmem((const void*)cs_group_pcg_kernel, c->groupSmem));
             int perSM = 0;
             CS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, cs_group_pcg_kernel, c->groupThreads, c->groupSmem));

@@ -12,9 +12,10 @@
 //   * A CTA holds its tile's SELL-32 panels in shared memory (what exceeds it, spread evenly over
 //     the slices, is read from L2), one row per thread with the CG vectors in registers, as
 //     resident.cu does, and runs the same iteration: Chronopoulos-Gear CG with one fused
-//     reduction, the tile-local Chebyshev preconditioner, the additive coarse-space correction
-//     (one constant per segment of a tile and component, its residual carried by recurrence
-//     within the reduction), FP64 residual replacements with the search direction kept.
+//     reduction, the levels of levels.cuh where the tile's rows are in octet order (else the tile-local
+//     Chebyshev preconditioner), the additive coarse-space correction (one constant per segment of a
+//     tile and component, its residual carried by recurrence within the reduction), FP64 residual
+//     replacements with the search direction kept.
 //   * CTAs exchange values through global memory (L2) in 16-byte packets {three words, epoch},
 //     each written and read by one 128-bit access: a reader polls the packet itself, so a value's
 //     arrival needs no flag, fence or barrier.
@@ -28,11 +29,11 @@
 // Every wait is bounded; a CTA whose wait runs out sets the error word, which ends the others'
 // waits, and the host reports CS_ERR_TIMEOUT.
 //
-// What bounds it: per iteration two trips through L2 (halo, reduction) of about 1 us each and the
-// shared-memory reads of deg SpMVs over the tile.  Measured against the batched loop (whole steps,
-// B200): a sheet of 66,049 nodes at 1e-10 15.4 -> 4.2 ms, 10,201 nodes 9.1 -> 1.85 ms, a lone sheet of
-// 72 x 72 quads 8.1 -> 1.8 ms, an irregular sheet of 261 x 261 nodes 13.0 -> 4.3 ms, 64 sheets of 4 to
-// 128 quads a side 15.5 -> 9.9 ms.
+// What bounds it: per iteration two trips through L2 (halo, reduction) of about 1 us each, the chain of
+// instructions between them and the shared-memory reads of the tile.  Measured against the batched
+// loop (whole steps, B200): a sheet of 66,049 nodes at 1e-10 15.4 -> 3.6 ms (4.2 with Chebyshev-3), 10,201
+// nodes 9.1 -> 1.33 ms, a lone sheet of 72 x 72 quads 8.1 -> 0.92 ms, an irregular sheet of 261 x 261
+// nodes (Chebyshev-3) 13.0 -> 3.4 ms, 64 sheets of 4 to 128 quads a side 15.5 -> 8.1 ms.
 #include "cs_internal.h"
 #include "levels.cuh"
 
@@ -62,19 +63,6 @@ template <class T>
 __device__ __forceinline__ T gwarp_sum(T v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-// The warp's sums of three values with 6 exchanges instead of 15: each step halves the values a
-// lane carries.  Lanes 0-7 return the first sum, 8-15 the second, 16-23 the third.
-template <class T>
-__device__ __forceinline__ T gwarp_sum3(T a, T b, T c, int lane) {
-    const bool up = lane & 16, odd = lane & 8;
-    T x = __shfl_xor_sync(0xffffffffu, up ? a : c, 16), y = __shfl_xor_sync(0xffffffffu, up ? b : T(0), 16);
-    x += up ? c : a;
-    y += up ? T(0) : b;
-    T v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 __device__ __forceinline__ bool gfinite(double x) { return x == x && x < 1e300 && x > -1e300; }
@@ -112,60 +100,6 @@ struct GroupSm {
         ai = ce + ((CS_GROUP_CE_PARTS * B.g_ck3 + 3) & ~3);
     }
 };
-
-// w += (row of A) u over the row's slots of one kind (own rows, or halo copies), the first `ks`
-// slots in shared memory, fully unrolled so that their loads are in flight together, the others
-// (beyond the shared-memory budget) from global memory: the first of those, with its column in
-// `tidx`, is requested before the shared-memory slots and used after them.
-template <bool HALO>
-__device__ __forceinline__ void group_row(const float* __restrict__ sp, const float* __restrict__ gp, int ks, int width,
-                                          const uint32_t (&cw)[CS_GROUP_MAX_WIDTH / 2], int tidx,
-                                          const int* __restrict__ code, const float4* su, int halo0, int lane, float& q0,
-                                          float& q1, float& q2) {
-    const bool tail = ks < width && (tidx >= halo0) == HALO;
-    float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-    float t8 = 0.f;
-    if (tail) {
-        const float* pk = gp + (size_t)ks * CS_PANEL_FLOATS;
-        t0 = __ldg(reinterpret_cast<const float4*>(pk) + lane);
-        t1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + lane);
-        t8 = __ldg(pk + 256 + lane);
-    }
-#pragma unroll
-    for (int k = 0; k < CS_GROUP_MAX_WIDTH; k++) {
-        const int idx = (int)((cw[k >> 1] >> ((k & 1) * 16)) & 0xffffu);
-        if (k < ks && (idx >= halo0) == HALO) {
-            const float* pk = sp + k * CS_PANEL_FLOATS;
-            const float4 a0 = reinterpret_cast<const float4*>(pk)[lane];
-            const float4 a1 = reinterpret_cast<const float4*>(pk + 128)[lane];
-            const float a8 = pk[256 + lane];
-            const float4 pv = su[idx];
-            q0 += a0.x * pv.x + a0.y * pv.y + a0.z * pv.z;
-            q1 += a0.w * pv.x + a1.x * pv.y + a1.y * pv.z;
-            q2 += a1.z * pv.x + a1.w * pv.y + a8 * pv.z;
-        }
-    }
-    if (tail) {
-        const float4 pv = su[tidx];
-        q0 += t0.x * pv.x + t0.y * pv.y + t0.z * pv.z;
-        q1 += t0.w * pv.x + t1.x * pv.y + t1.y * pv.z;
-        q2 += t1.z * pv.x + t1.w * pv.y + t8 * pv.z;
-    }
-#pragma unroll 2
-    for (int k = ks + 1; k < width; k++) {
-        const int idx = __ldg(code + k * CS_SLICE + lane);
-        if ((idx >= halo0) == HALO) {
-            const float* pk = gp + (size_t)k * CS_PANEL_FLOATS;
-            const float4 a0 = __ldg(reinterpret_cast<const float4*>(pk) + lane);
-            const float4 a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + lane);
-            const float a8 = __ldg(pk + 256 + lane);
-            const float4 pv = su[idx];
-            q0 += a0.x * pv.x + a0.y * pv.y + a0.z * pv.z;
-            q1 += a0.w * pv.x + a1.x * pv.y + a1.y * pv.z;
-            q2 += a1.z * pv.x + a1.w * pv.y + a8 * pv.z;
-        }
-    }
-}
 
 }  // namespace
 
@@ -232,20 +166,19 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                 pub = B.gpub[gi.pub0 + slot];
             }
         }
-        if (!live) width = ks = 0;
         const int g = sh.node_off + row;
         const float* const spn = sm_panels + (size_t)lp * CS_PANEL_FLOATS;
         const float* const gpn = B.A + (size_t)gp * CS_PANEL_FLOATS;
         const int* const code = B.rcode + (size_t)tp * CS_SLICE;
+        // byte offsets of the u entries of the slots in shared memory (the zero entry before the halo's for
+        // others)
         uint32_t cw[CS_GROUP_MAX_WIDTH / 2];
+        if (tid == 0) su[halo0 - 1] = su_alt[halo0 - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < CS_GROUP_MAX_WIDTH / 2; j++) {
-            uint32_t a = 0, b = 0;
-            if (2 * j < width) a = (uint32_t)__ldg(code + 2 * j * CS_SLICE + lane);
-            if (2 * j + 1 < width) b = (uint32_t)__ldg(code + (2 * j + 1) * CS_SLICE + lane);
-            cw[j] = a | (b << 16);
+        for (int j = 0; j < CS_GROUP_MAX_WIDTH; j++) {
+            const uint32_t at = 16u * (uint32_t)(live && j < ks ? __ldg(code + j * CS_SLICE + lane) : halo0 - 1);
+            cw[j >> 1] = (j & 1) ? cw[j >> 1] | at << 16 : at;
         }
-        const int tidx = ks < width ? __ldg(code + ks * CS_SLICE + lane) : 0;
         const int h0 = B.ghalo_ptr[gi.halo0 + rank], nh = B.ghalo_ptr[gi.halo0 + rank + 1] - h0;
         const int my_halo = tid < nh ? __ldg(&B.ghalo[h0 + tid]) : 0;
         // the segment of this warp's rows: the tile's slices cut into K ranges
@@ -285,20 +218,26 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             }
             return v;
         };
-        // Group-wide sums of v (identical in every CTA) and, with `y`, R y into C.rw.  Packet i < 3 of
+        // The warp's part of a reduction: sums 0 and 2, sum 1, the restriction of y
+        auto put_sum02 = [&](double a, double c) {
+            const double t = tile_sum2(a, c);
+            if ((lane & 15) == 0) S.wsum[w][lane >> 3] = t;  // lane 0: sum 0, lane 16: sum 2
+        };
+        auto put_sum1 = [&](double a) {
+            a = gwarp_sum(a);
+            if (lane == 0) S.wsum[w][1] = a;
+        };
+        auto put_coarse = [&](const float (&y)[3]) {
+            const float t = tile_sum3(y[0], y[1], y[2]);
+            if ((lane & 7) == 0 && lane < 24) S.wseg[w][lane >> 3] = t;
+        };
+        // Group-wide sums v of the warps' (identical in every CTA) and, with `y`, R y into C.rw.  Packet i < 3 of
         // a CTA carries its part of sum i and component i of its first segment's sum of y, packet
         // 2 + k the three components of segment k > 0.
-        auto group_sum = [&](double (&v)[3], const float* y) -> bool {
+        auto group_sum = [&](double (&v)[3], bool y) -> bool {
             const uint32_t epoch = nred + 1, buf = nred & 1u;
             nred++;
             const int np = y ? rstride : 3;
-            const double vs = gwarp_sum3(v[0], v[1], v[2], lane);
-            float ys = 0.f;
-            if (y) ys = live ? gwarp_sum3(y[0], y[1], y[2], lane) : gwarp_sum3(0.f, 0.f, 0.f, lane);
-            if ((lane & 7) == 0 && lane < 24) {
-                S.wsum[w][lane >> 3] = vs;
-                S.wseg[w][lane >> 3] = ys;
-            }
             __syncthreads();
             uint4* const mine = rpk + ((size_t)buf * G + rank) * rstride;
             if (tid < 3) {
@@ -349,7 +288,8 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         };
         auto local_spmv = [&](const float4* buf, float (&q)[3]) {
             q[0] = q[1] = q[2] = 0.f;
-            group_row<false>(spn, gpn, ks, width, cw, tidx, code, buf, halo0, lane, q[0], q[1], q[2]);
+            row_times<CS_GROUP_MAX_WIDTH, 3, true>(spn, gpn, ks, width, cw, code, row_tail_load(gpn, ks, width, code, lane), buf,
+                                                   halo0, lane, live, q[0], q[1], q[2]);
         };
         auto cta_sum2 = [&](double& a, double& b) {
             a = gwarp_sum(a);
@@ -406,7 +346,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             }
             double lam = 0.0;
             for (int k = 0; k < CS_CHEB_POWER_ITERS; k++) {
-                if (live) su_alt[myslot] = make_float4(v[0], v[1], v[2], 0.f);
+                su_alt[myslot] = make_float4(v[0], v[1], v[2], 0.f);
                 __syncthreads();
                 float q[3], z[3];
                 local_spmv(su_alt, q);
@@ -468,7 +408,9 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                 if (!zero) {
                     // every CTA's rows of dv64 are written before any is read
                     __threadfence();
-                    ok = group_sum(v, nullptr);
+                    put_sum02(0.0, 0.0);
+                    put_sum1(0.0);
+                    ok = group_sum(v, false);
                     if (!ok) break;
                     __threadfence();
                 }
@@ -516,7 +458,10 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
 #pragma unroll
                 for (int c = 0; c < 3; c++) r[c] = rn[c];
                 // the coarse residual R r of the replaced r travels with the norms
-                ok = group_sum(v, coarse ? r : nullptr);
+                put_sum02(v[0], v[2]);
+                put_sum1(v[1]);
+                if (coarse) put_coarse(r);
+                ok = group_sum(v, coarse);
                 if (!ok) break;
                 if (coarse)
                     for (int q = tid; q < nc; q += blockDim.x) {
@@ -594,7 +539,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                 // write after the reads of the buffer's previous contents
                 for (int k = 1; k < cdeg; k++) {
                     float4* const buf = (k & 1) ? su : su_alt;
-                    if (live) buf[myslot] = make_float4(u[0], u[1], u[2], 0.f);
+                    buf[myslot] = make_float4(u[0], u[1], u[2], 0.f);
                     __syncthreads();
                     if (coarse && k == 1) coarse_matvec();
                     float q[3], t[3];
@@ -622,14 +567,14 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                     for (int q = 0; q < parts; q++) u[c] += C.ce[(3 * seg + c) * parts + q];
             }
             nhalo++;
-            if (live) {
-                su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
-                if (pub)
-                    put_packet(upk + slot, __float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), nhalo);
-            }
-            __syncthreads();
-            wv[0] = wv[1] = wv[2] = 0.f;
-            group_row<false>(spn, gpn, ks, width, cw, tidx, code, su, halo0, lane, wv[0], wv[1], wv[2]);
+            if (!live) u[0] = u[1] = u[2] = 0.f;  // an octet's correction reaches lanes without a row
+            su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
+            if (live && pub)
+                put_packet(upk + slot, __float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), nhalo);
+            // while the halo values travel: the sums r.u and r.r, the first slot in global memory
+            const RowTail tail = row_tail_load(gpn, ks, width, code, lane);
+            put_sum02((double)r[0] * u[0] + (double)r[1] * u[1] + (double)r[2] * u[2],
+                      (double)r[0] * r[0] + (double)r[1] * r[1] + (double)r[2] * r[2]);
             for (int i = tid; i < nh; i += blockDim.x) {
                 const uint4 x = wait_packet(upk + (i == tid ? my_halo : __ldg(&B.ghalo[h0 + i])), nhalo, ok);
                 su[halo0 + i] = make_float4(__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), 0.f);
@@ -637,14 +582,12 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             if (!ok) atomicExch(err, 1);
             ok = __syncthreads_and(ok ? 1 : 0) != 0;
             if (!ok) break;
-            group_row<true>(spn, gpn, ks, width, cw, tidx, code, su, halo0, lane, wv[0], wv[1], wv[2]);
-            double v[3] = {0.0, 0.0, 0.0};
-            if (live) {
-                v[0] = (double)r[0] * u[0] + (double)r[1] * u[1] + (double)r[2] * u[2];
-                v[1] = (double)wv[0] * u[0] + (double)wv[1] * u[1] + (double)wv[2] * u[2];
-                v[2] = (double)r[0] * r[0] + (double)r[1] * r[1] + (double)r[2] * r[2];
-            }
-            ok = group_sum(v, coarse ? wv : nullptr);
+            wv[0] = wv[1] = wv[2] = 0.f;
+            row_times<CS_GROUP_MAX_WIDTH, 3, false>(spn, gpn, ks, width, cw, code, tail, su, halo0, lane, live, wv[0], wv[1], wv[2]);
+            put_sum1((double)wv[0] * u[0] + (double)wv[1] * u[1] + (double)wv[2] * u[2]);
+            if (coarse) put_coarse(wv);
+            double v[3];
+            ok = group_sum(v, coarse);
             if (!ok) break;
             const double gnew = v[0], dnew = v[1], rr = v[2];
             if (tid == 0) {
@@ -666,7 +609,9 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                     }
                     double v2[3] = {0.0, 0.0, 0.0};
                     if (live) v2[0] = (double)p[0] * sv[0] + (double)p[1] * sv[1] + (double)p[2] * sv[2];
-                    ok = group_sum(v2, nullptr);
+                    put_sum02(v2[0], 0.0);
+                    put_sum1(0.0);
+                    ok = group_sum(v2, false);
                     if (!ok) break;
                     if (v2[0] > 0.0 && gfinite(v2[0]) && gfinite(gnew / v2[0])) {
                         gam = gnew;
@@ -712,8 +657,9 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             // PH_CG: the iteration's x and r updates are done; stopping test on ||r||
             iters += 1;
             sweep_iters += 1;
-            const double ti = P.inner_tol * S.res0, tt = 0.5 * P.tol * S.bn;
-            bool stop = rr <= ti * ti || rr <= tt * tt || sweep_iters >= P.sweep_cap;
+            // the last sweep goes below the tolerance, as in resident.cu
+            const double ti = P.inner_tol * S.res0, tt = P.tol * S.bn, t = ti > tt ? ti : CS_LAST_SWEEP * tt;
+            bool stop = rr <= t * t || sweep_iters >= P.sweep_cap;
             const double bd = gnew * inv_gam, na = gnew / (dnew - gnew * gnew * inv_ga);
             if (!gfinite((double)(float)bd) || !gfinite((double)(float)na) || !(gnew > 0.0) || !((float)na > 0.f)) {
                 flags |= CS_IF_BREAKDOWN;

@@ -1,4 +1,5 @@
-// Tile levels of the on-chip solvers' preconditioner (resident.cu, group.cu).  The loader orders a
+// Parts of the on-chip solvers (resident.cu, group.cu) that work on a tile: warp sums, the product of a
+// row with the tile's u array, and the preconditioner's levels.  The loader orders a
 // tile's rows by recursive bisection, so every eight consecutive rows (an octet of lanes) and every 32
 // (a slice, one warp) are a compact patch of the sheet.  With F and G summing a vector over the octets
 // and the slices, per component,
@@ -11,6 +12,99 @@
 #include "cs_internal.h"
 
 namespace {
+
+// Warp sums of two (lanes 0-15 return the first, 16-31 the second) and of three values (lanes 0-7, 8-15,
+// 16-23), by exchanges that halve the values a lane carries: 5 and 8 additions instead of 10 and 15.
+template <class T>
+__device__ __forceinline__ T tile_sum2(T a, T b) {
+    const bool up = threadIdx.x & 16;
+    T v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <class T>
+__device__ __forceinline__ T tile_sum3(T a, T b, T c) {
+    const bool up = threadIdx.x & 16, odd = threadIdx.x & 8;
+    T x = __shfl_xor_sync(0xffffffffu, up ? a : c, 16), y = __shfl_xor_sync(0xffffffffu, up ? b : T(0), 16);
+    x += up ? c : a;
+    y += up ? T(0) : b;
+    T v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ void block_times(const float4 a0, const float4 a1, const float a8, const float4 pv, float& q0,
+                                            float& q1, float& q2) {
+    q0 = fmaf(a0.z, pv.z, fmaf(a0.y, pv.y, fmaf(a0.x, pv.x, q0)));
+    q1 = fmaf(a1.y, pv.z, fmaf(a1.x, pv.y, fmaf(a0.w, pv.x, q1)));
+    q2 = fmaf(a8, pv.z, fmaf(a1.w, pv.y, fmaf(a1.z, pv.x, q2)));
+}
+
+// w += (row of A) u.  The first ks slots of a slice (uniform in the warp) are in shared memory, slots ks ..
+// width - 1 (beyond the budget, spread evenly over the slices) in global memory, the first of those
+// requested by row_tail_load before the halo wait.  A warp's time is its count of instructions and the
+// latencies between them, so the slots go CHUNK at a time without branches, a chunk's loads in flight
+// together, over own rows and halo copies alike (a pass over the own rows while the halo values travel
+// and a second over the halo's took longer than the wait it hid).  `cw`: the byte offsets of the slots'
+// entries in the u array, two 16-bit ones per word (of a zero entry for the slots beyond ks).
+struct RowTail {
+    float4 a0, a1;
+    float a8;
+    int idx;
+};
+__device__ __forceinline__ RowTail row_tail_load(const float* __restrict__ gp, int ks, int width, const int* __restrict__ code,
+                                                 int lane) {
+    RowTail t;
+    t.a0 = t.a1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    t.a8 = 0.f;
+    t.idx = 0;
+    if (ks < width) {
+        const float* pk = gp + (size_t)ks * CS_PANEL_FLOATS;
+        t.a0 = __ldg(reinterpret_cast<const float4*>(pk) + lane);
+        t.a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + lane);
+        t.a8 = __ldg(pk + 256 + lane);
+        t.idx = __ldg(code + ks * CS_SLICE + lane);
+    }
+    return t;
+}
+// LOCAL: only the columns that are the CTA's own rows (entries below `halo0`; the one before it is zero).
+template <int W, int CHUNK, bool LOCAL>
+__device__ __forceinline__ void row_times(const float* __restrict__ sp, const float* __restrict__ gp, int ks, int width,
+                                          const uint32_t (&cw)[W / 2], const int* __restrict__ code,
+                                          const RowTail& t, const float4* su, int halo0, int lane, bool live, float& q0, float& q1,
+                                          float& q2) {
+    static_assert(W % CHUNK == 0, "whole chunks");
+    const unsigned char* const sb = reinterpret_cast<const unsigned char*>(su);
+#pragma unroll
+    for (int k0 = 0; k0 < W; k0 += CHUNK) {
+        if (k0 >= ks) break;
+        float4 a0[CHUNK], a1[CHUNK], pv[CHUNK];
+        float a8[CHUNK];
+#pragma unroll
+        for (int j = 0; j < CHUNK; j++) {
+            const int k = k0 + j;
+            const float* pk = sp + (k < ks ? k : k0) * CS_PANEL_FLOATS;
+            const uint32_t at = (k & 1) ? cw[k >> 1] >> 16 : cw[k >> 1] & 0xffffu;
+            a0[j] = reinterpret_cast<const float4*>(pk)[lane];
+            a1[j] = reinterpret_cast<const float4*>(pk + 128)[lane];
+            a8[j] = pk[256 + lane];
+            pv[j] = *reinterpret_cast<const float4*>(sb + (LOCAL ? min(at, 16u * (halo0 - 1)) : at));
+        }
+#pragma unroll
+        for (int j = 0; j < CHUNK; j++) block_times(a0[j], a1[j], a8[j], pv[j], q0, q1, q2);
+    }
+    if (ks < width) {
+        if (live && (!LOCAL || t.idx < halo0)) block_times(t.a0, t.a1, t.a8, su[t.idx], q0, q1, q2);
+        for (int k = ks + 1; k < width; k++) {
+            const int idx = __ldg(code + k * CS_SLICE + lane);
+            if (!live || (LOCAL && idx >= halo0)) continue;
+            const float* pk = gp + (size_t)k * CS_PANEL_FLOATS;
+            block_times(__ldg(reinterpret_cast<const float4*>(pk) + lane), __ldg(reinterpret_cast<const float4*>(pk + 128) + lane),
+                        __ldg(pk + 256 + lane), su[idx], q0, q1, q2);
+        }
+    }
+}
 
 // The inverse of the symmetrised 3x3 sum `m` as the six entries 00 01 02 11 12 22 (FP64 inside);
 // zeros unless it is positive definite.

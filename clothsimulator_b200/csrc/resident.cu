@@ -205,31 +205,10 @@ struct CoarseSm {
     __device__ __forceinline__ int off(int q) const { return (q / k3) * cp + q % k3; }
 };
 
-// Warp sums of two (lanes 0-15 return the first, 16-31 the second) and of three values (lanes 0-7, 8-15,
-// 16-23), by exchanges that halve the values a lane carries: 5 and 8 additions instead of 10 and 15.
-template <class T>
-__device__ __forceinline__ T rwarp_sum2(T a, T b) {
-    const bool up = threadIdx.x & 16;
-    T v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-template <class T>
-__device__ __forceinline__ T rwarp_sum3(T a, T b, T c) {
-    const bool up = threadIdx.x & 16, odd = threadIdx.x & 8;
-    T x = __shfl_xor_sync(0xffffffffu, up ? a : c, 16), y = __shfl_xor_sync(0xffffffffu, up ? b : T(0), 16);
-    x += up ? c : a;
-    y += up ? T(0) : b;
-    T v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 // The warp's part of a reduction: sums 0 and 2, sum 1, or the coarse restriction of y, in shared memory.
 __device__ __forceinline__ void put_sum02(ResShared& S, double a, double c, bool fp32) {
     const int lane = threadIdx.x & 31;
-    const double t = fp32 ? (double)rwarp_sum2((float)a, (float)c) : rwarp_sum2(a, c);
+    const double t = fp32 ? (double)tile_sum2((float)a, (float)c) : tile_sum2(a, c);
     if ((lane & 15) == 0) S.wsum[threadIdx.x >> 5][lane >> 3] = t;  // lane 0: sum 0, lane 16: sum 2
 }
 __device__ __forceinline__ void put_sum1(ResShared& S, double a, bool fp32) {
@@ -238,7 +217,7 @@ __device__ __forceinline__ void put_sum1(ResShared& S, double a, bool fp32) {
 }
 __device__ __forceinline__ void put_coarse(ResShared& S, const float (&y)[3]) {
     const int lane = threadIdx.x & 31;
-    const float t = rwarp_sum3(y[0], y[1], y[2]);
+    const float t = tile_sum3(y[0], y[1], y[2]);
     if ((lane & 7) == 0 && lane < 24) S.wy[threadIdx.x >> 5][lane >> 3] = t;
 }
 // The sums over 16 lanes (each half of the warp) of three values, in FP64 or (fp32) in float.
@@ -358,78 +337,6 @@ __device__ __forceinline__ void mat3_vec(const float (&M)[9], const float (&x)[3
     y[0] = M[0] * x[0] + M[1] * x[1] + M[2] * x[2];
     y[1] = M[3] * x[0] + M[4] * x[1] + M[5] * x[2];
     y[2] = M[6] * x[0] + M[7] * x[1] + M[8] * x[2];
-}
-
-__device__ __forceinline__ void block_times(const float4 a0, const float4 a1, const float a8, const float4 pv, float& q0,
-                                            float& q1, float& q2) {
-    q0 = fmaf(a0.z, pv.z, fmaf(a0.y, pv.y, fmaf(a0.x, pv.x, q0)));
-    q1 = fmaf(a1.y, pv.z, fmaf(a1.x, pv.y, fmaf(a0.w, pv.x, q1)));
-    q2 = fmaf(a8, pv.z, fmaf(a1.w, pv.y, fmaf(a1.z, pv.x, q2)));
-}
-
-// w += (row of A) u.  The first ks slots of a slice (uniform in the warp) are in shared memory, slots ks ..
-// width - 1 (beyond the budget, spread evenly over the slices) in global memory, the first of those
-// requested by row_tail_load before the halo wait.  A warp's time is its count of instructions and the
-// latencies between them, so the slots go RES_CHUNK at a time without branches, a chunk's loads in flight
-// together, over own rows and halo copies alike (a pass over the own rows while the halo values travel
-// and a second over the halo's took longer than the wait it hid).  `cw`: the byte offsets of the slots'
-// entries in the u array, two 16-bit ones per word.
-#define RES_CHUNK 4
-struct RowTail {
-    float4 a0, a1;
-    float a8;
-    int idx;
-};
-__device__ __forceinline__ RowTail row_tail_load(const float* __restrict__ gp, int ks, int width, const int* __restrict__ code,
-                                                 int lane) {
-    RowTail t;
-    t.a0 = t.a1 = make_float4(0.f, 0.f, 0.f, 0.f);
-    t.a8 = 0.f;
-    t.idx = 0;
-    if (ks < width) {
-        const float* pk = gp + (size_t)ks * CS_PANEL_FLOATS;
-        t.a0 = __ldg(reinterpret_cast<const float4*>(pk) + lane);
-        t.a1 = __ldg(reinterpret_cast<const float4*>(pk + 128) + lane);
-        t.a8 = __ldg(pk + 256 + lane);
-        t.idx = __ldg(code + ks * CS_SLICE + lane);
-    }
-    return t;
-}
-// LOCAL: only the columns that are the CTA's own rows (entries below `halo0`; the one before it is zero).
-template <bool LOCAL>
-__device__ __forceinline__ void row_times(const float* __restrict__ sp, const float* __restrict__ gp, int ks, int width,
-                                          const uint32_t (&cw)[CS_RES_MAX_WIDTH / 2], const int* __restrict__ code,
-                                          const RowTail& t, const float4* su, int halo0, int lane, bool live, float& q0, float& q1,
-                                          float& q2) {
-    const unsigned char* const sb = reinterpret_cast<const unsigned char*>(su);
-#pragma unroll
-    for (int k0 = 0; k0 < CS_RES_MAX_WIDTH; k0 += RES_CHUNK) {
-        if (k0 >= ks) break;
-        float4 a0[RES_CHUNK], a1[RES_CHUNK], pv[RES_CHUNK];
-        float a8[RES_CHUNK];
-#pragma unroll
-        for (int j = 0; j < RES_CHUNK; j++) {
-            const int k = k0 + j;
-            const float* pk = sp + (k < ks ? k : k0) * CS_PANEL_FLOATS;
-            const uint32_t at = (k & 1) ? cw[k >> 1] >> 16 : cw[k >> 1] & 0xffffu;
-            a0[j] = reinterpret_cast<const float4*>(pk)[lane];
-            a1[j] = reinterpret_cast<const float4*>(pk + 128)[lane];
-            a8[j] = pk[256 + lane];
-            pv[j] = *reinterpret_cast<const float4*>(sb + (LOCAL ? min(at, 16u * (halo0 - 1)) : at));
-        }
-#pragma unroll
-        for (int j = 0; j < RES_CHUNK; j++) block_times(a0[j], a1[j], a8[j], pv[j], q0, q1, q2);
-    }
-    if (ks < width) {
-        if (live && (!LOCAL || t.idx < halo0)) block_times(t.a0, t.a1, t.a8, su[t.idx], q0, q1, q2);
-        for (int k = ks + 1; k < width; k++) {
-            const int idx = __ldg(code + k * CS_SLICE + lane);
-            if (!live || (LOCAL && idx >= halo0)) continue;
-            const float* pk = gp + (size_t)k * CS_PANEL_FLOATS;
-            block_times(__ldg(reinterpret_cast<const float4*>(pk) + lane), __ldg(reinterpret_cast<const float4*>(pk + 128) + lane),
-                        __ldg(pk + 256 + lane), su[idx], q0, q1, q2);
-        }
-    }
 }
 
 }  // namespace
@@ -614,7 +521,7 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         float4* const su_alt = su + B.res_alt;
         auto local_spmv = [&](const float4* buf, float (&q)[3]) {
             q[0] = q[1] = q[2] = 0.f;
-            row_times<true>(spn, gpn, ks, width, cw, code, row_tail_load(gpn, ks, width, code, lane), buf, halo0, lane, live,
+            row_times<CS_RES_MAX_WIDTH, 4, true>(spn, gpn, ks, width, cw, code, row_tail_load(gpn, ks, width, code, lane), buf, halo0, lane, live,
                             q[0], q[1], q[2]);
         };
         // The coarse images of the CG recurrences: with s = w + beta s and the next iteration's
@@ -928,7 +835,7 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
             nhalo++;
             if (!ok) break;
             wv[0] = wv[1] = wv[2] = 0.f;
-            row_times<false>(spn, gpn, ks, width, cw, code, tail, su, halo0, lane, live, wv[0], wv[1], wv[2]);
+            row_times<CS_RES_MAX_WIDTH, 4, false>(spn, gpn, ks, width, cw, code, tail, su, halo0, lane, live, wv[0], wv[1], wv[2]);
             double v[3] = {0.0, 0.0, 0.0};
             if (mixed)
                 put_sum1(S, (double)wv[0] * u[0] + (double)wv[1] * u[1] + (double)wv[2] * u[2], false);
