@@ -26,6 +26,9 @@ struct f3 {
 };
 __device__ __forceinline__ f3 mk(float x, float y, float z) { return {x, y, z}; }
 __device__ __forceinline__ f3 ld3(const float* p, int i) { return mk(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
+__device__ __forceinline__ f3 ldg3(const float* p, int i) {
+    return mk(__ldg(p + 3 * i), __ldg(p + 3 * i + 1), __ldg(p + 3 * i + 2));
+}
 __device__ __forceinline__ f3 sub(f3 a, f3 b) { return mk(a.x - b.x, a.y - b.y, a.z - b.z); }
 __device__ __forceinline__ f3 add(f3 a, f3 b) { return mk(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ f3 scl(float s, f3 a) { return mk(s * a.x, s * a.y, s * a.z); }
@@ -442,17 +445,41 @@ __global__ void __launch_bounds__(CS_GATHER_THREADS) cs_gather_kernel(Batch B) {
                 b1 += r[1];
                 b2 += r[2];
             }
+            // The next edge's record is requested while this one's blocks are added: a row's edges were a
+            // chain of dependent loads (a 16 x 16 sheet 36.7 -> 30.8 us, 400 of 64 x 64 1,334 -> 1,261, an
+            // irregular one of 301 x 301 nodes 140 -> 127; same sums in the same order).
+            int2 nc = e0 < e1 ? __ldg(&B.redge[e0]) : make_int2(0, 0);
+            float4 nq[4];
+            int4 nen = make_int4(0, 0, 0, 0);
+            f3 nv[4];
+            auto fetch = [&](int2 cc) {
+                const int e = sh.edge_off + (cc.x >> 2);
+                const float4* rec = B.edge_geo + 4 * (size_t)e;
+#pragma unroll
+                for (int k = 0; k < 4; k++) nq[k] = __ldg(rec + k);
+                nen = __ldg(&B.edge_nodes[e]);
+            };
+            auto fetchv = [&]() {
+                nv[0] = ldg3(B.v, nen.x);
+                nv[1] = ldg3(B.v, nen.y);
+                nv[2] = ldg3(B.v, nen.z);
+                nv[3] = ldg3(B.v, nen.w);
+            };
+            if (e0 < e1) {
+                fetch(nc);
+                if (e0 + 1 < e1) nc = __ldg(&B.redge[e0 + 1]);
+            }
+            int2 c = e0 < e1 ? __ldg(&B.redge[e0]) : make_int2(0, 0);
             for (int t = e0; t < e1; t++) {
-                const int2 c = __ldg(&B.redge[t]);
-                const int e = sh.edge_off + (c.x >> 2), a = c.x & 3;
-                float dth[12], coef, angle;
-                {
-                    const float4* rec = B.edge_geo + 4 * (size_t)e;
-                    const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2), q3 = __ldg(rec + 3);
-                    dth[0] = q0.x; dth[1] = q0.y; dth[2] = q0.z; coef = q0.w;
-                    dth[3] = q1.x; dth[4] = q1.y; dth[5] = q1.z; angle = q1.w;
-                    dth[6] = q2.x; dth[7] = q2.y; dth[8] = q2.z;
-                    dth[9] = q3.x; dth[10] = q3.y; dth[11] = q3.z;
+                const int a = c.x & 3;
+                const float dth[12] = {nq[0].x, nq[0].y, nq[0].z, nq[1].x, nq[1].y, nq[1].z,
+                                       nq[2].x, nq[2].y, nq[2].z, nq[3].x, nq[3].y, nq[3].z};
+                const float coef = nq[0].w, angle = nq[1].w;
+                fetchv();
+                const int2 cn = nc;
+                if (t + 1 < e1) {
+                    fetch(cn);
+                    if (t + 2 < e1) nc = __ldg(&B.redge[t + 2]);
                 }
                 // the row's node's gradient by selects (no indexed local arrays)
                 float da[3];
@@ -469,9 +496,8 @@ __global__ void __launch_bounds__(CS_GATHER_THREADS) cs_gather_kernel(Batch B) {
                         for (int hh = 0; hh < 3; hh++) d[(3 * kk + hh) * CS_SLICE] += s * (coef * (da[kk] * dth[3 * bb + hh]));
                 }
                 // dt (f + dt J v) of the row's node (PhysicsHelper.cu:351-352)
-                const int4 en = B.edge_nodes[e];
-                const f3 v0 = ld3(B.v, en.x), v1 = ld3(B.v, en.y), v2 = ld3(B.v, en.z), v3 = ld3(B.v, en.w);
-                const float vel[12] = {v0.x, v0.y, v0.z, v1.x, v1.y, v1.z, v2.x, v2.y, v2.z, v3.x, v3.y, v3.z};
+                const float vel[12] = {nv[0].x, nv[0].y, nv[0].z, nv[1].x, nv[1].y, nv[1].z,
+                                       nv[2].x, nv[2].y, nv[2].z, nv[3].x, nv[3].y, nv[3].z};
                 const float ca = coef * angle;
                 float r[3];
 #pragma unroll
@@ -484,6 +510,7 @@ __global__ void __launch_bounds__(CS_GATHER_THREADS) cs_gather_kernel(Batch B) {
                 b0 += r[0];
                 b1 += r[1];
                 b2 += r[2];
+                c = cn;
             }
             const float4 hd = B.handle[row];
             const int hc = (int)hd.w;
