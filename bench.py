@@ -14,9 +14,9 @@ One step = assembly + PCG to an FP64-checked relative residual of 1e-6 for every
 v += dv, x += dt v, with the state resident in HBM.
 
 Metric: node-steps/s (sum over sheets of nodes x steps / device time).  The line reports the
-mixed-precision solver (`value`: cluster-resident solve where a sheet fits, strip-local Chebyshev
-preconditioner of degree --precond-degree with the coarse-space correction, reliable updates; the
-workload's warm start) and, in `arms`, the same solver without the coarse correction, with
+mixed-precision solver (`value`: solved on chip where a sheet fits, the multilevel preconditioner
+that --precond-degree 3 selects with the coarse-space correction, reliable updates; the workload's
+warm start) and, in `arms`, the same solver without the coarse correction, with
 block-Jacobi, from other starts, at the tolerance that meets the dv bound, and plain FP32 PCG from
 a zero guess on the same GPU, each with its dv error against an FP64 solve of its own system on
 sampled sheets.  `--impl reference` times the reference's CPU path for the workload (the
@@ -72,8 +72,8 @@ def parse(argv=None):
     ap.add_argument("--solver", default="auto", choices=["auto", "batched"],
                     help="auto: sheets that fit a cluster's shared memory are solved cluster-resident")
     ap.add_argument("--precond-degree", type=int, default=3,
-                    help="cluster-resident solver's preconditioner: 1 block-Jacobi, odd 3..15 a strip-local "
-                         "Chebyshev polynomial of that degree (the batched loop always uses block-Jacobi)")
+                    help="on-chip solvers' preconditioner: 1 block-Jacobi, odd 3..15 multilevel or, with "
+                         "--no-coarse, a tile-local Chebyshev polynomial of that degree")
     ap.add_argument("--no-coarse", action="store_true", help="headline arm without the coarse-space correction")
     ap.add_argument("--no-tune", action="store_true", help="skip the autotuner (cs_tune)")
     ap.add_argument("--fixed-precond", action="store_true",
@@ -457,7 +457,7 @@ def train_warm_start(args, group, local):
                 "sheets_per_minibatch": args.train_batch,
                 "adam_steps": epochs * (steps - 2) * ((sheets + args.train_batch - 1) // args.train_batch),
                 "trajectories": f"windy{sheets}x{args.nq} per rank, seeds disjoint from the evaluated workload, "
-                                "solved without the learned start (mixed PCG, Chebyshev-3 + coarse correction)",
+                                "solved without the learned start (mixed PCG, multilevel preconditioner)",
                 "loss_first_steps": float(np.mean(first[:k])), "loss_last_steps": float(np.mean(last[-k:])),
                 "loss_epoch_means": [float(np.mean(c)) for c in curve]}
         if world > 1:
@@ -781,11 +781,11 @@ def run_ours(args):
                         "note": "algorithmic bytes = CG iterations x (stored blocks x 40 B + nodes x 48 B), what a "
                                 "streaming PCG would move; the kernel reads them from shared memory (roofline_smem)"}
             # shared-memory bytes: per CG iteration the full SpMV (36 B of block values + 16 B of
-            # the vector per stored block) and (degree - 1) strip-local SpMVs over the strip-local
-            # blocks; per solve the power iterations
+            # the vector per stored block) and, without the coarse correction, (degree - 1) tile-local
+            # SpMVs over the tile-local blocks; per solve the power iterations
             rb = ctx.resident_blocks()
             local_frac = rb["local_blocks"] / max(rb["blocks"], 1)
-            cheb = deg >= 3
+            cheb = deg >= 3 and args.no_coarse
             smem_bytes = float(np.sum(it_res * blocks_sheet * 52 * (1 + (deg - 1) * local_frac * cheb)
                                       + cheb * rb["power_iters"] * local_frac * blocks_sheet * 52))
             sm_mhz = clocks.get("sm_mhz") or 1965.0
@@ -849,8 +849,8 @@ def run_ours(args):
                 "scheme": "mixed FP32 PCG, FP64 dot products, FP64 residual replacements (reliable updates)",
                 "warm_start": args.warm,
                 "solver": args.solver,
-                "precond": ("strip-local Chebyshev degree %d over block-Jacobi%s" %
-                            (deg, " + coarse-space correction" if coarse else "")
+                "precond": (("multilevel: block-Jacobi, octets and slices of rows, coarse space" if coarse else
+                             "tile-local Chebyshev degree %d over block-Jacobi" % deg)
                             if deg >= 3 and args.solver == "auto" else "block-Jacobi"),
                 "l2": "inputs larger than L2 (system matrix %.2f GB per GPU)" % (sizes[3] * 36 / 1e9)
                       if sizes[3] * 36 > 126e6 else "system matrix %.3f GB per GPU: within L2" % (sizes[3] * 36 / 1e9),

@@ -127,7 +127,7 @@ struct SolverOptions {
     int maxIters = 2000;
     int precision = CS_PREC_MIXED;
     int warmStart = CS_WARM_PREVIOUS;
-    int precondDegree = 3;  // strip-local Chebyshev of the cluster-resident solver (1: block-Jacobi)
+    int precondDegree = 3;  // on-chip solvers: 3 or more multilevel or Chebyshev (clothstep.h), 1 block-Jacobi
     bool coarse = true;     // with it, the coarse-space correction of the cluster-resident solver
     bool warmScale = false; // the warm start replaced by its Galerkin multiple before the guard
     std::string network;  // weights for the learned warm start (CS_MLP_PARAMS floats, binary)
