@@ -488,7 +488,9 @@ __global__ void __launch_bounds__(CS_BC_THREADS) cs_bc_invert_cluster_kernel(Bat
 // F r, G r and R r: a block per aggregate, a warp per middle cell in it.  The warp sums r over the nodes
 // of a fine cell in FP64 (lane-strided, then a butterfly; CS_BC_UNROLL cells' loads together), the fine
 // cells' sums over the middle cell, and the block the middle cells' over the aggregate, each in a fixed
-// order; R r is stored in FP32, and the cells' D_F^-1 F r and D_G^-1 G r as the cells' corrections.
+// order; R r is stored in FP32, and the cells' D_F^-1 F r and D_G^-1 G r as the cells' corrections.  Launched
+// with as many warps a block as an aggregate has middle cells, at most CS_BC_RESTRICT_THREADS / 32 (with 16
+// always, 15 idled on batches of small sheets, whose aggregates have one).
 __global__ void __launch_bounds__(CS_BC_RESTRICT_THREADS) cs_bc_restrict_kernel(Batch B) {
     __shared__ double sh3[CS_BC_RESTRICT_THREADS / 32][3];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -498,7 +500,7 @@ __global__ void __launch_bounds__(CS_BC_RESTRICT_THREADS) cs_bc_restrict_kernel(
     const int* aptr = B.bc_aptr + sh.bc_agg_off + sa.y;
     const int* mptr = B.bc_mptr + sh.bc_fine_off;
     double t[3] = {0.0, 0.0, 0.0};
-    for (int mid = aptr[0] + wid; mid < aptr[1]; mid += CS_BC_RESTRICT_THREADS / 32) {
+    for (int mid = aptr[0] + wid; mid < aptr[1]; mid += (int)(blockDim.x >> 5)) {
         const int f0 = B.bc_fptr[sh.bc_mid_off + mid], f1 = B.bc_fptr[sh.bc_mid_off + mid + 1];
         double g[3] = {0.0, 0.0, 0.0};
         for (int f = f0; f < f1; f += CS_BC_UNROLL) {
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(CS_BC_RESTRICT_THREADS) cs_bc_restrict_kernel(
     __syncthreads();
     if (threadIdx.x < 3) {
         double x = 0.0;
-        for (int q = 0; q < CS_BC_RESTRICT_THREADS / 32; q++) x += sh3[q][threadIdx.x];
+        for (int q = 0; q < (int)(blockDim.x >> 5); q++) x += sh3[q][threadIdx.x];
         B.bc_rc[sh.bc_vec_off + 3 * sa.y + threadIdx.x] = (float)x;
     }
 }

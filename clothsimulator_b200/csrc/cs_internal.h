@@ -266,6 +266,7 @@ struct Batch {
     float* bc_ef = nullptr;      // per sheet fine cell: its correction, then the sum of all levels' (3)
     float* bc_em = nullptr;      // per sheet middle cell: its correction (3)
     int bc_max_nmid = 0;         // largest number of middle cells of a sheet
+    int bc_warps = 1;            // warps per block of the restriction: middle cells of an aggregate, at most 16
     int4* bc_pair = nullptr;     // per topology coarse pair: (a, b, contributor begin, end)
     int* bc_contrib = nullptr;   // topology slots (panel * 32 + lane) of the stored blocks of each pair
     float* bc_mat = nullptr;     // per sheet nc x nc: the coarse matrix R A R^T (then GJ's work)

@@ -1301,7 +1301,7 @@ void launchTrip(cs_ctx* c, cudaGraphConditionalHandle h) {
     cs_vector_kernel<<<g, 128, 0, c->stream>>>(B);
     if (B.bc_total_agg > 0 && c->tripCoarse) {
         // the coarse correction of z and the r.z, r.r partials it changes (coarse.cu)
-        cs_bc_restrict_kernel<<<B.bc_total_agg, CS_BC_RESTRICT_THREADS, 0, c->stream>>>(B);
+        cs_bc_restrict_kernel<<<B.bc_total_agg, 32 * B.bc_warps, 0, c->stream>>>(B);
         cs_bc_apply_kernel<<<B.bc_total_agg, CS_BC_APPLY_THREADS, 0, c->stream>>>(B);
         cs_bc_finish_kernel<<<g, 128, 0, c->stream>>>(B);
     }
@@ -2163,6 +2163,10 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     B.bc_total_agg = (int)hbc_agg.size();
     B.bc_max_npair = bcMaxPair;
     B.bc_max_nmid = bcMaxMid;
+    B.bc_warps = 1;
+    for (const BCPlan& P : bcplans)
+        for (int a = 0; a < P.na; a++) B.bc_warps = std::max(B.bc_warps, P.aptr[a + 1] - P.aptr[a]);
+    B.bc_warps = std::min(B.bc_warps, CS_BC_RESTRICT_THREADS / 32);
     B.bc_n_big = (int)hbc_big.size();
     c->bcMatFloats = bcMat;
     UP(row2slot, hrow2slot);
@@ -3283,7 +3287,7 @@ cs_status cs_profile_kernels(cs_ctx* c, const cs_step_params* p, int reps, float
         cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
         cudaEventRecord(c->ev0, c->stream);
         for (int r = 0; r < reps; r++) {
-            cs_bc_restrict_kernel<<<B.bc_total_agg, CS_BC_RESTRICT_THREADS, 0, c->stream>>>(B);
+            cs_bc_restrict_kernel<<<B.bc_total_agg, 32 * B.bc_warps, 0, c->stream>>>(B);
             cs_bc_apply_kernel<<<B.bc_total_agg, CS_BC_APPLY_THREADS, 0, c->stream>>>(B);
             cs_bc_finish_kernel<<<g, 128, 0, c->stream>>>(B);
         }
