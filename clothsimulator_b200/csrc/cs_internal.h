@@ -77,7 +77,7 @@ struct SliceDesc {
     int width;       // block slots per row
     int panel0;      // first global value panel
     int tpanel0;     // first per-topology panel (columns, contributor lists)
-    int pad;
+    int keep;        // block slots that the on-chip solvers hold in shared memory (panels.h)
 };
 
 // Solver phases of one instance (one sheet's system) inside the batched loop.

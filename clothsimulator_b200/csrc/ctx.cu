@@ -31,6 +31,7 @@
 
 #include "../../include/clothstep.h"
 #include "cs_internal.h"
+#include "panels.h"
 #include "mlp.h"
 
 // kernels (forces.cu, pcg.cu)
@@ -1782,7 +1783,19 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         const size_t optin = devProp.sharedMemPerBlockOptin - ga.sharedSizeBytes;
         auto r2 = [](size_t n) { return (n + 1) & ~(size_t)1; };
         auto r4 = [](size_t n) { return (n + 3) & ~(size_t)3; };
-        int warps = 0, panels = 0;
+        // the shared memory of a CTA that takes sheets of these largest sizes
+        struct Sizes {
+            int warps = 0, panels = 0, max = 0, halo = 0, cnc = 0, ck3 = 0, cai = 0;
+        } z;
+        auto uBytes = [&](const Sizes& q) { return (2 * ((size_t)q.warps * CS_SLICE + 1) + q.halo) * sizeof(float4); };
+        auto restBytes = [&](const Sizes& q) {
+            return (r2(3 * (size_t)q.max) + 2 * r2(q.cnc)) * sizeof(double) +
+                   (2 * r4(q.cnc) + r4(CS_GROUP_CE_PARTS * (size_t)q.ck3) + r4(q.cai)) * sizeof(float);
+        };
+        auto capOf = [&](const Sizes& q) {
+            const size_t other = uBytes(q) + restBytes(q);
+            return other < optin ? (int)std::min<size_t>(q.panels, (optin - other) / (CS_PANEL_FLOATS * sizeof(float))) : 0;
+        };
         for (size_t t = 0; t < topos.size(); t++) {
             const Topo& T = *topos[t];
             if (!T.group || topoResident[t]) continue;
@@ -1795,28 +1808,47 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                 (size_t)P.max_panels * 3 / 4 * CS_PANEL_FLOATS * sizeof(float) +
                         (2 * (size_t)P.max_own * CS_SLICE + P.max_halo) * sizeof(float4) + 24 * 1024 > optin)
                 continue;
+            // nor may the sheets that share the launch take that much of one another's
+            Sizes q = z;
+            q.warps = std::max(q.warps, P.max_own);
+            q.panels = std::max(q.panels, P.max_panels);
+            q.max = std::max(q.max, T.tile_ctas);
+            q.halo = std::max(q.halo, P.max_halo);
+            q.cnc = std::max(q.cnc, nc);
+            q.ck3 = std::max(q.ck3, 3 * T.tile_segs);
+            q.cai = std::max(q.cai, 3 * T.tile_segs * nc);
+            if (4 * (long long)capOf(q) < 3 * (long long)q.panels) continue;
+            z = q;
             topoGroup[t] = 1;
-            B.g_max = std::max(B.g_max, T.tile_ctas);
-            warps = std::max(warps, P.max_own);
-            panels = std::max(panels, P.max_panels);
-            B.g_halo = std::max(B.g_halo, P.max_halo);
-            B.g_cnc = std::max(B.g_cnc, nc);
-            B.g_ck3 = std::max(B.g_ck3, 3 * T.tile_segs);
-            B.g_cai = std::max(B.g_cai, 3 * T.tile_segs * nc);
         }
-        if (warps > 0) {
-            B.g_own = warps * CS_SLICE + 1;  // a zero entry before the halo
-            const size_t u = (2 * (size_t)B.g_own + B.g_halo) * sizeof(float4);
-            const size_t rest = (r2(3 * (size_t)B.g_max) + 2 * r2(B.g_cnc)) * sizeof(double) +
-                                (2 * r4(B.g_cnc) + r4(CS_GROUP_CE_PARTS * (size_t)B.g_ck3) + r4(B.g_cai)) * sizeof(float);
-            B.g_cap = (int)std::min<size_t>(panels, (optin - u - rest) / (CS_PANEL_FLOATS * sizeof(float)));
-            B.g_coff = (int)(B.g_cap * CS_PANEL_FLOATS * sizeof(float) + u);
+        if (z.warps > 0) {
+            B.g_max = z.max;
+            B.g_halo = z.halo;
+            B.g_cnc = z.cnc;
+            B.g_ck3 = z.ck3;
+            B.g_cai = z.cai;
+            B.g_own = z.warps * CS_SLICE + 1;  // a zero entry before the halo
+            const size_t rest = restBytes(z);
+            B.g_cap = capOf(z);
+            B.g_coff = (int)(B.g_cap * CS_PANEL_FLOATS * sizeof(float) + uBytes(z));
             c->groupSmem = B.g_coff + rest;
-            c->groupThreads = warps * CS_SLICE;
+            c->groupThreads = z.warps * CS_SLICE;
             CS_CUDA(raiseDynSmem((const void*)cs_group_pcg_kernel, c->groupSmem));
             int perSM = 0;
             CS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, cs_group_pcg_kernel, c->groupThreads, c->groupSmem));
             if (perSM < 1) std::fill(topoGroup.begin(), topoGroup.end(), 0);
+        }
+    }
+    // the panels of every CTA's slices that its shared memory holds
+    std::vector<std::vector<int>> topoKeep(topos.size());
+    for (size_t t = 0; t < topos.size(); t++) {
+        const Topo& T = *topos[t];
+        const int ctas = topoResident[t] ? res.cl : topoGroup[t] ? T.tile_ctas : 0, cap = topoResident[t] ? resCap : B.g_cap;
+        topoKeep[t].assign(T.n_slices, 0);
+        for (int k = 0; k < ctas; k++) {
+            const int lo = topoResident[t] ? plans[t].split[k] : (int)((long long)T.n_slices * k / ctas);
+            const int hi = topoResident[t] ? plans[t].split[k + 1] : (int)((long long)T.n_slices * (k + 1) / ctas);
+            keptPanels(T.slice_width.data() + lo, hi - lo, cap, topoKeep[t].data() + lo);
         }
     }
     c->resCL = c->resThreads = c->resClusters = 0;
@@ -2001,6 +2033,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             sl.row0 = node_off;  // rows: row0 + rowmap[topo_slice * 32 + lane]
             sl.rows = T.slice_rows[t];
             sl.width = T.slice_width[t];
+            sl.keep = topoKeep[sheetTopoId[s]][t];
             sl.panel0 = panel_off + T.slice_tpanel0[t];
             sl.tpanel0 = topoPanel0[sheetTopoId[s]] + T.slice_tpanel0[t];
             hslices.push_back(sl);

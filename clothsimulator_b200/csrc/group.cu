@@ -133,16 +133,14 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         const int rstride = K + 2;
         __syncthreads();  // the previous item's shared memory is free
         // this thread's row: slice lo + w, lane.  The panels beyond the shared-memory budget are
-        // the last slots of the slices, spread evenly.
+        // the last slots of the slices (the loader chose how many of each, panels.h).
         bool live = false;
         int width = 0, ks = 0, lp = 0, gp = 0, tp = 0, row = 0, slot = 0, pub = 0;
         {
             const SliceDesc* sl = B.slices + sh.slice_off + lo;
-            const int panels = nsl > 0 ? sl[nsl - 1].panel0 + sl[nsl - 1].width - sl[0].panel0 : 0;
-            const int over = max(panels - B.g_cap, 0);
             int at = 0;
             for (int j = 0; j < nsl; j++) {
-                const int wd = sl[j].width, out = min(wd, (over * (j + 1)) / nsl - (over * j) / nsl), keep = wd - out;
+                const int wd = sl[j].width, keep = sl[j].keep;
                 // cooperative copy of the slice's kept panels
                 const float4* src = reinterpret_cast<const float4*>(B.A + (size_t)sl[j].panel0 * CS_PANEL_FLOATS);
                 float4* dst = reinterpret_cast<float4*>(cs_group_smem) + (size_t)at * (CS_PANEL_FLOATS / 4);

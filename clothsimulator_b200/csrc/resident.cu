@@ -396,17 +396,14 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         const int lo = B.rsplit[tb + rank], hi = B.rsplit[tb + rank + 1];
         const int nsl = hi - lo;
         // this CTA's panels into shared memory, up to the budget: what exceeds it are
-        // the last slots of the slices, spread evenly
+        // the last slots of the slices (the loader chose how many of each, panels.h)
         bool live = false;
         int width = 0, ks = 0, lp = 0, gp = 0, tp = 0, row = 0;
         {
             const SliceDesc* sl = B.slices + sh.slice_off + lo;
-            const int panels = nsl > 0 ? sl[nsl - 1].panel0 + sl[nsl - 1].width - sl[0].panel0 : 0;
-            const int over = max(panels - cap, 0);
             int at = 0;
             for (int j = 0; j < nsl; j++) {
-                const int wd = sl[j].width, p0 = sl[j].panel0;
-                const int out = min(wd, (over * (j + 1)) / nsl - (over * j) / nsl), keep = wd - out;
+                const int wd = sl[j].width, p0 = sl[j].panel0, keep = sl[j].keep;
                 const float4* src = reinterpret_cast<const float4*>(B.A + (size_t)p0 * CS_PANEL_FLOATS);
                 float4* dst = reinterpret_cast<float4*>(cs_res_smem) + (size_t)at * (CS_PANEL_FLOATS / 4);
                 for (int i = tid; i < keep * (CS_PANEL_FLOATS / 4); i += blockDim.x) dst[i] = __ldg(src + i);
