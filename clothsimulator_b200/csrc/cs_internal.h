@@ -40,9 +40,15 @@ __host__ __device__ inline uint32_t cs_code(int is_edge, int elem, int a, int b)
 // fit four warps in a CTA's shared memory gets fewer.  (One-warp CTAs, 15 warps per SM instead
 // of 12, measured slower on the windy batch: 3.82 against 3.35 ms.)
 #define CS_GATHER_THREADS 128
-// threads (rows) per block of the proximity row kernel, and its shared memory: a row's blocks and columns
+// Rows (threads) per block of the proximity row kernel: a warp's, fewer where the blocks and columns of that
+// many rows of `width` blocks exceed the shared memory of a block (from 182 blocks a row; the gather
+// takes up to 201); and that shared memory.
 #define CS_PROX_ROW_THREADS 32
-inline size_t cs_prox_row_smem(int width) { return (size_t)width * 10 * CS_PROX_ROW_THREADS * sizeof(float); }
+inline size_t cs_prox_row_smem(int width, int rows) { return (size_t)width * 10 * rows * sizeof(float); }
+inline int cs_prox_rows(int width, size_t smem) {
+    const size_t rows = smem / cs_prox_row_smem(width > 0 ? width : 1, 1);
+    return rows < CS_PROX_ROW_THREADS ? (int)rows : CS_PROX_ROW_THREADS;
+}
 
 struct SheetDesc {
     int node_off, n_nodes;

@@ -980,6 +980,7 @@ struct cs_ctx {
     int gatherGrid = 1;  // persistent assembly gather: a few warps per SM walk the slices
     size_t gatherSmem = 0;  // its dynamic shared memory (slot accumulators)
     int gatherWarps = 1;    // its warps per CTA
+    int proxRows = CS_PROX_ROW_THREADS;  // rows per block of the proximity row kernel
     // learned warm start
     MlpDev mlp;
     bool mlpInit = false;
@@ -1134,7 +1135,7 @@ int launchAssembly(cs_ctx* c) {
         // proximity terms after the handles (Cloth.cu:676-684): records, then per row the
         // blocks, right-hand side and block-Jacobi inverse, then the ||b|| partials
         cs_prox_kernel<<<nblk(B.n_pinst, 128), 128, 0, c->stream>>>(B);
-        cs_prox_row_kernel<<<nblk(B.N, CS_PROX_ROW_THREADS), CS_PROX_ROW_THREADS, cs_prox_row_smem(B.gather_width), c->stream>>>(B);
+        cs_prox_row_kernel<<<nblk(B.N, c->proxRows), c->proxRows, cs_prox_row_smem(B.gather_width, c->proxRows), c->stream>>>(B);
         cs_slice_bnorm_kernel<<<nblk((long long)B.n_slices * 32, 128), 128, 0, c->stream>>>(B);
         n += 3;
     }
@@ -2290,7 +2291,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             return fail(c, CS_ERR_INVALID_ARG, "slices of %d block slots exceed the assembly's shared memory", B.gather_width);
         c->gatherSmem = (size_t)c->gatherWarps * perWarp;
         CS_CUDA(raiseDynSmem((const void*)cs_gather_kernel, c->gatherSmem));
-        CS_CUDA(raiseDynSmem((const void*)cs_prox_row_kernel, cs_prox_row_smem(B.gather_width)));
+        c->proxRows = cs_prox_rows(B.gather_width, prop.sharedMemPerBlockOptin);
+        CS_CUDA(raiseDynSmem((const void*)cs_prox_row_kernel, cs_prox_row_smem(B.gather_width, c->proxRows)));
         const int threads = 32 * c->gatherWarps;
         int perSM = 0;
         CS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, cs_gather_kernel, threads, c->gatherSmem));

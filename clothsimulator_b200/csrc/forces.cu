@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(128) cs_prox_kernel(Batch B) {
 // after the gather's handle terms.  Blocks on the mesh pattern are summed onto their slot,
 // others onto the row's side list (zeroed first); the row's block-Jacobi inverse is redone.
 // The sums are a serial chain per row, so the row's blocks and columns are copied to shared memory
-// first (entry e of slot k of a thread at [(9 k + e) * CS_PROX_ROW_THREADS + thread]: no conflicts),
+// first (entry e of slot k of a thread at [(9 k + e) * rows + thread], rows the block's: no conflicts),
 // summed there and written back: summed in place through L2, a step of two 64 x 64 layers (18,600
 // proximities) took 317 us.
 extern __shared__ float cs_prox_acc[];
@@ -696,17 +696,18 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
     const int* cp = B.tcsr_ptr + sd.csr_ptr_off;
     const int li = row - sd.node_off;
     const int c0 = cp[li], nc = cp[li + 1] - c0;
+    const int R = blockDim.x;
     float* const acc = cs_prox_acc + threadIdx.x;
-    int* const cols = reinterpret_cast<int*>(cs_prox_acc + 9 * (size_t)B.gather_width * CS_PROX_ROW_THREADS) + threadIdx.x;
+    int* const cols = reinterpret_cast<int*>(cs_prox_acc + 9 * (size_t)B.gather_width * R) + threadIdx.x;
     int diag = 0;
     for (int k = 0; k < nc; k++) {
         const int col = B.tcsr_col[c0 + k] + sd.node_off;
-        cols[k * CS_PROX_ROW_THREADS] = col;
+        cols[k * R] = col;
         if (col == row) diag = k;
         float a[9];
         load_slot(B.A, sd.panel_off * CS_SLICE + B.tcsr_slot[c0 + k], a);
 #pragma unroll
-        for (int e = 0; e < 9; e++) acc[(9 * k + e) * CS_PROX_ROW_THREADS] = a[e];
+        for (int e = 0; e < 9; e++) acc[(9 * k + e) * R] = a[e];
     }
     const int x0 = B.xptr ? B.xptr[row] : 0, x1 = B.xptr ? B.xptr[row + 1] : 0;
     for (int m = x0; m < x1; m++)
@@ -726,10 +727,10 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
             int lo = 0, hi = nc;
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (cols[mid * CS_PROX_ROW_THREADS] < col) lo = mid + 1;
+                if (cols[mid * R] < col) lo = mid + 1;
                 else hi = mid;
             }
-            at[bb] = lo < nc && cols[lo * CS_PROX_ROW_THREADS] == col ? lo : -1;
+            at[bb] = lo < nc && cols[lo * R] == col ? lo : -1;
         }
         for (int fr = 0; fr < 2; fr++)
             for (int a = 0; a < 4; a++) {
@@ -743,11 +744,11 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
                     if (at[bb] == -2) continue;
                     const float* blk = rec + fr * 144 + (3 * a) * 12 + 3 * bb;
                     if (at[bb] >= 0) {
-                        float* d = acc + 9 * at[bb] * CS_PROX_ROW_THREADS;
+                        float* d = acc + 9 * at[bb] * R;
 #pragma unroll
                         for (int k = 0; k < 3; k++)
 #pragma unroll
-                            for (int h = 0; h < 3; h++) d[(3 * k + h) * CS_PROX_ROW_THREADS] += blk[k * 12 + h];
+                            for (int h = 0; h < 3; h++) d[(3 * k + h) * R] += blk[k * 12 + h];
                         continue;
                     }
                     int m = x0;
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
     for (int k = 0; k < nc; k++) {
         float a[9];
 #pragma unroll
-        for (int e = 0; e < 9; e++) a[e] = acc[(9 * k + e) * CS_PROX_ROW_THREADS];
+        for (int e = 0; e < 9; e++) a[e] = acc[(9 * k + e) * R];
         store_slot(B.A, sd.panel_off * CS_SLICE + B.tcsr_slot[c0 + k], a);
         if (k == diag) block_inverse(a, B.Pinv + 9 * (size_t)row);
     }
