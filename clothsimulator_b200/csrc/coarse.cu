@@ -88,7 +88,9 @@ __device__ __forceinline__ void bc_cell_inverse(const float (&a)[9], bool on, fl
 }
 
 // The diagonal blocks of F A F^T for the fine cells of middle cell `mid` of a sheet, and of G A G^T for
-// itself, inverted: a lane per node of a fine cell walks the node's row.
+// itself, inverted: a lane per node of a fine cell walks the node's row.  `B` is the kernel's own parameter
+// (__grid_constant__): a copy of it on every thread's stack would cost all threads 912 bytes of stores, 0.5 ms
+// a step of 1,024 sheets that the loop does not even solve.
 __device__ __noinline__ void bc_cell_blocks(const Batch& B, const SheetDesc& sh, int mid, int lane) {
     const int* fptr = B.bc_fptr + sh.bc_mid_off + mid;
     const int* mptr = B.bc_mptr + sh.bc_fine_off;
@@ -141,7 +143,7 @@ __device__ __forceinline__ bool bc_trip_on(const Batch& B, int s) {
 // contributor slots (lane-strided, then a butterfly: a fixed order) into rows 3a..3a+2,
 // columns 3b..3b+2 of the sheet's dense coarse matrix (zeroed before); further warps take the middle
 // cells and the fine cells in them.  Grid: x over pairs and middle cells, y over sheets.
-__global__ void __launch_bounds__(256) cs_bc_assemble_kernel(Batch B) {
+__global__ void __launch_bounds__(256) cs_bc_assemble_kernel(const __grid_constant__ Batch B) {
     const int s = blockIdx.y;
     if (!bc_sheet_on(B, s) || (B.inst[s].phase == PH_RESIDENT) != (B.bc_resident != 0)) return;
     const SheetDesc& sh = B.sheets[s];

@@ -52,7 +52,7 @@ static_assert(CS_SPMV_CANDIDATES == CS_TUNE_SPMV_SHAPES, "the tuner's result hol
 __global__ void cs_prox_kernel(Batch B);
 __global__ void cs_prox_row_kernel(Batch B);
 __global__ void cs_slice_bnorm_kernel(Batch B);
-__global__ void cs_bc_assemble_kernel(Batch B);
+__global__ void cs_bc_assemble_kernel(const __grid_constant__ Batch B);
 __global__ void cs_bc_invert_small_kernel(Batch B);
 __global__ void cs_bc_invert_cluster_kernel(Batch B);
 __global__ void cs_bc_restrict_kernel(Batch B);
