@@ -61,3 +61,24 @@ def test_sizes_against_fp64(n, per_row):
     # the residual's tolerance times the condition of the diagonally dominant system (below 1e3),
     # and the FP32 rounding of x
     assert np.linalg.norm(out[:3 * n] - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("nq,tol", [(40, 1e-7), (64, 1e-8), (100, 1e-8), (120, 1e-6)])
+def test_solution_overshoots_the_tolerance(ctx_factory, nq, tol):
+    """The last sweep ends at a quarter of the tolerance (and a tenth of that for the recursive residual's
+    drift), so that x is as close to the solution as that of a solver that stops anywhere below it."""
+    import torch
+
+    from clothsimulator_b200 import scenes
+
+    scene = scenes.hang(nq, 1)
+    ctx = ctx_factory(scene.sheets)
+    ctx.assemble(native.step_params(scene.dt, scene.gravity, scene.handle_stiffness))
+    rp, ci, val, b = ctx.system()
+    d = [torch.from_numpy(np.ascontiguousarray(a).reshape(-1)).cuda() for a in (rp, ci, val, b)]
+    x = torch.zeros(len(b), device="cuda")
+    torch.cuda.synchronize()
+    it, rr = ctypes.c_int(0), ctypes.c_double(-1.0)
+    st = native.load_library().cs_solve_block_csr_noalloc(len(rp) - 1, len(ci), *(t.data_ptr() for t in d), x.data_ptr(), tol,
+                                                          20000, None, ctypes.byref(it), ctypes.byref(rr))
+    assert st == native.CS_OK and rr.value <= 0.28 * tol
