@@ -65,7 +65,7 @@ def test_sizes_against_fp64(n, per_row):
 
 @pytest.mark.parametrize("nq,tol", [(40, 1e-7), (64, 1e-8), (100, 1e-8), (120, 1e-6)])
 def test_solution_overshoots_the_tolerance(ctx_factory, nq, tol):
-    """The last sweep ends at a quarter of the tolerance (and a tenth of that for the recursive residual's
+    """The last sweep ends at a fifth of the tolerance (and a tenth of that for the recursive residual's
     drift), so that x is as close to the solution as that of a solver that stops anywhere below it."""
     import torch
 
@@ -81,4 +81,4 @@ def test_solution_overshoots_the_tolerance(ctx_factory, nq, tol):
     it, rr = ctypes.c_int(0), ctypes.c_double(-1.0)
     st = native.load_library().cs_solve_block_csr_noalloc(len(rp) - 1, len(ci), *(t.data_ptr() for t in d), x.data_ptr(), tol,
                                                           20000, None, ctypes.byref(it), ctypes.byref(rr))
-    assert st == native.CS_OK and rr.value <= 0.28 * tol
+    assert st == native.CS_OK and rr.value <= 0.24 * tol
