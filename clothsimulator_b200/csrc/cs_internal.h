@@ -106,7 +106,7 @@ enum InstPhase : int {
 // Reliable updates keep the search direction only while the recursive residual has drifted
 // from the FP64 one by at most this fraction of the latter (larger drift: restart).
 #define CS_RELIABLE_DRIFT 0.1
-#define CS_LAST_SWEEP 0.3  // on-chip solvers: recursive residual that ends the last sweep, of the tolerance
+#define CS_LAST_SWEEP 0.3  // on-chip solvers beyond block-Jacobi: recursive residual that ends the last sweep, of the tolerance
 // power iterations per sheet solve for the tile-local Chebyshev bound
 #define CS_CHEB_POWER_ITERS 10
 // A sheet uses the tile-local Chebyshev preconditioner only if at least this share of its

@@ -655,8 +655,9 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             // PH_CG: the iteration's x and r updates are done; stopping test on ||r||
             iters += 1;
             sweep_iters += 1;
-            // the last sweep goes below the tolerance, as in resident.cu
-            const double ti = P.inner_tol * S.res0, tt = P.tol * S.bn, t = ti > tt ? ti : CS_LAST_SWEEP * tt;
+            // the sweep's end, as in resident.cu
+            const double ti = P.inner_tol * S.res0, tt = P.tol * S.bn;
+            const double t = P.cheb_degree >= 3 ? (ti > tt ? ti : CS_LAST_SWEEP * tt) : fmax(ti, 0.5 * tt);
             bool stop = rr <= t * t || sweep_iters >= P.sweep_cap;
             const double bd = gnew * inv_gam, na = gnew / (dnew - gnew * gnew * inv_ga);
             if (!gfinite((double)(float)bd) || !gfinite((double)(float)na) || !(gnew > 0.0) || !((float)na > 0.f)) {

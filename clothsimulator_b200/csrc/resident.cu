@@ -544,7 +544,8 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
         // then the coefficients of the Chebyshev iteration on [lmax / 30, lmax].  An odd
         // degree keeps the polynomial positive on all of (0, inf), so the preconditioner is
         // SPD whatever the estimate.
-        if (!levels && P.cheb_degree >= 3 && (B.rcheb[tb + rank] & 1)) {
+        const bool poly = !levels && P.cheb_degree >= 3 && (B.rcheb[tb + rank] & 1);  // uniform over the cluster
+        if (poly) {
             float v[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -852,10 +853,11 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
             const double gnew = v[0], dnew = v[1];
             rr = v[2];
             if (phase == PH_INIT) {
-                // the last sweep goes to CS_LAST_SWEEP of the tolerance: at equal residuals the levels leave
-                // up to 1.6 times the error in dv that a larger coarse space did (32 x 32 quads)
+                // a sweep ends when r fell by inner_tol, the last one at half the tolerance at the latest; with the
+                // levels or the polynomial it goes to CS_LAST_SWEEP of it: at equal residuals the levels
+                // leave up to 1.6 times the error in dv that a larger coarse space did (32 x 32 quads)
                 const double ti = mixed ? P.inner_tol * res0 : 0.0, tt = P.tol * bn;
-                const double t = ti > tt ? ti : (mixed ? CS_LAST_SWEEP : 1.0) * tt;
+                const double t = !mixed ? tt : levels || poly ? (ti > tt ? ti : CS_LAST_SWEEP * tt) : fmax(ti, 0.5 * tt);
                 thr = t * t;
             }
             if (phase == PH_INIT && cont) {
