@@ -171,7 +171,6 @@ void launchSpmvShape(const Batch& B, int shape, cudaStream_t st);
 // Group-resident solver (group.cu): block slots per row (column codes live in registers), slices
 // per CTA that a sheet's tiles are planned for, its fewest when a batch would leave the chip idle.
 #define CS_GROUP_MAX_WIDTH 18
-#define CS_GROUP_OCTET_PANELS 190  // a tile's panels up to which a group's rows take the octet order
 #define CS_GROUP_SLICES 14
 #define CS_GROUP_MAX_WARPS CS_RES_MAX_WARPS
 #define CS_GROUP_CE_PARTS 4    // warps that share a row of the coarse matrix-vector product, at most
@@ -250,7 +249,6 @@ struct ProxInst {
 struct GroupItem {
     int sheet, cta0, ctas, segs;
     int slot0, red0, pub0, halo0;
-    int octets;  // its rows are in octet order (levels.cuh)
     long long mat;
 };
 
@@ -314,6 +312,7 @@ struct Batch {
     int* nbr = nullptr;
     int* node_sheet = nullptr;   // sheet of every node
     int* rowmap = nullptr;       // per topology slice lane: sheet-local row
+    uint32_t* rcell = nullptr;   // per topology slice lane of a tiled sheet: LevelPlace (levels.cuh)
     int* row2slot = nullptr;     // per topology row: slice * 32 + lane
     // system
     float* A = nullptr;          // n_panels * 288

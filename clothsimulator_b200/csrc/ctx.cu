@@ -216,7 +216,10 @@ struct Topo {
     // CTAs its rows are tiled for (a cluster's, or a group's where `group`; 0: not tiled) and the
     // segments each tile is ordered by
     int tile_ctas = 0, tile_segs = 0;
-    bool group = false, octets = false;
+    bool group = false;
+    // per row slot of a tiled sheet: its place in its tile's cell order << 16 | the slot of the row at the place of
+    // this slot's number (levels.cuh)
+    std::vector<uint32_t> cell;
     // rest (uv) coordinates of every node, from the first sheet of this connectivity: the
     // geometry the coarse-space segments of the cluster-resident solver are cut along
     std::vector<float> node_uv;
@@ -242,12 +245,20 @@ uint64_t hashInts(const int32_t* a, size_t n, uint64_t h) {
 
 // Rows ordered by tiles for the solvers that hold a sheet on chip: the slices (32 rows) are dealt evenly to G
 // CTAs and within a CTA to K segments, and recursive bisection of the rest coordinates along the
-// longer axis gives every segment a compact piece of the sheet.  With `octets` the bisection goes on to
-// slices and to eights of rows, each compact; else the rows of a segment are ordered by block count
-// (descending, then by index), which keeps its slices' padding low.
-void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, bool octets, std::vector<int>& order) {
+// longer axis gives every segment a compact piece of the sheet, and on to 32 and to 8 rows, each compact: the
+// cells of the levels (levels.cuh); `cell`: LevelPlace, from the tile's first row on.  The rows of a segment are
+// stored by block count (descending, then by index).  Stored in cell order, every slice of a grid of
+// alternating diagonals held rows of 13 and of 9 blocks, 1.21 times the panels of a 64 x 64 sheet (1.04 by
+// count), 1.31 (1.07) on a sheet of random diagonals, and the assembly and the loop read the nodes in
+// patches of 8 x 4; by count the levels take two more barriers an iteration.  1,024 sheets of 64 x 64
+// quads, in cell order and by count: gather 4.27 and 3.63 ms, a step with block-Jacobi 113.9 and 109.6, with
+// Chebyshev-3 112 and 98, in the loop without coarse space 182 and 168, with the levels 59.4 and 60.2;
+// one sheet of 32 x 32 with the levels 0.360 and 0.378, a group of 72,900 nodes 5.25 and 4.59 (B200).
+void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, std::vector<int>& order,
+               std::vector<uint32_t>& cell) {
     const int n = (int)len.size(), ns = (n + CS_SLICE - 1) / CS_SLICE;
     order.resize(n);
+    cell.assign(n, 0);
     for (int i = 0; i < n; i++) order[i] = i;
     std::vector<int> cut{0};  // first row of every segment
     for (int c = 0; c < G; c++) {
@@ -280,11 +291,18 @@ void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G,
         const int r0 = cut[a], r1 = cut[b];
         if (r0 >= r1) return;
         if (b - a == 1) {
-            if (octets)
-                patches(r0, r1);
-            else
-                std::sort(order.begin() + r0, order.begin() + r1,
-                          [&](int x, int y) { return len[x] != len[y] ? len[x] > len[y] : x < y; });
+            patches(r0, r1);
+            std::vector<std::pair<int, int>> byCount(r1 - r0);  // place in cell order, row
+            for (int i = r0; i < r1; i++) byCount[i - r0] = {i, order[i]};
+            std::sort(byCount.begin(), byCount.end(), [&](const std::pair<int, int>& x, const std::pair<int, int>& y) {
+                return len[x.second] != len[y.second] ? len[x.second] > len[y.second] : x.second < y.second;
+            });
+            for (int i = r0; i < r1; i++) {
+                order[i] = byCount[i - r0].second;
+                const int base = cut[a / K * K], place = byCount[i - r0].first;
+                cell[i] |= (uint32_t)(place - base) << 16;
+                cell[place] |= (uint32_t)(i - base);
+            }
             return;
         }
         // tiles are halved before their segments are
@@ -296,9 +314,8 @@ void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G,
     bisect(0, G * K);
 }
 
-// tileCtas: CTAs to tile the rows for (0: none), at most `segs` segments per tile; octets: in
-// octet order whatever it pads.
-std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, bool octets, std::string& err) {
+// tileCtas: CTAs to tile the rows for (0: none), at most `segs` segments per tile.
+std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, std::string& err) {
     auto t = std::make_shared<Topo>();
     const int nn = s.n_nodes, nv = s.n_verts, nf = s.n_faces;
     t->n_nodes = nn;
@@ -495,32 +512,7 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     if (tileCtas > 0) {
         t->tile_ctas = tileCtas;
         t->tile_segs = std::max(1, std::min(segs, t->n_slices / tileCtas));
-        // Octet order mixes long and short rows in a slice: 1.2 times the panels on a grid of alternating
-        // diagonals, 1.3 times on an irregular mesh.  A group, whose tiles can fill the shared memory, takes
-        // it while a tile's panels about fit.
-        const int few = std::min(t->tile_segs, CS_COARSE_SEGS);
-        tileOrder(t->node_uv, len, t->tile_ctas, few, true, order);
-        t->octets = true;
-        if (!octets) {
-            auto mostPanels = [&](const std::vector<int>& o) {
-                int most = 0;
-                for (int c = 0; c < tileCtas; c++) {
-                    int n = 0;
-                    for (int sl = (int)((long long)t->n_slices * c / tileCtas); sl < (int)((long long)t->n_slices * (c + 1) / tileCtas); sl++) {
-                        int w = 0;
-                        for (int l = sl * CS_SLICE; l < std::min(nn, (sl + 1) * CS_SLICE); l++) w = std::max(w, len[o[l]]);
-                        n += w;
-                    }
-                    most = std::max(most, n);
-                }
-                return most;
-            };
-            if (mostPanels(order) > CS_GROUP_OCTET_PANELS) {
-                tileOrder(t->node_uv, len, t->tile_ctas, t->tile_segs, false, order);
-                t->octets = false;
-            }
-        }
-        if (t->octets) t->tile_segs = few;
+        tileOrder(t->node_uv, len, t->tile_ctas, t->tile_segs, order, t->cell);
     }
     t->rowmap.assign((size_t)t->n_slices * CS_SLICE, 0);
     t->row2slot.assign(nn, 0);
@@ -1502,7 +1494,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         } else {
             std::string err;
             const int G = groupCtasFor(d.n_nodes);
-            auto t = buildTopo(d, G, G > 0 ? std::min(CS_COARSE_MAX_K, CS_GROUP_NC / (3 * G)) : 0, false, err);
+            auto t = buildTopo(d, G, G > 0 ? std::min(CS_COARSE_SEGS, CS_GROUP_NC / (3 * G)) : 0, err);
             if (!t) return fail(c, CS_ERR_INVALID_ARG, "sheet %d: %s", s, err.c_str());
             t->group = G > 0;
             sheetTopoId[s] = (int)topos.size();
@@ -1551,6 +1543,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     std::vector<int2> hrface, hredge;
     int gatherWidth = 1;
     std::vector<int> hnbr_ptr, hnbr, hnode_sheet, hrowmap, hrow2slot;
+    std::vector<uint32_t> hcell;
     std::vector<int> topoRow2Slot0(topos.size());
     std::vector<int> topoNbrPtr0(topos.size()), topoNbr0(topos.size());
     std::vector<int> topoPanel0(topos.size()), topoSlice0(topos.size());
@@ -1676,7 +1669,9 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                 // (CS_CHEB_MIN_LOCAL), they take block-Jacobi
                 if (!est.resident[t] || topos[t]->n_slices < 2 * best) continue;
                 std::string err;
-                auto T = buildTopo(sheets[topoSheet[t]], best, std::max(1, coarseSegments(best)), true, err);
+                // (one segment where the coarse correction is not taken)
+                const int segs = topos[t]->n_slices >= CS_COARSE_MIN_SLICES * best ? std::max(1, coarseSegments(best)) : 1;
+                auto T = buildTopo(sheets[topoSheet[t]], best, segs, err);
                 if (!T) return fail(c, CS_ERR_INVALID_ARG, "sheet %d: %s", topoSheet[t], err.c_str());
                 topos[t] = T;
             }
@@ -1896,6 +1891,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             hredge.insert(hredge.end(), T.re.begin(), T.re.end());
             for (int w : T.slice_width) gatherWidth = std::max(gatherWidth, w);
             hrowmap.insert(hrowmap.end(), T.rowmap.begin(), T.rowmap.end());
+            hcell.insert(hcell.end(), T.cell.begin(), T.cell.end());
+            hcell.resize(hrowmap.size(), 0);
             topoRow2Slot0[t] = (int)hrow2slot.size();
             hrow2slot.insert(hrow2slot.end(), T.row2slot.begin(), T.row2slot.end());
             topoCsrPtr0[t] = (int)htcsr_ptr.size();
@@ -2119,7 +2116,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
                     best = o;
                 }
             }
-            GroupItem gi{s, best, G, K, gSlots, gRed, topoPub0[t], topoHalo0[t], topos[t]->octets ? 1 : 0, gMat};
+            GroupItem gi{s, best, G, K, gSlots, gRed, topoPub0[t], topoHalo0[t], gMat};
             for (int k = best; k < best + G; k++) {
                 busy[k] = when + std::sqrt((double)hs[s].n_nodes);
                 ctaItems[k].push_back((int)hgitem.size());
@@ -2177,6 +2174,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     UP(nbr, hnbr);
     UP(node_sheet, hnode_sheet);
     UP(rowmap, hrowmap);
+    UP(rcell, hcell);
     UP(bc_agg, hbc_agg);
     UP(bc_big, hbc_big);
     UP(bc_node_fine, hbc_fine);

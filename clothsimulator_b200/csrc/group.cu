@@ -12,7 +12,7 @@
 //   * A CTA holds its tile's SELL-32 panels in shared memory (what exceeds it, spread evenly over
 //     the slices, is read from L2), one row per thread with the CG vectors in registers, as
 //     resident.cu does, and runs the same iteration: Chronopoulos-Gear CG with one fused
-//     reduction, the levels of levels.cuh where the tile's rows are in octet order (else the tile-local
+//     reduction, the levels of levels.cuh (without the coarse correction the tile-local
 //     Chebyshev preconditioner), the additive coarse-space correction (one constant per segment of a
 //     tile and component, its residual carried by recurrence within the reduction), FP64 residual
 //     replacements with the search direction kept.
@@ -332,9 +332,14 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         };
         // The tile-local Chebyshev polynomial's interval: power iteration for P^-1 A_loc, as in
         // resident.cu (an odd degree keeps the preconditioner SPD whatever the estimate).
-        const bool levels = P.coarse && P.cheb_degree >= 3 && gi.octets;
+        const bool levels = P.coarse && P.cheb_degree >= 3;
         __syncthreads();
-        if (levels) level_blocks(spn, gpn, ks, width, code, w, lane, live, S.lev[w]);
+        LevelPlace at{(uint32_t)myslot * 0x10001u};
+        if (levels) {
+            const uint32_t* cells = B.rcell + (size_t)B.slices[sh.slice_off + lo].topo_slice * CS_SLICE;
+            if (live) at.v = __ldg(cells + myslot);
+            level_blocks(spn, gpn, ks, width, code, cells, halo0 - 1, at, lane, live, su_alt, S.lev[w]);
+        }
         if (!levels && P.cheb_degree >= 3) {
             float v[3];
 #pragma unroll
@@ -552,12 +557,14 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                         u[c] += d[c];
                     }
                 }
-            } else if (coarse) {
+            } else if (levels || coarse) {
+                if (levels) su[myslot] = make_float4(r[0], r[1], r[2], 0.f);
                 __syncthreads();
-                coarse_matvec();
+                if (coarse) coarse_matvec();
+                if (levels) level_sums(S.lev[w], su, su_alt, at, w, lane);
                 __syncthreads();
+                if (levels) level_add(su_alt, at, u);
             }
-            if (levels) level_correction(S.lev[w], r, lane, u);
             if (coarse && live) {
                 // u = C r + R^T A_c^-1 R r: the additive coarse-space correction
 #pragma unroll
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                     for (int q = 0; q < parts; q++) u[c] += C.ce[(3 * seg + c) * parts + q];
             }
             nhalo++;
-            if (!live) u[0] = u[1] = u[2] = 0.f;  // an octet's correction reaches lanes without a row
+            if (!live) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row
             su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
             if (live && pub)
                 put_packet(upk + slot, __float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), nhalo);

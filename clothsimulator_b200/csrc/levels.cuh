@@ -1,11 +1,13 @@
 // Parts of the on-chip solvers (resident.cu, group.cu) that work on a tile: warp sums, the product of a
 // row with the tile's u array, and the preconditioner's levels.  The loader orders a
-// tile's rows by recursive bisection, so every eight consecutive rows (an octet of lanes) and every 32
-// (a slice, one warp) are a compact patch of the sheet.  With F and G summing a vector over the octets
-// and the slices, per component,
+// tile's rows by recursive bisection into cells: every eight rows in that order (an octet) and every 32
+// (a patch) are a compact piece of the sheet.  Lane l of warp w holds place 32 w + l of that order; the rows
+// are stored by block count, so a vector's values go to their places and the corrections back through
+// shared memory.  With F and G summing a vector over the octets
+// and the patches, per component,
 //     z = D^-1 r + F^T D_F^-1 F r + G^T D_G^-1 G r (+ R^T A_c^-1 R r),
 // D_F and D_G the 3x3 diagonal blocks of F A F^T and G A G^T: additive, SPD, and 15 warp shuffles per
-// iteration with no barrier.  It takes the place of a Chebyshev polynomial in the tile's block of A
+// iteration with two barriers.  It takes the place of a Chebyshev polynomial in the tile's block of A
 // together with a larger coarse space: on a 64 x 64 sheet 76 CG iterations of one SpMV each instead of
 // 61 of one SpMV and two polynomial steps, and 54 coarse unknowns to invert instead of 162.
 #pragma once
@@ -128,29 +130,57 @@ __device__ __forceinline__ void level_apply(const float* inv, const float (&s)[3
     u[2] += a.z * s[0] + b.x * s[1] + b.y * s[2];
 }
 
-// The inverse diagonal blocks of one warp's octets (lev[0..3]) and of its slice (lev[4]), from the stored
-// blocks of its rows: the first ks slots in shared memory (sp), the others in global memory (gp), `code`
-// the slots' columns as row slots of the CTA (others from the halo's first slot on).
+// A thread's part in the levels: the octet of its row (its place in cell order / 8), and the slot of the row whose
+// place is the thread's number.  Threads without a row have their own number for both.
+struct LevelPlace {
+    uint32_t v;  // slot | place << 16
+    __device__ __forceinline__ int slot() const { return (int)(v & 0xffffu); }
+    __device__ __forceinline__ int place() const { return (int)(v >> 16); }
+    __device__ __forceinline__ int octet() const { return (int)(v >> 19); }
+};
+
+// The inverse diagonal blocks of the octets (lev[0..3]) and of the patch (lev[4]) at one warp's places in cell
+// order, from the stored blocks of the rows: the first ks slots of a slice in shared memory (sp), the others
+// in global memory (gp), `code` the slots' columns as row slots of the CTA (from `own` on: others).  `cells`: the
+// {slot, place} of all row slots; `buf`: room for a float4 per row slot.  Every thread of the CTA calls it.
 __device__ __forceinline__ void level_blocks(const float* sp, const float* gp, int ks, int width, const int* __restrict__ code,
-                                             int w, int lane, bool live, float (*lev)[8]) {
-    float a8[9], a32[9];
+                                             const uint32_t* __restrict__ cells, int own, LevelPlace at, int lane, bool live,
+                                             float4* buf,
+                                             float (*lev)[8]) {
+    float m[20];  // the row's part of its octet's block, of its patch's
 #pragma unroll
-    for (int e = 0; e < 9; e++) a8[e] = a32[e] = 0.f;
+    for (int e = 0; e < 20; e++) m[e] = 0.f;
     for (int k = 0; k < width; k++) {
-        const int at = __ldg(code + k * CS_SLICE + lane);
-        if (!live || (at >> 5) != w) continue;
+        const int col = __ldg(code + k * CS_SLICE + lane);
+        if (!live || col >= own) continue;
+        const int other = (int)(__ldg(cells + col) >> 16);
+        if ((other >> 5) != (at.place() >> 5)) continue;
         const float* pk = (k < ks ? sp : gp) + (size_t)k * CS_PANEL_FLOATS;
         const float4 b0 = reinterpret_cast<const float4*>(pk)[lane], b1 = reinterpret_cast<const float4*>(pk + 128)[lane];
         const float a[9] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w, pk[256 + lane]};
-        const float in8 = ((at ^ lane) & 24) == 0 ? 1.f : 0.f;
+        const float in8 = (other >> 3) == at.octet() ? 1.f : 0.f;
 #pragma unroll
         for (int e = 0; e < 9; e++) {
-            a32[e] += a[e];
-            a8[e] = fmaf(in8, a[e], a8[e]);
+            m[e] = fmaf(in8, a[e], m[e]);
+            m[9 + e] += a[e];
         }
     }
 #pragma unroll
+    for (int q = 0; q < 20; q += 4) {
+        __syncthreads();
+        buf[threadIdx.x] = make_float4(m[q], m[q + 1], m[q + 2], m[q + 3]);
+        __syncthreads();
+        const float4 x = buf[at.slot()];
+        m[q] = x.x;
+        m[q + 1] = x.y;
+        m[q + 2] = x.z;
+        m[q + 3] = x.w;
+    }
+    float a8[9], a32[9];
+#pragma unroll
     for (int e = 0; e < 9; e++) {
+        a8[e] = m[e];
+        a32[e] = m[9 + e];
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) a8[e] += __shfl_xor_sync(0xffffffffu, a8[e], o);
 #pragma unroll
@@ -158,22 +188,32 @@ __device__ __forceinline__ void level_blocks(const float* sp, const float* gp, i
     }
     if ((lane & 7) == 0) level_inverse(a8, lev[lane >> 3]);
     if (lane == 0) level_inverse(a32, lev[4]);
-    __syncwarp();
+    __syncthreads();  // `buf` is free
 }
 
-// u += the octet's and the slice's corrections of r (zero in lanes without a row)
-__device__ __forceinline__ void level_correction(const float (*lev)[8], const float (&r)[3], int lane, float (&u)[3]) {
-    float t[3] = {r[0], r[1], r[2]};
+// The corrections by the octets and the patch at one warp's places of the vector that every thread of the CTA
+// stored at its number in `r` (zero without a row), into `z`, a float4 per octet.  Between a barrier after
+// those stores and one before level_add; `r` may be overwritten after the second, `z` after the next.
+__device__ __forceinline__ void level_sums(const float (*lev)[8], const float4* r, float4* z, LevelPlace at, int w, int lane) {
+    const float4 x = r[at.slot()];
+    float t[3] = {x.x, x.y, x.z}, c[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int c = 0; c < 3; c++) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
-    level_apply(lev[lane >> 3], t, u);
+        for (int k = 0; k < 3; k++) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    level_apply(lev[lane >> 3], t, c);
 #pragma unroll
     for (int o = 8; o < 32; o <<= 1)
 #pragma unroll
-        for (int c = 0; c < 3; c++) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
-    level_apply(lev[4], t, u);
+        for (int k = 0; k < 3; k++) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    level_apply(lev[4], t, c);
+    if ((lane & 7) == 0) z[4 * w + (lane >> 3)] = make_float4(c[0], c[1], c[2], 0.f);
+}
+__device__ __forceinline__ void level_add(const float4* z, LevelPlace at, float (&u)[3]) {
+    const float4 y = z[at.octet()];
+    u[0] += y.x;
+    u[1] += y.y;
+    u[2] += y.z;
 }
 
 }  // namespace

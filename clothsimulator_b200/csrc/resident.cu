@@ -149,7 +149,7 @@ struct __align__(16) ResShared {
     int cheb_deg;
     float cheb_inv_th;
     float cheb_a[CS_PRECOND_MAX_DEGREE], cheb_b[CS_PRECOND_MAX_DEGREE];
-    // inverse diagonal blocks of the levels: per warp its four octets, then the slice (six entries)
+    // inverse diagonal blocks of the levels: per warp its four octets, then its patch (six entries)
     alignas(16) float lev[CS_RES_MAX_WARPS][5][8];
     double sc[CS_RES_MAX_WARPS][7];    // scalars of the solve, per warp
 };
@@ -532,12 +532,13 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 cr[h] -= alpha_c * cs[h];
             }
         };
-        // The levels' diagonal blocks: sums of the row's stored blocks whose column lies in the same octet
-        // or slice (of a tile's rows, every eight and every 32 are a compact patch of the sheet).
+        // The levels' diagonal blocks (levels.cuh); its first barrier also covers the panel copy
+        LevelPlace at{(uint32_t)myslot * 0x10001u};
         if (levels) {
-            __syncthreads();  // the panels are in place
-            level_blocks(spn, gpn, ks, width, code, w, lane, live, S.lev[w]);
-            __syncwarp();
+            __syncthreads();
+            const uint32_t* cells = B.rcell + (size_t)B.slices[sh.slice_off + lo].topo_slice * CS_SLICE;
+            if (live) at.v = __ldg(cells + myslot);
+            level_blocks(spn, gpn, ks, width, code, cells, halo0 - 1, at, lane, live, su_alt, S.lev[w]);
         }
         // Tile-local Chebyshev preconditioner: the largest eigenvalue of P^-1 A_loc by power
         // iteration from a hashed +-1 vector (the first barrier also covers the panel copy),
@@ -805,15 +806,19 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 }
             }
             if (levels) {
-                // + the octet's, the slice's and the segment's corrections (additive)
-                level_correction(S.lev[w], r, lane, u);
+                // + the segment's, the octet's and the patch's corrections (additive)
+                su[myslot] = make_float4(r[0], r[1], r[2], 0.f);
                 if (coarse) {
                     const float r0 = (float)cr[0], r1 = (float)cr[1];
 #pragma unroll
                     for (int c = 0; c < 3; c++) u[c] += rwarp_sum(fmaf(cai[64 * c + 32], r1, cai[64 * c] * r0));
                 }
+                __syncthreads();
+                level_sums(S.lev[w], su, su_alt, at, w, lane);
+                __syncthreads();
+                level_add(su_alt, at, u);
             }
-            if (!live) u[0] = u[1] = u[2] = 0.f;  // an octet's correction reaches lanes without a row
+            if (!live) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row
             su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
             __syncthreads();
             if (tid == 0) rbar_expect(hbar, halo_bytes);
