@@ -604,9 +604,13 @@ __global__ void __launch_bounds__(128) cs_bc_finish_kernel(Batch B) {
         const float* ec = B.bc_ef + 3 * (size_t)(sh.bc_fvec_off + B.bc_node_fine[sh.bc_node_off + local]);
         float r[3], z[3];
 #pragma unroll
+        for (int c = 0; c < 3; c++) r[c] = B.r[3 * row + c];
+        // a node without a face has an empty row, which no correction may move
+        bool moves = r[0] != 0.f || r[1] != 0.f || r[2] != 0.f;
+        for (int k = 0; k < 9 && !moves; k++) moves = B.Pinv[9 * (size_t)row + k] != 0.f;
+#pragma unroll
         for (int c = 0; c < 3; c++) {
-            r[c] = B.r[3 * row + c];
-            z[c] = B.z[3 * row + c] + ec[c];
+            z[c] = B.z[3 * row + c] + (moves ? ec[c] : 0.f);
             B.z[3 * row + c] = z[c];
         }
         if (mixed) {

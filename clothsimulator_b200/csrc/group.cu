@@ -196,6 +196,11 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
         if (live)
 #pragma unroll
             for (int c = 0; c < 3; c++) r[c] = B.b[3 * g + c];
+        // a node without a face has an empty row, which no correction may move
+        bool moves = false;
+#pragma unroll
+        for (int k = 0; k < 9; k++) moves |= Pi[k] != 0.f;
+        moves |= r[0] != 0.f || r[1] != 0.f || r[2] != 0.f;
         if (tid == 0) {
             S.bn = S.res0 = sqrt(B.inst[s].bnorm2);
             S.rr = S.delta = 0.0;
@@ -572,7 +577,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                     for (int q = 0; q < parts; q++) u[c] += C.ce[(3 * seg + c) * parts + q];
             }
             nhalo++;
-            if (!live) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row
+            if (!moves) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row and empty rows
             su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
             if (live && pub)
                 put_packet(upk + slot, __float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), nhalo);

@@ -477,6 +477,11 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
 #pragma unroll
             for (int k = 0; k < 9; k++) Pi[k] = 0.f;
         }
+        // a node without a face has an empty row, which no correction may move
+        bool moves = false;
+#pragma unroll
+        for (int k = 0; k < 9; k++) moves |= Pi[k] != 0.f;
+        moves |= r[0] != 0.f || r[1] != 0.f || r[2] != 0.f;
         // scalars used once per iteration or less live in shared memory, a copy per warp (every lane
         // writes the same value and reads its own write)
         double &bn = S.sc[w][0], &res0 = S.sc[w][1], &resnorm = S.sc[w][2], &first_res = S.sc[w][3], &rr = S.sc[w][4],
@@ -818,7 +823,7 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                 __syncthreads();
                 level_add(su_alt, at, u);
             }
-            if (!live) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row
+            if (!moves) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row and empty rows
             su[myslot] = make_float4(u[0], u[1], u[2], 0.f);
             __syncthreads();
             if (tid == 0) rbar_expect(hbar, halo_bytes);

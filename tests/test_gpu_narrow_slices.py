@@ -43,3 +43,17 @@ def test_unused_nodes_on_chip(ctx_factory, name):
         got, trips = dv(**kw)
         assert trips == 0
         assert np.linalg.norm(got - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("name", SCENES)
+def test_unused_nodes_stay(ctx_factory, name):
+    """A node without a face has an empty row of the system: no preconditioner moves it."""
+    scene = SCENES[name]()
+    ctx = ctx_factory(scene.sheets)
+    unused = np.concatenate([~np.isin(np.arange(len(s["x"])), s["fx"]) for s in scene.sheets])
+    for solver in (native.SOLVER_AUTO, native.SOLVER_BATCHED):
+        for degree, coarse in ((3, 1), (3, 0), (1, 1), (1, 0)):
+            p = native.step_params(scene.dt, scene.gravity, scene.handle_stiffness, tol=1e-7, max_iters=20000, advance=0,
+                                   solver=solver, precond_degree=degree, coarse=coarse)
+            stats, _ = ctx.step(p)
+            assert stats.converged == len(scene.sheets) and not np.any(ctx.get_dv()[unused])
