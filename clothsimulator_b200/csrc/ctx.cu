@@ -253,7 +253,7 @@ uint64_t hashInts(const int32_t* a, size_t n, uint64_t h) {
 // patches of 8 x 4; by count the levels take two more barriers an iteration.  1,024 sheets of 64 x 64
 // quads, in cell order and by count: gather 4.27 and 3.63 ms, a step with block-Jacobi 113.9 and 109.6, with
 // Chebyshev-3 112 and 98, in the loop without coarse space 182 and 168, with the levels 59.4 and 60.2;
-// one sheet of 32 x 32 with the levels 0.360 and 0.378, a group of 72,900 nodes 5.25 and 4.59 (B200).
+// one sheet of 32 x 32 with the levels 0.360 and 0.378, a group of 73,441 nodes 5.25 and 4.59 (B200).
 void tileOrder(const std::vector<float>& uv, const std::vector<int>& len, int G, int K, std::vector<int>& order,
                std::vector<uint32_t>& cell) {
     const int n = (int)len.size(), ns = (n + CS_SLICE - 1) / CS_SLICE;
