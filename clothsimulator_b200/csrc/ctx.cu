@@ -22,6 +22,7 @@
 #include <functional>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <unordered_map>
@@ -950,6 +951,7 @@ struct cs_ctx {
     // the resident solve (it overlaps the learned inference and the solve set-up)
     cudaStream_t side = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
+    cudaEvent_t evGroup = nullptr;  // end of the last step with group sheets (GroupTurn)
     std::string err;
     Batch B;
     bool loaded = false;
@@ -1255,6 +1257,37 @@ void launchGroup(cs_ctx* c) {
     cudaLaunchKernelEx(&cfg, cs_group_pcg_kernel, c->B);
 }
 
+// The CTAs of a group launch wait on one another, so all of them have to be on the chip at once.  Two such
+// launches from two contexts could each hold a part of it and wait for the rest until their waits run
+// out: the steps of contexts with group sheets take turns on a device.  Held while a step is enqueued;
+// the stream waits for the last such step of another context.
+struct GroupTurn {
+    static constexpr int kDevices = 64;
+    static std::mutex lock[kDevices];
+    static cs_ctx* last[kDevices];  // the context whose evGroup ends the last such step
+    cs_ctx* const c;
+    explicit GroupTurn(cs_ctx* ctx) : c(ctx->groupCtas > 0 ? ctx : nullptr) {
+        if (!c) return;
+        lock[c->device % kDevices].lock();
+        cs_ctx* l = last[c->device % kDevices];
+        if (l && l != c) cudaStreamWaitEvent(c->stream, l->evGroup, 0);
+    }
+    ~GroupTurn() {
+        if (!c) return;
+        cudaEventRecord(c->evGroup, c->stream);
+        last[c->device % kDevices] = c;
+        lock[c->device % kDevices].unlock();
+    }
+    GroupTurn(const GroupTurn&) = delete;
+    GroupTurn& operator=(const GroupTurn&) = delete;
+    static void forget(cs_ctx* ctx) {  // its stream has ended
+        std::lock_guard<std::mutex> g(lock[ctx->device % kDevices]);
+        if (last[ctx->device % kDevices] == ctx) last[ctx->device % kDevices] = nullptr;
+    }
+};
+std::mutex GroupTurn::lock[GroupTurn::kDevices];
+cs_ctx* GroupTurn::last[GroupTurn::kDevices] = {};
+
 int launchMlpInference(cs_ctx* c, float* pred);
 
 // The step up to its solve loop: assembly; the resident sheets' coarse matrices on the side
@@ -1396,7 +1429,8 @@ cs_status cs_create(cs_ctx** out, int device) {
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->evFork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->evGroup, cudaEventDisableTiming) != cudaSuccess) {
         delete c;
         return CS_ERR_CUDA;
     }
@@ -1413,6 +1447,8 @@ cs_status cs_destroy(cs_ctx* c) {
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->evFork);
     cudaEventDestroy(c->evJoin);
+    GroupTurn::forget(c);
+    cudaEventDestroy(c->evGroup);
     cudaStreamDestroy(c->side);
     cudaStreamDestroy(c->stream);
     delete c;
@@ -3095,6 +3131,7 @@ cs_status cs_step(cs_ctx* c, const cs_step_params* p, cs_step_stats* stats) {
     c->hostParams = d;
     CS_CUDA(cudaMemcpyAsync(c->B.params, &d, sizeof(d), cudaMemcpyHostToDevice, c->stream));
     if ((st = setTripCoarse(c, p->coarse != 0)) != CS_OK) return st;
+    const GroupTurn turn(c);
     CS_CUDA(cudaEventRecord(c->ev0, c->stream));
     const bool learned = p->warm_start == CS_WARM_LEARNED;
     // A graph holds the proximity lists it was captured with.  While they change from step to step
@@ -3386,6 +3423,7 @@ static float timeWholeSolve(cs_ctx* c, const cs_step_params& q) {
     if (setTripCoarse(c, q.coarse != 0) != CS_OK) return -1.f;
     if (cudaMemcpyAsync(B.params, &d, sizeof(d), cudaMemcpyHostToDevice, c->stream) != cudaSuccess) return -1.f;
     launchSolvePrologueAgain(c);
+    const GroupTurn turn(c);
     cudaEventRecord(c->ev0, c->stream);
     launchResident(c);
     launchGroup(c);
@@ -3643,6 +3681,7 @@ cs_status mlpEnergyPrepare(cs_ctx* c, const cs_step_params* p) {
     launchAssembly(c);
     cs_mlp_features_kernel<<<nblk(B.N, 256), 256, 0, c->stream>>>(B, M, M.feat);
     launchSolvePrologue(c);
+    const GroupTurn turn(c);
     launchResident(c);
     launchGroup(c);
     if ((st = hostLoop(c, d.loop_cap)) != CS_OK) return st;

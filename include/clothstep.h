@@ -136,7 +136,8 @@ typedef struct cs_step_params {
  * precision, by a group of CTAs over the whole chip while their rows and panels fit its shared
  * memory (about 80,000 nodes of a grid); the others by the batched loop.  CS_SOLVER_BATCHED: every sheet by the batched loop (the system streamed
  * from HBM every iteration).  Both run the same mixed/plain PCG to the same FP64-checked
- * tolerance. */
+ * tolerance.  Steps of different contexts on one device may be under way at the same time, except that
+ * those with sheets solved by a group take turns (the library orders them). */
 #define CS_SOLVER_AUTO 0
 #define CS_SOLVER_BATCHED 1
 
