@@ -359,6 +359,8 @@ struct Batch {
     // entries of a CTA's rows of the inverse coarse matrix),
     // panels per CTA in shared memory and the byte offset of what follows the u array there
     int n_group = 0, g_max = 0, g_own = 0, g_halo = 0, g_cap = 0, g_coff = 0, g_cnc = 0, g_ck3 = 0, g_cai = 0;
+    // polls of an exchange packet before a CTA gives up: within a solve, and for a sheet's first exchange
+    uint32_t g_polls = 1u << 19, g_polls_first = 1u << 27;
     GroupItem* gitem = nullptr;
     int *gcta_ptr = nullptr, *gcta_item = nullptr;
     unsigned char* gpub = nullptr;

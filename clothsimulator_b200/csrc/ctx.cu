@@ -2251,6 +2251,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
     UP(rcoarse, hrcoarse);
     UP(cpair, hcpair);
     UP(ccontrib, hccontrib);
+    // CS_GROUP_POLLS sets both limits of the groups' waits (tests of the path that a wait's end takes)
+    if (const char* ev = std::getenv("CS_GROUP_POLLS")) B.g_polls = B.g_polls_first = (uint32_t)std::max(0, std::atoi(ev));
     if (B.n_group > 0) {
         UP(gitem, hgitem);
         UP(gcta_ptr, hgcta_ptr);

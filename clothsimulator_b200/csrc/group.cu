@@ -26,8 +26,9 @@
 //     packets are zeroed before the launch and epochs start at 1.
 //   * Sums are deterministic: warp butterflies, warp partials in order, CTA partials in a fixed
 //     order that is the same in every CTA, so all take identical decisions.
-// Every wait is bounded; a CTA whose wait runs out sets the error word, which ends the others'
-// waits, and the host reports CS_ERR_TIMEOUT.
+// Every wait is bounded by a number of polls (Batch::g_polls: about 0.3 s; for a sheet's first exchange, whose
+// CTAs may still solve others, g_polls_first: more than a minute); a CTA whose wait runs out sets the error word,
+// which ends the others' waits, and the host reports CS_ERR_TIMEOUT.
 //
 // What bounds it: per iteration two trips through L2 (halo, reduction) of about 1 us each, the chain of
 // instructions between them and the shared-memory reads of the tile.  Measured against the batched
@@ -39,8 +40,6 @@
 
 namespace {
 
-constexpr uint32_t G_TRIES = 1u << 19;           // polls of a packet within a solve (about 0.3 s)
-constexpr uint32_t G_TRIES_FIRST = 1u << 27;     // for a sheet's first exchange: its CTAs may still solve others
 constexpr float G_LMAX_MARGIN = 1.1f;            // as in resident.cu
 constexpr float G_LMIN_RATIO = 1.0f / 30.0f;
 
@@ -206,7 +205,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             S.rr = S.delta = 0.0;
             S.resnorm = S.first_res = -1.0;
         }
-        uint32_t nred = 0, nhalo = 0, tries = G_TRIES_FIRST;
+        uint32_t nred = 0, nhalo = 0, tries = B.g_polls_first;
 
         // Waits for the packet at `q` to carry `epoch`; zeros with ok = false where that runs out.
         auto wait_packet = [&](const uint4* q, uint32_t epoch, bool& ok) -> uint4 {
@@ -274,7 +273,7 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
                     o[2] = __uint_as_float(x.z);
                 }
             }
-            tries = G_TRIES;
+            tries = B.g_polls;
             if (!ok) atomicExch(err, 1);
             if (!__syncthreads_and(ok ? 1 : 0)) return false;
             // with fewer than three warps, a warp takes more than one sum

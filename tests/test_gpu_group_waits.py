@@ -1,4 +1,8 @@
-"""Steps of several contexts with sheets of the group-resident solver at once."""
+"""Waits of the group-resident solver that run out, and steps of several contexts with such sheets at once.
+
+A wait's limit of zero polls makes the first exchange between CTAs give up: the kernel returns, the step
+reports CS_ERR_TIMEOUT, and the device goes on working.
+"""
 import threading
 
 import numpy as np
@@ -12,6 +16,24 @@ from clothsimulator_b200 import native, scenes
 def params_for(scene, **kw):
     return native.step_params(scene.dt, scene.gravity, scene.handle_stiffness, tol=1e-8, max_iters=20000, advance=0,
                               precond_degree=3, **kw)
+
+
+@pytest.mark.parametrize("use_graph", [0, 1])
+def test_wait_that_runs_out_is_reported(monkeypatch, use_graph):
+    scene = scenes.precision_sheet(101, seed=1)
+    monkeypatch.setenv("CS_GROUP_POLLS", "0")
+    ctx = native.Context(0).load(scene.sheets)
+    monkeypatch.delenv("CS_GROUP_POLLS")
+    for _ in range(2):
+        with pytest.raises(native.ClothStepError) as e:
+            ctx.step(params_for(scene, use_graph=use_graph))
+        assert e.value.status == native.CS_ERR_TIMEOUT
+    ctx.step(params_for(scene, solver=native.SOLVER_BATCHED))  # the context goes on: the loop has no such wait
+    dv = ctx.get_dv().astype(np.float64)
+    ctx.load(scene.sheets)
+    ctx.step(params_for(scene, use_graph=use_graph))
+    assert np.linalg.norm(ctx.get_dv() - dv) <= 1e-4 * np.linalg.norm(dv)
+    ctx.close()
 
 
 def test_contexts_with_group_sheets_take_turns():
