@@ -590,8 +590,9 @@ def run_ours(args):
         ctx.set_state(x0, v0)
         for _ in range(args.warmup):
             ctx.step(tp, allow_unconverged=True)
+        shape0 = tuple(ctx.solver_info()[k] for k in ("spmv_threads_per_block", "spmv_slices_per_warp", "spmv_slots_loaded_together"))
         t = ctx.tune(tp, reps=5)
-        default = next(x for x in t["spmv"] if (x["threads"], x["slices_per_warp"], x["unroll"]) == (128, 1, 1))
+        default = next(x for x in t["spmv"] if (x["threads"], x["slices_per_warp"], x["unroll"]) == shape0)
         tuning = {"spmv": {k: t["spmv"][t["best_spmv"]][k] for k in ("threads", "slices_per_warp", "unroll", "ms")},
                   "spmv_default_ms": default["ms"], "spmv_shapes_identical_bits": len({x["checksum"] for x in t["spmv"]}) == 1,
                   "precond": t["precond"][t["best_precond"]] if t["best_precond"] >= 0 else None,

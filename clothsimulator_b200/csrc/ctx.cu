@@ -1006,6 +1006,7 @@ struct cs_ctx {
     int residentProx = 0;       // those of them that a proximity touches
     int loopSheets = 0;         // sheets that the batched loop solves on the AUTO route
     int proxSteps = 0;          // steps since the proximities last changed
+    bool untiled = false;       // some sheet of the cluster solver is too small for tiles
     std::vector<long long> sheetBlocks, sheetLocalBlocks;  // per sheet: pattern blocks, tile-local ones
     // proximities (cs_set_proximities): their device lists, and the host copies of the
     // blocks outside the pattern that cs_get_system merges
@@ -1718,6 +1719,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         }
     }
     for (int s = 0; s < n_sheets; s++) c->sheetTopo[s] = topos[sheetTopoId[s]];
+    c->untiled = false;
+    for (size_t t = 0; t < topos.size(); t++) c->untiled |= res.resident[t] && topos[t]->tile_ctas == 0;
     std::vector<int> hrsplit(topos.size() * (CS_RES_MAX_CL + 1), 0), hrcode;
     std::vector<int> hrsendptr(topos.size() * (CS_RES_MAX_CL + 1), 0);
     std::vector<int> hrhalo(topos.size() * (CS_RES_MAX_CL + 1), 0);
@@ -3483,13 +3486,19 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
     }
     c->spmvShape = best;
     if (out) out->best_spmv = best;
-    // the resident solver's preconditioners: one whole solve of the resident sheets each
+    // the on-chip solvers' preconditioners: one whole solve of their sheets each.  With the coarse correction
+    // every degree is the same multilevel preconditioner on tiled sheets: one is timed for all unless
+    // some sheet is not tiled.
+    const bool onChip = c->resClusters > 0 || (c->groupCtas > 0 && p->precision == CS_PREC_MIXED);
+    float levelMs = 0.f;
     static const int degs[CS_TUNE_PRECONDS] = {1, 3, 3, 5, 5, 7}, coarse[CS_TUNE_PRECONDS] = {0, 0, 1, 0, 1, 1};
     int bestP = -1;
     float bestPm = 1e30f;
     for (int k = 0; k < CS_TUNE_PRECONDS; k++) {
         float ms = 0.f;
-        if (c->resClusters > 0) {
+        if (onChip && levelMs > 0.f && coarse[k] && !c->untiled) {
+            ms = levelMs;
+        } else if (onChip) {
             cs_step_params q = *p;
             q.precond_degree = degs[k];
             q.coarse = coarse[k];
@@ -3500,14 +3509,17 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
             const int nrep = reps < 3 ? reps : 3;
             for (int r = 0; r <= nrep; r++) {
                 launchSolvePrologueAgain(c);
+                const GroupTurn turn(c);
                 CS_CUDA(cudaEventRecord(c->ev0, c->stream));
                 launchResident(c);
+                launchGroup(c);
                 CS_CUDA(cudaEventRecord(c->ev1, c->stream));
                 CS_CUDA(cudaEventSynchronize(c->ev1));
                 float t = 0.f;
                 CS_CUDA(cudaEventElapsedTime(&t, c->ev0, c->ev1));
                 if (r > 0) ms += t / nrep;
             }
+            if (coarse[k] && degs[k] == 3) levelMs = ms;
             if (ms < bestPm) {
                 bestPm = ms;
                 bestP = k;
@@ -3522,9 +3534,9 @@ cs_status cs_tune(cs_ctx* c, const cs_step_params* p, int reps, cs_tune_result* 
     c->tunedDegree = bestP >= 0 ? degs[bestP] : 0;
     c->tunedCoarse = bestP >= 0 ? coarse[bestP] : 0;
     if (out) out->best_precond = bestP;
-    // the whole solve by each route: resident sheets on the cluster kernel (with the fastest
-    // preconditioner) and the rest in the batched loop, or every sheet in the batched loop
-    // (which wins when sheets too large for a cluster set the loop's trip count anyway)
+    // the whole solve by each route: what fits on chip there (with the fastest preconditioner) and the rest in
+    // the batched loop, or every sheet in the batched loop (which can win when sheets too large for the
+    // chip set the loop's trip count anyway)
     {
         cs_step_params q = *p;
         if (bestP >= 0) {

@@ -181,10 +181,11 @@ cs_status cs_get_solver_info(const cs_ctx* ctx, int* info);
  * algorithm (Cloth.cu:767-778, 790).  cs_tune times, with CUDA events on the context's stream and
  * on the loaded batch's system for the current state (params as for cs_step): every launch shape
  * of the batched SpMV -- threads per block, SELL slices per warp, block slots whose loads are
- * issued together -- reps launches each, and whole cluster-resident solves with each
- * preconditioner (block-Jacobi; strip-local Chebyshev of degree 3, 5 and 7 without and with the
- * coarse-space correction; one untimed, then the mean of min(reps, 3)), then whole solves by
- * either route (resident sheets on the cluster kernel and the rest in the batched loop, or all
+ * issued together -- reps launches each, and whole solves of the sheets solved on chip with each
+ * preconditioner (block-Jacobi; a Chebyshev polynomial of degree 3 and 5; with `coarse` degree 3, 5
+ * and 7, which are one multilevel preconditioner and timed once unless some sheet is too small
+ * for tiles; one untimed, then the mean of min(reps, 3)), then whole solves by
+ * either route (what fits on chip there and the rest in the batched loop, or all
  * in the batched loop; one untimed, then the mean of min(reps, 2)).  Every SpMV shape computes the same bits (out->spmv_checksum holds a
  * checksum of each shape's output); the fastest is used by the following steps.  The fastest
  * preconditioner is reported (cs_get_solver_info info[9], info[10]) for the caller's
@@ -197,7 +198,7 @@ typedef struct cs_tune_result {
     float spmv_ms[CS_TUNE_SPMV_SHAPES];
     uint32_t spmv_checksum[CS_TUNE_SPMV_SHAPES];
     int spmv_threads[CS_TUNE_SPMV_SHAPES], spmv_spw[CS_TUNE_SPMV_SHAPES], spmv_unroll[CS_TUNE_SPMV_SHAPES];
-    float precond_ms[CS_TUNE_PRECONDS];  /* 0 when no sheet is solved cluster-resident */
+    float precond_ms[CS_TUNE_PRECONDS];  /* 0 when no sheet is solved on chip */
     int precond_degree[CS_TUNE_PRECONDS], precond_coarse[CS_TUNE_PRECONDS];
     int best_spmv, best_precond;         /* indices; best_precond -1 without resident sheets */
     /* one whole solve of the system, with the fastest preconditioner: [0] CS_SOLVER_AUTO (0

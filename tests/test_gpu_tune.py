@@ -44,3 +44,16 @@ def test_tuner_shapes_agree_and_the_choice_is_applied(ctx_factory):
     ctx.set_state(x0, v0)
     ctx.step(p)
     assert np.array_equal(ctx.get_dv(), before)
+
+
+def test_tuner_times_each_preconditioner_once(ctx_factory):
+    """With the coarse correction every degree is one preconditioner on tiled sheets; sheets solved by groups
+    of CTAs are part of the timed solves."""
+    for scene in (scenes.windy_batch(3, 45, seed=503), scenes.precision_sheet(110, seed=504)):
+        ctx = ctx_factory(scene.sheets)
+        res = ctx.tune(native.step_params(scene.dt, scene.gravity, scene.handle_stiffness, tol=1e-7, max_iters=20000), reps=2)
+        ms = {(q["degree"], q["coarse"]): q["ms"] for q in res["precond"]}
+        assert all(t > 0 for t in ms.values())
+        assert ms[3, 1] == ms[5, 1] == ms[7, 1]
+        best = res["precond"][res["best_precond"]]
+        assert (best["degree"], best["coarse"]) not in ((5, 1), (7, 1))
