@@ -961,9 +961,9 @@ struct cs_ctx {
     std::vector<SliceDesc> slices;
     std::vector<std::shared_ptr<Topo>> sheetTopo;
     long long nnzb_pattern = 0;
-    // graphs of the step, per [learned warm start][coarse-correction kernels in the loop trips]
-    cudaGraphExec_t gexec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    cudaGraph_t gph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    // graphs of the step, per [learned warm start][coarse-correction kernels in the loop trips][batched loop]
+    cudaGraphExec_t gexec[2][2][2] = {};
+    cudaGraph_t gph[2][2][2] = {};
     // launchTrip launches the batched coarse correction's kernels (the step asks for it); the
     // launch counter's trips before the last change of this setting and their kernels
     bool tripCoarse = true;
@@ -1066,10 +1066,12 @@ void freeBatch(cs_ctx* c) {
     c->maxHandleMotion = -1;
     for (int l = 0; l < 2; l++)
         for (int k = 0; k < 2; k++) {
-            if (c->gexec[l][k]) cudaGraphExecDestroy(c->gexec[l][k]);
-            if (c->gph[l][k]) cudaGraphDestroy(c->gph[l][k]);
-            c->gexec[l][k] = nullptr;
-            c->gph[l][k] = nullptr;
+            for (int m = 0; m < 2; m++) {
+                if (c->gexec[l][k][m]) cudaGraphExecDestroy(c->gexec[l][k][m]);
+                if (c->gph[l][k][m]) cudaGraphDestroy(c->gph[l][k][m]);
+                c->gexec[l][k][m] = nullptr;
+                c->gph[l][k][m] = nullptr;
+            }
         }
     c->tripCoarse = true;
     c->tripsBase = c->tripLaunchBase = 0;
@@ -1195,10 +1197,11 @@ cs_status setTripCoarse(cs_ctx* c, bool on) {
     return CS_OK;
 }
 
-void launchSolvePrologue(cs_ctx* c, cudaGraphConditionalHandle h = 0) {
+// `loop`: some sheet may need the batched loop, which takes its correction's set-up
+void launchSolvePrologue(cs_ctx* c, cudaGraphConditionalHandle h = 0, bool loop = true) {
     Batch& B = c->B;
     cs_solve_setup_kernel<<<B.S, 128, 0, c->stream>>>(B, h);
-    launchBatchedCoarseSetup(c);
+    if (loop) launchBatchedCoarseSetup(c);
     cs_solve_prologue_kernel<<<nblk(3LL * B.N, 256), 256, 0, c->stream>>>(B);
 }
 
@@ -1294,7 +1297,7 @@ int launchMlpInference(cs_ctx* c, float* pred);
 // The step up to its solve loop: assembly; the resident sheets' coarse matrices on the side
 // stream while the learned inference (when asked) and the solve set-up run on the main stream;
 // the join; the cluster-resident solve.  Captured into the step graph, or launched directly.
-void launchPrelude(cs_ctx* c, bool learned, cudaGraphConditionalHandle h = 0) {
+void launchPrelude(cs_ctx* c, bool learned, bool loop, cudaGraphConditionalHandle h = 0) {
     launchAssembly(c);
     const bool fork = c->resClusters > 0 && c->B.res_cnc > 0 && c->B.n_resident > 0;
     if (fork) {
@@ -1304,7 +1307,7 @@ void launchPrelude(cs_ctx* c, bool learned, cudaGraphConditionalHandle h = 0) {
         cudaEventRecord(c->evJoin, c->side);
     }
     if (learned) launchMlpInference(c, c->B.warm);
-    launchSolvePrologue(c, h);
+    launchSolvePrologue(c, h, loop);
     if (fork) cudaStreamWaitEvent(c->stream, c->evJoin, 0);
     launchResident(c, false);
     launchGroup(c);
@@ -1349,19 +1352,31 @@ cs_status hostLoop(cs_ctx* c, int loop_cap) {
     return CS_OK;
 }
 
-cs_status buildGraph(cs_ctx* c, bool learned) {
-    cudaGraphExec_t& exec = c->gexec[learned][c->tripCoarse];
+// Whether a step with these parameters may need the batched loop: it does not when every sheet is solved on
+// chip, as cs_solve_setup_kernel decides on the device.
+bool needsLoop(const cs_ctx* c, const DevParams& d) {
+    return d.solver != CS_SOLVER_AUTO_DEV || c->loopSheets > 0 || (!d.mixed && c->groupCtas > 0);
+}
+
+cs_status buildGraph(cs_ctx* c, bool learned, bool loop) {
+    cudaGraphExec_t& exec = c->gexec[learned][c->tripCoarse][loop];
     if (exec) return CS_OK;
     cudaGraph_t graph;
     CS_CUDA(cudaGraphCreate(&graph, 0));
-    c->gph[learned][c->tripCoarse] = graph;
+    c->gph[learned][c->tripCoarse][loop] = graph;
     // the loop's condition: set by the solve set-up (no trip when every sheet is solved on chip) and
     // by each trip
-    cudaGraphConditionalHandle handle;
-    CS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
+    cudaGraphConditionalHandle handle = 0;
+    if (loop) CS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
     // prelude: assembly (+ learned warm start) + solve setup, captured into the graph
     CS_CUDA(cudaStreamBeginCaptureToGraph(c->stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launchPrelude(c, learned, handle);
+    launchPrelude(c, learned, loop, handle);
+    if (!loop) {
+        cs_advance_kernel<<<nblk(3LL * c->B.N, 256), 256, 0, c->stream>>>(c->B);
+        CS_CUDA(cudaStreamEndCapture(c->stream, &graph));
+        CS_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+        return CS_OK;
+    }
     cudaStreamCaptureStatus cst;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
@@ -2181,6 +2196,8 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
         }
     }
     B.n_group = (int)hgitem.size();
+    c->loopSheets = 0;
+    for (int s = 0; s < n_sheets; s++) c->loopSheets += hs[s].resident == 0 ? 1 : 0;
     c->sheets = hs;
     c->slices = hslices;
 
@@ -2401,10 +2418,12 @@ namespace {
 void destroyGraphs(cs_ctx* c) {
     for (int l = 0; l < 2; l++)
         for (int k = 0; k < 2; k++) {
-            if (c->gexec[l][k]) cudaGraphExecDestroy(c->gexec[l][k]);
-            if (c->gph[l][k]) cudaGraphDestroy(c->gph[l][k]);
-            c->gexec[l][k] = nullptr;
-            c->gph[l][k] = nullptr;
+            for (int m = 0; m < 2; m++) {
+                if (c->gexec[l][k][m]) cudaGraphExecDestroy(c->gexec[l][k][m]);
+                if (c->gph[l][k][m]) cudaGraphDestroy(c->gph[l][k][m]);
+                c->gexec[l][k][m] = nullptr;
+                c->gph[l][k][m] = nullptr;
+            }
         }
 }
 
@@ -3139,22 +3158,20 @@ cs_status cs_step(cs_ctx* c, const cs_step_params* p, cs_step_stats* stats) {
     const GroupTurn turn(c);
     CS_CUDA(cudaEventRecord(c->ev0, c->stream));
     const bool learned = p->warm_start == CS_WARM_LEARNED;
+    const bool loop = needsLoop(c, d);
     // A graph holds the proximity lists it was captured with.  While they change from step to step
     // (detection before every step), capturing one per step would cost more than it saves: such a
     // step launches its kernels directly, where none of its sheets needs the loop.
-    const bool direct = p->use_graph && c->prox.n > 0 && c->proxSteps == 0 && p->precision == CS_PREC_MIXED &&
-                        p->solver == CS_SOLVER_AUTO && c->loopSheets == 0;
+    const bool direct = p->use_graph && c->prox.n > 0 && c->proxSteps == 0 && !loop;
+    const int fixed = assemblyKernels(c) + 3 + (learned ? 3 : 0) + (loop ? bcSetupKernels(c) : 0) + residentKernels(c);
     c->proxSteps++;
-    if (direct) {
-        launchPrelude(c, learned);
-        cs_advance_kernel<<<nblk(3LL * c->B.N, 256), 256, 0, c->stream>>>(c->B);
-    } else if (p->use_graph) {
-        if ((st = buildGraph(c, learned)) != CS_OK) return st;
-        CS_CUDA(cudaGraphLaunch(c->gexec[learned][c->tripCoarse], c->stream));
+    if (p->use_graph && !direct) {
+        if ((st = buildGraph(c, learned, loop)) != CS_OK) return st;
+        CS_CUDA(cudaGraphLaunch(c->gexec[learned][c->tripCoarse][loop], c->stream));
     } else {
-        c->hostLaunches += assemblyKernels(c) + 3 + bcSetupKernels(c) + residentKernels(c) + (learned ? 3 : 0);
-        launchPrelude(c, learned);
-        if ((st = hostLoop(c, d.loop_cap)) != CS_OK) return st;
+        if (!p->use_graph) c->hostLaunches += fixed;
+        launchPrelude(c, learned, loop);
+        if (loop && (st = hostLoop(c, d.loop_cap)) != CS_OK) return st;
         cs_advance_kernel<<<nblk(3LL * c->B.N, 256), 256, 0, c->stream>>>(c->B);
     }
     CS_CUDA(cudaGetLastError());
@@ -3163,7 +3180,7 @@ cs_status cs_step(cs_ctx* c, const cs_step_params* p, cs_step_stats* stats) {
     c->steps++;
     if (p->use_graph) {
         c->graphSteps++;
-        c->graphLaunchesFixed += assemblyKernels(c) + 3 + (learned ? 3 : 0) + bcSetupKernels(c) + residentKernels(c);
+        c->graphLaunchesFixed += fixed;
     }
     if (!stats) return CS_OK;
     return fillStepStats(c, stats, d.loop_cap, true);

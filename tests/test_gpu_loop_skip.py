@@ -24,3 +24,25 @@ def test_loop_runs_only_for_sheets_that_need_it(ctx_factory, scene):
             assert (stats.loop_trips > 0) == (solver == native.SOLVER_BATCHED)
             out[solver, graph] = ctx.get_dv().copy()
         assert np.array_equal(out[solver, 1], out[solver, 0])
+
+
+def test_steps_on_chip_launch_nothing_of_the_loop(ctx_factory):
+    """Where every sheet is solved on chip, a step's launches are the assembly's two, the solve set-up's two, the
+    solver's and the state update's, whether captured or not; the same steps by the loop take more."""
+    scene = scenes.hang(32, 1)
+    ctx = ctx_factory(scene.sheets)
+    made = {}
+    for solver in (native.SOLVER_AUTO, native.SOLVER_BATCHED, native.SOLVER_AUTO):
+        for graph in (1, 0):
+            p = native.step_params(scene.dt, scene.gravity, scene.handle_stiffness, tol=1e-7, max_iters=20000, advance=0,
+                                   precond_degree=3, solver=solver, use_graph=graph)
+            c0 = ctx.counters()["launches"]
+            stats, _ = ctx.step(p)
+            assert stats.converged == 1
+            made[solver, graph] = ctx.counters()["launches"] - c0
+            dv = ctx.get_dv().copy()
+            if solver == native.SOLVER_AUTO:
+                assert stats.loop_trips == 0
+                assert np.array_equal(dv, made.setdefault("dv", dv))
+    assert made[native.SOLVER_AUTO, 0] == made[native.SOLVER_AUTO, 1] == 6
+    assert min(made[native.SOLVER_BATCHED, g] for g in (0, 1)) > 50
