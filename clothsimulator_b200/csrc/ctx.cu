@@ -341,16 +341,21 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
             }
     }
     // Edges: first appearance order, nodes[0] < nodes[1]; sides per Edge::initialize.
-    std::unordered_map<uint64_t, int> map;
-    map.reserve(3 * (size_t)nf);
+    // (found by an open-addressed table of edge numbers, at most half full)
+    size_t tabSize = 16;
+    while (tabSize < 6 * (size_t)nf) tabSize *= 2;
+    std::vector<int> tab(tabSize, -1);
     std::vector<int> eN, eF, eV, eO;
+    for (auto* v : {&eN, &eF, &eO}) v->reserve(4 * (size_t)nf);
+    eV.reserve(8 * (size_t)nf);
     auto find = [&](int a, int b) {
         if (a > b) std::swap(a, b);
-        uint64_t key = (uint64_t)(uint32_t)a << 32 | (uint32_t)b;
-        auto it = map.find(key);
-        if (it != map.end()) return it->second;
-        int id = (int)eN.size() / 2;
-        map.emplace(key, id);
+        const uint64_t key = (uint64_t)(uint32_t)a << 32 | (uint32_t)b;
+        size_t h = (size_t)((key * 0x9E3779B97F4A7C15ull) >> 20) & (tabSize - 1);
+        for (; tab[h] >= 0; h = (h + 1) & (tabSize - 1))
+            if (eN[2 * tab[h]] == a && eN[2 * tab[h] + 1] == b) return tab[h];
+        const int id = (int)eN.size() / 2;
+        tab[h] = id;
         eN.push_back(a); eN.push_back(b);
         eF.push_back(-1); eF.push_back(-1);
         for (int i = 0; i < 4; i++) eV.push_back(-1);
@@ -449,13 +454,14 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
                 rc[fill[i]++] = ((uint64_t)(uint32_t)j << 32) | cs_code(1, e, a, b);
             }
     // per row: columns (diagonal first, then ascending) and contributor ranges
-    std::vector<std::vector<int>> rowCols(nn);
-    std::vector<std::vector<std::pair<int, int>>> rowRanges(nn);
+    std::vector<int> cols, rowBase(nn + 1, 0);  // row i's from rowBase[i] on
+    std::vector<std::pair<int, int>> ranges;
+    cols.reserve(16 * (size_t)nn);
+    ranges.reserve(16 * (size_t)nn);
     for (int i = 0; i < nn; i++) {
-        auto beg = rc.begin() + cnt[i], end = rc.begin() + cnt[i + 1];
-        std::stable_sort(beg, end, [](uint64_t a, uint64_t b) { return (a >> 32) < (b >> 32); });
-        std::vector<int> cols;
-        std::vector<std::pair<int, int>> ranges;
+        // by column, then by code: the codes of one (row, column) ascend in the reference's order
+        std::sort(rc.begin() + cnt[i], rc.begin() + cnt[i + 1]);
+        const size_t diag = cols.size();
         cols.push_back(i);
         ranges.push_back({0, 0});
         for (int p = cnt[i]; p < cnt[i + 1];) {
@@ -463,21 +469,20 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
             int q = p;
             while (q < cnt[i + 1] && (int)(rc[q] >> 32) == j) q++;
             if (j == i)
-                ranges[0] = {p, q};
+                ranges[diag] = {p, q};
             else {
                 cols.push_back(j);
                 ranges.push_back({p, q});
             }
             p = q;
         }
-        rowCols[i] = std::move(cols);
-        rowRanges[i] = std::move(ranges);
+        rowBase[i + 1] = (int)cols.size();
     }
     // SELL-32 slices.  Rows are sorted by block count (descending, stable) within windows of
     // sigma rows; sigma is chosen from {32, 64, 128, 256} to minimise the padded slots (the
     // SpMV reads every slot of a slice's width), the smaller window on ties to keep locality.
     std::vector<int> len(nn);
-    for (int i = 0; i < nn; i++) len[i] = (int)rowCols[i].size();
+    for (int i = 0; i < nn; i++) len[i] = rowBase[i + 1] - rowBase[i];
     auto orderFor = [&](int sigma) {
         std::vector<int> order(nn);
         for (int i = 0; i < nn; i++) order[i] = i;
@@ -525,7 +530,7 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     for (int s = 0; s < t->n_slices; s++) {
         int r0 = s * CS_SLICE, rows = std::min(CS_SLICE, nn - r0);
         int w = 1;
-        for (int l = 0; l < rows; l++) w = std::max(w, (int)rowCols[order[r0 + l]].size());
+        for (int l = 0; l < rows; l++) w = std::max(w, len[order[r0 + l]]);
         t->slice_rows.push_back(rows);
         t->slice_width.push_back(w);
         t->slice_tpanel0.push_back(tp);
@@ -537,9 +542,7 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     t->tcontrib.clear();
     t->tcontrib.reserve(rc.size());
     std::vector<int> slotOf;  // per (row, column position)
-    std::vector<int> rowSlotBase(nn + 1, 0);
-    for (int i = 0; i < nn; i++) rowSlotBase[i + 1] = rowSlotBase[i] + (int)rowCols[i].size();
-    slotOf.assign(rowSlotBase[nn], -1);
+    slotOf.assign(rowBase[nn], -1);
     for (int s = 0; s < t->n_slices; s++) {
         int r0 = s * CS_SLICE;
         for (int k = 0; k < t->slice_width[s]; k++)
@@ -548,11 +551,11 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
                 t->tcptr[slot] = (int)t->tcontrib.size();
                 if (l < t->slice_rows[s]) {
                     int i = order[r0 + l];
-                    if (k < (int)rowCols[i].size()) {
-                        t->tcol[slot] = rowCols[i][k];
-                        auto rg = rowRanges[i][k];
+                    if (k < len[i]) {
+                        t->tcol[slot] = cols[rowBase[i] + k];
+                        const auto rg = ranges[rowBase[i] + k];
                         for (int p = rg.first; p < rg.second; p++) t->tcontrib.push_back((uint32_t)(rc[p] & 0xffffffffu));
-                        slotOf[rowSlotBase[i] + k] = (int)slot;
+                        slotOf[rowBase[i] + k] = (int)slot;
                     } else {
                         t->tcol[slot] = i;  // padding: zero block on the diagonal column
                     }
@@ -566,13 +569,12 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     // by corner).
     {
         auto slotIn = [&](int i, int j) {
-            const auto& cols = rowCols[i];
-            for (size_t k = 0; k < cols.size(); k++)
-                if (cols[k] == j) return (int)k;
+            for (int k = rowBase[i]; k < rowBase[i + 1]; k++)
+                if (cols[k] == j) return k - rowBase[i];
             return -1;
         };
         for (int i = 0; i < nn; i++)
-            if (rowCols[i].size() > 255) {
+            if (len[i] > 255) {
                 err = "a node couples to more than 255 nodes";
                 return nullptr;
             }
@@ -604,32 +606,36 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
     }
     // block-CSR view
     t->csr_ptr.assign(nn + 1, 0);
-    t->csr_col.clear();
-    t->csr_slot.clear();
+    t->csr_col.reserve(cols.size());
+    t->csr_slot.reserve(cols.size());
     for (int i = 0; i < nn; i++) {
-        std::vector<std::pair<int, int>> cs;
-        for (size_t k = 0; k < rowCols[i].size(); k++) cs.push_back({rowCols[i][k], slotOf[rowSlotBase[i] + k]});
-        std::sort(cs.begin(), cs.end());
-        for (auto& c : cs) {
-            t->csr_col.push_back(c.first);
-            t->csr_slot.push_back(c.second);
-        }
+        // the columns but the first, the diagonal, ascend
+        int k = rowBase[i] + 1;
+        auto put = [&](int q) {
+            t->csr_col.push_back(cols[q]);
+            t->csr_slot.push_back(slotOf[q]);
+        };
+        while (k < rowBase[i + 1] && cols[k] < i) put(k++);
+        put(rowBase[i]);
+        while (k < rowBase[i + 1]) put(k++);
         t->csr_ptr[i + 1] = (int)t->csr_col.size();
     }
     t->nnzb = (long long)t->csr_col.size();
     // one-ring neighbours
     {
-        std::vector<std::vector<int>> nb(nn);
+        std::vector<int> nb(6 * (size_t)nf), at(nn);  // two entries of each face at each of its nodes
+        for (int i = 0; i < nn; i++) at[i] = 2 * t->nf_ptr[i];
         for (int f = 0; f < nf; f++)
             for (int a = 0; a < 3; a++)
                 for (int b = 0; b < 3; b++)
-                    if (a != b) nb[t->fx[3 * f + a]].push_back(t->fx[3 * f + b]);
+                    if (a != b) nb[at[t->fx[3 * f + a]]++] = t->fx[3 * f + b];
         t->nbr_ptr.assign(nn + 1, 0);
+        t->nbr.reserve(8 * (size_t)nn);
         for (int i = 0; i < nn; i++) {
-            std::sort(nb[i].begin(), nb[i].end());
-            nb[i].erase(std::unique(nb[i].begin(), nb[i].end()), nb[i].end());
-            t->nbr_ptr[i + 1] = t->nbr_ptr[i] + (int)nb[i].size();
-            t->nbr.insert(t->nbr.end(), nb[i].begin(), nb[i].end());
+            const auto beg = nb.begin() + 2 * t->nf_ptr[i], end = nb.begin() + 2 * t->nf_ptr[i + 1];
+            std::sort(beg, end);
+            t->nbr.insert(t->nbr.end(), beg, std::unique(beg, end));
+            t->nbr_ptr[i + 1] = (int)t->nbr.size();
         }
     }
     return t;
@@ -674,24 +680,38 @@ size_t coarseSmemBytes(int ncta, int K) {
 
 // The pairs of aggregates and their stored blocks (slots with contributors; padding has none).
 void coarsePairs(const Topo& T, BCPlan& P) {
-    std::vector<std::pair<uint64_t, int>> blk;
-    blk.reserve(T.nnzb);
+    // every block's pair, numbered as they appear; then a counting sort by (a, b), slots ascending in each
+    std::vector<int> id((size_t)P.na * P.na, -1), pairOf, slotOf, count;
+    std::vector<int2> ab;
+    pairOf.reserve(T.nnzb);
+    slotOf.reserve(T.nnzb);
     for (int sl = 0; sl < T.n_slices; sl++)
         for (int k = 0; k < T.slice_width[sl]; k++)
             for (int l = 0; l < T.slice_rows[sl]; l++) {
                 const int slot = (T.slice_tpanel0[sl] + k) * CS_SLICE + l;
                 if (T.tcptr[slot + 1] == T.tcptr[slot]) continue;
-                blk.emplace_back((uint64_t)P.agg[T.rowmap[sl * CS_SLICE + l]] << 32 | (uint32_t)P.agg[T.tcol[slot]], slot);
+                const int a = P.agg[T.rowmap[sl * CS_SLICE + l]], b = P.agg[T.tcol[slot]];
+                int& p = id[(size_t)a * P.na + b];
+                if (p < 0) {
+                    p = (int)ab.size();
+                    ab.push_back(make_int2(a, b));
+                    count.push_back(0);
+                }
+                count[p]++;
+                pairOf.push_back(p);
+                slotOf.push_back(slot);
             }
-    std::sort(blk.begin(), blk.end());
-    for (size_t i = 0; i < blk.size();) {
-        size_t j = i;
-        while (j < blk.size() && blk[j].first == blk[i].first) j++;
-        P.pairs.push_back(make_int4((int)(blk[i].first >> 32), (int)(uint32_t)blk[i].first, (int)P.contrib.size(),
-                                    (int)(P.contrib.size() + (j - i))));
-        for (size_t q = i; q < j; q++) P.contrib.push_back(blk[q].second);
-        i = j;
+    std::vector<int> by(ab.size()), at(ab.size());
+    for (size_t i = 0; i < by.size(); i++) by[i] = (int)i;
+    std::sort(by.begin(), by.end(), [&](int x, int y) { return ab[x].x != ab[y].x ? ab[x].x < ab[y].x : ab[x].y < ab[y].y; });
+    int n = 0;
+    for (int p : by) {
+        P.pairs.push_back(make_int4(ab[p].x, ab[p].y, n, n + count[p]));
+        at[p] = n;
+        n += count[p];
     }
+    P.contrib.resize(n);
+    for (size_t i = 0; i < pairOf.size(); i++) P.contrib[at[pairOf[i]]++] = slotOf[i];
 }
 
 // Coarse space of the batched loop for one topology (coarse.cu): the nodes binned by their rest
