@@ -340,6 +340,9 @@ std::shared_ptr<Topo> buildTopo(const cs_sheet_desc& s, int tileCtas, int segs, 
                 t->node_uv[2 * t->fx[i] + 1] = s.uv[2 * t->fu[i] + 1];
             }
     }
+    // coordinates that are not finite have no order (their faces are refused later, by their areas)
+    for (float& q : t->node_uv)
+        if (!std::isfinite(q)) q = 0.0f;
     // Edges: first appearance order, nodes[0] < nodes[1]; sides per Edge::initialize.
     // (found by an open-addressed table of edge numbers, at most half full)
     size_t tabSize = 16;
