@@ -1026,7 +1026,6 @@ struct cs_ctx {
     Batch groupCoarse;
     std::vector<int> rlistAll;  // resident sheets before the proximity filter
     std::vector<int> rlistCur;  // resident sheets now
-    int residentProx = 0;       // those of them that a proximity touches
     int loopSheets = 0;         // sheets that the batched loop solves on the AUTO route
     int proxSteps = 0;          // steps since the proximities last changed
     bool untiled = false;       // some sheet of the cluster solver is too small for tiles
@@ -1123,7 +1122,6 @@ void freeBatch(cs_ctx* c) {
     c->sheetGroupDev = nullptr;
     c->rlistAll.clear();
     c->rlistCur.clear();
-    c->residentProx = 0;
     c->groupCtas = c->groupThreads = 0;
     c->groupSmem = c->groupPkBytes = 0;
     c->groupCoarse = Batch();
@@ -2386,7 +2384,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
 cs_status cs_get_solver_info(const cs_ctx* c, int* info) {
     if (!c || !info) return CS_ERR_INVALID_ARG;
     if (!c->loaded) return CS_ERR_STATE;
-    info[0] = c->B.n_resident - c->residentProx;
+    info[0] = c->B.n_resident;
     info[1] = c->resCL;
     info[2] = c->resThreads;
     info[3] = c->resClusters;
@@ -2560,12 +2558,8 @@ cs_status applyProximities(cs_ctx* c, int n, float thickness) {
     // sheets whose proximities couple nodes outside the mesh pattern leave the resident kernels for
     // the batched loop (only its SpMV reads such blocks); others keep the pattern and stay
     std::vector<int> rl;
-    c->residentProx = 0;
     for (int s : c->rlistAll)
-        if (!(touched[s] & 2)) {
-            rl.push_back(s);
-            c->residentProx += touched[s] ? 1 : 0;
-        }
+        if (!(touched[s] & 2)) rl.push_back(s);
     c->proxSteps = 0;
     c->loopSheets = 0;
     for (int s = 0; s < B.S; s++) c->loopSheets += (c->sheets[s].resident == 0 || (touched[s] & 2)) ? 1 : 0;

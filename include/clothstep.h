@@ -100,8 +100,9 @@ typedef struct cs_step_params {
                                  between CTAs), except where those rows are too thin a strip.
                                  The batched loop uses block-Jacobi (with the coarse
                                  correction when `coarse`). */
-    int coarse;               /* 1 adds a coarse-space correction, 0 leaves it out.  On-chip
-                                 solvers with a degree of 3 or more: one constant per component
+    int coarse;               /* 1 adds a coarse-space correction, 0 leaves it out.  A sheet
+                                 solved by a cluster with a degree of 3 or more, or by a group
+                                 with any: one constant per component
                                  on each of a few segments of every CTA's tile of rows, on sheets
                                  large enough for it.  Batched loop: one per aggregate of 256
                                  nodes or more (the rest (u, v) binned into at most 16 x 16
@@ -169,7 +170,8 @@ cs_status cs_load_batch(cs_ctx* ctx, const cs_material_desc* materials, int n_ma
  * it while proximities are set). */
 cs_status cs_get_sizes(const cs_ctx* ctx, long long* sizes);
 
-/* info[0..10] = sheets solved cluster-resident (that no proximity touches), CTAs per cluster, threads per CTA, clusters
+/* info[0..10] = sheets solved by a cluster (not those that proximities couple
+ * outside their mesh pattern, while set), CTAs per cluster, threads per CTA, clusters
  * in the persistent grid, SELL panels per CTA in shared memory, dynamic shared memory bytes
  * per CTA; the batched SpMV's launch shape (threads per block, slices per warp, slots loaded
  * together; cs_tune); the fastest resident preconditioner cs_tune found (degree, coarse
