@@ -128,8 +128,16 @@ enum InstPhase : int {
 // one CTA in shared memory, larger ones by a cluster of CS_BC_CLUSTER CTAs
 #define CS_BC_NODES_PER_AGG 256
 #define CS_BC_MAX_G 16
-#define CS_BC_BIG_NODES (1 << 18)  // sheets up to this size take at most 8 x 8 cells
-// the finer grids' cells (coarse.cu): nodes of a fine cell, fine cells along the side of a middle one
+// Sheets up to this size take at most 8 x 8 cells.  Steps with at most 8 x 8 / 16 x 16 (B200, tol 1e-6): an
+// irregular sheet of 301 x 301 nodes 5.9 / 7.1 ms, 401 x 401 9.5 / 13.7, 501 x 501 13.8 / 13.8, 601 x 601
+// 19.8 / 19.9, 801 x 801 39.3 / 32.3, 1,001 x 1,001 62 / 51; at tol 1e-8, where the iterations are many,
+// a sheet of 301 x 301 18.6 / 19.8 and of 451 x 451 52 / 41.
+#define CS_BC_BIG_NODES (1 << 18)
+// the finer grids' cells (coarse.cu): nodes of a fine cell, fine cells along the side of a middle one.  Steps
+// with 15, 30, 60 nodes (B200, tol 1e-6): irregular 301 x 301 nodes 5.3, 5.9, 8.5 ms, 401 x 401 10.2, 9.5, 11.7,
+// 501 x 501 14.4, 13.8, 16.1, 1,001 x 1,001 50.3, 50.7, 65.9, 60 sheets of 64 x 64 in the loop 11.3, 10.8,
+// 12.0 (a precision sheet of 601 x 601 at 1e-8 77, 96, 128); with a split of 2, 4, 6: 301 x 301 5.1, 5.9, 9.3,
+// 401 x 401 10.5, 9.5, 11.4, 501 x 501 14.8, 13.8, 16.9, 1,001 x 1,001 54, 51, 55 (601 x 601 73, 96, 108).
 #define CS_BC_NODES_PER_FINE 30
 #define CS_BC_FINE_SPLIT 4
 #define CS_BC_RESTRICT_THREADS 512
@@ -145,8 +153,10 @@ enum InstPhase : int {
 #define CS_COARSE_MAX_K 8
 #define CS_COARSE_SEGS 2
 #define CS_COARSE_AGGS 21
-// slices per CTA from which the coarse correction is worth its set-up: with 7.6 (48 x 48 quads) it saves
-// 15 of 79 iterations, with 3.5 (32 x 32) one of 58
+// Slices per CTA from which the cluster solver takes the coarse correction.  A step without / with it (B200, tol
+// 1e-6): one sheet of 32 x 32 quads (3.5 slices) 0.36 / 0.47 ms, of 40 x 40 (5.3) 0.42 / 0.50, of 48 x 48 (7.6)
+// 0.50 / 0.57, where a lone sheet waits for the set-up; 90 sheets of 32 x 32 1.27 / 1.45, of 40 x 40
+// 2.02 / 1.99, of 48 x 48 3.15 / 3.05, where it runs beside others.
 #define CS_COARSE_MIN_SLICES 5
 // Threads of the per-sheet set-up kernel that forms and inverts the coarse matrix, and its
 // dynamic shared memory: the nc x nc matrix with rows padded to 16 bytes, then one pivot block.

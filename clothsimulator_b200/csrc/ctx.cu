@@ -51,7 +51,7 @@ __global__ void cs_resident_pcg_kernel(Batch B);
 __global__ void cs_coarse_setup_kernel(Batch B);
 static_assert(CS_SPMV_CANDIDATES == CS_TUNE_SPMV_SHAPES, "the tuner's result holds every SpMV shape");
 __global__ void cs_prox_kernel(Batch B);
-__global__ void cs_prox_row_kernel(Batch B);
+__global__ void cs_prox_row_kernel(const __grid_constant__ Batch B);
 __global__ void cs_slice_bnorm_kernel(Batch B);
 __global__ void cs_bc_assemble_kernel(const __grid_constant__ Batch B);
 __global__ void cs_bc_invert_small_kernel(Batch B);

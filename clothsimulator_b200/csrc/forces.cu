@@ -687,7 +687,9 @@ __global__ void __launch_bounds__(128) cs_prox_kernel(Batch B) {
 // summed there and written back: summed in place through L2, a step of two 64 x 64 layers (18,600
 // proximities) took 317 us.
 extern __shared__ float cs_prox_acc[];
-__global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch B) {
+// ROWS: the block's rows where they are known when compiling (0: blockDim.x): a serial chain of indexes.
+template <int ROWS>
+__device__ __forceinline__ void prox_row(const Batch& B) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= B.N) return;
     const int q0 = B.prow_ptr[row], q1 = B.prow_ptr[row + 1];
@@ -696,7 +698,7 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
     const int* cp = B.tcsr_ptr + sd.csr_ptr_off;
     const int li = row - sd.node_off;
     const int c0 = cp[li], nc = cp[li + 1] - c0;
-    const int R = blockDim.x;
+    const int R = ROWS > 0 ? ROWS : (int)blockDim.x;
     float* const acc = cs_prox_acc + threadIdx.x;
     int* const cols = reinterpret_cast<int*>(cs_prox_acc + 9 * (size_t)B.gather_width * R) + threadIdx.x;
     int diag = 0;
@@ -770,6 +772,10 @@ __global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(Batch 
         store_slot(B.A, sd.panel_off * CS_SLICE + B.tcsr_slot[c0 + k], a);
         if (k == diag) block_inverse(a, B.Pinv + 9 * (size_t)row);
     }
+}
+__global__ void __launch_bounds__(CS_PROX_ROW_THREADS) cs_prox_row_kernel(const __grid_constant__ Batch B) {
+    if (blockDim.x == CS_PROX_ROW_THREADS) prox_row<CS_PROX_ROW_THREADS>(B);
+    else prox_row<0>(B);
 }
 
 // ||b||^2 per slice after the proximity right-hand sides (the gather's partials otherwise).

@@ -8,7 +8,7 @@
 //     z = D^-1 r + F^T D_F^-1 F r + G^T D_G^-1 G r (+ R^T A_c^-1 R r),
 // D_F and D_G the 3x3 diagonal blocks of F A F^T and G A G^T: additive, SPD, and 15 warp shuffles per
 // iteration with two barriers.  It takes the place of a Chebyshev polynomial in the tile's block of A
-// together with a larger coarse space: on a 64 x 64 sheet 76 CG iterations of one SpMV each instead of
+// together with a larger coarse space: on a 64 x 64 sheet about 75 CG iterations of one SpMV each instead of
 // 61 of one SpMV and two polynomial steps, and 54 coarse unknowns to invert instead of 162.
 #pragma once
 #include "cs_internal.h"

@@ -34,8 +34,8 @@
 // only one after start-up), so no CTA exits while another may still address its memory.
 //
 // What bounds it: the chain of latencies of one iteration -- its instructions in the slowest warp, two
-// exchanges through the cluster (halo, reduction), FP64 sums -- about 6 us for a 64 x 64 sheet on 9 CTAs
-// of 15 warps, 4 us for a 16 x 16 one.  Measured on the B200 (tol 1e-6, whole steps) against strips of
+// exchanges through the cluster (halo, reduction), FP64 sums -- about 8 us for a 64 x 64 sheet on 9 CTAs
+// of 15 warps with the levels and the coarse space, 6 us without them, 4 us for a 16 x 16 one.  Measured on the B200 (tol 1e-6, whole steps) against strips of
 // rows with a strip-local Chebyshev-3, 162 coarse unknowns and sums by every thread: a lone sheet of 64 x
 // 64 quads 1.14 -> 0.82 ms, 48 x 48 0.92 -> 0.52, 32 x 32 0.85 -> 0.34, 16 x 16 0.38 -> 0.30; 96 sheets of
 // 45 x 45 4.3 -> 2.9 ms, 700 of 64 x 64 46.0 -> 39.9 ms.
