@@ -564,8 +564,8 @@ __global__ void __launch_bounds__(CS_GROUP_MAX_WARPS * 32, 1) cs_group_pcg_kerne
             } else if (levels || coarse) {
                 if (levels) su[myslot] = make_float4(r[0], r[1], r[2], 0.f);
                 __syncthreads();
+                if (levels) level_sums(S.lev[w], su[at.slot()], su_alt, w, lane);
                 if (coarse) coarse_matvec();
-                if (levels) level_sums(S.lev[w], su, su_alt, at, w, lane);
                 __syncthreads();
                 if (levels) level_add(su_alt, at, u);
             }

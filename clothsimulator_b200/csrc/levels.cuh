@@ -191,11 +191,10 @@ __device__ __forceinline__ void level_blocks(const float* sp, const float* gp, i
     __syncthreads();  // `buf` is free
 }
 
-// The corrections by the octets and the patch at one warp's places of the vector that every thread of the CTA
-// stored at its number in `r` (zero without a row), into `z`, a float4 per octet.  Between a barrier after
-// those stores and one before level_add; `r` may be overwritten after the second, `z` after the next.
-__device__ __forceinline__ void level_sums(const float (*lev)[8], const float4* r, float4* z, LevelPlace at, int w, int lane) {
-    const float4 x = r[at.slot()];
+// The corrections by the octets and the patch at one warp's places of a vector, into `z`, a float4 per octet.  `x`:
+// the value of the row whose place is the thread's, which that row's thread stored in shared memory before a
+// barrier (zero without a row).  A barrier then lies before level_add; `z` may be overwritten after the next.
+__device__ __forceinline__ void level_sums(const float (*lev)[8], const float4 x, float4* z, int w, int lane) {
     float t[3] = {x.x, x.y, x.z}, c[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1)

@@ -180,6 +180,9 @@ __device__ __forceinline__ bool res_wait(ResShared& S, uint32_t bar, uint32_t pa
     return __syncthreads_and(res_poll<CLUSTER>(S, bar, parity) ? 1 : 0) != 0;
 }
 
+// Barrier of the first n warps of the CTA.
+__device__ __forceinline__ void warps_sync(int n) { asm volatile("bar.sync 1, %0;" ::"r"(32 * n) : "memory"); }
+
 // Raises the abort flag in every CTA of the cluster and the error word for the host.
 __device__ __forceinline__ void res_abort(const cg::cluster_group& cl, ResShared& S, int ncta, int* err) {
     if (threadIdx.x == 0) {
@@ -810,17 +813,18 @@ __global__ void __launch_bounds__(CS_RES_MAX_WARPS * 32, 1) cs_resident_pcg_kern
                     }
                 }
             }
-            if (levels) {
-                // + the segment's, the octet's and the patch's corrections (additive)
+            if (levels && w < nsl) {
+                // + the segment's, the octet's and the patch's corrections (additive); the barriers are of the
+                // warps with a slice alone, few of a small sheet's in a batch with large ones
                 su[myslot] = make_float4(r[0], r[1], r[2], 0.f);
                 if (coarse) {
                     const float r0 = (float)cr[0], r1 = (float)cr[1];
 #pragma unroll
                     for (int c = 0; c < 3; c++) u[c] += rwarp_sum(fmaf(cai[64 * c + 32], r1, cai[64 * c] * r0));
                 }
-                __syncthreads();
-                level_sums(S.lev[w], su, su_alt, at, w, lane);
-                __syncthreads();
+                warps_sync(nsl);
+                level_sums(S.lev[w], su[at.slot()], su_alt, w, lane);
+                warps_sync(nsl);
                 level_add(su_alt, at, u);
             }
             if (!moves) u[0] = u[1] = u[2] = 0.f;  // the corrections reach lanes without a row and empty rows
