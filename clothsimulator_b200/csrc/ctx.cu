@@ -1904,7 +1904,7 @@ cs_status cs_load_batch(cs_ctx* c, const cs_material_desc* mats, int n_mats, con
             q.cnc = std::max(q.cnc, nc);
             q.ck3 = std::max(q.ck3, 3 * T.tile_segs);
             q.cai = std::max(q.cai, 3 * T.tile_segs * nc);
-            if (4 * (long long)capOf(q) < 3 * (long long)q.panels) continue;
+            if (4 * (long long)capOf(q) < 3 * (long long)q.panels || q.warps * CS_SLICE + 1 + q.halo >= 4096) continue;
             z = q;
             topoGroup[t] = 1;
         }
