@@ -850,7 +850,7 @@ def run_ours(args):
                 "scheme": "mixed FP32 PCG, FP64 dot products, FP64 residual replacements (reliable updates)",
                 "warm_start": args.warm,
                 "solver": args.solver,
-                "precond": (("multilevel: block-Jacobi, octets and slices of rows, coarse space" if coarse else
+                "precond": (("multilevel: block-Jacobi, octets and patches of rows, coarse space" if coarse else
                              "tile-local Chebyshev degree %d over block-Jacobi" % deg)
                             if deg >= 3 and args.solver == "auto" else "block-Jacobi"),
                 "l2": "inputs larger than L2 (system matrix %.2f GB per GPU)" % (sizes[3] * 36 / 1e9)
